@@ -147,7 +147,9 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
 
     // This thread's row and the columns it may see: DQ a query and its interval of keys, DK / DV a
     // key and the interval of queries that see it (empty for a padded key).
-    const int lane_base = 32 * (warp & 3), r = lane_base + lane, row = row0 + r;
+    // Query tiles are 128 >> pack tokens of 1 << pack heads of a group, row (or column) = token << pack | head.
+    const int pack = a.pack, qt = ROWS >> pack;
+    const int lane_base = 32 * (warp & 3), r = lane_base + lane, row = row0 + (ROWS_ARE_QUERIES ? r >> pack : r);
     int lo = 0, hi = 0;
     if (warp >= 2 && warp < AUX_WARP) {
         if (ROWS_ARE_QUERIES) {
@@ -180,12 +182,12 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         int qfirst, qend;
         query_range(a.mask, row0, min(row0 + ROWS, a.tk), a.tq, a.tk, qfirst, qend);
         col_first = qfirst;
-        tiles = qend > qfirst ? (qend - qfirst + ROWS - 1) / ROWS : 0;
+        tiles = qend > qfirst ? (qend - qfirst + qt - 1) / qt : 0;
         head0 = res_head * group;
     }
-    const int steps = aborted ? 0 : (ROWS_ARE_QUERIES ? tiles : tiles * group);
-    auto step_head = [&](int t) { return ROWS_ARE_QUERIES ? head0 : head0 + t / tiles; };
-    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t : t % tiles) * ROWS; };
+    const int steps = aborted ? 0 : (ROWS_ARE_QUERIES ? tiles : tiles * (group >> pack));
+    auto step_head = [&](int t) { return ROWS_ARE_QUERIES ? head0 : head0 + ((t / tiles) << pack); };
+    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t * ROWS : (t % tiles) * qt); };
     bool failed = aborted;
     constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 256;
 
@@ -221,8 +223,8 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 const int h = step_head(t), q0 = step_col0(t);
 #pragma unroll
                 for (int i = 0; i < RPL; ++i) {
-                    const int q = min(q0 + lane + 32 * i, a.tq - 1);
-                    const int64_t at = ((int64_t)b * a.tq + q) * a.hq + h;
+                    const int c = lane + 32 * i, q = min(q0 + (c >> pack), a.tq - 1);
+                    const int64_t at = ((int64_t)b * a.tq + q) * a.hq + h + (c & ((1 << pack) - 1));
                     lse_n[i] = a.lse[at];
                     dl_n[i] = a.delta[at];
                 }
@@ -233,7 +235,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 float l2v[RPL], dlv[RPL];
 #pragma unroll
                 for (int i = 0; i < RPL; ++i) {
-                    const bool in = q0 + lane + 32 * i < a.tq;
+                    const bool in = q0 + ((lane + 32 * i) >> pack) < a.tq;
                     l2v[i] = (!in || lse_n[i] == -INFINITY) ? INFINITY : lse_n[i] * LOG2E;
                     dlv[i] = in ? dl_n[i] : 0.f;
                 }
@@ -334,18 +336,22 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
         const bool padded = ROWS_ARE_QUERIES && a.mask.kind == 1;
         float l2 = INFINITY, dl = 0.f;   // DQ: this query's log-sum-exp (base 2) and delta
+        const int head = ROWS_ARE_QUERIES ? res_head + (r & ((1 << pack) - 1)) : res_head;   // of this thread's row
         if (ROWS_ARE_QUERIES && row < a.tq) {
-            const int64_t at = ((int64_t)b * a.tq + row) * a.hq + res_head;
+            const int64_t at = ((int64_t)b * a.tq + row) * a.hq + head;
             const float x = a.lse[at];
             l2 = x == -INFINITY ? INFINITY : x * LOG2E;
             dl = a.delta[at];
         }
         for (int t = 0; t < steps && !failed; ++t) {
             const int st = t & 1, ph2 = (t >> 1) & 1;
-            const int c0 = step_col0(t) + col0;   // the first of this thread's columns (a key of DQ, a query of DK / DV)
+            // The step's columns this thread's row sees, [ca, cb): keys (DQ), or tokens << pack | head (DK / DV).
+            const int s0 = step_col0(t), c0 = col0;   // c0: the first of this thread's columns
+            const int span = ROWS_ARE_QUERIES ? ROWS : qt, shift = ROWS_ARE_QUERIES ? 0 : pack;
+            const int ca = min(max(lo - s0, 0), span) << shift, cb = min(max(hi - s0, 0), span) << shift;
             uint32_t pb = 0;
             if (padded) {
-                const int key = c0 + lane;
+                const int key = s0 + c0 + lane;
                 pb = __ballot_sync(0xffffffffu, key >= a.tk || key_padded(a.mask, b, key));
             }
             if (!ROWS_ARE_QUERIES && !__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.aux_full[st]), ph2))) { failed = true; break; }
@@ -361,12 +367,12 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 __syncwarp();
                 if (lane == 0) mbar_arrive(BAR(sh.bar.s_free));
             }
-            const bool clear = !padded && c0 >= lo && c0 + CW <= hi;
+            const bool clear = !padded && c0 >= ca && c0 + CW <= cb;
             if (!__all_sync(0xffffffffu, clear)) {
                 // A row that sees none of these columns (it belongs to another sequence of the packed batch, or
                 // its interval ends before them) needs no comparisons: where every row of the warp sees all or
                 // none, those rows are simply set.
-                const bool none = !padded && (hi <= c0 || lo >= c0 + CW || hi <= lo);
+                const bool none = !padded && (cb <= c0 || ca >= c0 + CW || cb <= ca);
                 if (__all_sync(0xffffffffu, clear || none)) {
                     if (none) {
 #pragma unroll
@@ -375,7 +381,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 } else {
 #pragma unroll
                     for (int c = 0; c < CW; ++c)
-                        p[c] = (c0 + c >= lo && c0 + c < hi && !((pb >> c) & 1u)) ? p[c] : -INFINITY;
+                        p[c] = (c0 + c >= ca && c0 + c < cb && !((pb >> c) & 1u)) ? p[c] : -INFINITY;
                 }
             }
             const ColumnAux &aux = sh.aux[st];
@@ -421,7 +427,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         bool in_range;
         float factor = a.scale;
         if (PASS == PASS_DQ) {
-            dst = static_cast<T *>(a.dq) + (((int64_t)b * a.tq + row) * a.hq + res_head) * HD;
+            dst = static_cast<T *>(a.dq) + (((int64_t)b * a.tq + row) * a.hq + head) * HD;
             in_range = row < a.tq;
         } else {
             dst = static_cast<T *>(PASS == PASS_DK ? a.dk : a.dv) + (((int64_t)b * a.tk + row) * a.hkv + res_head) * HD;
@@ -478,7 +484,7 @@ bwd256_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const Sm100BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem256[];
     const int qt = gridDim.y - 1 - blockIdx.y;   // later (longer, under causality) tiles first
-    bwd256_pass<T, PASS_DQ>(&tm_q, &tm_do, &tm_k, &tm_v, a, smem256, blockIdx.z, qt * ROWS, blockIdx.x);
+    bwd256_pass<T, PASS_DQ>(&tm_q, &tm_do, &tm_k, &tm_v, a, smem256, blockIdx.z, qt * (ROWS >> a.pack), blockIdx.x << a.pack);
 }
 
 // blockIdx.x: the (key block, key-value head) unit in the plan's order; blockIdx.y: 0 the dK pass (the
@@ -505,7 +511,8 @@ cudaError_t launch256_t(const Sm100BwdMaps &m, Sm100BwdArgs a, cudaStream_t stre
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(bwd256_dkdv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 gq(a.hq, (a.tq + ROWS - 1) / ROWS, a.b);
+    const int tokens = ROWS >> a.pack;
+    dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
     bwd256_dq_kernel<T><<<gq, THREADS, smem, stream>>>(m.q128, m.do128, m.k128, m.v128, a);
     *launches += 1;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

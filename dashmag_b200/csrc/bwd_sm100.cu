@@ -4,12 +4,12 @@
 // repeat from run to run (the contract's default, crates/dash-contract/src/attention.rs:96-102):
 //
 //   dkdv   one block per (128 keys, key-value head).  K_j and V_j stay in shared memory; the block
-//          sweeps the query heads of the group and, in steps of 128, the queries that see the key
-//          block.  Per step:  S^T = K_j Q^T and dP^T = V_j dO^T on the tensor cores (TMEM lane =
+//          sweeps, in steps of 128 rows (128 / P tokens x P heads), the queries of the group's heads
+//          that see the key block.  Per step:  S^T = K_j Q^T and dP^T = V_j dO^T on the tensor cores (TMEM lane =
 //          key), P^T = exp2(S^T sl - lse) and dS^T = P^T (dP^T - delta) elementwise, rounded to the
 //          input dtype back into tensor memory, then dV += P^T dO and dK += dS^T Q with the A
 //          operand read from tensor memory, accumulated in TMEM over the whole sweep.
-//   dq     one block per (128 queries, query head).  Q_i and dO_i stay in shared memory; the block
+//   dq     one block per tile of 128 query rows (128 / P tokens x P heads of a group, see pack_log2).  Q_i and dO_i stay in shared memory; the block
 //          sweeps, in steps of 64, the keys its queries see.  Per step: S = Q_i K^T, dP = dO_i V^T,
 //          dS = P (dP - delta), then dQ += dS K.
 //
@@ -331,8 +331,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     tc_fence_after_sync();
     const uint32_t tmem = sh.tmem_base;
     const bool aborted = sh.abort != 0;
-    const int tiles = (!aborted && qend > qfirst) ? (qend - qfirst + QS - 1) / QS : 0;
-    const int steps = tiles * group;
+    // A streamed tile of 128 rows: `qt` tokens of 1 << pack heads of the group, row = token << pack | head.
+    const int pack = a.pack, qt = QS >> pack;
+    const int tiles = (!aborted && qend > qfirst) ? (qend - qfirst + qt - 1) / qt : 0;
+    const int steps = tiles * (group >> pack);
     bool failed = aborted;
     // TMEM columns: S^T at 0, dP^T at 128 (each with its 16-bit twin over the first half of every
     // group of 32 columns: columns 32 g + [0, 16) hold queries 32 g + [0, 32)), dV at 256, dK at 384.
@@ -343,7 +345,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if (lane == 0 && steps > 0) {
             for (int t = 0; t < steps; ++t) {
                 const int st = t & 1, ph = (t >> 1) & 1;
-                const int h = hk * group + t / tiles, q0 = qfirst + (t % tiles) * QS;
+                const int h = hk * group + ((t / tiles) << pack), q0 = qfirst + (t % tiles) * qt;
                 // Q first (S^T of the step is issued before dP^T); its stage is also the later to come free.
                 if (!mbar_wait(BAR(sh.bar.q_empty[st]), ph ^ 1)) { failed = true; break; }
                 const uint32_t qf = BAR(sh.bar.q_full[st]), qd = smem_u32(q_s + st * BIG_BYTES);
@@ -365,11 +367,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         constexpr int RPL = QS / 32;   // rows per lane
         float lse_n[RPL], dl_n[RPL];
         auto gather = [&](int t) {
-            const int h = hk * group + t / tiles, q0 = qfirst + (t % tiles) * QS;
+            const int h = hk * group + ((t / tiles) << pack), q0 = qfirst + (t % tiles) * qt;
 #pragma unroll
             for (int i = 0; i < RPL; ++i) {
-                const int q = min(q0 + lane + 32 * i, a.tq - 1);
-                const int64_t at = ((int64_t)b * a.tq + q) * a.hq + h;
+                const int c = lane + 32 * i, q = min(q0 + (c >> pack), a.tq - 1);
+                const int64_t at = ((int64_t)b * a.tq + q) * a.hq + h + (c & ((1 << pack) - 1));
                 lse_n[i] = a.lse[at];
                 dl_n[i] = a.delta[at];
             }
@@ -377,7 +379,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if (steps > 0) gather(0);
         for (int t = 0; t < steps; ++t) {
             const int st = t & 1, ph = (t >> 1) & 1;
-            const int q0 = qfirst + (t % tiles) * QS;
+            const int q0 = qfirst + (t % tiles) * qt;
             float lse_c[RPL], dl_c[RPL];
 #pragma unroll
             for (int i = 0; i < RPL; ++i) { lse_c[i] = lse_n[i]; dl_c[i] = dl_n[i]; }
@@ -385,7 +387,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             float l2v[RPL], dlv[RPL];
 #pragma unroll
             for (int i = 0; i < RPL; ++i) {
-                const bool in = q0 + lane + 32 * i < a.tq;
+                const bool in = q0 + ((lane + 32 * i) >> pack) < a.tq;
                 l2v[i] = (!in || lse_c[i] == -INFINITY) ? INFINITY : lse_c[i] * LOG2E;
                 dlv[i] = in ? dl_c[i] : 0.f;
             }
@@ -517,7 +519,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
         const bool issuer = warp == KRED_WARP && lane == 0;
         for (int t = 0; t < steps && !failed; ++t) {
-            const int h = hk * group + t / tiles, q0 = qfirst + (t % tiles) * QS;
+            const int h = hk * group + ((t / tiles) << pack), q0 = qfirst + (t % tiles) * qt;
             if (!__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.dq_done), t & 1))) { failed = true; break; }
             tc_fence_after_sync();
 #pragma unroll
@@ -565,7 +567,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if (key < a.tk && !key_padded(a.mask, b, key)) queries_of_key(qmask, key, a.tq, a.tk, qa, qb);
         for (int t = 0; t < steps && !failed; ++t) {
             const int st = t & 1, aph = (t >> 1) & 1, ph = t & 1;
-            const int c0 = qfirst + (t % tiles) * QS + col0;   // the first query of this thread's columns
+            // The step's columns whose query sees this thread's key: [ca, cb), from the tokens' interval.
+            const int q0 = qfirst + (t % tiles) * qt, c0 = col0;   // c0: the first of this thread's columns
+            const int ca = min(max(qa - q0, 0), qt) << pack, cb = min(max(qb - q0, 0), qt) << pack;
             if (!__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.aux_full[st]), aph) && mbar_wait(BAR(sh.bar.s_full), ph))) {
                 failed = true;
                 break;
@@ -575,14 +579,14 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             tmem_ld32(t_lane + COL_ST + col0, *reinterpret_cast<uint32_t(*)[32]>(&p[0]));
             tmem_ld_wait();
             const QAux &aux = sh.aux[st];
-            const bool all_of_them = c0 >= qa && c0 + KQW <= qb;
+            const bool all_of_them = c0 >= ca && c0 + KQW <= cb;
             if (!__all_sync(0xffffffffu, all_of_them)) {
                 // Some key of the warp is not seen by all of these queries: hide what it is not seen by
                 // before the exponentials, in a pass of its own so that the common, unmasked step pays
                 // nothing for it.  A key that is seen by NONE of them - a key of another sequence of the
                 // packed batch, in a block of keys that straddles two - needs no comparisons: where every key
                 // of the warp is seen by all or by none, those rows are simply set.
-                const bool none_of_them = c0 + KQW <= qa || c0 >= qb || qb <= qa;
+                const bool none_of_them = c0 + KQW <= ca || c0 >= cb || cb <= ca;
                 if (__all_sync(0xffffffffu, all_of_them || none_of_them)) {
                     if (none_of_them) {
 #pragma unroll
@@ -590,7 +594,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     }
                 } else {
 #pragma unroll
-                    for (int c = 0; c < KQW; ++c) p[c] = (c0 + c >= qa && c0 + c < qb) ? p[c] : -INFINITY;
+                    for (int c = 0; c < KQW; ++c) p[c] = (c0 + c >= ca && c0 + c < cb) ? p[c] : -INFINITY;
                 }
             }
             // P^T over the first half of the f32 columns this thread has just read, in two halves of
@@ -741,11 +745,13 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     DqTail &sh = *reinterpret_cast<DqTail *>(v_s + 2 * BIG_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.x;
+    // The tile: 128 >> pack tokens from m0 on, of 1 << pack heads from h0 on; row = token << pack | head.
+    const int pack = a.pack;
+    const int h0 = blockIdx.x << pack;
     const int qt = gridDim.y - 1 - blockIdx.y;
     const int b = blockIdx.z;
-    const int hk = h / (a.hq / a.hkv);
-    const int m0 = qt * BIG;
+    const int hk = h0 / (a.hq / a.hkv);
+    const int m0 = qt * (BIG >> pack);
     auto BAR = [&](uint64_t &x) { return smem_u32(&x); };
 
     if (threadIdx.x == 0) {
@@ -776,10 +782,10 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // for them at the end: shared memory must not be written behind a block that has left.)
         const uint32_t full = BAR(sh.bar.res_full);
         mbar_expect_tx(full, 2 * BIG_BYTES);
-        tma_load_4d(smem_u32(q_s), &tm_q, full, 0, h, m0, b);
-        if constexpr (HD > 64) tma_load_4d(smem_u32(q_s + BIG_HALF), &tm_q, full, 64, h, m0, b);
-        tma_load_4d(smem_u32(do_s), &tm_do, full, 0, h, m0, b);
-        if constexpr (HD > 64) tma_load_4d(smem_u32(do_s + BIG_HALF), &tm_do, full, 64, h, m0, b);
+        tma_load_4d(smem_u32(q_s), &tm_q, full, 0, h0, m0, b);
+        if constexpr (HD > 64) tma_load_4d(smem_u32(q_s + BIG_HALF), &tm_q, full, 64, h0, m0, b);
+        tma_load_4d(smem_u32(do_s), &tm_do, full, 0, h0, m0, b);
+        if constexpr (HD > 64) tma_load_4d(smem_u32(do_s + BIG_HALF), &tm_do, full, 64, h0, m0, b);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&sh.tmem_base), 512);
@@ -790,7 +796,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int r = lane_base + lane;
     int lo = a.tk, hi = 0;
     if (warp >= 2) {
-        row_bounds_warp(a.mask, m0 + r, a.tq, a.tk, lo, hi);
+        row_bounds_warp(a.mask, m0 + (r >> pack), a.tq, a.tk, lo, hi);
         int wlo = warp_min_i(hi > lo ? lo : a.tk), whi = warp_max_i(hi > lo ? hi : 0);
         if (lane == 0) { sh.red_lo[sw] = wlo; sh.red_hi[sw] = whi; }
     }
@@ -886,7 +892,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
     } else {
         // ---------------- elementwise: a query row and QW of the step's keys per thread ----------------
-        const int row = m0 + r;
+        const int row = m0 + (r >> pack), h = h0 + (r & ((1 << pack) - 1));
         const int cg = sw >> 2, col0 = cg * QW;
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
         const bool padded = a.mask.kind == 1;
@@ -998,8 +1004,8 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             fence_proxy_async_smem();
             named_barrier(1, QEW_THREADS);
             if (sw == 0 && lane == 0 && sh.tile_bad == 0) {
-                tma_store_4d(&tm_dq, smem_u32(q_s), 0, h, m0, b);
-                if constexpr (HD > 64) tma_store_4d(&tm_dq, smem_u32(q_s + BIG_HALF), 64, h, m0, b);
+                tma_store_4d(&tm_dq, smem_u32(q_s), 0, h0, m0, b);
+                if constexpr (HD > 64) tma_store_4d(&tm_dq, smem_u32(q_s + BIG_HALF), 64, h0, m0, b);
                 tma_store_commit();
                 tma_store_wait_read();
             }
@@ -1054,7 +1060,8 @@ static cudaError_t launch_t(const Sm100BwdMaps &m, Sm100BwdArgs a, cudaStream_t 
     } else {
         e = cudaFuncSetAttribute(bwd_dq_sm100_kernel<T, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq<HD>());
         if (e != cudaSuccess) return e;
-        dim3 gq(a.hq, (a.tq + BIG - 1) / BIG, a.b);
+        const int tokens = BIG >> a.pack;
+        dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
         bwd_dq_sm100_kernel<T, HD><<<gq, DQ_THREADS, smem_dq<HD>(), stream>>>(m.q128, m.do128, m.k128, m.v128, m.dq128, a);
         *launches += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

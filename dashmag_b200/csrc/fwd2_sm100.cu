@@ -2,9 +2,8 @@
 // head dimension 128 or 64 (the text below gives the sizes at 128; at 64 the Q / K / V tiles and the O
 // accumulators are half as wide and P V runs 128 x 64 x 16).
 //
-// A block owns TWO tiles of 128 queries that sweep the same keys - two query heads of one
-// key-value group over the same rows (grouped heads, even group size), or two consecutive row
-// tiles of one head - so that every K / V tile fetched from L2 feeds twice the arithmetic, and it
+// A block owns TWO tiles of 128 query rows that sweep the same keys - consecutive tiles of 128 / P
+// tokens x P heads of one key-value group, P the power of two sm100.cu picks (pack_log2) - so that every K / V tile fetched from L2 feeds twice the arithmetic, and it
 // runs two softmax warpgroups, one per tile, so that every scheduler has two warps of elementwise
 // work to interleave.  384 threads:
 //   warp 0, 10  one lane each issues the TMA tile loads: warp 0 both Q tiles once and then the K
@@ -140,13 +139,12 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qt = gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
     const int b = blockIdx.z;
-    // Tile t of the block: head h0 + t over rows m0 (paired heads), or head h0 over rows m0 + 128 t.
-    const int pair = a.pair_heads;
-    const int h0 = pair ? 2 * blockIdx.x : blockIdx.x;
+    // Tile t of the block: BT = 128 >> pack tokens from m_base + t BT on, of 1 << pack heads from h0 on.
+    const int pack = a.pack, bt = BM >> pack;
+    const int h0 = blockIdx.x << pack;
     const int hk = h0 / (a.hq / a.hkv);
-    const int m_base = pair ? qt * BM : qt * NT * BM;
-    auto tile_head = [&](int t) { return pair ? h0 + t : h0; };
-    auto tile_row0 = [&](int t) { return pair ? m_base : m_base + t * BM; };
+    const int m_base = qt * NT * bt;
+    auto tile_row0 = [&](int t) { return m_base + t * bt; };
     auto BAR = [&](uint64_t &x) { return smem_u32(&x); };
 
     if (threadIdx.x == 0) {
@@ -182,7 +180,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             const uint32_t dst = smem_u32(q_s + t * Q_BYTES);
 #pragma unroll
             for (int half = 0; half < HALVES; ++half)
-                tma_load_4d(dst + half * Q_HALF, &tm_q, qf, 64 * half, tile_head(t), tile_row0(t), b);
+                tma_load_4d(dst + half * Q_HALF, &tm_q, qf, 64 * half, h0, tile_row0(t), b);
         }
     }
     if (warp == 1) {
@@ -198,7 +196,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int r = lane_base + lane;                // row of the tile
     int lo = a.tk, hi = 0;
     if (warp >= 2 && warp < 2 + 4 * NT) {
-        row_bounds_warp(a.mask, tile_row0(tile) + r, a.tq, a.tk, lo, hi);
+        row_bounds_warp(a.mask, tile_row0(tile) + (r >> pack), a.tq, a.tk, lo, hi);
         int wlo = warp_min_i(hi > lo ? lo : a.tk), whi = warp_max_i(hi > lo ? hi : 0);
         if (lane == 0) { sh.red_lo[sw] = wlo; sh.red_hi[sw] = whi; }
     }
@@ -336,8 +334,8 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
     } else {
         // ---------------- softmax of one tile, one row per thread ----------------
-        const int t = tile, h = tile_head(t);
-        const int row = tile_row0(t) + r;
+        const int t = tile, h = h0 + (r & ((1 << pack) - 1));
+        const int row = tile_row0(t) + (r >> pack);
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
         const bool padded = a.mask.kind == 1;
         const float2 sl2 = make_float2(a.scale_log2, a.scale_log2);
@@ -504,7 +502,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 uint8_t *stage = q_s + t * Q_BYTES;
 #pragma unroll
                 for (int half = 0; half < HALVES; ++half)
-                    tma_store_4d(&tm_o, smem_u32(stage + half * Q_HALF), 64 * half, h, tile_row0(t), b);
+                    tma_store_4d(&tm_o, smem_u32(stage + half * Q_HALF), 64 * half, h0, tile_row0(t), b);
                 tma_store_commit();
                 tma_store_wait_read();
             }
@@ -536,7 +534,8 @@ cudaError_t launch_fwd2_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &t
 
 cudaError_t launch_fwd2_sm100(int dtype, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv,
                               const CUtensorMap &to, const Sm100FwdArgs &a, cudaStream_t stream) {
-    dim3 grid(a.pair_heads ? a.hq / 2 : a.hq, a.pair_heads ? (a.tq + BM - 1) / BM : (a.tq + NT * BM - 1) / (NT * BM), a.b);
+    const int tokens = (NT * BM) >> a.pack;   // per block
+    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
     if (dtype == DASH_ATTN_BF16)
         return a.d == 64 ? launch_fwd2_t<__nv_bfloat16, 64>(grid, tq, tk, tv, to, a, stream)
                          : launch_fwd2_t<__nv_bfloat16, 128>(grid, tq, tk, tv, to, a, stream);

@@ -106,11 +106,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     Shared &sh = *reinterpret_cast<Shared *>(v_s + NS * TILE_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.x;
+    // The tile: 128 >> pack tokens from m0 on, of 1 << pack heads from h0 on; row = token << pack | head.
+    const int pack = a.pack;
+    const int h0 = blockIdx.x << pack;
     const int qt = gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
     const int b = blockIdx.z;
-    const int hk = h / (a.hq / a.hkv);
-    const int m0 = qt * BM;
+    const int hk = h0 / (a.hq / a.hkv);
+    const int m0 = qt * (BM >> pack);
 
     const uint32_t q_full = smem_u32(&sh.bar.q_full), o_ready = smem_u32(&sh.bar.o_ready);
     auto BAR = [&](uint64_t (&arr)[2], int i) { return smem_u32(&arr[i]); };
@@ -144,7 +146,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int r = lane_base + lane;                // row of the tile (softmax threads)
     int lo = a.tk, hi = 0;
     if (warp >= 2 && warp < 6) {
-        row_bounds_warp(a.mask, m0 + r, a.tq, a.tk, lo, hi);
+        row_bounds_warp(a.mask, m0 + (r >> pack), a.tq, a.tk, lo, hi);
         int wlo = warp_min_i(hi > lo ? lo : a.tk), whi = warp_max_i(hi > lo ? hi : 0);
         if (lane == 0) { sh.red_lo[sw] = wlo; sh.red_hi[sw] = whi; }
     }
@@ -166,7 +168,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (lane == 0 && n_tiles > 0) {
             mbar_expect_tx(q_full, TILE_BYTES);
 #pragma unroll
-            for (int part = 0; part < PARTS; ++part) tma_load_4d(smem_u32(q_s + part * HALF_BYTES), &tm_q, q_full, 64 * part, h, m0, b);
+            for (int part = 0; part < PARTS; ++part) tma_load_4d(smem_u32(q_s + part * HALF_BYTES), &tm_q, q_full, 64 * part, h0, m0, b);
             for (int j = 0; j < n_tiles && !failed; ++j) {
                 const int st = j % NS, ph = (j / NS) & 1, k0 = kmin + j * BN;
                 if (!mbar_wait(BAR(sh.bar.k_empty, st), ph ^ 1)) { failed = true; break; }
@@ -246,7 +248,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
     } else {
         // ---------------- softmax, one row per thread ----------------
-        const int row = m0 + r;
+        const int row = m0 + (r >> pack), h = h0 + (r & ((1 << pack) - 1));
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
         const bool padded = a.mask.kind == 1;
         float m_ref = -INFINITY, l = 0.f;
@@ -425,7 +427,8 @@ cudaError_t launch_fwd_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk
 
 cudaError_t launch_fwd_sm100(int dtype, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv,
                              const Sm100FwdArgs &a, cudaStream_t stream) {
-    dim3 grid(a.hq, (a.tq + BM - 1) / BM, a.b);
+    const int tokens = BM >> a.pack;
+    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
     if (dtype == DASH_ATTN_BF16)
         return a.d == 256 ? launch_fwd_t<__nv_bfloat16, 256>(grid, tq, tk, tv, a, stream)
                           : launch_fwd_t<__nv_bfloat16, 128>(grid, tq, tk, tv, a, stream);

@@ -16,7 +16,7 @@ struct Sm100FwdArgs {
     void *out;         // [B,Tq,Hq,D] contiguous, the inputs' dtype
     float *lse;        // [B,Tq,Hq]
     MaskArgs mask;
-    int pair_heads;    // two-tile kernel: the block's tiles are two heads of one group (else two row tiles)
+    int pack;          // a tile of 128 rows is 128 >> pack tokens of 1 << pack heads of one group, row = token << pack | head
 };
 
 struct Sm100BwdArgs {
@@ -29,6 +29,7 @@ struct Sm100BwdArgs {
     MaskArgs mask;
     int *order;          // scratch: the (key block, key-value head) units in launch order, [B * ceil(Tk / 128) * Hkv]
     float *dq_acc;       // scratch [B,Tq,Hq,D] f32, or null: the query gradient summed by reductions in L2 (the fused form)
+    int pack;            // a tile of 128 query rows is 128 >> pack tokens of 1 << pack heads of one group
 };
 
 // Tensor maps of the backward: every tensor with boxes of 128 rows, resident or streamed.
