@@ -485,6 +485,7 @@ bwd256_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     extern __shared__ __align__(1024) uint8_t smem256[];
     const int qt = gridDim.y - 1 - blockIdx.y;   // later (longer, under causality) tiles first
     bwd256_pass<T, PASS_DQ>(&tm_q, &tm_do, &tm_k, &tm_v, a, smem256, blockIdx.z, qt * (ROWS >> a.pack), blockIdx.x << a.pack);
+    end_beside();
 }
 
 // blockIdx.x: the (key block, key-value head) unit in the plan's order; blockIdx.y: 0 the dK pass (the
@@ -494,6 +495,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 bwd256_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do, const Sm100BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem256[];
+    allow_beside();   // dq
     const int nkb = (a.tk + ROWS - 1) / ROWS;
     const int unit = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
     const int item = unit / a.hkv, hk = unit - item * a.hkv;
@@ -504,25 +506,24 @@ bwd256_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
 namespace {
 template <typename T>
-cudaError_t launch256_t(const Sm100BwdMaps &m, Sm100BwdArgs a, cudaStream_t stream, int *launches) {
+cudaError_t launch256_t(const Sm100BwdMaps &m, const Sm100BwdArgs &a, cudaStream_t stream, int *launches) {
     constexpr size_t smem = smem_bytes(PASS_DQ);
     static_assert(smem_bytes(PASS_DK) == smem && smem_bytes(PASS_DV) <= smem, "one size for the three passes");
     cudaError_t e = cudaFuncSetAttribute(bwd256_dq_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(bwd256_dkdv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int tokens = ROWS >> a.pack;
-    dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
-    bwd256_dq_kernel<T><<<gq, THREADS, smem, stream>>>(m.q128, m.do128, m.k128, m.v128, a);
-    *launches += 1;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = launch_bwd_plan(a, stream, launches)) != cudaSuccess) return e;
     const long long units = (long long)a.b * ((a.tk + ROWS - 1) / ROWS) * a.hkv;
     if (units > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     dim3 gk((unsigned)units, 2, 1);
     bwd256_dkdv_kernel<T><<<gk, THREADS, smem, stream>>>(m.k128, m.v128, m.q128, m.do128, a);
     *launches += 1;
-    return cudaGetLastError();
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // dq's short blocks beside the last waves of dk and dv (see bwd_sm100.cu).
+    const int tokens = ROWS >> a.pack;
+    dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
+    *launches += 1;
+    return launch_beside(bwd256_dq_kernel<T>, gq, THREADS, smem, stream, true, m.q128, m.do128, m.k128, m.v128, a);
 }
 }  // namespace
 

@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) bwd_plan_kernel(const Sm100BwdAr
     __shared__ int work[PLAN_MAX], seq[PLAN_MAX], run_top[PLAN_MAX];
     __shared__ unsigned short run_of[PLAN_MAX], run_first[PLAN_MAX], run_len[PLAN_MAX];   // all below PLAN_MAX
     __shared__ int runs;
+    allow_beside();   // delta, which reads nothing of this
     const int nkb = (a.tk + BIG - 1) / BIG;
     if (threadIdx.x == 0) runs = 0;
     for (int i = threadIdx.x; i < items; i += PLAN_THREADS) {
@@ -259,6 +260,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     Tail &sh = *reinterpret_cast<Tail *>(FUSED ? red_s + 2 * RED_SLOT : do_s + DOS * BIG_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (!FUSED) allow_beside();   // dq
     // Units are taken in the order the plan kernel left (without one: in index order, the heads of a
     // key block side by side).
     const int nkb = (a.tk + BIG - 1) / BIG;
@@ -1020,6 +1022,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         tc_fence_after_sync();
         tmem_dealloc(tmem, 512);
     }
+    end_beside();
 }
 
 // =================================================================================================
@@ -1057,21 +1060,25 @@ static cudaError_t launch_t(const Sm100BwdMaps &m, Sm100BwdArgs a, cudaStream_t 
     if (fused) {
         // The accumulator starts at zero; every key block adds its share as it gets there.
         if ((e = cudaMemsetAsync(a.dq_acc, 0, sizeof(float) * (size_t)dq_elems, stream)) != cudaSuccess) return e;
-    } else {
+    }
+    const long long items = (long long)a.b * ((a.tk + BIG - 1) / BIG);
+    if (items * a.hkv > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    e = fused ? launch_dkdv<T, HD, true>(m, a, items, stream) : launch_dkdv<T, HD, false>(m, a, items, stream);
+    *launches += 1;
+    if (e != cudaSuccess) return e;
+    if (!fused) {
+        // dq's blocks are short (a tile of queries), dkdv's as long as their key block's sweep over the whole group:
+        // launched first, in falling order of work, dkdv leaves multiprocessors idle only at its end, and dq fills them.  (8 packed sequences,
+        // 16384 tokens, 32 / 8 heads: the step 1898 -> 1859 us; one sequence of 16384, 8 / 1 heads - 128 units, the longest
+        // of which takes as long as all of them spread evenly take twice over: 2699 -> 2248 us; D 256, 6144 tokens, 8 / 2
+        // heads: 894 -> 761 us.)
         e = cudaFuncSetAttribute(bwd_dq_sm100_kernel<T, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq<HD>());
         if (e != cudaSuccess) return e;
         const int tokens = BIG >> a.pack;
         dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
-        bwd_dq_sm100_kernel<T, HD><<<gq, DQ_THREADS, smem_dq<HD>(), stream>>>(m.q128, m.do128, m.k128, m.v128, m.dq128, a);
         *launches += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return launch_beside(bwd_dq_sm100_kernel<T, HD>, gq, DQ_THREADS, smem_dq<HD>(), stream, true, m.q128, m.do128, m.k128, m.v128, m.dq128, a);
     }
-    const long long items = (long long)a.b * ((a.tk + BIG - 1) / BIG);
-    if ((e = launch_bwd_plan(a, stream, launches)) != cudaSuccess) return e;
-    if (items * a.hkv > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    e = fused ? launch_dkdv<T, HD, true>(m, a, items, stream) : launch_dkdv<T, HD, false>(m, a, items, stream);
-    *launches += 1;
-    if (e != cudaSuccess || !fused) return e;
     const long long n8 = dq_elems / 8;
     bwd_dq_finish_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(a.dq_acc, static_cast<T *>(a.dq), a.scale, n8);
     *launches += 1;

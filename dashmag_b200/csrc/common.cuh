@@ -165,6 +165,35 @@ __device__ __forceinline__ int warp_max_i(int x) {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Kernels of one call that run side by side
+// ---------------------------------------------------------------------------------------------
+// A kernel launched with launch_beside may start as soon as every block of the kernel in front of it
+// has run allow_beside (or has left): its blocks take the multiprocessors that kernel's last wave leaves
+// idle.  It must not touch what that kernel writes, and what both read was complete before either
+// began.  Whatever comes next in the stream waits for the second kernel only, so that kernel's last block waits
+// for the first before it leaves (end_beside; a no-op in an ordinary launch).
+__device__ __forceinline__ void allow_beside() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void end_beside() {
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_beside(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool beside, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Arguments of the generic kernels
 // ---------------------------------------------------------------------------------------------
 struct TrainArgs {

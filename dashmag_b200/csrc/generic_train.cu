@@ -186,14 +186,16 @@ __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq;
     int64_t row = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
-    if (row >= rows) return;
-    int h = (int)(row % a.hq);
-    int64_t bt = row / a.hq;
-    int t = (int)(bt % a.tq), b = (int)(bt / a.tq);
-    float sum = 0.f;
-    for (int c = lane; c < a.d; c += 32) sum = fmaf(load_f32<T>(a.dout, b, t, h, c), load_f32<T>(a.o, b, t, h, c), sum);
-    sum = warp_sum(sum);
-    if (lane == 0) a.delta[row] = sum;
+    if (row < rows) {
+        int h = (int)(row % a.hq);
+        int64_t bt = row / a.hq;
+        int t = (int)(bt % a.tq), b = (int)(bt / a.tq);
+        float sum = 0.f;
+        for (int c = lane; c < a.d; c += 32) sum = fmaf(load_f32<T>(a.dout, b, t, h, c), load_f32<T>(a.o, b, t, h, c), sum);
+        sum = warp_sum(sum);
+        if (lane == 0) a.delta[row] = sum;
+    }
+    end_beside();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -544,6 +546,7 @@ __global__ void __launch_bounds__(THREADS) delta_rows_kernel(TrainArgs a) {
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
     if (row < rows && sub == 0) a.delta[row] = sum;
+    end_beside();
 }
 
 // Whether every row of the view starts on a 16-byte boundary and is contiguous.
@@ -552,29 +555,26 @@ static bool rows_16b(const View4 &v) {
 }
 
 template <typename T>
-static cudaError_t delta_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
+static cudaError_t delta_t(const TrainArgs &a, cudaStream_t stream, int *launches, bool beside) {
     int64_t rows = (int64_t)a.b * a.tq * a.hq;
     if (sizeof(T) == 2 && (a.d == 64 || a.d == 128 || a.d == 256) && rows_16b(a.dout) && rows_16b(a.o)) {
         const int64_t per_block = (32 / (a.d / 8)) * (THREADS / 32);
         const unsigned blocks = (unsigned)((rows + per_block - 1) / per_block);
-        if (a.d == 64) delta_rows_kernel<T, 64><<<blocks, THREADS, 0, stream>>>(a);
-        else if (a.d == 128) delta_rows_kernel<T, 128><<<blocks, THREADS, 0, stream>>>(a);
-        else delta_rows_kernel<T, 256><<<blocks, THREADS, 0, stream>>>(a);
         *launches += 1;
-        return cudaGetLastError();
+        return launch_beside(a.d == 64 ? delta_rows_kernel<T, 64> : a.d == 128 ? delta_rows_kernel<T, 128> : delta_rows_kernel<T, 256>,
+                             dim3(blocks), THREADS, 0, stream, beside, a);
     }
     unsigned blocks = (unsigned)((rows + THREADS / 32 - 1) / (THREADS / 32));
-    generic_delta_kernel<T><<<blocks, THREADS, 0, stream>>>(a);
     *launches += 1;
-    return cudaGetLastError();
+    return launch_beside(generic_delta_kernel<T>, dim3(blocks), THREADS, 0, stream, beside, a);
 }
 
 // delta = rowsum(dO * O) alone, for the tensor-core backward.
-cudaError_t launch_generic_delta(int dtype, const TrainArgs &a, cudaStream_t stream, int *launches) {
+cudaError_t launch_generic_delta(int dtype, const TrainArgs &a, cudaStream_t stream, int *launches, bool beside) {
     switch (dtype) {
-        case 0: return delta_t<float>(a, stream, launches);
-        case 1: return delta_t<__nv_bfloat16>(a, stream, launches);
-        default: return delta_t<__half>(a, stream, launches);
+        case 0: return delta_t<float>(a, stream, launches, beside);
+        case 1: return delta_t<__nv_bfloat16>(a, stream, launches, beside);
+        default: return delta_t<__half>(a, stream, launches, beside);
     }
 }
 

@@ -241,8 +241,6 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
         err = "attention_backward: the driver refused a TMA tensor map over the inputs";
         return cudaSuccess;
     }
-    cudaError_t e = launch_generic_delta(p->dtype, a, stream, launches);
-    if (e != cudaSuccess) return e;
     Sm100BwdArgs f{};
     f.b = p->b; f.tq = p->tq; f.tk = p->tk; f.hq = p->hq; f.hkv = p->hkv; f.d = p->d;
     f.scale = a.scale;
@@ -254,6 +252,11 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
     f.order = static_cast<int *>(workspace);
     f.dq_acc = dq_acc;
     f.pack = pack;
+    // The plan's one block and delta run side by side; then dkdv, and dq beside its last waves (neither reads what
+    // the other writes).
+    cudaError_t e = launch_bwd_plan(f, stream, launches);
+    if (e == cudaSuccess) e = launch_generic_delta(p->dtype, a, stream, launches, f.order != nullptr);
+    if (e != cudaSuccess) return e;
     if (p->d == 256) return launch_bwd256_sm100(p->dtype, m, f, stream, launches);
     return launch_bwd_sm100(p->dtype, m, f, stream, launches);
 }
