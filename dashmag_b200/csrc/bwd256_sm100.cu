@@ -164,7 +164,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         }
     }
     tc_fence_before_sync();
-    __syncthreads();
+    const int any_row = __syncthreads_or(hi > lo);   // a block of padding keys has no gradient to sum
     tc_fence_after_sync();
     const uint32_t tmem = sh.tmem_base;
     const bool aborted = sh.abort != 0;
@@ -175,6 +175,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         int cmin = a.tk, cmax = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) { cmin = min(cmin, sh.red_lo[i]); cmax = max(cmax, sh.red_hi[i]); }
+        if (a.mask.kind == 1) trim_padded(a.mask, b, cmin, cmax);
         col_first = cmin;
         tiles = cmax > cmin ? (cmax - cmin + ROWS - 1) / ROWS : 0;
         head0 = res_head / group;
@@ -182,7 +183,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         int qfirst, qend;
         query_range(a.mask, row0, min(row0 + ROWS, a.tk), a.tq, a.tk, qfirst, qend);
         col_first = qfirst;
-        tiles = qend > qfirst ? (qend - qfirst + qt - 1) / qt : 0;
+        tiles = any_row && qend > qfirst ? (qend - qfirst + qt - 1) / qt : 0;
         head0 = res_head * group;
     }
     const int steps = aborted ? 0 : (ROWS_ARE_QUERIES ? tiles : tiles * (group >> pack));
@@ -343,6 +344,10 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
             l2 = x == -INFINITY ? INFINITY : x * LOG2E;
             dl = a.delta[at];
         }
+        // The padding flags of a step, asked for one step ahead (as in the forward).
+        bool hidden = false;
+        auto flags = [&](int key) { hidden = key >= a.tk || key_padded(a.mask, b, key); };
+        if (padded && steps > 0) flags(step_col0(0) + col0 + lane);
         for (int t = 0; t < steps && !failed; ++t) {
             const int st = t & 1, ph2 = (t >> 1) & 1;
             // The step's columns this thread's row sees, [ca, cb): keys (DQ), or tokens << pack | head (DK / DV).
@@ -351,8 +356,8 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
             const int ca = min(max(lo - s0, 0), span) << shift, cb = min(max(hi - s0, 0), span) << shift;
             uint32_t pb = 0;
             if (padded) {
-                const int key = s0 + c0 + lane;
-                pb = __ballot_sync(0xffffffffu, key >= a.tk || key_padded(a.mask, b, key));
+                pb = __ballot_sync(0xffffffffu, hidden);
+                if (t + 1 < steps) flags(s0 + ROWS + c0 + lane);
             }
             if (!ROWS_ARE_QUERIES && !__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.aux_full[st]), ph2))) { failed = true; break; }
             const uint32_t s_at = PASS == PASS_DV ? st * 128 : COL_S;
@@ -367,12 +372,12 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 __syncwarp();
                 if (lane == 0) mbar_arrive(BAR(sh.bar.s_free));
             }
-            const bool clear = !padded && c0 >= ca && c0 + CW <= cb;
+            const bool clear = pb == 0 && c0 >= ca && c0 + CW <= cb;
             if (!__all_sync(0xffffffffu, clear)) {
                 // A row that sees none of these columns (it belongs to another sequence of the packed batch, or
                 // its interval ends before them) needs no comparisons: where every row of the warp sees all or
                 // none, those rows are simply set.
-                const bool none = !padded && (cb <= c0 || ca >= c0 + CW || cb <= ca);
+                const bool none = pb == 0xffffffffu || cb <= c0 || ca >= c0 + CW || cb <= ca;
                 if (__all_sync(0xffffffffu, clear || none)) {
                     if (none) {
 #pragma unroll

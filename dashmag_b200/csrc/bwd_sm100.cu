@@ -315,6 +315,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     int qfirst, qend;
     query_range(a.mask, k0, k1, a.tq, a.tk, qfirst, qend);
+    // A key block that is padding from end to end has no gradient to sum.
+    const bool open = threadIdx.x < BIG && k0 + (int)threadIdx.x < k1 && !key_padded(a.mask, b, k0 + threadIdx.x);
     // The per-query vectors of every step need each query's key interval, a binary search over the
     // sequences' offsets: from shared memory when they fit, so that it costs tens of cycles a probe
     // instead of a trip to L2.
@@ -329,13 +331,13 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         qmask.idx_bytes = 4;
     }
     tc_fence_before_sync();
-    __syncthreads();
+    const int any_open = __syncthreads_or(open);
     tc_fence_after_sync();
     const uint32_t tmem = sh.tmem_base;
     const bool aborted = sh.abort != 0;
     // A streamed tile of 128 rows: `qt` tokens of 1 << pack heads of the group, row = token << pack | head.
     const int pack = a.pack, qt = QS >> pack;
-    const int tiles = (!aborted && qend > qfirst) ? (qend - qfirst + qt - 1) / qt : 0;
+    const int tiles = (!aborted && any_open && qend > qfirst) ? (qend - qfirst + qt - 1) / qt : 0;
     const int steps = tiles * (group >> pack);
     bool failed = aborted;
     // TMEM columns: S^T at 0, dP^T at 128 (each with its 16-bit twin over the first half of every
@@ -710,7 +712,7 @@ constexpr int DQ_KS = 3;   // stages of the K ring: a K tile serves S of its ste
 constexpr int QCG = 2;
 constexpr int QW = BIG / QCG;
 constexpr int QEW_THREADS = 32 * 4 * QCG;
-static_assert(QW % 32 == 0, "whole 32-column TMEM loads per thread");
+static_assert(QW == 64, "two 32-column TMEM loads and two words of padding flags per thread");
 
 struct DqBarriers {
     uint64_t res_full;
@@ -810,6 +812,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     int kmin = a.tk, kmax = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }  // the first four warps cover every row
+    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
     const int steps = (!aborted && kmax > kmin) ? (kmax - kmin + BIG - 1) / BIG : 0;
     bool failed = aborted;
     // TMEM columns: S at 0, dP[2] at 128 / 256 (dS over the first half of every group of 32 columns), dQ at 384.
@@ -905,16 +908,23 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             l2 = x == -INFINITY ? INFINITY : x * LOG2E;
             dl = a.delta[at];
         }
-        for (int t = 0; t < steps && !failed; ++t) {
-            const int st = t & 1, c0 = kmin + t * BIG + col0;
-            uint32_t pb[QW / 32];
+        // The padding flags of a step, asked for one step ahead (as in the forward).
+        bool hidden[QW / 32] = {false, false};
+        auto flags = [&](int c0) {
 #pragma unroll
             for (int g = 0; g < QW / 32; ++g) {
-                pb[g] = 0;
-                if (padded) {
-                    const int key = c0 + 32 * g + lane;
-                    pb[g] = __ballot_sync(0xffffffffu, key >= a.tk || key_padded(a.mask, b, key));
-                }
+                const int key = c0 + 32 * g + lane;
+                hidden[g] = key >= a.tk || key_padded(a.mask, b, key);
+            }
+        };
+        if (padded && steps > 0) flags(kmin + col0);
+        for (int t = 0; t < steps && !failed; ++t) {
+            const int st = t & 1, c0 = kmin + t * BIG + col0;
+            uint32_t pb[QW / 32] = {0, 0};
+            if (padded) {
+#pragma unroll
+                for (int g = 0; g < QW / 32; ++g) pb[g] = __ballot_sync(0xffffffffu, hidden[g]);
+                if (t + 1 < steps) flags(c0 + BIG);
             }
             if (!__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.s_full), t & 1))) { failed = true; break; }
             tc_fence_after_sync();
@@ -926,11 +936,11 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(sh.bar.s_free));
 
-            const bool clear = !padded && c0 >= lo && c0 + QW <= hi;
+            const bool clear = (pb[0] | pb[1]) == 0 && c0 >= lo && c0 + QW <= hi;
             // ... or sees none of them: a row of another sequence of the packed batch (a tile that straddles two
             // sequences sweeps the first one's keys for the second one's rows too), or one whose interval ends
             // before these keys.  Such a row needs no masking pass: against +inf its exponentials are exact zeros.
-            const bool none = !padded && (hi <= c0 || lo >= c0 + QW || hi <= lo);
+            const bool none = (pb[0] & pb[1]) == 0xffffffffu || hi <= c0 || lo >= c0 + QW || hi <= lo;
             if (!__all_sync(0xffffffffu, clear || none)) {
 #pragma unroll
                 for (int c = 0; c < QW; ++c) {

@@ -143,6 +143,37 @@ __device__ __forceinline__ bool key_padded(const MaskArgs &m, int b, int key) {
                            : static_cast<const unsigned char *>(m.kp)[at] != 0;
 }
 
+// (declared below)
+__device__ __forceinline__ int warp_max_i(int x);
+__device__ __forceinline__ int warp_min_i(int x);
+
+// A block's sweep [kmin, kmax) without the padded keys at its ends: right- and left-padded batches are swept no further
+// than their tokens go.  All 32 lanes call and get one answer, the same in every warp; 256 flags a look, from either
+// end, so that a sweep that is not padded there pays one trip to memory.  (kmax <= kmin: no key is left.)
+static __device__ __noinline__ void trim_padded(const MaskArgs &m, int b, int &kmin, int &kmax) {
+    const int lane = threadIdx.x & 31;
+    int last = -1;
+    while (kmax > kmin && last < 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int key = kmax - 1 - 32 * i - lane;
+            if (key >= kmin && !key_padded(m, b, key)) last = max(last, key);
+        }
+        last = warp_max_i(last);
+        kmax = last >= 0 ? last + 1 : kmax - 256;
+    }
+    int first = 2147483647;
+    while (kmax > kmin && first == 2147483647) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int key = kmin + 32 * i + lane;
+            if (key < kmax && !key_padded(m, b, key)) first = min(first, key);
+        }
+        first = warp_min_i(first);
+        kmin = first != 2147483647 ? first : kmin + 256;
+    }
+}
+
 __device__ __forceinline__ float warp_max(float x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));

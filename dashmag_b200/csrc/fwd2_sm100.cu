@@ -66,6 +66,7 @@ template <int HD> struct Geo {
 constexpr int THREADS = 384;
 constexpr int V_WARP = 10;
 constexpr int MMA_WARP0 = 1, MMA_WARP1 = 11;   // the issuers of tile 0 and of tile 1, on two schedulers
+static_assert(SN == 64, "two words of padding flags per sub-step");
 constexpr float RESCALE_LOG2 = 8.0f;
 // A row that sees at most this many keys keeps the exact running maximum instead of the lazy one:
 // with few keys one of them often carries most of the weight, and only against the exact maximum is
@@ -207,6 +208,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     int kmin = a.tk, kmax = 0;
 #pragma unroll
     for (int i = 0; i < 4 * NT; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
+    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
     const bool aborted = sh.abort != 0;
     const int subs = (!aborted && kmax > kmin) ? (kmax - kmin + SN - 1) / SN : 0;   // sub-steps of 64 keys
     const int steps = (subs + 1) / 2;                                                // K / V tiles of 128 keys
@@ -341,15 +343,24 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const float2 sl2 = make_float2(a.scale_log2, a.scale_log2);
         float m_ref = -INFINITY, l = 0.f;
         const float rescale_at = hi - lo <= EXACT_KEYS ? 0.f : RESCALE_LOG2;
+        // The padding flags of a sub-step are asked for one sub-step ahead: a trip to memory between the wait for S and
+        // the maximum would be the longest link of the step.
+        bool hidden[SN / 32] = {false, false};
+        auto flags = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < SN / 32; ++i) {
+                const int key = k0 + i * 32 + lane;
+                hidden[i] = key >= a.tk || key_padded(a.mask, b, key);
+            }
+        };
+        if (padded && subs > 0) flags(kmin);
         for (int u = 0; u < subs && !failed; ++u) {
             const int k0 = kmin + u * SN, buf = u & 1;
             uint32_t pb[SN / 32] = {0, 0};
             if (padded) {
 #pragma unroll
-                for (int i = 0; i < SN / 32; ++i) {
-                    const int key = k0 + i * 32 + lane;
-                    pb[i] = __ballot_sync(0xffffffffu, key >= a.tk || key_padded(a.mask, b, key));
-                }
+                for (int i = 0; i < SN / 32; ++i) pb[i] = __ballot_sync(0xffffffffu, hidden[i]);
+                if (u + 1 < subs) flags(k0 + SN);
             }
             if (!__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.s_full[t][buf]), (u >> 1) & 1))) { failed = true; break; }
             tc_fence_after_sync();
@@ -358,12 +369,12 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             for (int c = 0; c < SN / 32; ++c) tmem_ld32(t_lane + COL_S(t, buf) + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
             tmem_ld_wait();
 
-            const bool clear = !padded && k0 >= lo && k0 + SN <= hi;  // the row sees the whole sub-step
+            const bool clear = (pb[0] | pb[1]) == 0 && k0 >= lo && k0 + SN <= hi;  // the row sees the whole sub-step
             // ... or nothing of it: a row of another sequence of the packed batch (a tile that straddles two
             // sequences sweeps the first one's keys for the second one's rows too), or one whose interval ends
             // before the sub-step.  Such a row needs no look at its scores: its maximum is -inf and its
             // exponentials are taken against -inf, which makes them exact zeros.
-            const bool none = !padded && (hi <= k0 || lo >= k0 + SN || hi <= lo);
+            const bool none = (pb[0] & pb[1]) == 0xffffffffu || hi <= k0 || lo >= k0 + SN || hi <= lo;
             if (!__all_sync(0xffffffffu, clear || none)) {
 #pragma unroll
                 for (int c = 0; c < SN; ++c) {

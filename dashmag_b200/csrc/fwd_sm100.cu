@@ -157,6 +157,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int kmin = a.tk, kmax = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
+    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
     // Once a bounded wait has run out anywhere, later blocks do nothing: the call has failed and
     // the host will say so; there is no point in timing out thousands of times.
     const bool aborted = sh.abort != 0;
@@ -253,17 +254,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const bool padded = a.mask.kind == 1;
         float m_ref = -INFINITY, l = 0.f;
         const float rescale_at = hi - lo <= EXACT_KEYS ? 0.f : RESCALE_LOG2;
+        // The tile's 128 padding flags as four words; every warp gathers its own copy, so that no softmax
+        // warp ever waits on another, and asks for it one tile ahead.
+        bool hidden[4] = {false, false, false, false};
+        auto flags = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int key = k0 + i * 32 + lane;
+                hidden[i] = key >= a.tk || key_padded(a.mask, b, key);
+            }
+        };
+        if (padded && n_tiles > 0) flags(kmin);
         for (int j = 0; j < n_tiles && !failed; ++j) {
             const int st = j & 1, ph = (j >> 1) & 1, k0 = kmin + j * BN;
             uint32_t pb[4] = {0, 0, 0, 0};
             if (padded) {
-                // The tile's 128 padding flags as four words; every warp gathers its own copy, so
-                // that no softmax warp ever waits on another.
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int key = k0 + i * 32 + lane;
-                    pb[i] = __ballot_sync(0xffffffffu, key >= a.tk || key_padded(a.mask, b, key));
-                }
+                for (int i = 0; i < 4; ++i) pb[i] = __ballot_sync(0xffffffffu, hidden[i]);
+                if (j + 1 < n_tiles) flags(k0 + BN);
             }
             if (!__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.s_full, st), ph))) { failed = true; break; }
             tc_fence_after_sync();
@@ -272,11 +280,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             for (int c = 0; c < 4; ++c) tmem_ld32(t_lane + st * BN + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
             tmem_ld_wait();
 
-            const bool clear = !padded && k0 >= lo && k0 + BN <= hi;  // the row sees the whole tile
+            const bool clear = (pb[0] | pb[1] | pb[2] | pb[3]) == 0 && k0 >= lo && k0 + BN <= hi;  // the row sees the whole tile
             // ... or nothing of it (a row of another sequence of the packed batch, or one whose interval ends
             // before the tile): no look at its scores is needed, its maximum is -inf and its exponentials are
             // taken against -inf, which makes them exact zeros.
-            const bool none = !padded && (hi <= k0 || lo >= k0 + BN || hi <= lo);
+            const bool none = (pb[0] & pb[1] & pb[2] & pb[3]) == 0xffffffffu || hi <= k0 || lo >= k0 + BN || hi <= lo;
             if (!__all_sync(0xffffffffu, clear || none)) {
 #pragma unroll
                 for (int c = 0; c < BN; ++c) {
