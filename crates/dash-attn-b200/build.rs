@@ -14,6 +14,7 @@ const SOURCES: &[&str] = &[
     "sm100.cu",
     "fwd_sm100.cu",
     "fwd2_sm100.cu",
+    "fwd_merge.cu",
     "bwd_sm100.cu",
     "bwd256_sm100.cu",
 ];

@@ -309,15 +309,12 @@ int dash_attn_forward(const dash_attn_params *p, const void *q, const void *k, c
         return DASH_ATTN_OK;
     }
     if (!q || !k || !v || !o || !lse) return fail(DASH_ATTN_INVALID, "%s: a tensor pointer is null", op);
-    size_t need = dash_attn_forward_workspace(p);
-    if ((rc = check_workspace(op, workspace, workspace_bytes, need)) != DASH_ATTN_OK) return rc;
-
     dash::TrainArgs a = train_args(p, q, k, v);
     a.out = o;
     a.lse = lse;
     cudaError_t e;
     if (train_path(p, q, k, v, 0) == 1 && aligned16({o})) {
-        e = dash::sm100_forward(p, a, workspace, stream, &launches, g_error);
+        e = dash::sm100_forward(p, a, workspace, workspace_bytes, stream, &launches, g_error);
         if (e == cudaSuccess && !g_error.empty()) return DASH_ATTN_CUDA;
         g_probe[DASH_ATTN_PROBE_TENSOR_CORE_RUNS] += 1;
     } else {

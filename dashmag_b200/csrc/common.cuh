@@ -209,6 +209,10 @@ __device__ __forceinline__ void end_beside() {
         asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A kernel launched with launch_beside that does read what the kernel in front of it writes: its blocks are brought in
+// under that kernel's end and wait here.
+__device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename... P, typename... A>
 inline cudaError_t launch_beside(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool beside, A... args) {
     cudaLaunchConfig_t cfg = {};

@@ -138,7 +138,9 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     Shared &sh = *reinterpret_cast<Shared *>(v_s + NS * KV_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qt = gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
+    const int split = blockIdx.y % a.splits;
+    const int qt = (gridDim.y - 1 - blockIdx.y) / a.splits;  // later (longer, under causality) tiles first
+    if (a.splits > 1) allow_beside();   // the merge
     const int b = blockIdx.z;
     // Tile t of the block: BT = 128 >> pack tokens from m_base + t BT on, of 1 << pack heads from h0 on.
     const int pack = a.pack, bt = BM >> pack;
@@ -209,6 +211,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
     for (int i = 0; i < 4 * NT; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
     if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
+    split_keys(split, a.splits, BN, kmin, kmax);
     const bool aborted = sh.abort != 0;
     const int subs = (!aborted && kmax > kmin) ? (kmax - kmin + SN - 1) / SN : 0;   // sub-steps of 64 keys
     const int steps = (subs + 1) / 2;                                                // K / V tiles of 128 keys
@@ -459,8 +462,38 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // ---------------- epilogue ----------------
         T *out = static_cast<T *>(a.out);
         const int64_t base = ((int64_t)b * a.tq + row) * a.hq + h;
-        if (subs == 0 || failed) {
-            if (row < a.tq && !failed) {
+        if (a.splits > 1 && !failed) {
+            // A part of the row's keys: the normalised f32 row and its log-sum-exp, for the merge.
+            const int64_t at = (int64_t)split * gridDim.z * a.tq * a.hq + base;
+            if (subs == 0) {
+                if (row < a.tq) a.part_lse[at] = -INFINITY;
+            } else if (__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.o_done[t]), 0))) {
+                tc_fence_after_sync();
+                const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll 1
+                for (int c = 0; c < HD / 32; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(t_lane + COL_O(t) + c * 32, o);
+                    tmem_ld_wait();
+                    if (row < a.tq) {
+                        float4 *po = reinterpret_cast<float4 *>(a.part_o + at * HD + c * 32);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            po[e] = make_float4(__uint_as_float(o[4 * e]) * inv, __uint_as_float(o[4 * e + 1]) * inv,
+                                                __uint_as_float(o[4 * e + 2]) * inv, __uint_as_float(o[4 * e + 3]) * inv);
+                    }
+                }
+                if (row < a.tq) {   // (as below)
+                    const float used = __fmul_rn(m_ref, a.scale_log2);
+                    const double slip = (double)used - (double)m_ref * (double)a.scale_log2;
+                    a.part_lse[at] = l > 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
+                }
+                tc_fence_before_sync();
+            } else {
+                failed = true;
+            }
+        } else if (subs == 0 || failed) {
+            if (row < a.tq && !failed && a.splits == 1) {
                 const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
                 for (int c = 0; c < HD / 8; ++c) reinterpret_cast<uint4 *>(out + base * HD)[c] = z;
@@ -503,7 +536,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         } else {
             failed = true;
         }
-        if (steps > 0) {
+        if (steps > 0 && a.splits == 1) {
             // Every warp of the tile gets here (all waits are bounded), whatever became of it: one
             // that gave up marks the tile, and nothing is stored from a tile that is not whole.
             if (failed && lane == 0) sh.tile_bad[t] = 1;
@@ -546,7 +579,7 @@ cudaError_t launch_fwd2_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &t
 cudaError_t launch_fwd2_sm100(int dtype, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv,
                               const CUtensorMap &to, const Sm100FwdArgs &a, cudaStream_t stream) {
     const int tokens = (NT * BM) >> a.pack;   // per block
-    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
+    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens * a.splits, a.b);
     if (dtype == DASH_ATTN_BF16)
         return a.d == 64 ? launch_fwd2_t<__nv_bfloat16, 64>(grid, tq, tk, tv, to, a, stream)
                          : launch_fwd2_t<__nv_bfloat16, 128>(grid, tq, tk, tv, to, a, stream);

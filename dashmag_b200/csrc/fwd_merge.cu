@@ -1,0 +1,66 @@
+// The second half of a forward whose keys were split over blocks (forward_splits, sm100.cu): each row's partial outputs,
+// normalised f32, weighed by their log-sum-exp and rounded once to the queries' dtype.
+//
+// A warp a row, a lane D / 32 neighbouring features, so that a part is one coalesced read; the parts of a row are summed
+// in their order, so the bits repeat.  Bound by launch and latency at the sizes that split (the parts of 500 queries x 32
+// heads x 128 in 4 splits are 33 MB, still in L2): the blocks are brought in under the sweep's last wave.
+// Side by side: 500 queries against 8200 keys, 32 / 8 heads of 128 (64 tiles, two splits) 131 -> 86 us, merge included.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "sm100.h"
+#include "sm100_kernels.h"
+
+namespace dash {
+namespace {
+
+constexpr int MERGE_THREADS = 256;
+
+template <typename T, int HD>
+__global__ void __launch_bounds__(MERGE_THREADS) fwd_merge_kernel(const Sm100FwdArgs a) {
+    constexpr int PER = HD / 32;
+    wait_before();
+    const int lane = threadIdx.x & 31;
+    const int64_t rows = (int64_t)a.b * a.tq * a.hq, row = (int64_t)blockIdx.x * (MERGE_THREADS / 32) + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    float mx = -INFINITY;
+    for (int s = 0; s < a.splits; ++s) mx = fmaxf(mx, a.part_lse[s * rows + row]);
+    float num[PER], den = 0.f;
+#pragma unroll
+    for (int c = 0; c < PER; ++c) num[c] = 0.f;
+    if (mx != -INFINITY) {
+        for (int s = 0; s < a.splits; ++s) {
+            const float w = expf(a.part_lse[s * rows + row] - mx);
+            if (w == 0.f) continue;   // a part that saw no key left nothing
+            const float *po = a.part_o + (s * rows + row) * HD + lane * PER;
+            den += w;
+#pragma unroll
+            for (int c = 0; c < PER; c += 2) {
+                const float2 x = *reinterpret_cast<const float2 *>(po + c);
+                num[c] = fmaf(w, x.x, num[c]);
+                num[c + 1] = fmaf(w, x.y, num[c + 1]);
+            }
+        }
+    }
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    T *out = static_cast<T *>(a.out) + row * HD + lane * PER;
+#pragma unroll
+    for (int c = 0; c < PER; ++c) out[c] = Num<T>::from_f32(num[c] * inv);
+    if (lane == 0) a.lse[row] = den > 0.f ? (float)((double)mx + log((double)den)) : -INFINITY;
+}
+
+template <typename T>
+cudaError_t merge_t(const Sm100FwdArgs &a, cudaStream_t stream) {
+    const int64_t rows = (int64_t)a.b * a.tq * a.hq;
+    const dim3 grid((unsigned)((rows + MERGE_THREADS / 32 - 1) / (MERGE_THREADS / 32)));
+    return launch_beside(a.d == 64 ? fwd_merge_kernel<T, 64> : a.d == 128 ? fwd_merge_kernel<T, 128> : fwd_merge_kernel<T, 256>, grid,
+                         MERGE_THREADS, 0, stream, true, a);
+}
+
+}  // namespace
+
+cudaError_t launch_fwd_merge(int dtype, const Sm100FwdArgs &a, cudaStream_t stream) {
+    return dtype == DASH_ATTN_BF16 ? merge_t<__nv_bfloat16>(a, stream) : merge_t<__half>(a, stream);
+}
+
+}  // namespace dash

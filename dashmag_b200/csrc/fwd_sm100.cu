@@ -109,7 +109,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // The tile: 128 >> pack tokens from m0 on, of 1 << pack heads from h0 on; row = token << pack | head.
     const int pack = a.pack;
     const int h0 = blockIdx.x << pack;
-    const int qt = gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
+    const int split = blockIdx.y % a.splits;
+    const int qt = (gridDim.y - 1 - blockIdx.y) / a.splits;  // later (longer, under causality) tiles first
+    if (a.splits > 1) allow_beside();   // the merge
     const int b = blockIdx.z;
     const int hk = h0 / (a.hq / a.hkv);
     const int m0 = qt * (BM >> pack);
@@ -158,6 +160,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
     for (int i = 0; i < 4; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
     if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
+    split_keys(split, a.splits, BN, kmin, kmax);
     // Once a bounded wait has run out anywhere, later blocks do nothing: the call has failed and
     // the host will say so; there is no point in timing out thousands of times.
     const bool aborted = sh.abort != 0;
@@ -370,7 +373,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // ---------------- epilogue ----------------
         T *out = static_cast<T *>(a.out);
         const int64_t base = ((int64_t)b * a.tq + row) * a.hq + h;
-        if (n_tiles == 0 || failed) {
+        const bool part = a.splits > 1;   // a part of the row's keys: the normalised f32 row and its log-sum-exp, for the merge
+        const int64_t at = (int64_t)split * gridDim.z * a.tq * a.hq + base;
+        float *lse_at = part ? a.part_lse + at : a.lse + base;
+        if (part && n_tiles == 0) {
+            if (row < a.tq && !failed) *lse_at = -INFINITY;
+        } else if (n_tiles == 0 || failed) {
             if (row < a.tq && !failed) {
                 uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
@@ -385,7 +393,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 uint32_t o[32];
                 tmem_ld32(t_lane + 256 + c * 32, o);
                 tmem_ld_wait();
-                if (row < a.tq) {
+                if (row < a.tq && part) {
+                    float4 *po = reinterpret_cast<float4 *>(a.part_o + at * HD + c * 32);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        po[e] = make_float4(__uint_as_float(o[4 * e]) * inv, __uint_as_float(o[4 * e + 1]) * inv,
+                                            __uint_as_float(o[4 * e + 2]) * inv, __uint_as_float(o[4 * e + 3]) * inv);
+                } else if (row < a.tq) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         uint4 v;
@@ -403,7 +417,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (row < a.tq) {
                 const float used = __fmul_rn(m_ref, a.scale_log2);   // what the loop subtracted from every exponent
                 const double slip = (double)used - (double)m_ref * (double)a.scale_log2;
-                a.lse[base] = l > 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
+                *lse_at = l > 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
             }
             tc_fence_before_sync();
         } else {
@@ -436,7 +450,7 @@ cudaError_t launch_fwd_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk
 cudaError_t launch_fwd_sm100(int dtype, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv,
                              const Sm100FwdArgs &a, cudaStream_t stream) {
     const int tokens = BM >> a.pack;
-    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
+    dim3 grid(a.hq >> a.pack, (a.tq + tokens - 1) / tokens * a.splits, a.b);
     if (dtype == DASH_ATTN_BF16)
         return a.d == 256 ? launch_fwd_t<__nv_bfloat16, 256>(grid, tq, tk, tv, a, stream)
                           : launch_fwd_t<__nv_bfloat16, 128>(grid, tq, tk, tv, a, stream);

@@ -4,6 +4,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -180,7 +181,51 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
     return true;
 }
 
-size_t sm100_forward_workspace(const dash_attn_params *) { return 0; }
+// Over how many blocks the forward splits the keys of a tile of queries.  A call of few queries - a chunk of a prompt
+// against a long cache - has fewer tiles than the GPU has multiprocessors, each a long sweep: cut into runs of keys they
+// fill it.  Estimated in steps of 64 keys (128 at D 256): a block's share of its sweep plus what a block costs however
+// short its sweep (set-up, the first tiles' flight, the output: about six steps of the two-tile kernel, three of the
+// other's, which are twice as long), times the waves of blocks; a split also pays for its partial rows and the merge
+// (about five and three steps).  The sweep is the longest tile's; under causality with as many queries as keys the mean
+// is half of it, so the waves are counted on the mean and the longest tile is a bound of its own.  Packed batches, whose
+// lengths the host does not know, are not split.  A chunk of 500 queries against 8200 keys, 32 / 8 heads (64 tiles):
+// see the figures at fwd_merge.cu.
+int forward_splits(const dash_attn_params *p) {
+    if (p->mask_kind == DASH_ATTN_MASK_PACKED || p->hkv <= 0 || p->tq <= 0) return 1;
+    const bool one = p->d == 256;
+    const int pack = pack_log2(p->hq / p->hkv, p->tq);
+    const int64_t tokens = (one ? 128 : 256) >> pack, step = one ? 128 : 64, sms = 148;
+    const int64_t tiles = (p->tq + tokens - 1) / tokens, blocks = tiles * (p->hq >> pack) * p->b;
+    if (blocks >= 2 * sms) return 1;
+    int64_t longest = p->tk, mean = p->tk;
+    const int64_t right = p->causal ? 0 : p->has_window && p->window_right >= 0 ? p->window_right : -1;
+    if (right >= 0) {   // query i sees keys up to i + tk - tq + right
+        const int64_t last = std::min<int64_t>(p->tk, p->tk + right), first = std::min<int64_t>(p->tk, std::max<int64_t>(p->tk - p->tq + right + tokens, 0));
+        longest = last;
+        mean = (first + last) / 2;
+    }
+    if (p->has_window && p->window_left >= 0) {
+        const int64_t reach = (int64_t)p->window_left + std::max<int64_t>(right, 0) + tokens;
+        longest = std::min(longest, right < 0 ? p->tk : reach);
+        mean = std::min(mean, longest);
+    }
+    const int64_t l = (longest + step - 1) / step, m = (mean + step - 1) / step, fixed = one ? 3 : 6, merge = one ? 4 : 8;
+    auto cost = [&](int64_t s) {
+        const int64_t waves = (blocks * s + sms - 1) / sms;
+        return std::max(waves * ((m + s - 1) / s + fixed), (l + s - 1) / s + fixed) + (s > 1 ? merge : 0);
+    };
+    int best = 1;
+    for (int s = 2; s <= 32 && l / s >= 2 && tiles * s <= 65535; ++s)
+        if (cost(s) * 10 < cost(1) * 9 && cost(s) < cost(best)) best = s;
+    return best;
+}
+static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }
+static size_t split_lse_bytes(const dash_attn_params *p, int splits) { return (sizeof(float) * split_rows(p, splits) + 255) & ~size_t(255); }
+size_t sm100_forward_workspace(const dash_attn_params *p) {
+    const bool takes = (p->dtype == DASH_ATTN_BF16 || p->dtype == DASH_ATTN_F16) && (p->d == 64 || p->d == 128 || p->d == 256);
+    const int splits = takes ? forward_splits(p) : 1;
+    return splits > 1 ? split_lse_bytes(p, splits) + sizeof(float) * split_rows(p, splits) * p->d : 0;
+}
 // Whether a backward call takes the five-product form that adds dQ by reductions in L2: only when the
 // caller gave up the fixed order of summation, and only where that form exists (D = 64, 128).
 static bool fused_backward(const dash_attn_params *p) { return !p->deterministic && (p->d == 128 || p->d == 64); }
@@ -191,8 +236,8 @@ size_t sm100_backward_workspace(const dash_attn_params *p) {
     return bwd_sm100_order_bytes(p->b, p->tk, p->hkv) + (fused_backward(p) ? dq_acc_bytes(p) : 0);
 }
 
-cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *, cudaStream_t stream, int *launches,
-                          std::string &err) {
+cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream,
+                          int *launches, std::string &err) {
     // The two-tile kernel shares every K / V tile between two query tiles; DASH_ATTN_FWD_TILES=1
     // keeps the one-tile kernel (for comparison runs).
     static const bool one_tile = [] { const char *e = std::getenv("DASH_ATTN_FWD_TILES"); return e && std::atoi(e) == 1; }();
@@ -216,8 +261,20 @@ cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *,
     f.lse = a.lse;
     f.mask = a.mask;
     f.pack = pack;
+    // Without scratch for the parts (or with less than the query asks for) the keys stay in one block.
+    const size_t need = sm100_forward_workspace(p);
+    const bool split = need > 0 && workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && !one_tile;
+    f.splits = split ? forward_splits(p) : 1;
+    if (split) {
+        f.part_lse = static_cast<float *>(workspace);
+        f.part_o = reinterpret_cast<float *>(static_cast<char *>(workspace) + split_lse_bytes(p, f.splits));
+    }
     cudaError_t e = ((one_tile && p->d == 128) || p->d == 256) ? launch_fwd_sm100(p->dtype, tq, tk, tv, f, stream) : launch_fwd2_sm100(p->dtype, tq, tk, tv, to, f, stream);
     *launches += 1;
+    if (e == cudaSuccess && split) {
+        e = launch_fwd_merge(p->dtype, f, stream);
+        *launches += 1;
+    }
     return e;
 }
 

@@ -17,10 +17,11 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
 // How many tensor maps the driver has encoded for this process (repeated calls reuse theirs).
 uint64_t sm100_tensor_map_encodes();
 // Extra scratch the tensor-core path needs beyond what the C ABI layer itself plans.
+// (The forward runs without it too, its keys then not split over blocks.)
 size_t sm100_forward_workspace(const dash_attn_params *p);
 size_t sm100_backward_workspace(const dash_attn_params *p);
 // Launchers: add to *launches; a failure that is not a CUDA error code is reported through `err`.
-cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *workspace, cudaStream_t stream,
+cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream,
                           int *launches, std::string &err);
 cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *workspace, cudaStream_t stream,
                            int *launches, bool *atomic, std::string &err);

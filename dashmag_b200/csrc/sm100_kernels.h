@@ -17,7 +17,20 @@ struct Sm100FwdArgs {
     float *lse;        // [B,Tq,Hq]
     MaskArgs mask;
     int pack;          // a tile of 128 rows is 128 >> pack tokens of 1 << pack heads of one group, row = token << pack | head
+    // Keys split over `splits` blocks a tile: each sweeps its run of the tile's keys and leaves its normalised f32 output and
+    // its log-sum-exp for fwd_merge.  1: one block sweeps them all and writes the result.
+    int splits;
+    float *part_o;     // [splits][B,Tq,Hq,D]
+    float *part_lse;   // [splits][B,Tq,Hq]
 };
+
+// The run of a tile's keys [kmin, kmax) that falls to split `s`, in whole `step`s.
+__device__ __forceinline__ void split_keys(int s, int splits, int step, int &kmin, int &kmax) {
+    if (splits <= 1 || kmax <= kmin) return;
+    const int per = ((kmax - kmin + step - 1) / step + splits - 1) / splits * step;
+    kmin = (int)min((long long)kmin + (long long)s * per, (long long)kmax);
+    kmax = min(kmin + per, kmax);
+}
 
 struct Sm100BwdArgs {
     int b, tq, tk, hq, hkv;
@@ -48,6 +61,8 @@ cudaError_t launch_bwd256_sm100(int dtype, const Sm100BwdMaps &m, const Sm100Bwd
 cudaError_t read_sm100_bwd256_status(unsigned int *status, bool clear);
 size_t bwd_sm100_fused_shared_bytes(int d);
 
+// Combines the partial results of a split forward by their log-sum-exp (fwd_merge.cu).
+cudaError_t launch_fwd_merge(int dtype, const Sm100FwdArgs &a, cudaStream_t stream);
 cudaError_t launch_fwd_sm100(int dtype, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv,
                              const Sm100FwdArgs &a, cudaStream_t stream);
 // The two-tile forward: tq with boxes of 128 rows, tk / tv with boxes of 64 rows.

@@ -111,7 +111,9 @@ typedef struct dash_attn_decode_params {
     float scale;
 } dash_attn_decode_params;
 
-/* Bytes of device scratch each call needs (0 is possible).  256-byte aligned workspace. */
+/* Bytes of device scratch each call needs (0 is possible).  256-byte aligned workspace.  The forward
+ * also runs without its scratch, or with less (it then does not split a tile's keys over blocks, and
+ * a call of few queries against many keys takes longer). */
 size_t dash_attn_forward_workspace(const dash_attn_params *p);
 size_t dash_attn_backward_workspace(const dash_attn_params *p);
 size_t dash_attn_decode_workspace(const dash_attn_decode_params *p);
