@@ -199,8 +199,26 @@ void decode_plan(const dash_attn_decode_params *p, int *chunk, int *splits) {
         const char *env = std::getenv("DASH_ATTN_DECODE_CHUNK");
         return env ? std::atoll(env) : 0LL;
     }();
+    // Units a multiprocessor works on at a time: warps of the tensor-core pass (two a unit at D 256), or of the FMA pass.
+    const int group = p->hkv > 0 ? p->hq / p->hkv : 1;
+    const bool mma = p->dtype != DASH_ATTN_F32 && group >= 2 && (p->d == 64 || p->d == 128 || p->d == 256);
+    const long long slots = 148LL * (!mma ? 12 : p->d == 256 ? 4 : p->d == 128 ? 8 : 16);
+    const long long heads = (long long)p->b * p->hkv * (mma ? (group + 15) / 16 : (group + 3) / 4);   // units of one chunk
     long long c = 512;
-    if (fixed > 0) {
+    const bool few = heads > 0 && heads * ((p->s + (p->lengths ? 127 : 511)) / (p->lengths ? 128 : 512)) <= (p->lengths ? 1 : 4) * slots;
+    if (fixed <= 0 && few) {
+        // A few waves of units at most (with lengths, which the host does not know, one: what then runs in later waves is
+        // anybody's guess): the chunk whose waves are shortest, each costing its keys plus what a unit costs whatever its
+        // length - its set-up and first trip to HBM, about 48 keys' worth: a full batch slows by that law from chunks of
+        // 512 (627 us) over 256 (663) and 128 (740) down to 64 (957) - and half a key a split for the merge.  Eight caches
+        // of 6144 keys, 2 heads of 256: 48 splits of 128 keys in two waves 33 us, 35 of 176 in one 26 us.
+        long long best = -1;
+        for (long long t = 64; t <= 512; t += 16) {
+            const long long n = (p->s + t - 1) / t, waves = (heads * n + slots - 1) / slots;
+            const long long cost = waves * (t + 48) * 2 + n;
+            if (best < 0 || cost < best) { best = cost; c = t; }
+        }
+    } else if (fixed > 0) {
         c = fixed;
     } else {
         // Chunks of 128 to 512 keys, as long as they still leave units (a chunk of a key-value head;
@@ -374,12 +392,20 @@ int dash_attn_backward(const dash_attn_params *p, const void *q, const void *k, 
     return DASH_ATTN_OK;
 }
 
+// Whether the decoding step's inputs can be read 16 bytes at a time.
+static bool decode_vectors(const dash_attn_decode_params *p, const void *q, const void *k_new, const void *v_new, const void *k_cache, const void *v_cache) {
+    const size_t eb = elem_bytes(p->dtype);
+    return (p->d == 64 || p->d == 128 || p->d == 256) && vector_readable(q, p->q_stride, 3, eb) &&
+           vector_readable(k_cache, p->k_stride, 4, eb) && vector_readable(v_cache, p->v_stride, 4, eb) &&
+           (!k_new || (reinterpret_cast<uintptr_t>(k_new) % 16 == 0 && reinterpret_cast<uintptr_t>(v_new) % 16 == 0));
+}
+
 // The decoding step, with (k_new, v_new set) or without the new row written into the cache first.
 // The split pass's partial outputs go to the caller's workspace, or (`library_array`) to the array the
 // library itself holds on the device.
 static int decode_impl(const char *op, const dash_attn_decode_params *p, const void *q, const void *k_new, const void *v_new,
                        const void *k_cache, const void *v_cache, void *out, void *workspace, size_t workspace_bytes,
-                       dash_attn_stream_t stream_, bool library_array = false) {
+                       dash_attn_stream_t stream_, bool library_array = false, const dash::DecodeArgs *rope = nullptr) {
     g_error.clear();
     int rc = check_decode(p, op);
     if (rc != DASH_ATTN_OK) return rc;
@@ -434,9 +460,11 @@ static int decode_impl(const char *op, const dash_attn_decode_params *p, const v
     int64_t none = (int64_t)p->s + 1;
     a.left = (int)((p->has_window && p->window_left >= 0 && p->window_left < none) ? p->window_left : none);
     a.out = out;
-    bool vec = (p->d == 64 || p->d == 128 || p->d == 256) && vector_readable(q, p->q_stride, 3, eb) &&
-               vector_readable(k_cache, p->k_stride, 4, eb) && vector_readable(v_cache, p->v_stride, 4, eb) &&
-               (!k_new || (reinterpret_cast<uintptr_t>(k_new) % 16 == 0 && reinterpret_cast<uintptr_t>(v_new) % 16 == 0));
+    const bool vec = decode_vectors(p, q, k_new, v_new, k_cache, v_cache);
+    if (rope) {
+        a.rope_cos = rope->rope_cos; a.rope_sin = rope->rope_sin; a.rope_pos = rope->rope_pos;
+        a.rope_dim = rope->rope_dim; a.rope_pos_bytes = rope->rope_pos_bytes; a.rope_len = rope->rope_len;
+    }
     int launches = 0;
     cudaError_t e = dash::launch_decode(p->dtype, a, vec, stream, &launches);
     g_probe[DASH_ATTN_PROBE_KERNEL_LAUNCHES] += launches;
@@ -548,6 +576,14 @@ int dash_attn_decode_append_rope(const dash_attn_decode_params *p, const dash_ro
     if (p->q_stride[2] != 1) return fail(DASH_ATTN_UNSUPPORTED, "%s: the query's features must be contiguous", op);
     const size_t need = dash_attn_decode_append_rope_workspace(p);
     if ((rc = check_workspace(op, workspace, workspace_bytes, need)) != DASH_ATTN_OK) return rc;
+    // Where the split pass can rotate on its way, the step is that pass and the merge; else a launch of the rotation goes first.
+    dash::DecodeArgs f{};
+    f.hq = p->hq; f.hkv = p->hkv; f.d = p->d;
+    f.rope_cos = r->cos; f.rope_sin = r->sin; f.rope_dim = r->dim; f.rope_len = r->len;
+    f.rope_pos = positions ? positions : p->lengths;
+    f.rope_pos_bytes = positions ? positions_elem_bytes : p->lengths_elem_bytes;
+    if (r->len > 0 && k_cache && v_cache && dash::decode_fuses_rope(p->dtype, f, decode_vectors(p, q, k_new, v_new, k_cache, v_cache)))
+        return decode_impl(op, p, q, k_new, v_new, k_cache, v_cache, out, workspace, workspace_bytes, stream_, false, &f);
     char *q_rot = static_cast<char *>(workspace) + rope_scratch_offset(p);
     char *k_rot = q_rot + align256((size_t)p->b * p->hq * p->d * eb);
 

@@ -258,6 +258,11 @@ struct DecodeArgs {
     // The step that also appends: the new key and value rows [B,Hkv,D] (contiguous) go to
     // position lengths[b] of the cache, where the step already sees them.  Null otherwise.
     const void *k_new, *v_new;
+    // The step that also rotates: the queries and the new key are rotated by the row of the tables [rope_len, rope_dim] at
+    // rope_pos[b] as they are read (decode_fuses_rope says which calls).  rope_cos null otherwise.
+    const void *rope_cos, *rope_sin, *rope_pos;
+    int rope_dim, rope_pos_bytes;
+    int64_t rope_len;
 };
 
 // Where the appending step writes sequence b's new row: its length before the step, or -1 when

@@ -14,6 +14,9 @@
 //   * scores are reduced across the D / 8 lanes with shuffles, the softmax is kept online in f32
 //     per query head, lane groups are merged with shuffles at the end, and each warp writes one
 //     normalised partial output and its log-sum-exp;
+//     (dash_attn_decode_append_rope: the pass also rotates the queries and the new key as it reads them;
+//     one sequence of 2047 keys, the whole step on the device 19.2 -> 13.5 us with that, the chunk of 64
+//     keys the planner now picks and the merge brought in under the pass's end);
 //   * the merge kernel combines the partials of each (sequence, query head) by their log-sum-exp
 //     and rounds to the queries' dtype.  Chunks past a sequence's length or before its window are
 //     never touched.
@@ -131,6 +134,7 @@ __device__ __forceinline__ void slot8<__half>(const uint4 *slot, float (&x)[8]) 
 // with three steps each on the way from HBM.
 template <typename T, int D, int GH>
 __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_kernel(DecodeArgs a) {
+    allow_beside();   // the merge
     constexpr int LPK = D / 8;                    // lanes per key
     constexpr int KPW = 32 / LPK;                 // keys per warp in one load
     constexpr int VPK = sizeof(T) == 4 ? 2 : 1;   // 16-byte vectors per eight values
@@ -301,12 +305,12 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_kernel(DecodeArgs
 // every lane copies 16-byte pieces of the tile's 16 key rows and 16 value rows asynchronously, two
 // tiles ahead, into rows (256 bytes at D = 128) whose 16-byte chunks are XOR-swizzled by the row, and ldmatrix
 // reads the fragments from there without bank conflicts (transposed for V).
-constexpr int DM_WARPS = 8;     // warps per block
 constexpr int DM_STAGES = 3;    // tiles of the per-warp ring
 constexpr int DM_KEYS = 16;     // keys per tile
 
 template <typename T> struct MmaType;
 template <> struct MmaType<__nv_bfloat16> {
+    using Two = __nv_bfloat162;
     static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -319,6 +323,7 @@ template <> struct MmaType<__nv_bfloat16> {
     static __device__ __forceinline__ float hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 };
 template <> struct MmaType<__half> {
+    using Two = __half2;
     static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
         asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -341,8 +346,27 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 // features - its half of the scores' sum over the features, which the two exchange through shared
 // memory and add (in one order, so both hold the same bits), its half of Q, of every K and V row
 // and of the output; the accumulators of a whole row of 256 would not fit a thread's registers.
-template <typename T, int D, int PARTS>
-__global__ void __launch_bounds__(DM_WARPS * 32) decode_split_mma_kernel(DecodeArgs a) {
+//
+// WARPS warps to a block: eight, or two where blocks of eight would leave multiprocessors without one (a block is a
+// multiprocessor's worth of shared memory: 256 units of one sequence's 8 heads in blocks of eight are 32 blocks).  The warps
+// resident at a time are the same.  Blocks of two up to two waves of warps, where they measured ahead (one sequence of 2047
+// keys with rotation and append: 15.5 us with blocks of eight, 13.5 with two); beyond, eight (64 sequences of up to 4096:
+// 91 against 102 us): its warps read neighbouring heads of the same keys at the same time.
+//
+// Two columns rotated in the dtype's own arithmetic, as rope_kernel does it (each product and the sum rounded once): `low` for
+// the first half of the rotated features, whose partner enters with its sign turned.
+template <typename T>
+__device__ __forceinline__ uint32_t rotate_two(uint32_t x, uint32_t partner, uint32_t c, uint32_t s, bool low) {
+    using P2 = typename MmaType<T>::Two;
+    const P2 px = *reinterpret_cast<P2 *>(&x), pp = *reinterpret_cast<P2 *>(&partner), pc = *reinterpret_cast<P2 *>(&c), ps = *reinterpret_cast<P2 *>(&s);
+    P2 r = __hadd2_rn(__hmul2_rn(px, pc), __hmul2_rn(low ? __hneg2(pp) : pp, ps));
+    return *reinterpret_cast<uint32_t *>(&r);
+}
+
+template <typename T, int D, int PARTS, int WARPS, bool ROPE>
+__global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs a) {
+    constexpr int DM_WARPS = WARPS;
+    allow_beside();   // the merge
     constexpr int DFULL = D * PARTS;            // the head dimension; D is what one warp takes of it
     constexpr int ROWB = 2 * D;                 // bytes of a warp's part of a cache row: 256 at D = 128, 128 at D = 64
     constexpr int CH = D / 8;                   // its 16-byte chunks
@@ -384,6 +408,36 @@ __global__ void __launch_bounds__(DM_WARPS * 32) decode_split_mma_kernel(DecodeA
             qa[ks][3] = live1 ? *reinterpret_cast<const uint32_t *>(q1 + ks * 16 + 8 + 2 * t) : 0u;
         }
     }
+    // The rotation's row of the tables (no such row: every rotated feature is a NaN, as rope_kernel has it).
+    const int half = a.rope_dim / 2;
+    const T *cos_row = nullptr, *sin_row = nullptr;
+    if constexpr (ROPE) {
+        const int64_t at = a.rope_pos_bytes == 8 ? static_cast<const long long *>(a.rope_pos)[b] : static_cast<const int *>(a.rope_pos)[b];
+        if (at >= 0 && at < a.rope_len) {
+            cos_row = static_cast<const T *>(a.rope_cos) + at * a.rope_dim;
+            sin_row = static_cast<const T *>(a.rope_sin) + at * a.rope_dim;
+        }
+        const T *qg = static_cast<const T *>(a.q) + (int64_t)b * a.q_sb + (int64_t)(hk * group) * a.q_sh;
+        const int64_t r0 = (int64_t)min(g_base + g, group - 1) * a.q_sh, r1 = (int64_t)min(g_base + g + 8, group - 1) * a.q_sh;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {   // columns c, c + 1 of rows g and g + 8
+                const int c = d0 + ks * 16 + 4 * j + 2 * t;
+                if (c >= a.rope_dim) continue;
+                const bool low = c < half;
+                const int other = low ? c + half : c - half;
+                if (cos_row) {
+                    const uint32_t cs = *reinterpret_cast<const uint32_t *>(cos_row + c), sn = *reinterpret_cast<const uint32_t *>(sin_row + c);
+                    qa[ks][j] = rotate_two<T>(qa[ks][j], *reinterpret_cast<const uint32_t *>(qg + r0 + other), cs, sn, low);
+                    qa[ks][j + 1] = rotate_two<T>(qa[ks][j + 1], *reinterpret_cast<const uint32_t *>(qg + r1 + other), cs, sn, low);
+                } else {
+                    qa[ks][j] = qa[ks][j + 1] = 0x7fff7fffu;   // a NaN in either dtype
+                }
+                if (g_base + g >= group) qa[ks][j] = 0u;
+                if (g_base + g + 8 >= group) qa[ks][j + 1] = 0u;
+            }
+    }
     const T *kbase = static_cast<const T *>(a.k.ptr) + (int64_t)b * a.k.sb + (int64_t)hk * a.k.sh + d0;
     const T *vbase = static_cast<const T *>(a.v.ptr) + (int64_t)b * a.v.sb + (int64_t)hk * a.v.sh + d0;
     const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(dm_ring)) + (uint32_t)wib * DM_STAGES * 2 * DM_TILE;
@@ -396,10 +450,25 @@ __global__ void __launch_bounds__(DM_WARPS * 32) decode_split_mma_kernel(DecodeA
     const int pos = decode_append_at(a, b);
     const T *knew = static_cast<const T *>(a.k_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
     const T *vnew = static_cast<const T *>(a.v_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
-    if (pos >= c0 && pos < c1 && lane < 2 * CH && g_base == 0) {
-        const T *src = (lane < CH ? knew : vnew) + cp_chunk * 8;
-        T *dst = const_cast<T *>(lane < CH ? kbase + (int64_t)pos * a.k.st : vbase + (int64_t)pos * a.v.st) + cp_chunk * 8;
-        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(src);
+    uint4 row_chunk = make_uint4(0, 0, 0, 0);   // lanes below CH: this lane's chunk of the new key row, rotated if the step rotates
+    if (pos >= c0 && pos < c1 && lane < 2 * CH) {
+        row_chunk = *reinterpret_cast<const uint4 *>((lane < CH ? knew : vnew) + cp_chunk * 8);
+        const int c = d0 + cp_chunk * 8;
+        if (ROPE && lane < CH && c < a.rope_dim) {
+            const bool low = c < half;
+            if (cos_row) {
+                const uint4 o4 = *reinterpret_cast<const uint4 *>(knew - d0 + (low ? c + half : c - half));
+                const uint4 cs = *reinterpret_cast<const uint4 *>(cos_row + c), sn = *reinterpret_cast<const uint4 *>(sin_row + c);
+                row_chunk = make_uint4(rotate_two<T>(row_chunk.x, o4.x, cs.x, sn.x, low), rotate_two<T>(row_chunk.y, o4.y, cs.y, sn.y, low),
+                                       rotate_two<T>(row_chunk.z, o4.z, cs.z, sn.z, low), rotate_two<T>(row_chunk.w, o4.w, cs.w, sn.w, low));
+            } else {
+                row_chunk = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+            }
+        }
+        if (g_base == 0) {
+            T *dst = const_cast<T *>(lane < CH ? kbase + (int64_t)pos * a.k.st : vbase + (int64_t)pos * a.v.st) + cp_chunk * 8;
+            *reinterpret_cast<uint4 *>(dst) = row_chunk;
+        }
     }
     const int pos_it = (pos >= c0 && pos < c1) ? (pos - c0) / DM_KEYS : -1;   // the tile of the new row, if this chunk holds it
     auto issue = [&](int it) {
@@ -436,6 +505,12 @@ __global__ void __launch_bounds__(DM_WARPS * 32) decode_split_mma_kernel(DecodeA
         __syncwarp();   // ... and sees the other lanes' pieces of this tile
         const uint32_t kt = ring + (uint32_t)(it % DM_STAGES) * 2 * DM_TILE, vt = kt + DM_TILE;
         const int key0 = c0 + it * DM_KEYS;
+        if (ROPE && it == pos_it) {   // the new key arrived as it was given: the rotated row takes its place in the tile
+            const int row = pos - key0;
+            if (lane < CH) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(kt + (uint32_t)(row * ROWB + ((cp_chunk ^ (row & 7)) << 4))),
+                                        "r"(row_chunk.x), "r"(row_chunk.y), "r"(row_chunk.z), "r"(row_chunk.w) : "memory");
+            __syncwarp();
+        }
 
         // S[16 heads x 16 keys] as two N tiles of 8 keys.
         float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -538,6 +613,7 @@ __global__ void __launch_bounds__(DM_WARPS * 32) decode_split_mma_kernel(DecodeA
 // lane owning the head dimensions `lane + 32 i`, keys in order.
 template <typename T>
 __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_scalar_kernel(DecodeArgs a) {
+    allow_beside();   // the merge
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
     long long unit = (long long)blockIdx.x * DEC_WARPS + (threadIdx.x >> 5);
@@ -609,6 +685,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) decode_merge_kernel(DecodeArgs a) {
     __shared__ float w[MERGE_MAX];
     __shared__ float red[4];
+    wait_before();   // the split pass
     const int bh = blockIdx.x;
     const int b = bh / a.hq;
     int first, len;
@@ -720,16 +797,21 @@ static cudaError_t split_vec(const DecodeArgs &a, cudaStream_t stream) {
     return split_vec_g<T, D, 1>(a, grid, stream);
 }
 
+template <typename T, int DFULL, int WARPS>
+static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, cudaStream_t stream) {
+    constexpr int PARTS = DFULL > 128 ? 2 : 1, D = DFULL / PARTS;
+    constexpr size_t smem = (size_t)WARPS * DM_STAGES * 2 * DM_KEYS * 2 * D + (PARTS == 2 ? (size_t)WARPS * 32 * 8 * sizeof(float) : 0);
+    const auto kernel = a.rope_cos ? decode_split_mma_kernel<T, D, PARTS, WARPS, true> : decode_split_mma_kernel<T, D, PARTS, WARPS, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    dim3 grid((unsigned)((warps + WARPS - 1) / WARPS), a.b);
+    kernel<<<grid, WARPS * 32, smem, stream>>>(a);
+    return cudaGetLastError();
+}
 template <typename T, int DFULL>
 static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream) {
-    constexpr int PARTS = DFULL > 128 ? 2 : 1, D = DFULL / PARTS;
-    constexpr size_t smem = (size_t)DM_WARPS * DM_STAGES * 2 * DM_KEYS * 2 * D + (PARTS == 2 ? (size_t)DM_WARPS * 32 * 8 * sizeof(float) : 0);
-    cudaError_t e = cudaFuncSetAttribute(decode_split_mma_kernel<T, D, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const long long units = (long long)a.splits * a.hkv * PARTS * ((a.hq / a.hkv + 15) / 16);
-    dim3 grid((unsigned)((units + DM_WARPS - 1) / DM_WARPS), a.b);
-    decode_split_mma_kernel<T, D, PARTS><<<grid, DM_WARPS * 32, smem, stream>>>(a);
-    return cudaGetLastError();
+    const long long warps = (long long)a.splits * a.hkv * (DFULL > 128 ? 2 : 1) * ((a.hq / a.hkv + 15) / 16);   // of one sequence
+    return warps * a.b < 148LL * 8 * 2 ? split_mma_w<T, DFULL, 2>(a, warps, stream) : split_mma_w<T, DFULL, 8>(a, warps, stream);
 }
 template <> cudaError_t split_mma<float, 128>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }   // never taken: 16-bit caches only
 template <> cudaError_t split_mma<float, 64>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }
@@ -741,10 +823,19 @@ static bool decode_force_scalar_pass() {
     return off;
 }
 
+static bool decode_uses_mma(size_t elem, const DecodeArgs &a, bool vector_ok) {
+    return vector_ok && elem == 2 && a.hq / a.hkv >= 2 && !decode_force_scalar_pass();
+}
+bool decode_fuses_rope(int dtype, const DecodeArgs &a, bool vector_ok) {
+    auto aligned = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    // Halves of whole 16-byte chunks: a pair's two columns then sit in chunks (and fragments) of their own.
+    return dtype != 0 && decode_uses_mma(2, a, vector_ok) && a.rope_dim % 16 == 0 && aligned(a.rope_cos) && aligned(a.rope_sin);
+}
+
 template <typename T>
 static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches) {
     cudaError_t e;
-    const bool mma = vector_ok && sizeof(T) == 2 && a.hq / a.hkv >= 2 && !decode_force_scalar_pass();
+    const bool mma = decode_uses_mma(sizeof(T), a, vector_ok);
     if (mma && a.d == 128) e = split_mma<T, 128>(a, stream);
     else if (mma && a.d == 64) e = split_mma<T, 64>(a, stream);
     else if (mma && a.d == 256) e = split_mma<T, 256>(a, stream);
@@ -759,9 +850,8 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
     }
     *launches += 1;
     if (e != cudaSuccess) return e;
-    decode_merge_kernel<T><<<a.b * a.hq, 128, 0, stream>>>(a);
     *launches += 1;
-    return cudaGetLastError();
+    return launch_beside(decode_merge_kernel<T>, dim3(a.b * a.hq), 128, 0, stream, true, a);
 }
 
 cudaError_t launch_decode(int dtype, const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches) {
