@@ -150,14 +150,19 @@ __device__ __forceinline__ int warp_min_i(int x);
 // A block's sweep [kmin, kmax) without the padded keys at its ends: right- and left-padded batches are swept no further
 // than their tokens go.  All 32 lanes call and get one answer, the same in every warp; 256 flags a look, from either
 // end, so that a sweep that is not padded there pays one trip to memory.  (kmax <= kmin: no key is left.)
-static __device__ __noinline__ void trim_padded(const MaskArgs &m, int b, int &kmin, int &kmax) {
+// (By value, in and out: a reference would put the caller's arguments on the stack.)
+static __device__ __noinline__ int2 trim_padded_span(const void *kp, int kp_bytes, int64_t sb, int64_t st, int b, int kmin, int kmax) {
     const int lane = threadIdx.x & 31;
+    auto padded = [&](int key) {
+        const int64_t at = (int64_t)b * sb + (int64_t)key * st;
+        return kp_bytes == 4 ? static_cast<const int *>(kp)[at] != 0 : static_cast<const unsigned char *>(kp)[at] != 0;
+    };
     int last = -1;
     while (kmax > kmin && last < 0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int key = kmax - 1 - 32 * i - lane;
-            if (key >= kmin && !key_padded(m, b, key)) last = max(last, key);
+            if (key >= kmin && !padded(key)) last = max(last, key);
         }
         last = warp_max_i(last);
         kmax = last >= 0 ? last + 1 : kmax - 256;
@@ -167,11 +172,17 @@ static __device__ __noinline__ void trim_padded(const MaskArgs &m, int b, int &k
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int key = kmin + 32 * i + lane;
-            if (key < kmax && !key_padded(m, b, key)) first = min(first, key);
+            if (key < kmax && !padded(key)) first = min(first, key);
         }
         first = warp_min_i(first);
         kmin = first != 2147483647 ? first : kmin + 256;
     }
+    return make_int2(kmin, kmax);
+}
+__device__ __forceinline__ void trim_padded(const MaskArgs &m, int b, int &kmin, int &kmax) {
+    const int2 span = trim_padded_span(m.kp, m.kp_bytes, m.kp_sb, m.kp_st, b, kmin, kmax);
+    kmin = span.x;
+    kmax = span.y;
 }
 
 __device__ __forceinline__ float warp_max(float x) {

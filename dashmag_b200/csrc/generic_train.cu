@@ -7,69 +7,158 @@
 // recomputes the scores tile by tile from the saved log-sum-exp, and sums every gradient in a
 // fixed order (no atomics), so its results are the same bits on every run.
 //
-// Work split: a block of 256 threads owns 32 rows (queries, or keys in the key/value gradient
-// kernel), four per warp; the other side streams through shared memory in tiles of 32, one per
-// lane.  A lane forms the dot products of its tile row with the warp's four rows, the warp
-// reduces the softmax statistics with shuffles, and for the second product each lane owns the
-// head dimensions `lane + 32 i`.
+// Work split: a block of eight warps owns 8 RPW rows (queries, or keys in the key/value gradient
+// kernel), RPW to a warp; the other side streams through shared memory in tiles of 32, one row per
+// lane, double-buffered: the next tile is on its way (16-byte asynchronous copies for f32 rows that allow
+// them) while this one is worked on.  A lane forms the dot products of its tile row with the warp's rows - four
+// features at a time, from rows whose stride is an odd number of 16-byte chunks, so that eight lanes
+// meet all banks - the warp reduces the maxima with shuffles, and for the second product each lane
+// owns the head dimensions `lane + 32 i`.
+//
+// RPW is four where the rows fill the GPU that way (a tile row read from shared memory then serves four
+// products), one where they do not: small calls are bound by the length of a block's chain of tiles, not
+// by throughput.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
+// Two packed sequences of 384 tokens, four heads of 64, f32: the step 254 ->
+// 68 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
+// another; launch and host time are most of what is left).
+#include "bwd_common.cuh"
 #include "common.cuh"
 #include "launch.h"
 
 namespace dash {
 
-constexpr int ROWS = 32;      // rows per block
-constexpr int RPW = 4;        // rows per warp
 constexpr int TILE = 32;      // streamed rows per tile (one per lane)
 constexpr int THREADS = 256;
-constexpr int MAXI = 8;       // ceil(256 / 32) owned head dimensions per lane
+constexpr int WARPS = THREADS / 32;
 
 __host__ __device__ inline int padded_d(int d) { return (d + 3) & ~3; }
+// Floats between two rows of a tile: whole 16-byte chunks, an odd number of them.
+__host__ __device__ inline int tile_stride(int d) { return padded_d(d) % 8 == 0 ? padded_d(d) + 4 : padded_d(d); }
 
-// Copies rows [r0, r0 + 32) of one head into shared memory as f32, zero past `limit` and past d.
+__device__ __forceinline__ void copy_async(float *dst, const void *src, bool valid, int bytes16) {
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if (bytes16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// Copies rows [r0, r0 + rows) of one head into shared memory as f32, zero past `limit` and past d.  `vec`: every row of the
+// source can be read 16 bytes at a time and d is whole 16-byte vectors (f32: asynchronously, complete after copies_wait).
 template <typename T>
-__device__ __forceinline__ void stage_rows(float *dst, int stride, const View4 &src, int b, int h,
-                                           int r0, int limit, int d, int dp) {
-    for (int idx = threadIdx.x; idx < TILE * dp; idx += THREADS) {
-        int r = idx / dp, c = idx - r * dp;
+__device__ __forceinline__ void stage_rows(float *dst, int stride, const View4 &src, int b, int h, int r0, int rows, int limit, int d, bool vec) {
+    const T *base = static_cast<const T *>(src.ptr) + (int64_t)b * src.sb + (int64_t)h * src.sh;
+    if (vec) {
+        constexpr int V = 16 / sizeof(T);
+        const int per = d / V, total = rows * per;
+        for (int i0 = threadIdx.x; i0 < total; i0 += 2 * THREADS) {
+            uint4 raw[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = i0 + u * THREADS, r = i / per, c = (i - r * per) * V;
+                const bool in = i < total, valid = in && r0 + r < limit;
+                const T *from = base + (int64_t)(valid ? r0 + r : 0) * src.st + (valid ? c : 0);
+                if constexpr (sizeof(T) == 4) {
+                    if (in) copy_async(dst + r * stride + c, from, valid, 1);
+                } else {
+                    raw[u] = make_uint4(0, 0, 0, 0);
+                    if (valid) raw[u] = *reinterpret_cast<const uint4 *>(from);
+                }
+            }
+            if constexpr (sizeof(T) == 2) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int i = i0 + u * THREADS, r = i / per, c = (i - r * per) * V;
+                    if (i >= total) continue;
+                    const T *e = reinterpret_cast<const T *>(&raw[u]);
+                    float4 *to = reinterpret_cast<float4 *>(dst + r * stride + c);
+                    to[0] = make_float4(Num<T>::to_f32(e[0]), Num<T>::to_f32(e[1]), Num<T>::to_f32(e[2]), Num<T>::to_f32(e[3]));
+                    to[1] = make_float4(Num<T>::to_f32(e[4]), Num<T>::to_f32(e[5]), Num<T>::to_f32(e[6]), Num<T>::to_f32(e[7]));
+                }
+            }
+        }
+        return;
+    }
+    const int dp = padded_d(d);
+    for (int idx = threadIdx.x; idx < rows * dp; idx += THREADS) {
+        const int r = idx / dp, c = idx - r * dp;
         float x = 0.f;
-        if (r0 + r < limit && c < d) x = load_f32<T>(src, b, r0 + r, h, c);
+        if (r0 + r < limit && c < d) x = Num<T>::to_f32(base[(int64_t)(r0 + r) * src.st + (int64_t)c * src.sd]);
         dst[r * stride + c] = x;
     }
 }
 
-// dot[r] = sum_c rows[(w*4 + r)][c] * tile[lane][c], the four rows read as broadcast float4.
-__device__ __forceinline__ void dots4(const float *rows, int row_stride, const float *tile_row,
-                                      int dp, float (&acc)[RPW]) {
+// dot[r] = sum_c rows[r][c] * tile_row[c]: the warp's rows as broadcast float4, four partial sums a row.
+template <int RPW>
+__device__ __forceinline__ void dots(const float *rows, int row_stride, const float *tile_row, int dp, float (&out)[RPW]) {
+    float4 acc[RPW];
 #pragma unroll
-    for (int r = 0; r < RPW; ++r) acc[r] = 0.f;
+    for (int r = 0; r < RPW; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (int c = 0; c < dp; c += 4) {
-        float t0 = tile_row[c], t1 = tile_row[c + 1], t2 = tile_row[c + 2], t3 = tile_row[c + 3];
+        const float4 t = *reinterpret_cast<const float4 *>(tile_row + c);
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            float4 x = *reinterpret_cast<const float4 *>(rows + r * row_stride + c);
-            acc[r] = fmaf(x.x, t0, acc[r]);
-            acc[r] = fmaf(x.y, t1, acc[r]);
-            acc[r] = fmaf(x.z, t2, acc[r]);
-            acc[r] = fmaf(x.w, t3, acc[r]);
+            const float4 x = *reinterpret_cast<const float4 *>(rows + r * row_stride + c);
+            acc[r].x = fmaf(x.x, t.x, acc[r].x);
+            acc[r].y = fmaf(x.y, t.y, acc[r].y);
+            acc[r].z = fmaf(x.z, t.z, acc[r].z);
+            acc[r].w = fmaf(x.w, t.w, acc[r].w);
         }
+    }
+#pragma unroll
+    for (int r = 0; r < RPW; ++r) out[r] = (acc[r].x + acc[r].y) + (acc[r].z + acc[r].w);
+}
+
+// acc[r][i] += sum_j weight[j][r] * tile[j][lane + 32 i] over the tile's 32 rows.
+template <int RPW, int NI>
+__device__ __forceinline__ void accumulate(const float *weight, const float *tile, int stride, int dp, float (&acc)[RPW][NI]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 8
+    for (int j = 0; j < TILE; ++j) {
+        float w[RPW];
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) w[r] = weight[j * RPW + r];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int c = lane + 32 * i;
+            const float v = c < dp ? tile[j * stride + c] : 0.f;
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) acc[r][i] = fmaf(w[r], v, acc[r][i]);
+        }
+    }
+}
+
+// The block's first row, and what each of its rows sees: the queries' key intervals (warp 0 places them) and their union.
+struct RowSpans {
+    int lo[32], hi[32];
+    int kmin, kmax;
+};
+__device__ __forceinline__ void place_rows(RowSpans &sp, const MaskArgs &m, int row0, int rows, int tq, int tk) {
+    if (threadIdx.x < 32) {
+        int lo, hi;
+        row_bounds_warp(m, row0 + (int)threadIdx.x, tq, tk, lo, hi);
+        if ((int)threadIdx.x >= rows) { lo = tk; hi = 0; }
+        sp.lo[threadIdx.x] = lo;
+        sp.hi[threadIdx.x] = hi;
+        const int kmin = warp_min_i(hi > lo ? lo : tk), kmax = warp_max_i(hi > lo ? hi : 0);
+        if (threadIdx.x == 0) { sp.kmin = kmin; sp.kmax = kmax; }
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a) {
+template <typename T, int RPW, int NI>
+__global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    const int dp = padded_d(a.d);
-    float *qs = smem;                          // [32][dp]
-    float *ks = qs + ROWS * dp;                // [32][dp + 1]
-    float *vs = ks + TILE * (dp + 1);          // [32][dp]
-    float *ps = vs + TILE * dp;                // [8 warps][32 keys][4 rows]
-    int *los = reinterpret_cast<int *>(ps + 8 * TILE * RPW);  // [32]
-    int *his = los + ROWS;                     // [32]
-    int *pad = his + ROWS;                     // [32] key padding flags of the tile
-    __shared__ int span[2];
+    constexpr int ROWS = WARPS * RPW;
+    const int dp = padded_d(a.d), sp = tile_stride(a.d);
+    float *qs = smem;                          // [ROWS][dp]
+    float *kv = qs + ROWS * dp;                // [2 buffers][K, V][32][sp]
+    float *ps = kv + 4 * TILE * sp;            // [8 warps][32 keys][RPW]
+    __shared__ RowSpans rs;
+    __shared__ int pad[2][TILE];               // key padding flags of the tile
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int qt = gridDim.x - 1 - blockIdx.x;  // long (late) causal rows first
@@ -77,104 +166,87 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a) {
     const int hk = h / (a.hq / a.hkv);
     const int row0 = qt * ROWS;
 
-    stage_rows<T>(qs, dp, a.q, b, h, row0, a.tq, a.d, dp);
-    if (threadIdx.x < ROWS) {
-        int lo, hi;
-        row_bounds(a.mask, row0 + threadIdx.x, a.tq, a.tk, lo, hi);
-        los[threadIdx.x] = lo;
-        his[threadIdx.x] = hi;
-        int kmin = warp_min_i(hi > lo ? lo : a.tk);
-        int kmax = warp_max_i(hi > lo ? hi : 0);
-        if (threadIdx.x == 0) { span[0] = kmin; span[1] = kmax; }
-    }
+    stage_rows<T>(qs, dp, a.q, b, h, row0, ROWS, a.tq, a.d, vec);
+    place_rows(rs, a.mask, row0, ROWS, a.tq, a.tk);
     __syncthreads();
-    const int kmin = span[0], kmax = span[1];
+    int kmin = rs.kmin, kmax = rs.kmax;
+    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
 
     int lo[RPW], hi[RPW];
     int wlo = a.tk, whi = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        lo[r] = los[w * RPW + r];
-        hi[r] = his[w * RPW + r];
+        lo[r] = rs.lo[w * RPW + r];
+        hi[r] = rs.hi[w * RPW + r];
         if (hi[r] > lo[r]) { wlo = min(wlo, lo[r]); whi = max(whi, hi[r]); }
     }
-    float m[RPW], l[RPW], acc[RPW][MAXI];
+    float m[RPW], l[RPW], acc[RPW][NI];   // l: this lane's share of the row's sum
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
         m[r] = -INFINITY;
         l[r] = 0.f;
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) acc[r][i] = 0.f;
+        for (int i = 0; i < NI; ++i) acc[r][i] = 0.f;
     }
-    const int ni = (dp + 31) / 32;
-
-    for (int k0 = (kmin / TILE) * TILE; k0 < kmax; k0 += TILE) {
-        __syncthreads();
-        stage_rows<T>(ks, dp + 1, a.k, b, hk, k0, a.tk, a.d, dp);
-        stage_rows<T>(vs, dp, a.v, b, hk, k0, a.tk, a.d, dp);
+    auto stage = [&](int k0, int buf) {
+        stage_rows<T>(kv + (2 * buf) * TILE * sp, sp, a.k, b, hk, k0, TILE, a.tk, a.d, vec);
+        stage_rows<T>(kv + (2 * buf + 1) * TILE * sp, sp, a.v, b, hk, k0, TILE, a.tk, a.d, vec);
         if (threadIdx.x < TILE) {
-            int key = k0 + threadIdx.x;
-            pad[threadIdx.x] = key < a.tk ? (key_padded(a.mask, b, key) ? 1 : 0) : 1;
+            const int key = k0 + threadIdx.x;
+            pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
-        __syncthreads();
+        copies_commit();
+    };
+    const int first = kmin / TILE * TILE;
+    if (kmax > kmin) stage(first, 0);
+    for (int k0 = first, buf = 0; k0 < kmax; k0 += TILE, buf ^= 1) {
+        copies_wait();
+        __syncthreads();   // the tile is whole, and every warp is done with the other buffer
+        if (k0 + TILE < kmax) stage(k0 + TILE, buf ^ 1);
         if (k0 + TILE <= wlo || k0 >= whi) continue;  // no row of this warp sees the tile
+        const float *ks = kv + (2 * buf) * TILE * sp, *vs = ks + TILE * sp;
 
         float s[RPW];
-        dots4(qs + w * RPW * dp, dp, ks + lane * (dp + 1), dp, s);
+        dots<RPW>(qs + w * RPW * dp, dp, ks + lane * sp, dp, s);
         const int key = k0 + lane;
-        const bool open = pad[lane] == 0;
-        float4 p4;
-        float *pp = reinterpret_cast<float *>(&p4);
+        const bool open = pad[buf][lane] == 0;
+        float *pw = ps + w * TILE * RPW;
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            bool vis = open && key >= lo[r] && key < hi[r];
-            float sr = vis ? s[r] * a.scale : -INFINITY;
-            float mt = warp_max(sr);
-            float mn = fmaxf(m[r], mt);
+            const bool vis = open && key >= lo[r] && key < hi[r];
+            const float sr = vis ? s[r] * a.scale : -INFINITY;
+            const float mn = fmaxf(m[r], warp_max(sr));
             float p = 0.f, alpha = 1.f;
             if (mn != -INFINITY) {
                 alpha = expf(m[r] - mn);  // exp(-inf) = 0 on the first visible tile
                 p = expf(sr - mn);
             }
-            l[r] = l[r] * alpha + warp_sum(p);
+            l[r] = l[r] * alpha + p;
 #pragma unroll
-            for (int i = 0; i < MAXI; ++i) acc[r][i] *= alpha;
+            for (int i = 0; i < NI; ++i) acc[r][i] *= alpha;
             m[r] = mn;
-            pp[r] = p;
+            pw[lane * RPW + r] = p;
         }
-        float4 *pw = reinterpret_cast<float4 *>(ps) + w * TILE;
-        pw[lane] = p4;
         __syncwarp();
-        for (int j = 0; j < TILE; ++j) {
-            float4 pj = pw[j];
-#pragma unroll
-            for (int i = 0; i < MAXI; ++i) {
-                if (i < ni) {
-                    int c = lane + 32 * i;
-                    float v = c < dp ? vs[j * dp + c] : 0.f;
-                    acc[0][i] = fmaf(pj.x, v, acc[0][i]);
-                    acc[1][i] = fmaf(pj.y, v, acc[1][i]);
-                    acc[2][i] = fmaf(pj.z, v, acc[2][i]);
-                    acc[3][i] = fmaf(pj.w, v, acc[3][i]);
-                }
-            }
-        }
+        accumulate<RPW, NI>(pw, vs, sp, dp, acc);
         __syncwarp();
     }
+    copies_wait();
 
     T *out = static_cast<T *>(a.out);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        int row = row0 + w * RPW + r;
+        const int row = row0 + w * RPW + r;
+        const float sum = warp_sum(l[r]);
         if (row >= a.tq) continue;
-        float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
-        int64_t base = (((int64_t)b * a.tq + row) * a.hq + h);
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        const int64_t base = (((int64_t)b * a.tq + row) * a.hq + h);
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) {
-            int c = lane + 32 * i;
-            if (i < ni && c < a.d) out[base * a.d + c] = Num<T>::from_f32(acc[r][i] * inv);
+        for (int i = 0; i < NI; ++i) {
+            const int c = lane + 32 * i;
+            if (c < a.d) out[base * a.d + c] = Num<T>::from_f32(acc[r][i] * inv);
         }
-        if (lane == 0) a.lse[base] = l[r] > 0.f ? m[r] + logf(l[r]) : -INFINITY;
+        if (lane == 0) a.lse[base] = sum > 0.f ? m[r] + logf(sum) : -INFINITY;
     }
 }
 
@@ -183,6 +255,7 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a) {
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
+    allow_beside();   // dkdv
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq;
     int64_t row = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
@@ -199,21 +272,19 @@ __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// dQ: each block of 32 queries sweeps, in order, the key tiles it sees.
+// dQ: each block of queries sweeps, in order, the key tiles it sees.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a) {
+template <typename T, int RPW, int NI>
+__global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    const int dp = padded_d(a.d);
-    float *qs = smem;                          // [32][dp]
-    float *gs = qs + ROWS * dp;                // [32][dp]   dO
-    float *ks = gs + ROWS * dp;                // [32][dp + 1]
-    float *vs = ks + TILE * (dp + 1);          // [32][dp + 1]
-    float *ps = vs + TILE * (dp + 1);          // [8][32][4]  dS
-    int *los = reinterpret_cast<int *>(ps + 8 * TILE * RPW);
-    int *his = los + ROWS;
-    int *pad = his + ROWS;
-    __shared__ int span[2];
+    constexpr int ROWS = WARPS * RPW;
+    const int dp = padded_d(a.d), sp = tile_stride(a.d);
+    float *qs = smem;                          // [ROWS][dp]
+    float *gs = qs + ROWS * dp;                // [ROWS][dp]   dO
+    float *kv = gs + ROWS * dp;                // [2 buffers][K, V][32][sp]
+    float *ps = kv + 4 * TILE * sp;            // [8][32][RPW]  dS
+    __shared__ RowSpans rs;
+    __shared__ int pad[2][TILE];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int qt = gridDim.x - 1 - blockIdx.x;
@@ -221,243 +292,191 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a) {
     const int hk = h / (a.hq / a.hkv);
     const int row0 = qt * ROWS;
 
-    stage_rows<T>(qs, dp, a.q, b, h, row0, a.tq, a.d, dp);
-    stage_rows<T>(gs, dp, a.dout, b, h, row0, a.tq, a.d, dp);
-    if (threadIdx.x < ROWS) {
-        int lo, hi;
-        row_bounds(a.mask, row0 + threadIdx.x, a.tq, a.tk, lo, hi);
-        los[threadIdx.x] = lo;
-        his[threadIdx.x] = hi;
-        int kmin = warp_min_i(hi > lo ? lo : a.tk);
-        int kmax = warp_max_i(hi > lo ? hi : 0);
-        if (threadIdx.x == 0) { span[0] = kmin; span[1] = kmax; }
-    }
+    stage_rows<T>(qs, dp, a.q, b, h, row0, ROWS, a.tq, a.d, vec);
+    stage_rows<T>(gs, dp, a.dout, b, h, row0, ROWS, a.tq, a.d, vec);
+    place_rows(rs, a.mask, row0, ROWS, a.tq, a.tk);
     __syncthreads();
-    const int kmin = span[0], kmax = span[1];
+    int kmin = rs.kmin, kmax = rs.kmax;
+    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
 
     int lo[RPW], hi[RPW];
     float lse[RPW], delta[RPW];
     int wlo = a.tk, whi = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        int row = row0 + w * RPW + r;
-        lo[r] = los[w * RPW + r];
-        hi[r] = his[w * RPW + r];
+        const int row = row0 + w * RPW + r;
+        lo[r] = rs.lo[w * RPW + r];
+        hi[r] = rs.hi[w * RPW + r];
         if (hi[r] > lo[r]) { wlo = min(wlo, lo[r]); whi = max(whi, hi[r]); }
         float x = INFINITY, dl = 0.f;
         if (row < a.tq) {
-            int64_t at = ((int64_t)b * a.tq + row) * a.hq + h;
+            const int64_t at = ((int64_t)b * a.tq + row) * a.hq + h;
             x = a.lse[at];
             dl = a.delta[at];
         }
         lse[r] = x == -INFINITY ? INFINITY : x;  // a query that saw no key: P = 0
         delta[r] = dl;
     }
-    float acc[RPW][MAXI];
+    float acc[RPW][NI];
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) acc[r][i] = 0.f;
-    const int ni = (dp + 31) / 32;
-
-    for (int k0 = (kmin / TILE) * TILE; k0 < kmax; k0 += TILE) {
-        __syncthreads();
-        stage_rows<T>(ks, dp + 1, a.k, b, hk, k0, a.tk, a.d, dp);
-        stage_rows<T>(vs, dp + 1, a.v, b, hk, k0, a.tk, a.d, dp);
+        for (int i = 0; i < NI; ++i) acc[r][i] = 0.f;
+    auto stage = [&](int k0, int buf) {
+        stage_rows<T>(kv + (2 * buf) * TILE * sp, sp, a.k, b, hk, k0, TILE, a.tk, a.d, vec);
+        stage_rows<T>(kv + (2 * buf + 1) * TILE * sp, sp, a.v, b, hk, k0, TILE, a.tk, a.d, vec);
         if (threadIdx.x < TILE) {
-            int key = k0 + threadIdx.x;
-            pad[threadIdx.x] = key < a.tk ? (key_padded(a.mask, b, key) ? 1 : 0) : 1;
+            const int key = k0 + threadIdx.x;
+            pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
+        copies_commit();
+    };
+    const int first = kmin / TILE * TILE;
+    if (kmax > kmin) stage(first, 0);
+    for (int k0 = first, buf = 0; k0 < kmax; k0 += TILE, buf ^= 1) {
+        copies_wait();
         __syncthreads();
+        if (k0 + TILE < kmax) stage(k0 + TILE, buf ^ 1);
         if (k0 + TILE <= wlo || k0 >= whi) continue;
+        const float *ks = kv + (2 * buf) * TILE * sp, *vs = ks + TILE * sp;
 
         float s[RPW], dpv[RPW];
-        dots4(qs + w * RPW * dp, dp, ks + lane * (dp + 1), dp, s);
-        dots4(gs + w * RPW * dp, dp, vs + lane * (dp + 1), dp, dpv);
+        dots<RPW>(qs + w * RPW * dp, dp, ks + lane * sp, dp, s);
+        dots<RPW>(gs + w * RPW * dp, dp, vs + lane * sp, dp, dpv);
         const int key = k0 + lane;
-        const bool open = pad[lane] == 0;
-        float4 d4;
-        float *dd = reinterpret_cast<float *>(&d4);
+        const bool open = pad[buf][lane] == 0;
+        float *pw = ps + w * TILE * RPW;
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            bool vis = open && key >= lo[r] && key < hi[r];
-            float p = vis ? expf(s[r] * a.scale - lse[r]) : 0.f;
-            dd[r] = p * (dpv[r] - delta[r]);
+            const bool vis = open && key >= lo[r] && key < hi[r];
+            const float p = vis ? expf(s[r] * a.scale - lse[r]) : 0.f;
+            pw[lane * RPW + r] = p * (dpv[r] - delta[r]);
         }
-        float4 *pw = reinterpret_cast<float4 *>(ps) + w * TILE;
-        pw[lane] = d4;
         __syncwarp();
-        for (int j = 0; j < TILE; ++j) {
-            float4 dj = pw[j];
-#pragma unroll
-            for (int i = 0; i < MAXI; ++i) {
-                if (i < ni) {
-                    int c = lane + 32 * i;
-                    float kv = c < dp ? ks[j * (dp + 1) + c] : 0.f;
-                    acc[0][i] = fmaf(dj.x, kv, acc[0][i]);
-                    acc[1][i] = fmaf(dj.y, kv, acc[1][i]);
-                    acc[2][i] = fmaf(dj.z, kv, acc[2][i]);
-                    acc[3][i] = fmaf(dj.w, kv, acc[3][i]);
-                }
-            }
-        }
+        accumulate<RPW, NI>(pw, ks, sp, dp, acc);
         __syncwarp();
     }
+    copies_wait();
 
     T *dq = static_cast<T *>(a.dq);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        int row = row0 + w * RPW + r;
+        const int row = row0 + w * RPW + r;
         if (row >= a.tq) continue;
-        int64_t base = (((int64_t)b * a.tq + row) * a.hq + h) * a.d;
+        const int64_t base = (((int64_t)b * a.tq + row) * a.hq + h) * a.d;
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) {
-            int c = lane + 32 * i;
-            if (i < ni && c < a.d) dq[base + c] = Num<T>::from_f32(acc[r][i] * a.scale);
+        for (int i = 0; i < NI; ++i) {
+            const int c = lane + 32 * i;
+            if (c < a.d) dq[base + c] = Num<T>::from_f32(acc[r][i] * a.scale);
         }
     }
+    end_beside();   // dkdv
 }
 
 // ---------------------------------------------------------------------------------------------
-// dK, dV: each block of 32 keys sweeps, in order, the query heads of its group and the query
-// tiles that see it; a warp owns four keys, a lane one query of the tile.
+// dK, dV: each block of keys sweeps, in order, the query heads of its group and the query
+// tiles that see it; a warp owns RPW keys, a lane one query of the tile.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a) {
+template <typename T, int RPW, int NI>
+__global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    const int dp = padded_d(a.d);
-    float *ks = smem;                          // [32][dp]
-    float *vs = ks + ROWS * dp;                // [32][dp]
-    float *qs = vs + ROWS * dp;                // [32][dp + 1]
-    float *gs = qs + TILE * (dp + 1);          // [32][dp + 1]  dO
-    float *ps = gs + TILE * (dp + 1);          // [8][32][4]  P
-    float *ds = ps + 8 * TILE * RPW;           // [8][32][4]  dS
-    float *lses = ds + 8 * TILE * RPW;         // [32]
-    float *deltas = lses + TILE;               // [32]
-    int *los = reinterpret_cast<int *>(deltas + TILE);
-    int *his = los + TILE;
-    __shared__ int span[2];
-    __shared__ int red[2][THREADS / 32];
+    constexpr int ROWS = WARPS * RPW;
+    const int dp = padded_d(a.d), sp = tile_stride(a.d);
+    float *ks = smem;                          // [ROWS][dp]
+    float *vs = ks + ROWS * dp;                // [ROWS][dp]
+    float *qg = vs + ROWS * dp;                // [2 buffers][Q, dO][32][sp]
+    float *ps = qg + 4 * TILE * sp;            // [8][32][RPW]  P
+    float *ds = ps + WARPS * TILE * RPW;       // [8][32][RPW]  dS
+    __shared__ float lses[2][TILE], deltas[2][TILE];
+    __shared__ int from[32], to[32];           // the queries that see each of the block's keys
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
     const int group = a.hq / a.hkv;
     const int key0 = kt * ROWS;
 
-    stage_rows<T>(ks, dp, a.k, b, hk, key0, a.tk, a.d, dp);
-    stage_rows<T>(vs, dp, a.v, b, hk, key0, a.tk, a.d, dp);
-
-    // The queries that see some key of [key0, key0 + 32): first and one past the last.
-    {
-        const int k1 = min(key0 + ROWS, a.tk);
-        int first = a.tq, end = 0;
-        for (int row = threadIdx.x; row < a.tq; row += THREADS) {
-            int lo, hi;
-            row_bounds(a.mask, row, a.tq, a.tk, lo, hi);
-            if (hi > lo && lo < k1 && hi > key0) { first = min(first, row); end = max(end, row + 1); }
-        }
-        first = warp_min_i(first);
-        end = warp_max_i(end);
-        if (lane == 0) { red[0][w] = first; red[1][w] = end; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int i = 1; i < THREADS / 32; ++i) { first = min(first, red[0][i]); end = max(end, red[1][i]); }
-            span[0] = first;
-            span[1] = end;
-        }
-        __syncthreads();
+    stage_rows<T>(ks, dp, a.k, b, hk, key0, ROWS, a.tk, a.d, vec);
+    stage_rows<T>(vs, dp, a.v, b, hk, key0, ROWS, a.tk, a.d, vec);
+    if (threadIdx.x < ROWS) {
+        const int key = key0 + threadIdx.x;
+        int qa = 0, qb = 0;
+        if (key < a.tk && !key_padded(a.mask, b, key)) queries_of_key(a.mask, key, a.tq, a.tk, qa, qb);
+        from[threadIdx.x] = qa;
+        to[threadIdx.x] = qb;
     }
-    const int qfirst = span[0], qend = span[1];
-
-    bool open[RPW];
+    // The queries that may see some key of the block: those that see none of them are masked key by key.
+    int qfirst, qend;
+    query_range(a.mask, key0, min(key0 + ROWS, a.tk), a.tq, a.tk, qfirst, qend);
+    wait_before();     // delta
+    allow_beside();    // dq
+    __syncthreads();
+    int qa[RPW], qb[RPW];
+    int wfrom = a.tq, wto = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        int key = key0 + w * RPW + r;
-        open[r] = key < a.tk && !key_padded(a.mask, b, key);
+        qa[r] = from[w * RPW + r];
+        qb[r] = to[w * RPW + r];
+        if (qb[r] > qa[r]) { wfrom = min(wfrom, qa[r]); wto = max(wto, qb[r]); }
     }
-    float acck[RPW][MAXI], accv[RPW][MAXI];
+    float acck[RPW][NI], accv[RPW][NI];
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) { acck[r][i] = 0.f; accv[r][i] = 0.f; }
-    const int ni = (dp + 31) / 32;
+        for (int i = 0; i < NI; ++i) { acck[r][i] = 0.f; accv[r][i] = 0.f; }
 
-    for (int g = 0; g < group; ++g) {
-        const int h = hk * group + g;
-        for (int q0 = (qfirst / TILE) * TILE; q0 < qend; q0 += TILE) {
-            __syncthreads();
-            stage_rows<T>(qs, dp + 1, a.q, b, h, q0, a.tq, a.d, dp);
-            stage_rows<T>(gs, dp + 1, a.dout, b, h, q0, a.tq, a.d, dp);
-            if (threadIdx.x < TILE) {
-                int row = q0 + threadIdx.x;
-                int lo, hi;
-                row_bounds(a.mask, row, a.tq, a.tk, lo, hi);
-                los[threadIdx.x] = lo;
-                his[threadIdx.x] = hi;
-                float x = INFINITY, dl = 0.f;
-                if (row < a.tq) {
-                    int64_t at = ((int64_t)b * a.tq + row) * a.hq + h;
-                    x = a.lse[at];
-                    dl = a.delta[at];
-                }
-                lses[threadIdx.x] = x == -INFINITY ? INFINITY : x;
-                deltas[threadIdx.x] = dl;
-            }
-            __syncthreads();
-
-            float s[RPW], dpv[RPW];
-            dots4(ks + w * RPW * dp, dp, qs + lane * (dp + 1), dp, s);
-            dots4(vs + w * RPW * dp, dp, gs + lane * (dp + 1), dp, dpv);
-            const int lo = los[lane], hi = his[lane];
-            const float lse = lses[lane], delta = deltas[lane];
-            float4 p4, d4;
-            float *pp = reinterpret_cast<float *>(&p4), *dd = reinterpret_cast<float *>(&d4);
-#pragma unroll
-            for (int r = 0; r < RPW; ++r) {
-                int key = key0 + w * RPW + r;
-                bool vis = open[r] && key >= lo && key < hi;
-                float p = vis ? expf(s[r] * a.scale - lse) : 0.f;
-                pp[r] = p;
-                dd[r] = p * (dpv[r] - delta);
-            }
-            float4 *pw = reinterpret_cast<float4 *>(ps) + w * TILE;
-            float4 *dw = reinterpret_cast<float4 *>(ds) + w * TILE;
-            pw[lane] = p4;
-            dw[lane] = d4;
-            __syncwarp();
-            for (int j = 0; j < TILE; ++j) {
-                float4 pj = pw[j], dj = dw[j];
-#pragma unroll
-                for (int i = 0; i < MAXI; ++i) {
-                    if (i < ni) {
-                        int c = lane + 32 * i;
-                        float gv = c < dp ? gs[j * (dp + 1) + c] : 0.f;
-                        float qv = c < dp ? qs[j * (dp + 1) + c] : 0.f;
-                        accv[0][i] = fmaf(pj.x, gv, accv[0][i]);
-                        accv[1][i] = fmaf(pj.y, gv, accv[1][i]);
-                        accv[2][i] = fmaf(pj.z, gv, accv[2][i]);
-                        accv[3][i] = fmaf(pj.w, gv, accv[3][i]);
-                        acck[0][i] = fmaf(dj.x, qv, acck[0][i]);
-                        acck[1][i] = fmaf(dj.y, qv, acck[1][i]);
-                        acck[2][i] = fmaf(dj.z, qv, acck[2][i]);
-                        acck[3][i] = fmaf(dj.w, qv, acck[3][i]);
-                    }
-                }
-            }
-            __syncwarp();
+    const int first = qfirst / TILE * TILE, tiles = qend > qfirst ? (qend - first + TILE - 1) / TILE : 0, steps = tiles * group;
+    auto stage = [&](int t, int buf) {
+        const int h = hk * group + t / tiles, q0 = first + t % tiles * TILE;
+        stage_rows<T>(qg + (2 * buf) * TILE * sp, sp, a.q, b, h, q0, TILE, a.tq, a.d, vec);
+        stage_rows<T>(qg + (2 * buf + 1) * TILE * sp, sp, a.dout, b, h, q0, TILE, a.tq, a.d, vec);
+        if (threadIdx.x < 2 * TILE) {
+            const int row = q0 + (threadIdx.x & 31);
+            const bool in = row < a.tq;
+            const int64_t at = ((int64_t)b * a.tq + (in ? row : 0)) * a.hq + h;
+            if (threadIdx.x < TILE) copy_async(&lses[buf][threadIdx.x], a.lse + at, in, 0);
+            else copy_async(&deltas[buf][threadIdx.x - TILE], a.delta + at, in, 0);
         }
+        copies_commit();
+    };
+    if (steps > 0) stage(0, 0);
+    for (int t = 0; t < steps; ++t) {
+        const int buf = t & 1, q0 = first + t % tiles * TILE;
+        copies_wait();
+        __syncthreads();
+        if (t + 1 < steps) stage(t + 1, buf ^ 1);
+        if (q0 + TILE <= wfrom || q0 >= wto) continue;   // no key of this warp is seen from the tile
+        const float *qs = qg + (2 * buf) * TILE * sp, *gs = qs + TILE * sp;
+
+        float s[RPW], dpv[RPW];
+        dots<RPW>(ks + w * RPW * dp, dp, qs + lane * sp, dp, s);
+        dots<RPW>(vs + w * RPW * dp, dp, gs + lane * sp, dp, dpv);
+        const int row = q0 + lane;
+        const float x = lses[buf][lane], lse = x == -INFINITY ? INFINITY : x, delta = deltas[buf][lane];
+        float *pw = ps + w * TILE * RPW, *dw = ds + w * TILE * RPW;
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) {
+            const bool vis = row >= qa[r] && row < qb[r];
+            const float p = vis ? expf(s[r] * a.scale - lse) : 0.f;
+            pw[lane * RPW + r] = p;
+            dw[lane * RPW + r] = p * (dpv[r] - delta);
+        }
+        __syncwarp();
+        accumulate<RPW, NI>(pw, gs, sp, dp, accv);
+        accumulate<RPW, NI>(dw, qs, sp, dp, acck);
+        __syncwarp();
     }
+    copies_wait();
 
     T *dk = static_cast<T *>(a.dk), *dv = static_cast<T *>(a.dv);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        int key = key0 + w * RPW + r;
+        const int key = key0 + w * RPW + r;
         if (key >= a.tk) continue;
-        int64_t base = (((int64_t)b * a.tk + key) * a.hkv + hk) * a.d;
+        const int64_t base = (((int64_t)b * a.tk + key) * a.hkv + hk) * a.d;
 #pragma unroll
-        for (int i = 0; i < MAXI; ++i) {
-            int c = lane + 32 * i;
-            if (i < ni && c < a.d) {
+        for (int i = 0; i < NI; ++i) {
+            const int c = lane + 32 * i;
+            if (c < a.d) {
                 dk[base + c] = Num<T>::from_f32(acck[r][i] * a.scale);
                 dv[base + c] = Num<T>::from_f32(accv[r][i]);
             }
@@ -468,59 +487,65 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a) {
 // ---------------------------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------------------------
-static size_t forward_smem(int d) {
-    int dp = padded_d(d);
-    return sizeof(float) * (ROWS * dp + TILE * (dp + 1) + TILE * dp + 8 * TILE * RPW) + sizeof(int) * 3 * ROWS;
+// Rows per warp: four, or one where blocks of 32 rows would leave multiprocessors without work.
+static int rows_per_warp(int64_t rows, int64_t heads) { return (rows + 31) / 32 * heads >= 148 ? 4 : 1; }
+
+// Whether every row of the view can be read 16 bytes at a time.
+template <typename T>
+static bool rows_readable(const View4 &v, int d) {
+    const int64_t per = 16 / sizeof(T);
+    return v.sd == 1 && d % per == 0 && reinterpret_cast<uintptr_t>(v.ptr) % 16 == 0 && v.sb % per == 0 && v.st % per == 0 && v.sh % per == 0;
 }
-static size_t dq_smem(int d) {
-    int dp = padded_d(d);
-    return sizeof(float) * (2 * ROWS * dp + 2 * TILE * (dp + 1) + 8 * TILE * RPW) + sizeof(int) * 3 * ROWS;
+
+// `own`: tensors whose rows the block keeps; `probs`: arrays of a tile's weights.
+static size_t generic_smem(int d, int rpw, int own, int probs) {
+    return sizeof(float) * ((size_t)own * WARPS * rpw * padded_d(d) + 4 * TILE * tile_stride(d) + (size_t)probs * WARPS * TILE * rpw);
 }
-static size_t dkdv_smem(int d) {
-    int dp = padded_d(d);
-    return sizeof(float) * (2 * ROWS * dp + 2 * TILE * (dp + 1) + 2 * 8 * TILE * RPW + 2 * TILE) + sizeof(int) * 2 * TILE;
+
+using GenericKernel = void (*)(TrainArgs, int);
+static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, cudaStream_t stream, bool beside, const TrainArgs &a, bool vec) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_beside(kernel, grid, THREADS, smem, stream, beside, a, (int)vec);
 }
+// The instance for the rows per warp and the head dimension.
+#define GENERIC_PICK(kernel, T, rpw, d)                                                                    \
+    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2> : (d) <= 128 ? kernel<T, 4, 4> : kernel<T, 4, 8>)           \
+                : ((d) <= 64 ? kernel<T, 1, 2> : (d) <= 128 ? kernel<T, 1, 4> : kernel<T, 1, 8>))
 
 template <typename T>
 static cudaError_t forward_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
-    size_t smem = forward_smem(a.d);
-    cudaError_t e = cudaFuncSetAttribute(generic_forward_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid((a.tq + ROWS - 1) / ROWS, a.hq, a.b);
-    generic_forward_kernel<T><<<grid, THREADS, smem, stream>>>(a);
+    const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b), rows = WARPS * rpw;
+    const bool vec = rows_readable<T>(a.q, a.d) && rows_readable<T>(a.k, a.d) && rows_readable<T>(a.v, a.d);
     *launches += 1;
-    return cudaGetLastError();
+    return launch_generic(GENERIC_PICK(generic_forward_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 1, 1), stream,
+                          false, a, vec);
 }
 
 template <typename T>
 static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
+    const bool vec = rows_readable<T>(a.q, a.d) && rows_readable<T>(a.k, a.d) && rows_readable<T>(a.v, a.d) && rows_readable<T>(a.dout, a.d);
     cudaError_t e;
     {
-        int64_t rows = (int64_t)a.b * a.tq * a.hq;
-        unsigned blocks = (unsigned)((rows + THREADS / 32 - 1) / (THREADS / 32));
+        const int64_t rows = (int64_t)a.b * a.tq * a.hq;
+        const unsigned blocks = (unsigned)((rows + THREADS / 32 - 1) / (THREADS / 32));
+        *launches += 1;
         generic_delta_kernel<T><<<blocks, THREADS, 0, stream>>>(a);
-        *launches += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    {
-        size_t smem = dq_smem(a.d);
-        e = cudaFuncSetAttribute(generic_dq_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    {   // brought in under delta's end; waits for it before it reads it
+        const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b), rows = WARPS * rpw;
+        *launches += 1;
+        e = launch_generic(GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3((a.tk + rows - 1) / rows, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
+                           true, a, vec);
         if (e != cudaSuccess) return e;
-        dim3 grid((a.tq + ROWS - 1) / ROWS, a.hq, a.b);
-        generic_dq_kernel<T><<<grid, THREADS, smem, stream>>>(a);
-        *launches += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    {
-        size_t smem = dkdv_smem(a.d);
-        e = cudaFuncSetAttribute(generic_dkdv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        dim3 grid((a.tk + ROWS - 1) / ROWS, a.hkv, a.b);
-        generic_dkdv_kernel<T><<<grid, THREADS, smem, stream>>>(a);
+    {   // beside dkdv, whose blocks let it in only once delta is complete
+        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b), rows = WARPS * rpw;
         *launches += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return launch_generic(GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
+                              true, a, vec);
     }
-    return cudaSuccess;
 }
 
 // The same for 16-bit rows of D = 64, 128 or 256 elements that can be read 16 bytes at a time: D / 8
