@@ -32,6 +32,7 @@ class Unsupported(NotImplementedError):
 
 
 _DTYPES = {torch.float32: DType.F32, torch.bfloat16: DType.BF16, torch.float16: DType.F16}
+_CODES = {dtype: int(code) for dtype, code in _DTYPES.items()}
 
 
 def _raise(code: int) -> None:
@@ -44,21 +45,34 @@ def _raise(code: int) -> None:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None or t.numel() == 0 else ctypes.c_void_p(t.data_ptr())
+    return None if t is None or t.numel() == 0 else t.data_ptr()
 
 
-def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+# The current stream's handle without a Stream object around it, where this torch has it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _stream(device) -> int:
+    return _raw_stream(device.index) if _raw_stream is not None else torch.cuda.current_stream(device).cuda_stream
+
+
+class _Here:
+    """The tensors' device is the current one already: nothing to switch, nothing to switch back."""
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
 
 
 def _on(device):
     """Makes the tensors' device the current one for the call: the library launches on the current
     device, and the caller's may be another (one process driving several GPUs)."""
-    return torch.cuda.device(device)
-
-
-def _strides(t: torch.Tensor, n: int):
-    return (ctypes.c_int64 * n)(*t.stride())
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _index_bytes(t: torch.Tensor, what: str) -> int:
@@ -90,53 +104,48 @@ def make_params(op: str, query, key, value, mask: AttentionMask, options: Attent
         raise AttentionError(f"{op}: queries, keys and values share one dtype")
     p = _lib.Params()
     keep = []
-    p.dtype = int(_DTYPES[query.dtype])
-    p.b, p.tq, p.hq, p.d = query.shape
-    p.k_b, p.tk, p.hkv, p.k_d = key.shape
-    if value.shape[0] != key.shape[0]:
+    b, tq, hq, d = query.shape
+    k_b, tk, hkv, k_d = key.shape
+    if value.shape[0] != k_b:
         raise AttentionError(f"{op}: key and value must have one shape")
-    _, p.v_tk, p.v_hkv, p.v_d = value.shape
-    p.q_stride, p.k_stride, p.v_stride = _strides(query, 4), _strides(key, 4), _strides(value, 4)
-    if output is not None:
-        p.o_stride = _strides(output, 4)
-    if grad_output is not None:
-        p.do_stride = _strides(grad_output, 4)
+    _, v_tk, v_hkv, v_d = value.shape
+    kp_ptr, kp_bytes, kp_shape, kp_stride = 0, 0, (0, 0), (0, 0)
+    cq_ptr, ck_ptr, cq_len, ck_len, index_bytes = 0, 0, 0, 0, 0
     if mask.kind == "key_padding":
         kp = mask.key_padding_mask
         if kp.dim() != 2:
-            raise AttentionError(f"{op}: the key padding mask is [B, Tk] = [{p.b}, {p.tk}]")
+            raise AttentionError(f"{op}: the key padding mask is [B, Tk] = [{b}, {tk}]")
         if kp.dtype in (torch.bool, torch.uint8, torch.int8):
-            p.key_padding_elem_bytes = 1
+            kp_bytes = 1
         elif kp.dtype == torch.int32:
-            p.key_padding_elem_bytes = 4
+            kp_bytes = 4
         else:
             raise AttentionError(f"{op}: the key padding mask holds 1-byte booleans or 4-byte integers")
-        p.mask_kind = _lib.MASK_KEY_PADDING
-        p.key_padding = kp.data_ptr()
-        p.key_padding_shape = (ctypes.c_int32 * 2)(*kp.shape)
-        p.key_padding_stride = (ctypes.c_int64 * 2)(*kp.stride())
+        mask_kind = _lib.MASK_KEY_PADDING
+        kp_ptr, kp_shape, kp_stride = kp.data_ptr(), kp.shape, kp.stride()
         keep.append(kp)
     elif mask.kind == "packed":
         cq, ck = mask.cu_seqlens_q, mask.cu_seqlens_k
         if cq.dim() != 1 or ck.dim() != 1 or cq.dtype != ck.dtype:
             raise AttentionError(
                 f"{op}: cu_seqlens_q and cu_seqlens_k are [S + 1], one S, got {list(cq.shape)}, {list(ck.shape)}")
-        p.mask_kind = _lib.MASK_PACKED
-        p.index_elem_bytes = _index_bytes(cq, f"{op}: cu_seqlens")
+        mask_kind = _lib.MASK_PACKED
+        index_bytes = _index_bytes(cq, f"{op}: cu_seqlens")
         cq, ck = cq.contiguous(), ck.contiguous()
-        p.cu_seqlens_q, p.cu_seqlens_k = cq.data_ptr(), ck.data_ptr()
-        p.cu_seqlens_q_len, p.cu_seqlens_k_len = cq.shape[0], ck.shape[0]
+        cq_ptr, ck_ptr, cq_len, ck_len = cq.data_ptr(), ck.data_ptr(), cq.shape[0], ck.shape[0]
         keep += [cq, ck]
     else:
-        p.mask_kind = _lib.MASK_NONE
-    p.causal = int(options.causal)
+        mask_kind = _lib.MASK_NONE
+    left = right = 0
     if options.window is not None:
-        p.has_window = 1
-        p.window_left = -1 if options.window.left is None else int(options.window.left)
-        p.window_right = -1 if options.window.right is None else int(options.window.right)
-    if options.scale is not None:
-        p.has_scale, p.scale = 1, float(options.scale)
-    p.deterministic = int(options.deterministic)
+        left = -1 if options.window.left is None else int(options.window.left)
+        right = -1 if options.window.right is None else int(options.window.right)
+    none = (0, 0, 0, 0)
+    _lib.fill(p, _lib.PARAMS_FORMAT, _CODES[query.dtype], b, tq, tk, hq, hkv, d, v_tk, v_hkv, v_d, k_b, k_d,
+              *query.stride(), *key.stride(), *value.stride(), *(none if output is None else output.stride()),
+              *(none if grad_output is None else grad_output.stride()), mask_kind, kp_ptr, kp_bytes, *kp_shape, *kp_stride,
+              cq_ptr, ck_ptr, cq_len, ck_len, index_bytes, int(options.causal), int(options.window is not None), left, right,
+              int(options.scale is not None), 0.0 if options.scale is None else float(options.scale), int(options.deterministic))
     return p, keep
 
 
@@ -215,25 +224,22 @@ def make_decode_params(query, key, value, cache_lengths, options: AttentionOptio
         raise AttentionError(f"{op}: queries, keys and values share one dtype")
     p = _lib.DecodeParams()
     keep = []
-    p.dtype = int(_DTYPES[query.dtype])
-    p.b, p.hq, p.d = query.shape
-    p.k_b, p.s, p.hkv, p.k_d = key.shape
-    p.v_b, p.v_s, p.v_hkv, p.v_d = value.shape
-    p.q_stride = _strides(query, 3)
-    p.k_stride, p.v_stride = _strides(key, 4), _strides(value, 4)
+    b, hq, d = query.shape
+    k_b, s, hkv, k_d = key.shape
+    lengths, lengths_len, lengths_bytes = 0, 0, 0
     if cache_lengths is not None:
         if cache_lengths.dim() != 1:
-            raise AttentionError(f"{op}: the cache lengths are [B] = [{p.b}]")
+            raise AttentionError(f"{op}: the cache lengths are [B] = [{b}]")
         cache_lengths = cache_lengths.contiguous()
-        p.lengths = cache_lengths.data_ptr()
-        p.lengths_len = cache_lengths.shape[0]
-        p.lengths_elem_bytes = _index_bytes(cache_lengths, f"{op}: the cache lengths")
+        lengths, lengths_len = cache_lengths.data_ptr(), cache_lengths.shape[0]
+        lengths_bytes = _index_bytes(cache_lengths, f"{op}: the cache lengths")
         keep.append(cache_lengths)
+    left = 0
     if options.window is not None:
-        p.has_window = 1
-        p.window_left = -1 if options.window.left is None else int(options.window.left)
-    if options.scale is not None:
-        p.has_scale, p.scale = 1, float(options.scale)
+        left = -1 if options.window.left is None else int(options.window.left)
+    _lib.fill(p, _lib.DECODE_PARAMS_FORMAT, _CODES[query.dtype], b, s, hq, hkv, d, k_b, k_d, *value.shape,
+              *query.stride(), *key.stride(), *value.stride(), lengths, lengths_len, lengths_bytes,
+              int(options.window is not None), left, int(options.scale is not None), 0.0 if options.scale is None else float(options.scale))
     return p, keep
 
 

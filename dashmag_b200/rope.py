@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .attention import (AttentionError, AttentionOptions, _check_device, _DTYPES, _index_bytes, _ptr, _raise, _stream,
+from .attention import (AttentionError, AttentionOptions, _check_device, _DTYPES, _index_bytes, _on, _ptr, _raise, _stream,
                         _workspace, make_decode_params)
 
 
@@ -95,7 +95,7 @@ class Rope:
         else:
             p.start, p.period = where["start"], where["period"]
         tables = self.tables()
-        with torch.cuda.device(x.device):   # the library launches on the current device
+        with _on(x.device):
             rc = _lib.lib().dash_rope_apply(ctypes.byref(tables), ctypes.byref(p), _ptr(tensors[0]), _ptr(outs[0]),
                                             _ptr(tensors[1]) if other is not None else None,
                                             _ptr(outs[1]) if other is not None else None, _stream(x.device))
@@ -166,7 +166,7 @@ def attention_decode_append_rope(rope: Rope, query, new_key, new_value, key, val
     out = torch.empty(query.shape, dtype=query.dtype, device=query.device)
     ws = _workspace(lib.dash_attn_decode_append_rope_workspace(ctypes.byref(p)), query.device)
     tables = rope.tables()
-    with torch.cuda.device(query.device):   # the library launches on the current device
+    with _on(query.device):
         rc = lib.dash_attn_decode_append_rope(ctypes.byref(p), ctypes.byref(tables),
                                               _ptr(positions.contiguous()) if positions is not None else None,
                                               positions.element_size() if positions is not None else 0,

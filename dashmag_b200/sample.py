@@ -14,7 +14,7 @@ from typing import Sequence
 import torch
 
 from . import _lib
-from .attention import AttentionError, _check_device, _DTYPES, _ptr, _raise, _stream, _workspace
+from .attention import AttentionError, _check_device, _DTYPES, _on, _ptr, _raise, _stream, _workspace
 
 
 @dataclasses.dataclass(frozen=True)
@@ -72,7 +72,7 @@ def sample(logits: torch.Tensor, options: SampleOptions = SampleOptions(), token
     out = Sampled(torch.empty(b, dtype=token_dtype, device=dev), *(torch.empty(b, dtype=torch.float32, device=dev) for _ in range(3)))
     lib = _lib.lib()
     ws = _workspace(lib.dash_sample_workspace(ctypes.byref(p)), dev)
-    with torch.cuda.device(dev):   # the library launches on the current device
+    with _on(dev):
         rc = lib.dash_sample(ctypes.byref(p), _ptr(logits), _ptr(out.tokens), _ptr(out.logprob), _ptr(out.tempered_logprob),
                              _ptr(out.sampling_logprob), _ptr(ws), 0 if ws is None else ws.numel(), _stream(dev))
     if rc != _lib.OK:
