@@ -1,0 +1,44 @@
+"""What the forward's workspace query says about splitting a tile's keys, without a GPU: a pure function of the shape, nothing
+for packed batches, f32 or calls that fill the GPU, and never more rows of parts than a few waves of tiles."""
+import ctypes
+import random
+
+import torch
+
+from dashmag_b200 import _lib
+from dashmag_b200 import attention as A
+from dashmag_b200.contract import AttentionMask, AttentionOptions
+
+C, N = AttentionOptions.causal_(), AttentionOptions()
+
+
+def splits(b, hq, hkv, tq, tk, d, options=C, dtype=torch.bfloat16, mask=AttentionMask.none()):
+    q, k = torch.empty(b, tq, hq, d, dtype=dtype, device="meta"), torch.empty(b, tk, hkv, d, dtype=dtype, device="meta")
+    p, _ = A.make_params("attention", q, k, k, mask, options)
+    need = _lib.lib().dash_attn_forward_workspace(ctypes.byref(p))
+    rows = b * tq * hq
+    if need == 0:
+        return 1
+    n = need // (4 * rows * (d + 1))
+    assert need == 4 * n * rows * d + (4 * n * rows + 255) // 256 * 256, "parts and their log-sum-exps, nothing else"
+    return n
+
+
+def test_who_is_split():
+    assert splits(1, 32, 8, 500, 8200, 128) > 1 and splits(1, 32, 8, 16, 4000, 64) > 1 and splits(1, 8, 2, 130, 4000, 256) > 1
+    assert splits(1, 32, 8, 500, 8200, 128, dtype=torch.float32) == 1 and splits(1, 32, 8, 500, 8200, 96) == 1
+    cu = torch.tensor([0, 500], dtype=torch.int32)
+    assert splits(1, 32, 8, 500, 500, 128, mask=AttentionMask.packed(cu, cu)) == 1
+    assert splits(1, 32, 8, 16384, 16384, 128) == 1 and splits(16, 12, 12, 509, 509, 64, N) == 1
+    assert splits(1, 32, 8, 500, 60, 128) == 1   # too few keys to share
+
+
+def test_the_parts_stay_a_few_waves():
+    rng = random.Random(5)
+    for _ in range(2000):
+        hkv, group, d = rng.choice([1, 2, 3, 8]), rng.choice([1, 2, 3, 4, 8, 16]), rng.choice([64, 128, 256])
+        b, tq, tk = rng.choice([1, 1, 2, 9]), rng.randint(1, 3000), rng.randint(1, 40000)
+        options = rng.choice([C, N, C.with_window(rng.randint(0, 5000), 0), N.with_window(rng.randint(0, 900), rng.randint(0, 900))])
+        n = splits(b, hkv * group, hkv, tq, tk, d, options)
+        assert 1 <= n <= 32 and n * 64 <= max(tk, 64), "a part has a sub-step's keys at least"
+        assert n == splits(b, hkv * group, hkv, tq, tk, d, options)
