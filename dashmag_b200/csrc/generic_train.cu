@@ -16,11 +16,13 @@
 // owns the head dimensions `lane + 32 i`.
 //
 // RPW is four where the rows fill the GPU that way (a tile row read from shared memory then serves four
-// products), one where they do not: small calls are bound by the length of a block's chain of tiles, not
-// by throughput.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
+// products), two or one where they do not (rows_per_warp): small calls are bound by the length of a block's chain of
+// tiles, not by throughput.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
 // Two packed sequences of 384 tokens, four heads of 64, f32: the step 254 ->
-// 68 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
+// 61 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
 // another; launch and host time are most of what is left).
+#include <algorithm>
+
 #include "bwd_common.cuh"
 #include "common.cuh"
 #include "launch.h"
@@ -255,7 +257,6 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
-    allow_beside();   // dkdv
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq;
     int64_t row = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
@@ -407,7 +408,6 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
     // The queries that may see some key of the block: those that see none of them are masked key by key.
     int qfirst, qend;
     query_range(a.mask, key0, min(key0 + ROWS, a.tk), a.tq, a.tk, qfirst, qend);
-    wait_before();     // delta
     allow_beside();    // dq
     __syncthreads();
     int qa[RPW], qb[RPW];
@@ -487,8 +487,6 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
 // ---------------------------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------------------------
-// Rows per warp: four, or one where blocks of 32 rows would leave multiprocessors without work.
-static int rows_per_warp(int64_t rows, int64_t heads) { return (rows + 31) / 32 * heads >= 148 ? 4 : 1; }
 
 // Whether every row of the view can be read 16 bytes at a time.
 template <typename T>
@@ -502,6 +500,20 @@ static size_t generic_smem(int d, int rpw, int own, int probs) {
     return sizeof(float) * ((size_t)own * WARPS * rpw * padded_d(d) + 4 * TILE * tile_stride(d) + (size_t)probs * WARPS * TILE * rpw);
 }
 
+// Rows per warp: the fewest of one, two and four whose blocks all run at once - as many to a multiprocessor as its shared
+// memory holds, up to two and a half (beyond, the reads of shared memory that more rows would share are what it waits for) -
+// else four.  Measured (rows per warp 1 | 2 | 4, us): forward of 130 tokens x 4 heads of 64 (68 | 36 | 20 blocks) 10 | 12 | 15;
+// 300 x 8 of 128 (304 | 152 | 80) 27 | 25 | 27; 1000 x 8 of 64 (1000 | 504 | 256) 190 | 122 | 124; 60 queries x 32 heads of
+// 256 against 2060 keys, one block to a multiprocessor (256 | 128 | 64) 648 | 374 | 525; 100 against 9100 (416 | 224 | 128)
+// 4339 | 3272 | 2320; backward of 300 x 8 / 2 heads of 128 122 | 144 | 180, of 1400 x 4 of 128 257 | 190 | 212.
+static int rows_per_warp(int64_t rows, int64_t heads, int d, int own, int probs) {
+    for (int rpw = 1; rpw < 4; rpw *= 2) {
+        const int64_t blocks = (rows + WARPS * rpw - 1) / (WARPS * rpw) * heads, fit = (227 * 1024) / (int64_t)generic_smem(d, rpw, own, probs);
+        if (blocks <= std::min<int64_t>(148 * fit, 370)) return rpw;
+    }
+    return 4;
+}
+
 using GenericKernel = void (*)(TrainArgs, int);
 static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, cudaStream_t stream, bool beside, const TrainArgs &a, bool vec) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -511,11 +523,12 @@ static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, 
 // The instance for the rows per warp and the head dimension.
 #define GENERIC_PICK(kernel, T, rpw, d)                                                                    \
     ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2> : (d) <= 128 ? kernel<T, 4, 4> : kernel<T, 4, 8>)           \
+     : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2> : (d) <= 128 ? kernel<T, 2, 4> : kernel<T, 2, 8>)         \
                 : ((d) <= 64 ? kernel<T, 1, 2> : (d) <= 128 ? kernel<T, 1, 4> : kernel<T, 1, 8>))
 
 template <typename T>
 static cudaError_t forward_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
-    const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b), rows = WARPS * rpw;
+    const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 1, 1), rows = WARPS * rpw;
     const bool vec = rows_readable<T>(a.q, a.d) && rows_readable<T>(a.k, a.d) && rows_readable<T>(a.v, a.d);
     *launches += 1;
     return launch_generic(GENERIC_PICK(generic_forward_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 1, 1), stream,
@@ -533,15 +546,16 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
         generic_delta_kernel<T><<<blocks, THREADS, 0, stream>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    {   // brought in under delta's end; waits for it before it reads it
-        const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b), rows = WARPS * rpw;
+    {
+        const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b, a.d, 2, 2), rows = WARPS * rpw;
         *launches += 1;
         e = launch_generic(GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3((a.tk + rows - 1) / rows, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
-                           true, a, vec);
+                           false, a, vec);
         if (e != cudaSuccess) return e;
     }
-    {   // beside dkdv, whose blocks let it in only once delta is complete
-        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b), rows = WARPS * rpw;
+    {   // beside dkdv.  (dkdv itself brought in under delta's end, to wait there, made the whole twice as slow: 1000 tokens, 4 / 2
+        // heads of 64 327 against 213 us.)
+        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), rows = WARPS * rpw;
         *launches += 1;
         return launch_generic(GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
                               true, a, vec);

@@ -1,4 +1,4 @@
-"""The CUDA-core training kernels where their tiles can go wrong: blocks of 8 and of 32 rows (calls on both sides of the line,
+"""The CUDA-core training kernels where their tiles can go wrong: blocks of 8, 16 and 32 rows (calls on both sides of the lines,
 by tokens and by heads), tiles of 32 with remainders, head dimensions on both sides of 64 and 128, of whole and of broken
 16-byte vectors, inputs no vector can read, padding and packed batches, against the f64 oracle; repeats to the bit."""
 import numpy as np
@@ -25,9 +25,9 @@ def adapter():
 
 def generic_cases():
     out = []
-    # b, hq, hkv, tq, tk, d: one query (of five keys: with one, dQ and dK are zero); a tile's edges; 147 and 148 blocks of 32 rows; several tiles a side
-    for i, (dims, options) in enumerate([((1, 2, 1, 1, 5, 64), N), ((2, 3, 3, 31, 33, 51), C), ((1, 4, 2, 65, 64, 96), C), ((1, 1, 1, 4704, 40, 4), N),
-                                         ((1, 1, 1, 4705, 40, 4), N), ((1, 148, 4, 32, 96, 66), C), ((1, 2, 1, 130, 257, 256), C.with_window(50, 0)),
+    # b, hq, hkv, tq, tk, d: one query (of five keys: with one, dQ and dK are zero); a tile's edges; 370 and 371 blocks of 8 rows, 371 of 16; several tiles a side
+    for i, (dims, options) in enumerate([((1, 2, 1, 1, 5, 64), N), ((2, 3, 3, 31, 33, 51), C), ((1, 4, 2, 65, 64, 96), C), ((1, 1, 1, 2960, 40, 4), N),
+                                         ((1, 1, 1, 2961, 40, 4), N), ((1, 1, 1, 5925, 40, 4), N), ((1, 148, 4, 32, 96, 66), C), ((1, 2, 1, 130, 257, 256), C.with_window(50, 0)),
                                          ((3, 50, 50, 70, 70, 128), C), ((1, 4, 4, 300, 300, 200), N.with_window(20, 90)), ((1, 6, 2, 40, 5000, 72), C)]):
         out.append(K.seeded(f"{dims}", list(dims), AttentionMask.none(), options, 9000 + 10 * i))
     pad = np.zeros((3, 100), dtype=bool)

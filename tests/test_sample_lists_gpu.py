@@ -35,8 +35,12 @@ def rows(kind, b, v, dtype):
 def test_lists(kind, b, v, dtype):
     z = rows(kind, b, v, dtype)
     top = tuple(int(i) for i in np.argsort(-z[0], kind="stable")[:7])
+    # The nucleus ends where the kept mass reaches p of all of it; the oracle's f32 sums know that to some 1e-6 of the mass.  With
+    # forty tokens left, p = 0.9999 puts tokens of about that weight at the edge (a row of 9001 differed, with the passes over
+    # the row as with the list), p = 0.99 none of less than 1e-4.
+    nearly_all = 0.99 if kind == "ruled out" else 0.9999
     for options in (SampleOptions(top_k=50, top_p=0.9, temperature=0.7, seed=1), SampleOptions(top_k=1, seed=2), SampleOptions(top_k=20, seed=3),
-                    SampleOptions(top_k=3000, top_p=0.5, seed=4), SampleOptions(top_p=0.9, temperature=0.7, seed=5), SampleOptions(top_p=0.9999, seed=6),
+                    SampleOptions(top_k=3000, top_p=0.5, seed=4), SampleOptions(top_p=0.9, temperature=0.7, seed=5), SampleOptions(top_p=nearly_all, seed=6),
                     SampleOptions(top_k=30, top_p=0.95, masked=top, seed=7), SampleOptions(top_p=0.6, masked=top, seed=8)):
         got, want = run(z, dtype, options), oracle_of(z, options)
         tau = float(S.inverse_temperature(options.temperature))
