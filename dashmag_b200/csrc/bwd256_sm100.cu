@@ -94,7 +94,7 @@ namespace {
 
 // One block's pass.  `r1` / `r2` are the tensor maps of the resident tensors (r2 unused by DV),
 // `s1` / `s2` those of the streamed ones: DQ (Q, dO | K, V), DK and DV (K, V | Q, dO).
-template <typename T, int PASS>
+template <typename T, int PASS, bool SPLIT>
 __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtensorMap *r2, const CUtensorMap *s1,
                                             const CUtensorMap *s2, const Sm100BwdArgs &a, uint8_t *smem, int b, int row0,
                                             int res_head) {
@@ -186,9 +186,13 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         tiles = any_row && qend > qfirst ? (qend - qfirst + qt - 1) / qt : 0;
         head0 = res_head * group;
     }
-    const int steps = aborted ? 0 : (ROWS_ARE_QUERIES ? tiles : tiles * (group >> pack));
-    auto step_head = [&](int t) { return ROWS_ARE_QUERIES ? head0 : head0 + ((t / tiles) << pack); };
-    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t * ROWS : (t % tiles) * qt); };
+    // SPLIT (DK / DV): the two blocks of a cluster share the sweep, the first half of the steps and the second, and meet at the end.
+    const int all_steps = ROWS_ARE_QUERIES ? tiles : tiles * (group >> pack), first_half = SPLIT ? (all_steps + 1) / 2 : all_steps;
+    const uint32_t part = SPLIT ? cluster_rank() : 0u;
+    const int t0 = part ? first_half : 0;
+    const int steps = aborted ? 0 : part ? all_steps - first_half : first_half;
+    auto step_head = [&](int t) { return ROWS_ARE_QUERIES ? head0 : head0 + (((t + t0) / tiles) << pack); };
+    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t * ROWS : ((t + t0) % tiles) * qt); };
     bool failed = aborted;
     constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 256;
 
@@ -427,6 +431,40 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 if (!ROWS_ARE_QUERIES) mbar_arrive(BAR(sh.bar.aux_free[st]));
             }
         }
+        // The accumulator is complete before the blocks meet.
+        if (SPLIT && steps > 0 && !failed && !__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.acc_ready), 0))) failed = true;
+    }
+    if constexpr (SPLIT) {
+        // The second block's share of the f32 sums goes into the first one's shared memory, whose tiles are dead once both
+        // have got here: thread by thread, 16 bytes apart, so that a warp's stores are contiguous.  The first block adds
+        // the two shares in one order and writes the result.  Every thread of both blocks passes both meetings.
+        constexpr int EW_THREADS = 32 * EW_WARPS;
+        __syncwarp();
+        cluster_sync();
+        if (part == 1 && steps > 0 && warp >= 2 && warp < AUX_WARP) {
+            const int cg = (warp - 2) >> 2;
+            const uint32_t at = cluster_map(smem_u32(smem), 0) + (uint32_t)(threadIdx.x - 64) * 16;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t o[32];
+                tmem_ld32(tmem + (static_cast<uint32_t>(lane_base) << 16) + COL_ACC + cg * 64 + c * 32, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    cluster_store4(at + (uint32_t)((c * 8 + e) * EW_THREADS * 16), o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+            }
+            tc_fence_before_sync();
+        }
+        __syncwarp();
+        cluster_sync();
+    }
+    if (warp >= 2 && warp < AUX_WARP && part == 0) {
+        const int cg = (warp - 2) >> 2;
+        const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
+        const int head = ROWS_ARE_QUERIES ? res_head + (r & ((1 << pack) - 1)) : res_head;
+        const bool shared_sweep = SPLIT && all_steps > first_half;   // the second block had steps
+        const uint4 *theirs = reinterpret_cast<const uint4 *>(smem) + (threadIdx.x - 64);
         // ---------------- epilogue: 64 columns of the row per thread ----------------
         T *dst;
         bool in_range;
@@ -453,6 +491,16 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
                 uint32_t o[32];
                 tmem_ld32(t_lane + COL_ACC + cg * 64 + c * 32, o);
                 tmem_ld_wait();
+                if (shared_sweep) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const uint4 x = theirs[(c * 8 + e) * 32 * EW_WARPS];
+                        o[4 * e + 0] = __float_as_uint(__uint_as_float(o[4 * e + 0]) + __uint_as_float(x.x));
+                        o[4 * e + 1] = __float_as_uint(__uint_as_float(o[4 * e + 1]) + __uint_as_float(x.y));
+                        o[4 * e + 2] = __float_as_uint(__uint_as_float(o[4 * e + 2]) + __uint_as_float(x.z));
+                        o[4 * e + 3] = __float_as_uint(__uint_as_float(o[4 * e + 3]) + __uint_as_float(x.w));
+                    }
+                }
                 if (in_range) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -489,24 +537,27 @@ bwd256_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const Sm100BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem256[];
     const int qt = gridDim.y - 1 - blockIdx.y;   // later (longer, under causality) tiles first
-    bwd256_pass<T, PASS_DQ>(&tm_q, &tm_do, &tm_k, &tm_v, a, smem256, blockIdx.z, qt * (ROWS >> a.pack), blockIdx.x << a.pack);
+    bwd256_pass<T, PASS_DQ, false>(&tm_q, &tm_do, &tm_k, &tm_v, a, smem256, blockIdx.z, qt * (ROWS >> a.pack), blockIdx.x << a.pack);
     end_beside();
 }
 
-// blockIdx.x: the (key block, key-value head) unit in the plan's order; blockIdx.y: 0 the dK pass (the
+// SPLIT: a cluster of two blocks a unit and pass, each half of the unit's steps: with few units the longest of them - all
+// queries that see the key block, of all heads of the group, in steps of 2.6 us - is the kernel's length.  Where units fill the
+// GPU without it the second set-up and the meeting only cost (figures at the launch).
+// blockIdx.x: the (key block, key-value head) unit in the plan's order (SPLIT: twice); blockIdx.y: 0 the dK pass (the
 // longer one: three products a step), 1 the dV pass.
-template <typename T>
+template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 bwd256_dkdv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do, const Sm100BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem256[];
     allow_beside();   // dq
     const int nkb = (a.tk + ROWS - 1) / ROWS;
-    const int unit = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
+    const int at = SPLIT ? blockIdx.x >> 1 : blockIdx.x, unit = a.order ? a.order[at] : at;
     const int item = unit / a.hkv, hk = unit - item * a.hkv;
     const int b = item / nkb, kt = item - b * nkb;
-    if (blockIdx.y == 0) bwd256_pass<T, PASS_DK>(&tm_k, &tm_v, &tm_q, &tm_do, a, smem256, b, kt * ROWS, hk);
-    else bwd256_pass<T, PASS_DV>(&tm_k, &tm_v, &tm_q, &tm_do, a, smem256, b, kt * ROWS, hk);
+    if (blockIdx.y == 0) bwd256_pass<T, PASS_DK, SPLIT>(&tm_k, &tm_v, &tm_q, &tm_do, a, smem256, b, kt * ROWS, hk);
+    else bwd256_pass<T, PASS_DV, SPLIT>(&tm_k, &tm_v, &tm_q, &tm_do, a, smem256, b, kt * ROWS, hk);
 }
 
 namespace {
@@ -516,14 +567,28 @@ cudaError_t launch256_t(const Sm100BwdMaps &m, const Sm100BwdArgs &a, cudaStream
     static_assert(smem_bytes(PASS_DK) == smem && smem_bytes(PASS_DV) <= smem, "one size for the three passes");
     cudaError_t e = cudaFuncSetAttribute(bwd256_dq_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(bwd256_dkdv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     const long long units = (long long)a.b * ((a.tk + ROWS - 1) / ROWS) * a.hkv;
-    if (units > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    dim3 gk((unsigned)units, 2, 1);
-    bwd256_dkdv_kernel<T><<<gk, THREADS, smem, stream>>>(m.k128, m.v128, m.q128, m.do128, a);
+    if (units > 0x3fffffffLL) return cudaErrorInvalidConfiguration;
+    // Two blocks a unit while all of them, two passes each, are fewer than the multiprocessors twice over.  (One sequence of
+    // 2000 tokens, 8 / 2 heads - 32 units: 208 -> 146 us a step; 700 in two, 12 units: 85 -> 68.  But 6144 tokens, 96 units: 643
+    // -> 639; 4000 in four, 4 / 4 heads, 128 units: 156 -> 191; 8192 in four, 32 / 16 heads, 1024 units: 2123 -> 2333.)
+    const bool split = units <= 74;
+    const auto kernel = split ? bwd256_dkdv_kernel<T, true> : bwd256_dkdv_kernel<T, false>;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)units * (split ? 2 : 1), 2, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = split ? 1 : 0;
     *launches += 1;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = cudaLaunchKernelEx(&cfg, kernel, m.k128, m.v128, m.q128, m.do128, a)) != cudaSuccess) return e;
     // dq's short blocks beside the last waves of dk and dv (see bwd_sm100.cu).
     const int tokens = ROWS >> a.pack;
     dim3 gq(a.hq >> a.pack, (a.tq + tokens - 1) / tokens, a.b);
