@@ -211,9 +211,10 @@ int dash_rope_apply(const dash_rope_tables *rope, const dash_rope_params *p, con
  * positions, e.g. for a cache that slides), then the step is dash_attn_decode_append with the
  * rotated query and key - the reference's caller does Rope::apply_at on the query, Rope::apply_at
  * on the key, two put_along_axis_owned and attention_decode, five dispatches, where this is one
- * call that launches the rotation (both tensors at once, into the workspace) and the decoding
- * step's own kernels.  The result is bit-identical to dash_rope_apply followed by
- * dash_attn_decode_append.  q's last stride must be 1.
+ * call: the split pass rotates what it reads where it can (16-bit, a rotated width of whole
+ * 16-byte halves), else the rotation is launched first (both tensors at once, into the workspace).
+ * The result is bit-identical to dash_rope_apply followed by dash_attn_decode_append.  q's last
+ * stride must be 1.
  */
 size_t dash_attn_decode_append_rope_workspace(const dash_attn_decode_params *p);
 int dash_attn_decode_append_rope(const dash_attn_decode_params *p, const dash_rope_tables *rope,
