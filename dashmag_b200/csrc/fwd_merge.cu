@@ -4,7 +4,8 @@
 // A warp a row, a lane D / 32 neighbouring features, so that a part is one coalesced read; the parts of a row are summed
 // in their order, so the bits repeat.  Bound by launch and latency at the sizes that split (the parts of 500 queries x 32
 // heads x 128 in 4 splits are 33 MB, still in L2): the blocks are brought in under the sweep's last wave.
-// Side by side: 500 queries against 8200 keys, 32 / 8 heads of 128 (64 tiles, two splits) 131 -> 86 us, merge included.
+// Side by side: 500 queries against 8200 keys, 32 / 8 heads of 128 (64 tiles, two splits) 131 -> 84 us, merge included
+// (87 with a row's log-sum-exps read one after another and its features 8 bytes a lane).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -23,29 +24,37 @@ __global__ void __launch_bounds__(MERGE_THREADS) fwd_merge_kernel(const Sm100Fwd
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq, row = (int64_t)blockIdx.x * (MERGE_THREADS / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
-    float mx = -INFINITY;
-    for (int s = 0; s < a.splits; ++s) mx = fmaxf(mx, a.part_lse[s * rows + row]);
-    float num[PER], den = 0.f;
+    // Lane s weighs part s (there are at most 32); a part that saw no key left nothing and weighs nothing.
+    const float part = lane < a.splits ? a.part_lse[lane * rows + row] : -INFINITY, mx = warp_max(part);
+    const float weight = part != -INFINITY ? expf(part - mx) : 0.f, den = warp_sum(weight);
+    float num[PER];
 #pragma unroll
     for (int c = 0; c < PER; ++c) num[c] = 0.f;
-    if (mx != -INFINITY) {
-        for (int s = 0; s < a.splits; ++s) {
-            const float w = expf(a.part_lse[s * rows + row] - mx);
-            if (w == 0.f) continue;   // a part that saw no key left nothing
-            const float *po = a.part_o + (s * rows + row) * HD + lane * PER;
-            den += w;
+#pragma unroll 4
+    for (int s = 0; s < a.splits; ++s) {
+        const float w = __shfl_sync(0xffffffffu, weight, s);
+        if (w == 0.f) continue;
+        const float *po = a.part_o + (s * rows + row) * HD + lane * PER;
+        if constexpr (PER % 4 == 0) {
 #pragma unroll
-            for (int c = 0; c < PER; c += 2) {
-                const float2 x = *reinterpret_cast<const float2 *>(po + c);
+            for (int c = 0; c < PER; c += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(po + c);
                 num[c] = fmaf(w, x.x, num[c]);
                 num[c + 1] = fmaf(w, x.y, num[c + 1]);
+                num[c + 2] = fmaf(w, x.z, num[c + 2]);
+                num[c + 3] = fmaf(w, x.w, num[c + 3]);
             }
+        } else {
+            const float2 x = *reinterpret_cast<const float2 *>(po);
+            num[0] = fmaf(w, x.x, num[0]);
+            num[1] = fmaf(w, x.y, num[1]);
         }
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
-    T *out = static_cast<T *>(a.out) + row * HD + lane * PER;
+    struct alignas(2 * PER) Out { T e[PER]; } out;   // a lane's features in one store
 #pragma unroll
-    for (int c = 0; c < PER; ++c) out[c] = Num<T>::from_f32(num[c] * inv);
+    for (int c = 0; c < PER; ++c) out.e[c] = Num<T>::from_f32(num[c] * inv);
+    *reinterpret_cast<Out *>(static_cast<T *>(a.out) + row * HD + lane * PER) = out;
     if (lane == 0) a.lse[row] = den > 0.f ? (float)((double)mx + log((double)den)) : -INFINITY;
 }
 
