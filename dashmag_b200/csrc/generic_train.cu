@@ -116,19 +116,30 @@ __device__ __forceinline__ void dots(const float *rows, int row_stride, const fl
 template <int RPW, int NI>
 __device__ __forceinline__ void accumulate(const float *weight, const float *tile, int stride, int dp, float (&acc)[RPW][NI]) {
     const int lane = threadIdx.x & 31;
-#pragma unroll 8
-    for (int j = 0; j < TILE; ++j) {
-        float w[RPW];
+    constexpr int JS = 4 / RPW;   // rows whose weights are one 16-byte read
+#pragma unroll 8 / JS
+    for (int j0 = 0; j0 < TILE; j0 += JS) {
+        const float4 w4 = *reinterpret_cast<const float4 *>(weight + j0 * RPW);
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) w[r] = weight[j * RPW + r];
+        for (int jj = 0; jj < JS; ++jj)
 #pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int c = lane + 32 * i;
-            const float v = c < dp ? tile[j * stride + c] : 0.f;
+            for (int i = 0; i < NI; ++i) {
+                const int c = lane + 32 * i;
+                const float v = c < dp ? tile[(j0 + jj) * stride + c] : 0.f;
 #pragma unroll
-            for (int r = 0; r < RPW; ++r) acc[r][i] = fmaf(w[r], v, acc[r][i]);
-        }
+                for (int r = 0; r < RPW; ++r) acc[r][i] = fmaf(w[jj * RPW + r], v, acc[r][i]);
+            }
     }
+}
+
+// A lane's weights for the warp's rows, in one store.
+template <int RPW>
+__device__ __forceinline__ void put_weights(float *weight, const float (&w)[RPW]) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (RPW == 4) reinterpret_cast<float4 *>(weight)[lane] = make_float4(w[0], w[1], w[2], w[3]);
+    else if constexpr (RPW == 2) reinterpret_cast<float2 *>(weight)[lane] = make_float2(w[0], w[1]);
+    else weight[lane] = w[0];
 }
 
 // The block's first row, and what each of its rows sees: the queries' key intervals (warp 0 places them) and their union.
@@ -212,7 +223,7 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
         dots<RPW>(qs + w * RPW * dp, dp, ks + lane * sp, dp, s);
         const int key = k0 + lane;
         const bool open = pad[buf][lane] == 0;
-        float *pw = ps + w * TILE * RPW;
+        float *pw = ps + w * TILE * RPW, ps4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const bool vis = open && key >= lo[r] && key < hi[r];
@@ -227,8 +238,9 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
 #pragma unroll
             for (int i = 0; i < NI; ++i) acc[r][i] *= alpha;
             m[r] = mn;
-            pw[lane * RPW + r] = p;
+            ps4[r] = p;
         }
+        put_weights<RPW>(pw, ps4);
         __syncwarp();
         accumulate<RPW, NI>(pw, vs, sp, dp, acc);
         __syncwarp();
@@ -346,13 +358,14 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
         dots<RPW>(gs + w * RPW * dp, dp, vs + lane * sp, dp, dpv);
         const int key = k0 + lane;
         const bool open = pad[buf][lane] == 0;
-        float *pw = ps + w * TILE * RPW;
+        float *pw = ps + w * TILE * RPW, ds4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const bool vis = open && key >= lo[r] && key < hi[r];
             const float p = vis ? expf(s[r] * a.scale - lse[r]) : 0.f;
-            pw[lane * RPW + r] = p * (dpv[r] - delta[r]);
+            ds4[r] = p * (dpv[r] - delta[r]);
         }
+        put_weights<RPW>(pw, ds4);
         __syncwarp();
         accumulate<RPW, NI>(pw, ks, sp, dp, acc);
         __syncwarp();
@@ -452,14 +465,16 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
         dots<RPW>(vs + w * RPW * dp, dp, gs + lane * sp, dp, dpv);
         const int row = q0 + lane;
         const float x = lses[buf][lane], lse = x == -INFINITY ? INFINITY : x, delta = deltas[buf][lane];
-        float *pw = ps + w * TILE * RPW, *dw = ds + w * TILE * RPW;
+        float *pw = ps + w * TILE * RPW, *dw = ds + w * TILE * RPW, ps4[RPW], ds4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const bool vis = row >= qa[r] && row < qb[r];
             const float p = vis ? expf(s[r] * a.scale - lse) : 0.f;
-            pw[lane * RPW + r] = p;
-            dw[lane * RPW + r] = p * (dpv[r] - delta);
+            ps4[r] = p;
+            ds4[r] = p * (dpv[r] - delta);
         }
+        put_weights<RPW>(pw, ps4);
+        put_weights<RPW>(dw, ds4);
         __syncwarp();
         accumulate<RPW, NI>(pw, gs, sp, dp, accv);
         accumulate<RPW, NI>(dw, qs, sp, dp, acck);
