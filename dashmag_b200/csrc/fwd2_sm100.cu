@@ -483,10 +483,10 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                                                 __uint_as_float(o[4 * e + 2]) * inv, __uint_as_float(o[4 * e + 3]) * inv);
                     }
                 }
-                if (row < a.tq) {   // (as below)
+                if (row < a.tq) {   // (as below, but that a part which met a NaN leaves one: -inf is the mark of a part without keys)
                     const float used = __fmul_rn(m_ref, a.scale_log2);
                     const double slip = (double)used - (double)m_ref * (double)a.scale_log2;
-                    a.part_lse[at] = l > 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
+                    a.part_lse[at] = l != 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
                 }
                 tc_fence_before_sync();
             } else {

@@ -24,16 +24,18 @@ __global__ void __launch_bounds__(MERGE_THREADS) fwd_merge_kernel(const Sm100Fwd
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq, row = (int64_t)blockIdx.x * (MERGE_THREADS / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
-    // Lane s weighs part s (there are at most 32); a part that saw no key left nothing and weighs nothing.
+    // Lane s weighs part s (there are at most 32).  A part that saw no key (-inf) left nothing and is not read; every other one
+    // counts, whatever its weight: a NaN, in a part's sum or in its features, is a NaN of the row, as in the unsplit sweep.
     const float part = lane < a.splits ? a.part_lse[lane * rows + row] : -INFINITY, mx = warp_max(part);
     const float weight = part != -INFINITY ? expf(part - mx) : 0.f, den = warp_sum(weight);
+    const unsigned seen = __ballot_sync(0xffffffffu, part != -INFINITY);
     float num[PER];
 #pragma unroll
     for (int c = 0; c < PER; ++c) num[c] = 0.f;
 #pragma unroll 4
     for (int s = 0; s < a.splits; ++s) {
         const float w = __shfl_sync(0xffffffffu, weight, s);
-        if (w == 0.f) continue;
+        if (!(seen >> s & 1u)) continue;
         const float *po = a.part_o + (s * rows + row) * HD + lane * PER;
         if constexpr (PER % 4 == 0) {
 #pragma unroll

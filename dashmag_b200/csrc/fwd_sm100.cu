@@ -417,7 +417,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (row < a.tq) {
                 const float used = __fmul_rn(m_ref, a.scale_log2);   // what the loop subtracted from every exponent
                 const double slip = (double)used - (double)m_ref * (double)a.scale_log2;
-                *lse_at = l > 0.f ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
+                // (A part that met a NaN leaves one: -inf is the mark of a part without keys.)
+                *lse_at = (part ? l != 0.f : l > 0.f) ? (float)((double)m_ref * (double)a.scale + slip * 0.6931471805599453 + log((double)l)) : -INFINITY;
             }
             tc_fence_before_sync();
         } else {

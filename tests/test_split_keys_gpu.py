@@ -60,3 +60,24 @@ def test_split_forward(i, dtype):
     assert rc == _lib.OK
     assert np.max(np.abs(o1.float().cpu().numpy() - want_o)) <= OUTPUT * scale * np.max(np.abs(want_o))
     assert np.max(np.abs(lse1.cpu().numpy()[seen] - want_lse[seen])) <= SWEEP[1] * np.max(np.abs(want_lse[seen]))
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("where,bad", [("q", "nan"), ("k", "nan"), ("k", "inf"), ("v", "nan"), ("v", "inf")])
+def test_a_part_hides_no_nan(d, where, bad):
+    """A NaN or an infinity in a query, key or value comes out of the split forward where it comes out of the unsplit one."""
+    host = [oracle.seeded(s, 70 + j) for j, s in enumerate([(1, 150, 8, d), (1, 3000, 2, d), (1, 3000, 2, d)])]
+    q, k, v = (torch.from_numpy(x).cuda().to(torch.bfloat16) for x in host)
+    {"q": q, "k": k, "v": v}[where][0, 100, 0, 3] = float(bad)   # every query sees key 100
+    p, keep = A.make_params("attention", q, k, v, AttentionMask.none(), C)
+    assert _lib.lib().dash_attn_forward_workspace(ctypes.byref(p)) > 0
+    o, lse = A.attention_with_lse(q, k, v, AttentionMask.none(), C)
+    o1, lse1 = torch.zeros_like(o), torch.zeros_like(lse)
+    rc = _lib.lib().dash_attn_forward(ctypes.byref(p), A._ptr(q), A._ptr(k), A._ptr(v), A._ptr(o1), A._ptr(lse1), None, 0, A._stream(q.device))
+    assert rc == _lib.OK
+    assert not torch.isfinite(o1).all()
+    assert torch.equal(torch.isfinite(o), torch.isfinite(o1)) and torch.equal(torch.isfinite(lse), torch.isfinite(lse1))
+    if bad == "nan":
+        assert torch.equal(torch.isnan(o), torch.isnan(o1))
+    whole = torch.isfinite(o1)
+    assert torch.max(torch.abs(o[whole].float() - o1[whole].float())) <= 2 * OUTPUT * torch.max(torch.abs(o1[whole].float()))
