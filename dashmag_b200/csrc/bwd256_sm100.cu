@@ -192,7 +192,8 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
     const int t0 = part ? first_half : 0;
     const int steps = aborted ? 0 : part ? all_steps - first_half : first_half;
     auto step_head = [&](int t) { return ROWS_ARE_QUERIES ? head0 : head0 + (((t + t0) / tiles) << pack); };
-    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t * ROWS : ((t + t0) % tiles) * qt); };
+    // (DK / DV: the last queries first, as in bwd_sm100.cu: small terms before large ones.)
+    auto step_col0 = [&](int t) { return col_first + (ROWS_ARE_QUERIES ? t * ROWS : (tiles - 1 - (t + t0) % tiles) * qt); };
     bool failed = aborted;
     constexpr uint32_t COL_S = 0, COL_DP = 128, COL_ACC = 256;
 
