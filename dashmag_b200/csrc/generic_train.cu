@@ -42,8 +42,8 @@ __device__ __forceinline__ void copy_async(float *dst, const void *src, bool val
     if (bytes16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(valid ? 16 : 0) : "memory");
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src), "r"(valid ? 4 : 0) : "memory");
 }
-__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+// All of this thread's copies, the resident rows' too: a block with nothing to sweep must not leave with them in flight.
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Copies rows [r0, r0 + rows) of one head into shared memory as f32, zero past `limit` and past d.  `vec`: every row of the
 // source can be read 16 bytes at a time and d is whole 16-byte vectors (f32: asynchronously, complete after copies_wait).
@@ -208,7 +208,6 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
             const int key = k0 + threadIdx.x;
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
-        copies_commit();
     };
     const int first = kmin / TILE * TILE;
     if (kmax > kmin) stage(first, 0);
@@ -342,7 +341,6 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
             const int key = k0 + threadIdx.x;
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
-        copies_commit();
     };
     const int first = kmin / TILE * TILE;
     if (kmax > kmin) stage(first, 0);
@@ -449,7 +447,6 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
             if (threadIdx.x < TILE) copy_async(&lses[buf][threadIdx.x], a.lse + at, in, 0);
             else copy_async(&deltas[buf][threadIdx.x - TILE], a.delta + at, in, 0);
         }
-        copies_commit();
     };
     if (steps > 0) stage(0, 0);
     for (int t = 0; t < steps; ++t) {

@@ -92,3 +92,27 @@ def test_rows_no_vector_can_read():
         got = A.attention_with_lse(q, k, v, mask, C)
         got_g = A.attention_backward(q, k, v, *got, go, mask, C)
         assert all(torch.equal(x, y) for x, y in zip((*got, *got_g), (*want, *want_g))), lay.__name__
+
+
+# Rows whose blocks have nothing to sweep (their own rows still arrive asynchronously, and the block waits for them before it
+# leaves): b, hq, hkv, tq, tk, d with blocks of 8, 16 and 32 rows; all keys padded, or causal with more queries than keys.
+@pytest.mark.parametrize("shape", [(2, 4, 2, 40, 40, 64), (1, 8, 8, 700, 60, 128), (2, 16, 16, 600, 600, 64), (1, 2, 1, 33, 9, 256)], ids=str)
+@pytest.mark.parametrize("kind", ["all padding", "causal"])
+def test_blocks_with_nothing_to_sweep(shape, kind):
+    b, hq, hkv, tq, tk, d = shape
+    host = [oracle.seeded(s, 9600 + j) for j, s in enumerate([(b, tq, hq, d), (b, tk, hkv, d), (b, tk, hkv, d), (b, tq, hq, d)])]
+    q, k, v, g = (torch.from_numpy(x).cuda() for x in host)
+    if kind == "causal":
+        mask, options, blind = AttentionMask.none(), C, max(tq - tk, 0)
+    else:
+        mask, options, blind = AttentionMask.key_padding(torch.ones(b, tk, dtype=torch.bool, device="cuda")), N, tq
+    for _ in range(20):
+        o, lse = A.attention_with_lse(q, k, v, mask, options)
+        dq, dk, dv = A.attention_backward(q, k, v, o, lse, g, mask, options)
+        assert not o[:, :blind].any() and torch.isneginf(lse[:, :blind]).all() and not dq[:, :blind].any()
+        if blind == tq:
+            assert not dk.any() and not dv.any()
+    if kind == "causal":
+        want_o, want_lse = oracle.forward(*host[:3], causal=True)
+        assert np.max(np.abs(o.cpu().numpy() - want_o)) <= OWN[DType.F32][0] * np.max(np.abs(want_o))
+        assert torch.isfinite(lse[:, blind:]).all()
