@@ -79,6 +79,7 @@ struct Tail {
     uint32_t tmem_base;
     unsigned int abort;
     int red_lo[4], red_hi[4];
+    uint32_t share_whole[EW_WARPS];   // split: whether the second block's warp got through its sweep (written by that block)
 };
 constexpr size_t TAIL_BYTES = 3072;
 static_assert(sizeof(Tail) <= TAIL_BYTES, "the tail of the kernel's shared memory");
@@ -438,10 +439,14 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
     if constexpr (SPLIT) {
         // The second block's share of the f32 sums goes into the first one's shared memory, whose tiles are dead once both
         // have got here: thread by thread, 16 bytes apart, so that a warp's stores are contiguous.  The first block adds
-        // the two shares in one order and writes the result.  Every thread of both blocks passes both meetings.
+        // the two shares in one order and writes the result.  Every thread of both blocks passes both meetings.  With each
+        // warp's share goes whether it is whole: where a wait of the second block ran out (or it found the status raised) the first
+        // stores nothing either.
         constexpr int EW_THREADS = 32 * EW_WARPS;
         __syncwarp();
         cluster_sync();
+        if (part == 1 && warp >= 2 && warp < AUX_WARP && lane == 0)
+            cluster_store1(cluster_map(smem_u32(&sh.share_whole[warp - 2]), 0), failed ? 0u : 1u);
         if (part == 1 && steps > 0 && warp >= 2 && warp < AUX_WARP) {
             const int cg = (warp - 2) >> 2;
             const uint32_t at = cluster_map(smem_u32(smem), 0) + (uint32_t)(threadIdx.x - 64) * 16;
@@ -466,6 +471,7 @@ __device__ __forceinline__ void bwd256_pass(const CUtensorMap *r1, const CUtenso
         const int head = ROWS_ARE_QUERIES ? res_head + (r & ((1 << pack) - 1)) : res_head;
         const bool shared_sweep = SPLIT && all_steps > first_half;   // the second block had steps
         const uint4 *theirs = reinterpret_cast<const uint4 *>(smem) + (threadIdx.x - 64);
+        if (shared_sweep && sh.share_whole[warp - 2] == 0) failed = true;
         // ---------------- epilogue: 64 columns of the row per thread ----------------
         T *dst;
         bool in_range;

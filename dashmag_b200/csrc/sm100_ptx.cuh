@@ -97,6 +97,10 @@ __device__ __forceinline__ void cluster_store4(uint32_t addr, uint32_t x, uint32
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
+__device__ __forceinline__ void cluster_store1(uint32_t addr, uint32_t x) {
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
+}
+
 // ---- proxies and thread sync ---------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
