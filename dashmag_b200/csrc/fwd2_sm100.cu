@@ -536,6 +536,8 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         } else {
             failed = true;
         }
+        // A part whose waits ran out left nothing: its rows come out of the merge as NaN (and the status is raised).
+        if (a.splits > 1 && failed && row < a.tq) a.part_lse[(int64_t)split * gridDim.z * a.tq * a.hq + base] = __int_as_float(0x7fc00000);
         if (steps > 0 && a.splits == 1) {
             // Every warp of the tile gets here (all waits are bounded), whatever became of it: one
             // that gave up marks the tile, and nothing is stored from a tile that is not whole.

@@ -424,6 +424,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         } else {
             failed = true;
         }
+        // A part whose waits ran out left nothing: its rows come out of the merge as NaN (and the status is raised).
+        if (part && failed && row < a.tq) *lse_at = __int_as_float(0x7fc00000);
     }
 
     if (failed && !aborted) atomicOr(&g_sm100_status, 1u);
