@@ -89,6 +89,11 @@ def _check_device(op: str, *tensors):
             raise Unsupported(f"{op}: tensors must be on a CUDA device; this library has no CPU path")
 
 
+def _strides(t: Optional[torch.Tensor]):
+    """A [B, T, H, D] tensor's strides; zeros for none, and for one of another rank, which its caller refuses by its shape."""
+    return t.stride() if t is not None and t.dim() == 4 else (0, 0, 0, 0)
+
+
 def make_params(op: str, query, key, value, mask: AttentionMask, options: AttentionOptions,
                 output=None, grad_output=None) -> Tuple[_lib.Params, list]:
     """``dash_attn_params`` for a call, and the tensors it points to (kept alive by the caller)."""
@@ -140,10 +145,8 @@ def make_params(op: str, query, key, value, mask: AttentionMask, options: Attent
     if options.window is not None:
         left = -1 if options.window.left is None else int(options.window.left)
         right = -1 if options.window.right is None else int(options.window.right)
-    none = (0, 0, 0, 0)
     _lib.fill(p, _lib.PARAMS_FORMAT, _CODES[query.dtype], b, tq, tk, hq, hkv, d, v_tk, v_hkv, v_d, k_b, k_d,
-              *query.stride(), *key.stride(), *value.stride(), *(none if output is None else output.stride()),
-              *(none if grad_output is None else grad_output.stride()), mask_kind, kp_ptr, kp_bytes, *kp_shape, *kp_stride,
+              *query.stride(), *key.stride(), *value.stride(), *_strides(output), *_strides(grad_output), mask_kind, kp_ptr, kp_bytes, *kp_shape, *kp_stride,
               cq_ptr, ck_ptr, cq_len, ck_len, index_bytes, int(options.causal), int(options.window is not None), left, right,
               int(options.scale is not None), 0.0 if options.scale is None else float(options.scale), int(options.deterministic))
     return p, keep
