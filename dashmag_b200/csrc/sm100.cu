@@ -198,14 +198,17 @@ int forward_splits(const dash_attn_params *p) {
     const int64_t tiles = (p->tq + tokens - 1) / tokens, blocks = tiles * (p->hq >> pack) * p->b;
     if (blocks >= 2 * sms) return 1;
     int64_t longest = p->tk, mean = p->tk;
-    const int64_t right = p->causal ? 0 : p->has_window && p->window_right >= 0 ? p->window_right : -1;
+    // A side that reaches past every key is no bound (and must not be added to).
+    const int64_t none = (int64_t)p->tq + p->tk + 1;
+    auto side = [&](int64_t reach) { return p->has_window && reach >= 0 && reach < none ? reach : int64_t(-1); };
+    const int64_t left = side(p->window_left), right = p->causal ? 0 : side(p->window_right);
     if (right >= 0) {   // query i sees keys up to i + tk - tq + right
         const int64_t last = std::min<int64_t>(p->tk, p->tk + right), first = std::min<int64_t>(p->tk, std::max<int64_t>(p->tk - p->tq + right + tokens, 0));
         longest = last;
         mean = (first + last) / 2;
     }
-    if (p->has_window && p->window_left >= 0) {
-        const int64_t reach = (int64_t)p->window_left + std::max<int64_t>(right, 0) + tokens;
+    if (left >= 0) {
+        const int64_t reach = left + std::max<int64_t>(right, 0) + tokens;
         longest = std::min(longest, right < 0 ? p->tk : reach);
         mean = std::min(mean, longest);
     }

@@ -42,3 +42,13 @@ def test_the_parts_stay_a_few_waves():
         n = splits(b, hkv * group, hkv, tq, tk, d, options)
         assert 1 <= n <= 32 and n * 64 <= max(tk, 64), "a part has a sub-step's keys at least"
         assert n == splits(b, hkv * group, hkv, tq, tk, d, options)
+
+
+def test_sides_past_every_key_are_no_bound():
+    big = [2 ** 63 - 1, 2 ** 63 - 2, 2 ** 62, 2 ** 40]
+    for tq, tk, d in ((500, 8200, 128), (37, 3001, 64), (300, 3001, 256), (130, 4000, 128)):
+        for options, sides in ((C, [(x, 0) for x in big]), (C, [(x, y) for x in big for y in big]), (N, [(x, y) for x in big for y in big])):
+            for left, right in sides:
+                assert splits(1, 32, 8, tq, tk, d, options.with_window(left, right)) == splits(1, 32, 8, tq, tk, d, options), (options, left, right)
+        for x in big:
+            assert splits(1, 32, 8, tq, tk, d, N.with_window(200, x)) == splits(1, 32, 8, tq, tk, d, N.with_window(200, None))
