@@ -281,7 +281,7 @@ int dash_attn_kernels_take(const dash_attn_params *p, const void *q, const void 
 
 size_t dash_attn_forward_workspace(const dash_attn_params *p) {
     if (!p || check_train("attention", p) != DASH_ATTN_OK || degenerate(p)) return 0;
-    return dash::sm100_forward_workspace(p);
+    return g_force_generic.load() ? 0 : dash::sm100_forward_workspace(p, g_force_tensor.load() != 0);
 }
 
 size_t dash_attn_backward_workspace(const dash_attn_params *p) {

@@ -58,12 +58,13 @@ bool device_is_sm100() {
 
 // The reference's in-place rule (crates/dash-ops/src/attention/cube.rs:428-461), which is also what
 // a TMA tensor map needs: last stride 1, the others multiples of 16 bytes, base 16-byte aligned.
-bool tma_readable(const void *ptr, const int64_t *stride) {
-    if (reinterpret_cast<uintptr_t>(ptr) % 16 != 0 || stride[3] != 1) return false;
+bool tma_strides(const int64_t *stride) {
+    if (stride[3] != 1) return false;
     for (int i = 0; i < 3; ++i)
         if (stride[i] % 8 != 0 || stride[i] < 0) return false;
     return true;
 }
+bool tma_base(const void *ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; }
 
 // A [B, T, H, d] tensor of 16-bit elements (d = 64, 128 or 256) as a 4-D map (d, h, t, b) with boxes of
 // 64 x heads x (rows / heads) x 1 and the 128-byte swizzle: each load brings 128 rows of 128 bytes, of one
@@ -161,8 +162,9 @@ int pack_log2(int group, int tq) {
 
 uint64_t sm100_tensor_map_encodes() { return g_map_encodes.load(std::memory_order_relaxed); }
 
-bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const void *v, int backward, bool any_size) {
-    if (backward && !tma_readable(q, p->do_stride)) return false;  // dO's strides; its base is checked at launch
+// What sm100_takes asks of a call's parameters (of its pointers and of the device: there).
+static bool parameters_taken(const dash_attn_params *p, int backward, bool any_size) {
+    if (backward && !tma_strides(p->do_stride)) return false;  // dO's base is checked at launch
     if (p->dtype != DASH_ATTN_BF16 && p->dtype != DASH_ATTN_F16) return false;
     // Head dimensions 64 and 256 only from 128 queries and 128 keys on: below that there is a single
     // partial tile of queries or of keys (one block per head), the tensor cores gain nothing, and the
@@ -174,9 +176,13 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
     if (p->d != 128 && !((p->d == 64 || p->d == 256) && big)) return false;
     const float scale = resolved_scale(p);
     if (!(scale > 0.f) || !std::isfinite(scale)) return false;  // the row maximum is taken before scaling
-    if (!q || !k || !v) return false;
-    if (!tma_readable(q, p->q_stride) || !tma_readable(k, p->k_stride) || !tma_readable(v, p->v_stride)) return false;
-    if (p->hq > 65535 || p->b > 65535) return false;   // grid extents
+    if (!tma_strides(p->q_stride) || !tma_strides(p->k_stride) || !tma_strides(p->v_stride)) return false;
+    return p->hq <= 65535 && p->b <= 65535;   // grid extents
+}
+
+bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const void *v, int backward, bool any_size) {
+    if (!parameters_taken(p, backward, any_size)) return false;
+    if (!q || !k || !v || !tma_base(q) || !tma_base(k) || !tma_base(v)) return false;
     if (!device_is_sm100() || !encoder()) return false;
     return true;
 }
@@ -224,10 +230,11 @@ int forward_splits(const dash_attn_params *p) {
 }
 static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }
 static size_t split_lse_bytes(const dash_attn_params *p, int splits) { return (sizeof(float) * split_rows(p, splits) + 255) & ~size_t(255); }
-size_t sm100_forward_workspace(const dash_attn_params *p) {
-    const bool takes = (p->dtype == DASH_ATTN_BF16 || p->dtype == DASH_ATTN_F16) && (p->d == 64 || p->d == 128 || p->d == 256);
-    const int splits = takes ? forward_splits(p) : 1;
+static size_t split_bytes(const dash_attn_params *p, int splits) {
     return splits > 1 ? split_lse_bytes(p, splits) + sizeof(float) * split_rows(p, splits) * p->d : 0;
+}
+size_t sm100_forward_workspace(const dash_attn_params *p, bool any_size) {
+    return parameters_taken(p, 0, any_size) ? split_bytes(p, forward_splits(p)) : 0;   // a call the generic kernels take is not split
 }
 // Whether a backward call takes the five-product form that adds dQ by reductions in L2: only when the
 // caller gave up the fixed order of summation, and only where that form exists (D = 64, 128).
@@ -245,7 +252,6 @@ cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *w
     // keeps the one-tile kernel (for comparison runs).
     static const bool one_tile = [] { const char *e = std::getenv("DASH_ATTN_FWD_TILES"); return e && std::atoi(e) == 1; }();
     const int kv_rows = 128;
-    (void)one_tile;
     CUtensorMap tq, tk, tv, to;
     const int64_t o_stride[4] = {(int64_t)p->tq * p->hq * p->d, (int64_t)p->hq * p->d, p->d, 1};   // the output is contiguous
     const int pack = pack_log2(p->hq / p->hkv, p->tq);
@@ -265,9 +271,9 @@ cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *w
     f.mask = a.mask;
     f.pack = pack;
     // Without scratch for the parts (or with less than the query asks for) the keys stay in one block.
-    const size_t need = sm100_forward_workspace(p);
-    const bool split = need > 0 && workspace && workspace_bytes >= need && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && !one_tile;
-    f.splits = split ? forward_splits(p) : 1;
+    const int splits = forward_splits(p);
+    const bool split = splits > 1 && workspace && workspace_bytes >= split_bytes(p, splits) && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && !one_tile;
+    f.splits = split ? splits : 1;
     if (split) {
         f.part_lse = static_cast<float *>(workspace);
         f.part_o = reinterpret_cast<float *>(static_cast<char *>(workspace) + split_lse_bytes(p, f.splits));

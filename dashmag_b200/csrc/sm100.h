@@ -18,7 +18,7 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
 uint64_t sm100_tensor_map_encodes();
 // Extra scratch the tensor-core path needs beyond what the C ABI layer itself plans.
 // (The forward runs without it too, its keys then not split over blocks.)
-size_t sm100_forward_workspace(const dash_attn_params *p);
+size_t sm100_forward_workspace(const dash_attn_params *p, bool any_size);
 size_t sm100_backward_workspace(const dash_attn_params *p);
 // Launchers: add to *launches; a failure that is not a CUDA error code is reported through `err`.
 cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *workspace, size_t workspace_bytes, cudaStream_t stream,

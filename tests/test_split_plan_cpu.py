@@ -25,12 +25,22 @@ def splits(b, hq, hkv, tq, tk, d, options=C, dtype=torch.bfloat16, mask=Attentio
 
 
 def test_who_is_split():
-    assert splits(1, 32, 8, 500, 8200, 128) > 1 and splits(1, 32, 8, 16, 4000, 64) > 1 and splits(1, 8, 2, 130, 4000, 256) > 1
+    assert splits(1, 32, 8, 500, 8200, 128) > 1 and splits(1, 32, 8, 130, 4000, 64) > 1 and splits(1, 8, 2, 130, 4000, 256) > 1
+    assert splits(1, 32, 8, 16, 4000, 128) > 1
     assert splits(1, 32, 8, 500, 8200, 128, dtype=torch.float32) == 1 and splits(1, 32, 8, 500, 8200, 96) == 1
     cu = torch.tensor([0, 500], dtype=torch.int32)
     assert splits(1, 32, 8, 500, 500, 128, mask=AttentionMask.packed(cu, cu)) == 1
     assert splits(1, 32, 8, 16384, 16384, 128) == 1 and splits(16, 12, 12, 509, 509, 64, N) == 1
     assert splits(1, 32, 8, 500, 60, 128) == 1   # too few keys to share
+    # What the CUDA-core kernels take is never split, and no scratch is asked for: few queries at D 64 and 256, a scale the
+    # tensor-core kernels refuse, rows no tile load can read.
+    assert splits(1, 32, 8, 16, 4000, 64) == 1 and splits(1, 32, 8, 100, 9100, 256) == 1
+    assert splits(1, 32, 8, 500, 8200, 128, C.with_scale(-0.1)) == 1
+    q = torch.empty(1, 500, 32, 128, dtype=torch.bfloat16, device="meta")
+    for width, step in ((256, 2), (132, 1)):
+        k = torch.empty(1, 8200, 8, width, dtype=torch.bfloat16, device="meta")[..., : 128 * step : step]
+        p, _ = A.make_params("attention", q, k, k, AttentionMask.none(), C)
+        assert _lib.lib().dash_attn_forward_workspace(ctypes.byref(p)) == 0
 
 
 def test_the_parts_stay_a_few_waves():
