@@ -191,8 +191,11 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
 // against a long cache - has fewer tiles than the GPU has multiprocessors, each a long sweep: cut into runs of keys they
 // fill it.  Estimated in steps of 64 keys (128 at D 256): a block's share of its sweep plus what a block costs however
 // short its sweep (set-up, the first tiles' flight, the output: about six steps of the two-tile kernel, three of the
-// other's, which are twice as long), times the waves of blocks; a split also pays for its partial rows and the merge
-// (about five and three steps).  The sweep is the longest tile's; under causality with as many queries as keys the mean
+// other's, which are twice as long), times the waves of blocks; a split also pays for the merge's launch (five and three
+// steps) and for the f32 rows of its parts, written and read at about 2.5 TB/s (a step is 0.95 us, the other's 1.8).  Measured
+// at forced numbers of splits over 100 calls (130 to 4096 queries, D 64 to 256, 5 to 32 heads), the pick is never slower than
+// the unsplit call; with the parts unpriced 3000 tokens, 12 / 4 heads of 128, were split in two, 65.7 us against 53.4, and 256
+// queries against 30000 keys, 32 / 8 heads of 256, in nine, 313 us against 227 in two.  The sweep is the longest tile's; under causality with as many queries as keys the mean
 // is half of it, so the waves are counted on the mean and the longest tile is a bound of its own.  Packed batches, whose
 // lengths the host does not know, are not split.  A chunk of 500 queries against 8200 keys, 32 / 8 heads (64 tiles):
 // see the figures at fwd_merge.cu.
@@ -218,14 +221,15 @@ int forward_splits(const dash_attn_params *p) {
         longest = std::min(longest, right < 0 ? p->tk : reach);
         mean = std::min(mean, longest);
     }
-    const int64_t l = (longest + step - 1) / step, m = (mean + step - 1) / step, fixed = one ? 3 : 6, merge = one ? 4 : 8;
+    const int64_t l = (longest + step - 1) / step, m = (mean + step - 1) / step, fixed = one ? 3 : 6;
+    const double merge = one ? 3 : 5, part = (double)p->b * p->tq * p->hq * p->d * sizeof(float) / (one ? 4.5e6 : 2.4e6);
     auto cost = [&](int64_t s) {
         const int64_t waves = (blocks * s + sms - 1) / sms;
-        return std::max(waves * ((m + s - 1) / s + fixed), (l + s - 1) / s + fixed) + (s > 1 ? merge : 0);
+        return (double)std::max(waves * ((m + s - 1) / s + fixed), (l + s - 1) / s + fixed) + (s > 1 ? merge + s * part : 0.);
     };
     int best = 1;
     for (int s = 2; s <= 32 && l / s >= 2 && tiles * s <= 65535; ++s)
-        if (cost(s) * 10 < cost(1) * 9 && cost(s) < cost(best)) best = s;
+        if (cost(s) < 0.95 * cost(1) && cost(s) < cost(best)) best = s;
     return best;
 }
 static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }

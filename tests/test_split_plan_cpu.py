@@ -1,5 +1,5 @@
 """What the forward's workspace query says about splitting a tile's keys, without a GPU: a pure function of the shape, nothing
-for packed batches, f32 or calls that fill the GPU, and never more rows of parts than a few waves of tiles."""
+for packed batches, f32 or calls that fill the GPU, and never more parts than the sweep they shorten is worth."""
 import ctypes
 import random
 
@@ -43,15 +43,34 @@ def test_who_is_split():
         assert _lib.lib().dash_attn_forward_workspace(ctypes.byref(p)) == 0
 
 
-def test_the_parts_stay_a_few_waves():
+def test_the_parts_stay_bounded():
     rng = random.Random(5)
+    most = 0
     for _ in range(2000):
         hkv, group, d = rng.choice([1, 2, 3, 8]), rng.choice([1, 2, 3, 4, 8, 16]), rng.choice([64, 128, 256])
-        b, tq, tk = rng.choice([1, 1, 2, 9]), rng.randint(1, 3000), rng.randint(1, 40000)
+        b, tq, tk = rng.choice([1, 1, 2, 9]), rng.randint(130, 3000), rng.randint(130, 40000)
         options = rng.choice([C, N, C.with_window(rng.randint(0, 5000), 0), N.with_window(rng.randint(0, 900), rng.randint(0, 900))])
         n = splits(b, hkv * group, hkv, tq, tk, d, options)
-        assert 1 <= n <= 32 and n * 64 <= max(tk, 64), "a part has a sub-step's keys at least"
-        assert n == splits(b, hkv * group, hkv, tq, tk, d, options)
+        most = max(most, n)
+        if n == 1:
+            continue
+        pack = 1   # heads of a group in a tile
+        while pack < 8 and group % (2 * pack) == 0:
+            pack *= 2
+        rows, step, step_bytes = (128, 128, 4.5e6) if d == 256 else (256, 64, 2.4e6)   # of a block; keys of a step; f32 parts that cost one
+        blocks = -(-tq // (rows // pack)) * (hkv * group // pack) * b
+        steps = -(-tk // step)
+        assert n <= 32 and n <= steps // 2, "a part has two steps of keys at least"
+        assert blocks < 2 * 148, "a call that fills the GPU is not split"
+        waves = -(-blocks // 148)
+        assert 4 * n * b * tq * hkv * group * d <= step_bytes * waves * (steps + 6), "the parts cost less than the sweep they shorten"
+    assert most > 8
+
+
+def test_many_rows_are_not_split():
+    """Calls that measured slower in parts than whole: their f32 rows outweigh the shorter sweep."""
+    assert splits(1, 12, 4, 3000, 3000, 128) == 1 and splits(1, 12, 4, 1500, 1500, 128) == 1 and splits(1, 12, 4, 2048, 4096, 128) == 1
+    assert splits(1, 12, 4, 1000, 3000, 256) == 1 and splits(1, 5, 1, 3000, 3000, 256) == 1 and splits(1, 12, 4, 3000, 3000, 64) == 1
 
 
 def test_sides_past_every_key_are_no_bound():
