@@ -192,9 +192,10 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
 // fill it.  Estimated in steps of 64 keys (128 at D 256): a block's share of its sweep plus what a block costs however
 // short its sweep (set-up, the first tiles' flight, the output: about six steps of the two-tile kernel, three of the
 // other's, which are twice as long), times the waves of blocks; a split also pays for the merge's launch (five and three
-// steps) and for the f32 rows of its parts, written and read at about 2.5 TB/s (a step is 0.95 us, the other's 1.8).  Measured
-// at forced numbers of splits over 100 calls (130 to 4096 queries, D 64 to 256, 5 to 32 heads), the pick is never slower than
-// the unsplit call; with the parts unpriced 3000 tokens, 12 / 4 heads of 128, were split in two, 65.7 us against 53.4, and 256
+// steps) and for the f32 rows of its parts, written and read at about 2.5 TB/s (a step is 0.95 us, the other's 1.8).  Only
+// an estimate a tenth below the whole sweep's is taken: the last wave's blocks are the short ones, which the count of waves
+// does not know (2380 queries against 6897 keys, 8 / 2 heads of 256, 150 blocks: 123 us whole, 143 in three).  At forced
+// numbers of splits over 200 calls (130 to 5000 queries, D 64 to 256, 4 to 32 heads) the pick is never slower than the whole; with the parts unpriced 3000 tokens, 12 / 4 heads of 128, were split in two, 65.7 us against 53.4, and 256
 // queries against 30000 keys, 32 / 8 heads of 256, in nine, 313 us against 227 in two.  The sweep is the longest tile's; under causality with as many queries as keys the mean
 // is half of it, so the waves are counted on the mean and the longest tile is a bound of its own.  Packed batches, whose
 // lengths the host does not know, are not split.  A chunk of 500 queries against 8200 keys, 32 / 8 heads (64 tiles):
@@ -229,7 +230,7 @@ int forward_splits(const dash_attn_params *p) {
     };
     int best = 1;
     for (int s = 2; s <= 32 && l / s >= 2 && tiles * s <= 65535; ++s)
-        if (cost(s) < 0.95 * cost(1) && cost(s) < cost(best)) best = s;
+        if (cost(s) < 0.9 * cost(1) && cost(s) < cost(best)) best = s;
     return best;
 }
 static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }

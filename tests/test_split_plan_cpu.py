@@ -71,6 +71,7 @@ def test_many_rows_are_not_split():
     """Calls that measured slower in parts than whole: their f32 rows outweigh the shorter sweep."""
     assert splits(1, 12, 4, 3000, 3000, 128) == 1 and splits(1, 12, 4, 1500, 1500, 128) == 1 and splits(1, 12, 4, 2048, 4096, 128) == 1
     assert splits(1, 12, 4, 1000, 3000, 256) == 1 and splits(1, 5, 1, 3000, 3000, 256) == 1 and splits(1, 12, 4, 3000, 3000, 64) == 1
+    assert splits(1, 8, 2, 2380, 6897, 256) == 1   # 150 blocks: the second wave is two short ones
 
 
 def test_sides_past_every_key_are_no_bound():
