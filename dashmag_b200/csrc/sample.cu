@@ -14,12 +14,12 @@
 //      every token tied with the last one is kept by construction, as the definition wants.  Two
 //      passes for 16-bit logits (their keys are their own 16 bits), four for f32, and all but the
 //      first look only at the tokens that share the bytes found so far;
-//      A cut leaves few tokens of many, and a lower bound of its threshold is cheap: the k-th largest of the THREADS' maxima
-//      is a token at least k tokens reach (its top byte is enough), and a nucleus never reaches down to a weight that all
-//      tokens together could hold without filling 1 - p of the mass.  The tokens above the bound go into a list in shared
-//      memory - under top-k in the pass that sums the exponentials anyway - and the search and the draw look at the list;
-//      a list that would not fit leaves the passes over the row.  64 x 151936 bf16 logits, k = 50, p = 0.9: 74 -> 45 us
-//      side by side.
+//      Top-k leaves few tokens of many, and a lower bound of its threshold is cheap: the k-th largest of the THREADS' maxima
+//      is a token at least k tokens reach.  The tokens above the bound go into a list in shared memory, in the pass that sums
+//      the exponentials anyway, and the search and the draw look at the list; a list that would not fit leaves the passes over
+//      the row.  64 x 151936 bf16 logits, k = 50, p = 0.9: 74 -> 45 us side by side.  (A nucleus alone has no such bound
+//      without one more pass over the row, which cost more than the list gave at every spread of the logits: N(0, 10) 67.8
+//      us with it, 63.8 without.)
 //   4. argmax over the kept tokens of s_i + g_i, ties to the lowest id, four tokens per Philox call;
 //   5. the three log-probabilities, taken from one another where the definition says they are one
 //      number (tau = 1; nothing cut).
@@ -164,7 +164,7 @@ struct RadixSmem {
     uint32_t mass[3][8][256][4];
     uint32_t tcnt[256];
     unsigned long long tmass[256];
-    uint32_t sel, above_cnt;
+    uint32_t sel, above_cnt, reach;
     unsigned long long above_mass, target;
 };
 constexpr float MASS_ONE = 1099511627776.0f;   // 2^40: a weight in (0, 1] as an integer
@@ -175,26 +175,25 @@ constexpr float MASS_ONE = 1099511627776.0f;   // 2^40: a weight in (0, 1] as an
 // the tokens that share the bits found so far are looked at again.  Masked tokens count as -inf
 // for top-k (they sort last, as in the reference) and take no part in the masses.
 //
-// `each(f)` calls f(token, logit, whether it is masked) for this thread's tokens; `groups` of the copies of the bins are used
-// (eight for a row, one for a list's few tokens); `total` is the mass the tokens hold where the caller knows it to be more than
-// what `each` visits (else 0); `levels` the bytes to find.
-template <typename T, bool MASS, typename Each>
-__device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uint32_t floor_key, RadixSmem &sm, int groups, unsigned long long total_mass,
-                                    int levels) {
+// `each(f)` calls f(token, logit, whether it is masked) for this thread's tokens; GROUPS of the copies of the bins are used
+// (eight for a row, one for a list's few tokens).  The search ends early, with the low bits of T zero, once no more than
+// `enough` tokens reach T; `reaching` is how many do.
+template <typename T, bool MASS, int GROUPS, typename Each>
+__device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uint32_t floor_key, RadixSmem &sm, uint32_t enough, uint32_t &reaching) {
     cg::cluster_group cluster = cg::this_cluster();
     const int blocks = (int)cluster.num_blocks();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t key_ninf = Key<T>::of(Num<T>::from_f32(-INFINITY));
     uint32_t prefix = 0, above_cnt = 0;
     unsigned long long above_mass = 0, target = 0;
-    for (int level = 0; level < levels; ++level) {
+    for (int level = 0; level < Key<T>::BITS / 8; ++level) {
         const int shift = Key<T>::BITS - 8 * (level + 1);
-        for (int i = threadIdx.x; i < groups * 4 * 256; i += ST) {
+        for (int i = threadIdx.x; i < GROUPS * 4 * 256; i += ST) {
             (&sm.cnt[0][0][0])[i] = 0;
             if (MASS) { (&sm.mass[0][0][0][0])[i] = 0; (&sm.mass[1][0][0][0])[i] = 0; (&sm.mass[2][0][0][0])[i] = 0; }
         }
         __syncthreads();
-        const int copies = groups == 1 ? 0 : warp >> 2;
+        const int copies = GROUPS == 1 ? 0 : warp >> 2;
         each([&](int, T zi, bool gone) {
             if (MASS && gone) return;
             const uint32_t key = gone ? key_ninf : Key<T>::of(zi);
@@ -215,7 +214,7 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
         if (threadIdx.x < 256) {
             uint32_t c = 0;
             unsigned long long w = 0;
-            for (int x = 0; x < 4 * groups; ++x) {
+            for (int x = 0; x < 4 * GROUPS; ++x) {
                 c += sm.cnt[x >> 2][threadIdx.x][x & 3];
                 if (MASS) w += (unsigned long long)sm.mass[0][x >> 2][threadIdx.x][x & 3] + ((unsigned long long)sm.mass[1][x >> 2][threadIdx.x][x & 3] << 14) +
                                ((unsigned long long)sm.mass[2][x >> 2][threadIdx.x][x & 3] << 28);
@@ -250,7 +249,7 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
                 if (lane >= o) { c_before += cu; w_before += wu; }
             }
             if (MASS && level == 0) {
-                const unsigned long long seen = __shfl_sync(0xffffffffu, w_before, 31), total = total_mass ? total_mass : seen;
+                const unsigned long long total = __shfl_sync(0xffffffffu, w_before, 31);
                 target = __double2ull_ru((double)a.p * (double)total);
             }
             uint32_t run_c = above_cnt + c_before - c8;
@@ -269,6 +268,7 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
             const unsigned vote = __ballot_sync(0xffffffffu, hit >= 0);
             const int src = vote ? __ffs(vote) - 1 : 31;   // the lowest lane: the highest bin
             if (lane == src) {
+                sm.reach = run_c;   // up to the bin taken, or all of them
                 sm.sel = hit >= 0 ? (uint32_t)hit : 0u;
                 sm.above_cnt = hit >= 0 ? hit_c : run_c;
                 sm.above_mass = hit >= 0 ? hit_w : run_w;
@@ -277,15 +277,17 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
         }
         __syncthreads();
         prefix = (prefix << 8) | sm.sel;
+        reaching = sm.reach;
         above_cnt = sm.above_cnt;
         above_mass = sm.above_mass;
         target = sm.target;
         __syncthreads();   // read before the next level writes
+        if (enough > 0 && reaching <= enough) return prefix << shift;
     }
     return prefix;
 }
 
-// The tokens above a bound of the cuts' threshold: their ids and the bits of their logits.
+// The tokens above a bound of top-k's threshold: their ids and the bits of their logits.
 constexpr int LIST_MAX = 8192;   // per block
 struct TokenList {
     uint32_t id[LIST_MAX], bits[LIST_MAX];
@@ -301,7 +303,9 @@ template <typename T> __device__ __forceinline__ T from_bits(uint32_t u) {
     return x;
 }
 
-template <typename T>
+// LIST: top-k of at most half the row's threads, by the list of candidates.  (An instance of its own: the other calls paid 2 to
+// 4 us for code they never took.)
+template <typename T, bool LIST>
 __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     __shared__ unsigned long long us[32], uslot;
     __shared__ int listed_here;   // tokens that asked for a place in the block's list
@@ -332,28 +336,32 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     const bool tempered_differs = !a.greedy && a.tau != 1.0f;
     const bool cut = a.top_k > 0 || a.has_p;
     auto each_logit = [&](auto f) { for_each_logit(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) { f(i, zi, masked(i)); }); };
-    // Top-k's bound: the top byte of the k-th largest of the threads' maxima (at least k of them reach it).
-    const bool k_list = !a.greedy && !degenerate && a.top_k > 0 && a.top_k <= TS / 2;
-    uint32_t bound = 0;
-    if (k_list) {
-        auto each_maximum = [&](auto f) { if (mine != -INFINITY) f(0, Num<T>::from_f32(mine), false); };
-        bound = radix_threshold<T, false>(each_maximum, a, m, 0u, radix, 1, 0, 1) << (Key<T>::BITS - 8);
+    // Top-k's bound: the k-th largest of the threads' maxima (at least k of them reach it), as many bytes of it as it takes for no
+    // more than half the threads to reach it: the row's tokens that do are then about 0.7 of the threads' number, whatever the
+    // logits' offset and spread - where all bytes leave more, ties crowd at the cut and no list is made.  (One byte of a bf16
+    // key is a factor of four: of logits N(20, 3) it held nearly all.)  Below it -inf, which is never drawn and weighs nothing.
+    bool listed = LIST && !degenerate;
+    uint32_t bound = 0xffffffffu;
+    if constexpr (LIST) {
+        if (listed) {
+            auto each_maximum = [&](auto f) { if (mine != -INFINITY) f(0, Num<T>::from_f32(mine), false); };
+            uint32_t reaching = 0;
+            bound = max(radix_threshold<T, false, 1>(each_maximum, a, m, 0u, radix, TS / 2, reaching), key_ninf + 1);
+            listed = reaching <= TS / 2;
+            if (!listed) bound = 0xffffffffu;
+        }
+        if (threadIdx.x == 0) listed_here = 0;
+        __syncthreads();
     }
-    const bool p_list = !a.greedy && !degenerate && a.has_p && a.top_k == 0;
-    if (threadIdx.x == 0) listed_here = 0;
-    __syncthreads();
     float s1 = 0.f, wu = 0.f;
-    unsigned long long mass = 0;   // p_list: the tempered mass in the search's fixed point
     int first = a.v;   // the lowest unmasked id holding the maximum
     for_each_logit(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
         if (masked(i)) return;
         const float x = Num<T>::to_f32(zi);
-        const float e1 = expf(x - m), eu = tempered_differs ? expf(__fmul_rn(x - m, a.tau)) : e1;
-        s1 += e1;
-        if (tempered_differs) wu += eu;
+        s1 += expf(x - m);
+        if (tempered_differs) wu += expf((x - m) * a.tau);
         if (x == m && i < first) first = i;
-        if (p_list) mass += __float2ull_rn(eu * MASS_ONE);
-        if (k_list && Key<T>::of(zi) >= bound) {
+        if (LIST && Key<T>::of(zi) >= bound) {
             const int at = atomicAdd(&listed_here, 1);
             if (at < LIST_MAX) { list.id[at] = (uint32_t)i; list.bits[at] = bits_of(zi); }
         }
@@ -370,32 +378,20 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     } else {
         // 3. The cuts: one threshold T on the keys; 0 keeps every token.
         uint32_t t_keep = 0;
-        constexpr int LEVELS = Key<T>::BITS / 8;
-        bool listed = (k_list || p_list) && s1 == s1;   // a NaN among the logits: the passes over the row
-        if (p_list && listed) {
-            mass = row_reduce(mass, AddOp(), us, &uslot);
-            // V tokens of less than this weight hold less than half of 1 - p of the mass: the nucleus ends above it (by a
-            // margin that the rounding of weights and logarithm is far inside).
-            const float floor_s = logf(0.5f * (1.f - a.p) * (tempered_differs ? wu : s1) / (float)a.v) - 0.01f;
-            each_logit([&](int i, T zi, bool gone) {
-                if (gone || !(__fmul_rn(Num<T>::to_f32(zi) - m, a.tau) >= floor_s)) return;
-                const int at = atomicAdd(&listed_here, 1);
-                if (at < LIST_MAX) { list.id[at] = (uint32_t)i; list.bits[at] = bits_of(zi); }
-            });
-        }
-        if (k_list || p_list) {
+        uint32_t reaching = 0;
+        if constexpr (LIST) {
             __syncthreads();
             const int most = row_reduce(-listed_here, MinOp(), is, &islot);   // of any block of the row
-            listed = listed && -most <= LIST_MAX;
+            listed = listed && s1 == s1 && -most <= LIST_MAX;   // (a NaN among the logits: the passes over the row)
         }
         if (listed) {
             const int n = listed_here;
             auto each_listed = [&](auto f) { for (int j = threadIdx.x; j < n; j += ST) f((int)list.id[j], from_bits<T>(list.bits[j]), false); };
-            if (a.top_k > 0) t_keep = radix_threshold<T, false>(each_listed, a, m, 0u, radix, 1, 0, LEVELS);
-            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true>(each_listed, a, m, t_keep, radix, 1, p_list ? mass : 0, LEVELS));
+            t_keep = radix_threshold<T, false, 1>(each_listed, a, m, 0u, radix, 0, reaching);
+            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 1>(each_listed, a, m, t_keep, radix, 0, reaching));
         } else {
-            if (a.top_k > 0) t_keep = radix_threshold<T, false>(each_logit, a, m, 0u, radix, 8, 0, LEVELS);
-            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true>(each_logit, a, m, t_keep, radix, 8, 0, LEVELS));
+            if (a.top_k > 0) t_keep = radix_threshold<T, false, 8>(each_logit, a, m, 0u, radix, 0, reaching);
+            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 8>(each_logit, a, m, t_keep, radix, 0, reaching));
         }
 
         // 4. argmax of s + g over the kept tokens, ties to the lowest id; the kept tokens' mass.
@@ -539,15 +535,15 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
 
 }  // namespace
 
-template <typename T>
+template <typename T, bool LIST>
 static cudaError_t launch_t(const SampleArgs &a, int blocks, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(a.b * blocks), 1, 1);
     cfg.blockDim = dim3(ST, 1, 1);
     cfg.stream = stream;
-    constexpr size_t smem = sizeof(RadixSmem) + sizeof(TokenList);
+    constexpr size_t smem = sizeof(RadixSmem) + (LIST ? sizeof(TokenList) : 0);
     cfg.dynamicSmemBytes = smem;
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(sample_kernel<T, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -556,7 +552,7 @@ static cudaError_t launch_t(const SampleArgs &a, int blocks, cudaStream_t stream
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, sample_kernel<T>, a);
+    return cudaLaunchKernelEx(&cfg, sample_kernel<T, LIST>, a);
 }
 
 cudaError_t launch_sample(int dtype, const SampleArgs &a, cudaStream_t stream, int *launches) {
@@ -567,11 +563,16 @@ cudaError_t launch_sample(int dtype, const SampleArgs &a, cudaStream_t stream, i
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int blocks = 1;
     while (blocks < 8 && (int64_t)a.b * blocks * 2 <= sms && a.v >= blocks * 2 * ST * 4) blocks *= 2;
+    // The list's own search costs what two passes do over rows of one 16-byte load a thread (top-k alone, 16 rows of 32000 bf16
+    // logits: 22.4 us with the list, 20.6 without; with top-p behind it 26.7 against 30.8, and 24.7 -> 22.6 where the rows
+    // are read a logit at a time).
+    const bool list = !a.greedy && a.top_k > 0 && a.top_k <= blocks * ST / 2 &&
+                      (a.has_p || !a.vec || (int64_t)a.v > (int64_t)blocks * ST * (dtype == 0 ? 4 : 8));
     cudaError_t e;
     switch (dtype) {
-        case 0: e = launch_t<float>(a, blocks, stream); break;
-        case 1: e = launch_t<__nv_bfloat16>(a, blocks, stream); break;
-        default: e = launch_t<__half>(a, blocks, stream); break;
+        case 0: e = list ? launch_t<float, true>(a, blocks, stream) : launch_t<float, false>(a, blocks, stream); break;
+        case 1: e = list ? launch_t<__nv_bfloat16, true>(a, blocks, stream) : launch_t<__nv_bfloat16, false>(a, blocks, stream); break;
+        default: e = list ? launch_t<__half, true>(a, blocks, stream) : launch_t<__half, false>(a, blocks, stream); break;
     }
     *launches += 1;
     return e;
