@@ -125,7 +125,9 @@ __device__ __noinline__ void rescale_accumulator(uint32_t taddr, float factor) {
 
 }  // namespace
 
-template <typename T, int HD>
+// SPLIT: the block sweeps one of a.splits runs of its tiles' keys and leaves parts for the merge.  (An instance of its own: short
+// sweeps that are not split paid for its code, 20 packed sequences of 3000 tokens, 16 / 16 heads of 128, 30.3 us against 29.0.)
+template <typename T, int HD, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Sm100FwdArgs a) {
@@ -138,9 +140,9 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     Shared &sh = *reinterpret_cast<Shared *>(v_s + NS * KV_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = blockIdx.y % a.splits;
-    const int qt = (gridDim.y - 1 - blockIdx.y) / a.splits;  // later (longer, under causality) tiles first
-    if (a.splits > 1) allow_beside();   // the merge
+    const int split = SPLIT ? blockIdx.y % a.splits : 0;
+    const int qt = SPLIT ? (gridDim.y - 1 - blockIdx.y) / a.splits : gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
+    if constexpr (SPLIT) allow_beside();   // the merge
     const int b = blockIdx.z;
     // Tile t of the block: BT = 128 >> pack tokens from m_base + t BT on, of 1 << pack heads from h0 on.
     const int pack = a.pack, bt = BM >> pack;
@@ -211,7 +213,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
     for (int i = 0; i < 4 * NT; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
     if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
-    split_keys(split, a.splits, BN, kmin, kmax);
+    if constexpr (SPLIT) split_keys(split, a.splits, BN, kmin, kmax);
     const bool aborted = sh.abort != 0;
     const int subs = (!aborted && kmax > kmin) ? (kmax - kmin + SN - 1) / SN : 0;   // sub-steps of 64 keys
     const int steps = (subs + 1) / 2;                                                // K / V tiles of 128 keys
@@ -462,7 +464,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         // ---------------- epilogue ----------------
         T *out = static_cast<T *>(a.out);
         const int64_t base = ((int64_t)b * a.tq + row) * a.hq + h;
-        if (a.splits > 1 && !failed) {
+        if (SPLIT && !failed) {
             // A part of the row's keys: the normalised f32 row and its log-sum-exp, for the merge.
             const int64_t at = (int64_t)split * gridDim.z * a.tq * a.hq + base;
             if (subs == 0) {
@@ -493,7 +495,7 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                 failed = true;
             }
         } else if (subs == 0 || failed) {
-            if (row < a.tq && !failed && a.splits == 1) {
+            if (row < a.tq && !failed && !SPLIT) {
                 const uint4 z = make_uint4(0, 0, 0, 0);
 #pragma unroll
                 for (int c = 0; c < HD / 8; ++c) reinterpret_cast<uint4 *>(out + base * HD)[c] = z;
@@ -537,8 +539,8 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             failed = true;
         }
         // A part whose waits ran out left nothing: its rows come out of the merge as NaN (and the status is raised).
-        if (a.splits > 1 && failed && row < a.tq) a.part_lse[(int64_t)split * gridDim.z * a.tq * a.hq + base] = __int_as_float(0x7fc00000);
-        if (steps > 0 && a.splits == 1) {
+        if (SPLIT && failed && row < a.tq) a.part_lse[(int64_t)split * gridDim.z * a.tq * a.hq + base] = __int_as_float(0x7fc00000);
+        if (steps > 0 && !SPLIT) {
             // Every warp of the tile gets here (all waits are bounded), whatever became of it: one
             // that gave up marks the tile, and nothing is stored from a tile that is not whole.
             if (failed && lane == 0) sh.tile_bad[t] = 1;
@@ -571,9 +573,10 @@ template <typename T, int HD>
 cudaError_t launch_fwd2_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv, const CUtensorMap &to,
                           const Sm100FwdArgs &a, cudaStream_t stream) {
     constexpr size_t smem = Geo<HD>::SMEM_BYTES;
-    cudaError_t e = cudaFuncSetAttribute(fwd2_sm100_kernel<T, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = a.splits > 1 ? fwd2_sm100_kernel<T, HD, true> : fwd2_sm100_kernel<T, HD, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fwd2_sm100_kernel<T, HD><<<grid, THREADS, smem, stream>>>(tq, tk, tv, to, a);
+    kernel<<<grid, THREADS, smem, stream>>>(tq, tk, tv, to, a);
     return cudaGetLastError();
 }
 }  // namespace

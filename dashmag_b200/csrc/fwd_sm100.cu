@@ -93,7 +93,8 @@ template <> struct Pack<__half> {
 
 }  // namespace
 
-template <typename T, int HD>
+// SPLIT: the block sweeps one of a.splits runs of its tile's keys and leaves a part for the merge (as in the two-tile kernel).
+template <typename T, int HD, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const Sm100FwdArgs a) {
@@ -109,9 +110,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // The tile: 128 >> pack tokens from m0 on, of 1 << pack heads from h0 on; row = token << pack | head.
     const int pack = a.pack;
     const int h0 = blockIdx.x << pack;
-    const int split = blockIdx.y % a.splits;
-    const int qt = (gridDim.y - 1 - blockIdx.y) / a.splits;  // later (longer, under causality) tiles first
-    if (a.splits > 1) allow_beside();   // the merge
+    const int split = SPLIT ? blockIdx.y % a.splits : 0;
+    const int qt = SPLIT ? (gridDim.y - 1 - blockIdx.y) / a.splits : gridDim.y - 1 - blockIdx.y;  // later (longer, under causality) tiles first
+    if constexpr (SPLIT) allow_beside();   // the merge
     const int b = blockIdx.z;
     const int hk = h0 / (a.hq / a.hkv);
     const int m0 = qt * (BM >> pack);
@@ -160,7 +161,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
     for (int i = 0; i < 4; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
     if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
-    split_keys(split, a.splits, BN, kmin, kmax);
+    if constexpr (SPLIT) split_keys(split, a.splits, BN, kmin, kmax);
     // Once a bounded wait has run out anywhere, later blocks do nothing: the call has failed and
     // the host will say so; there is no point in timing out thousands of times.
     const bool aborted = sh.abort != 0;
@@ -373,7 +374,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // ---------------- epilogue ----------------
         T *out = static_cast<T *>(a.out);
         const int64_t base = ((int64_t)b * a.tq + row) * a.hq + h;
-        const bool part = a.splits > 1;   // a part of the row's keys: the normalised f32 row and its log-sum-exp, for the merge
+        constexpr bool part = SPLIT;   // a part of the row's keys: the normalised f32 row and its log-sum-exp, for the merge
         const int64_t at = (int64_t)split * gridDim.z * a.tq * a.hq + base;
         float *lse_at = part ? a.part_lse + at : a.lse + base;
         if (part && n_tiles == 0) {
@@ -443,9 +444,10 @@ template <typename T, int HD>
 cudaError_t launch_fwd_t(dim3 grid, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tv, const Sm100FwdArgs &a,
                          cudaStream_t stream) {
     constexpr size_t smem = Geo1<HD>::SMEM_BYTES;
-    cudaError_t e = cudaFuncSetAttribute(fwd_sm100_kernel<T, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = a.splits > 1 ? fwd_sm100_kernel<T, HD, HD == 256> : fwd_sm100_kernel<T, HD, false>;   // (D 128 here: a switch, never split)
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    fwd_sm100_kernel<T, HD><<<grid, THREADS, smem, stream>>>(tq, tk, tv, a);
+    kernel<<<grid, THREADS, smem, stream>>>(tq, tk, tv, a);
     return cudaGetLastError();
 }
 }  // namespace
