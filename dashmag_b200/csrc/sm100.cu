@@ -192,14 +192,14 @@ bool sm100_takes(const dash_attn_params *p, const void *q, const void *k, const 
 // fill it.  Estimated in steps of 64 keys (128 at D 256): a block's share of its sweep plus what a block costs however
 // short its sweep (set-up, the first tiles' flight, the output: about six steps of the two-tile kernel, three of the
 // other's, which are twice as long), times the waves of blocks; a split also pays for the merge's launch (five and three
-// steps) and for the f32 rows of its parts, written and read at about 2.5 TB/s (a step is 0.95 us, the other's 1.8).  Only
-// an estimate a tenth below the whole sweep's is taken: the last wave's blocks are the short ones, which the count of waves
-// does not know (2380 queries against 6897 keys, 8 / 2 heads of 256, 150 blocks: 123 us whole, 143 in three).  At forced
-// numbers of splits over 200 calls (130 to 5000 queries, D 64 to 256, 4 to 32 heads) the pick is never slower than the whole; with the parts unpriced 3000 tokens, 12 / 4 heads of 128, were split in two, 65.7 us against 53.4, and 256
-// queries against 30000 keys, 32 / 8 heads of 256, in nine, 313 us against 227 in two.  The sweep is the longest tile's; under causality with as many queries as keys the mean
-// is half of it, so the waves are counted on the mean and the longest tile is a bound of its own.  Packed batches, whose
-// lengths the host does not know, are not split.  A chunk of 500 queries against 8200 keys, 32 / 8 heads (64 tiles):
-// see the figures at fwd_merge.cu.
+// steps) and for the f32 rows of its parts, written and read at 2.3 TB/s (a step is 0.95 us, the other's 1.8).  Under
+// causality tiles differ, the long ones first: waves are counted on the mean, the last wave, where it is not full, goes
+// from the shortest towards the mean with its share of the multiprocessors, and the longest tile is a bound of its own.
+// Packed batches, whose lengths the host does not know, are not split.
+// At forced numbers of splits over 240 calls (130 to 5000 queries, D 64 to 256, 4 to 32 heads) the pick is never slower
+// than the whole sweep.  With the parts unpriced, 3000 tokens of 12 / 4 heads of 128 were split in two, 65.7 us against 53.4;
+// with the last wave as long as the others, 2380 queries against 6897 keys, 8 / 2 heads of 256 (150 blocks), in three, 143
+// against 123.  (A chunk of 500 queries against 8200 keys, 32 / 8 heads, 64 tiles: the figures at fwd_merge.cu.)
 int forward_splits(const dash_attn_params *p) {
     if (p->mask_kind == DASH_ATTN_MASK_PACKED || p->hkv <= 0 || p->tq <= 0) return 1;
     const bool one = p->d == 256;
@@ -207,7 +207,7 @@ int forward_splits(const dash_attn_params *p) {
     const int64_t tokens = (one ? 128 : 256) >> pack, step = one ? 128 : 64, sms = 148;
     const int64_t tiles = (p->tq + tokens - 1) / tokens, blocks = tiles * (p->hq >> pack) * p->b;
     if (blocks >= 2 * sms) return 1;
-    int64_t longest = p->tk, mean = p->tk;
+    int64_t longest = p->tk, mean = p->tk, shortest = p->tk;
     // A side that reaches past every key is no bound (and must not be added to).
     const int64_t none = (int64_t)p->tq + p->tk + 1;
     auto side = [&](int64_t reach) { return p->has_window && reach >= 0 && reach < none ? reach : int64_t(-1); };
@@ -216,21 +216,24 @@ int forward_splits(const dash_attn_params *p) {
         const int64_t last = std::min<int64_t>(p->tk, p->tk + right), first = std::min<int64_t>(p->tk, std::max<int64_t>(p->tk - p->tq + right + tokens, 0));
         longest = last;
         mean = (first + last) / 2;
+        shortest = first;
     }
     if (left >= 0) {
         const int64_t reach = left + std::max<int64_t>(right, 0) + tokens;
         longest = std::min(longest, right < 0 ? p->tk : reach);
         mean = std::min(mean, longest);
+        shortest = std::min(shortest, longest);
     }
-    const int64_t l = (longest + step - 1) / step, m = (mean + step - 1) / step, fixed = one ? 3 : 6;
-    const double merge = one ? 3 : 5, part = (double)p->b * p->tq * p->hq * p->d * sizeof(float) / (one ? 4.5e6 : 2.4e6);
+    const int64_t l = (longest + step - 1) / step, m = (mean + step - 1) / step, n = (shortest + step - 1) / step, fixed = one ? 3 : 6;
+    const double merge = one ? 3 : 5, part = (double)p->b * p->tq * p->hq * p->d * sizeof(float) / (one ? 4.1e6 : 2.2e6);
     auto cost = [&](int64_t s) {
-        const int64_t waves = (blocks * s + sms - 1) / sms;
-        return (double)std::max(waves * ((m + s - 1) / s + fixed), (l + s - 1) / s + fixed) + (s > 1 ? merge + s * part : 0.);
+        const int64_t full = blocks * s / sms, rest = blocks * s % sms, ms = (m + s - 1) / s, ns = (n + s - 1) / s;
+        const double last = rest ? ns + (ms - ns) * ((double)rest / sms) + fixed : 0.;
+        return std::max(full * (ms + fixed) + last, (double)((l + s - 1) / s + fixed)) + (s > 1 ? merge + s * part : 0.);
     };
     int best = 1;
     for (int s = 2; s <= 32 && l / s >= 2 && tiles * s <= 65535; ++s)
-        if (cost(s) < 0.9 * cost(1) && cost(s) < cost(best)) best = s;
+        if (cost(s) < 0.93 * cost(1) && cost(s) < cost(best)) best = s;
     return best;
 }
 static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }

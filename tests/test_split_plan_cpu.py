@@ -57,7 +57,7 @@ def test_the_parts_stay_bounded():
         pack = 1   # heads of a group in a tile
         while pack < 8 and group % (2 * pack) == 0:
             pack *= 2
-        rows, step, step_bytes = (128, 128, 4.5e6) if d == 256 else (256, 64, 2.4e6)   # of a block; keys of a step; f32 parts that cost one
+        rows, step, step_bytes = (128, 128, 4.1e6) if d == 256 else (256, 64, 2.2e6)   # of a block; keys of a step; f32 parts that cost one
         blocks = -(-tq // (rows // pack)) * (hkv * group // pack) * b
         steps = -(-tk // step)
         assert n <= 32 and n <= steps // 2, "a part has two steps of keys at least"
