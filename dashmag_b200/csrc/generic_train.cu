@@ -513,14 +513,18 @@ static size_t generic_smem(int d, int rpw, int own, int probs) {
 }
 
 // Rows per warp: the fewest of one, two and four whose blocks all run at once - as many to a multiprocessor as its shared
-// memory holds, up to two and a half (beyond, the reads of shared memory that more rows would share are what it waits for) -
-// else four.  Measured (rows per warp 1 | 2 | 4, us): forward of 130 tokens x 4 heads of 64 (68 | 36 | 20 blocks) 10 | 12 | 15;
-// 300 x 8 of 128 (304 | 152 | 80) 27 | 25 | 27; 1000 x 8 of 64 (1000 | 504 | 256) 190 | 122 | 124; 60 queries x 32 heads of
-// 256 against 2060 keys, one block to a multiprocessor (256 | 128 | 64) 648 | 374 | 525; 100 against 9100 (416 | 224 | 128)
-// 4339 | 3272 | 2320; backward of 300 x 8 / 2 heads of 128 122 | 144 | 180, of 1400 x 4 of 128 257 | 190 | 212.
+// memory holds (a block also takes its static arrays and the kilobyte the system keeps for it), up to two and a half (beyond,
+// the reads of shared memory that more rows would share are what it waits for) - else four.  Measured, f32, causal (rows per
+// warp 1 | 2 | 4, us): forward of 130 tokens x 4 heads of 64 (68 | 36 | 20 blocks) 12 | 14 | 16; 300 x 8 of 128
+// (304 | 152 | 80) 45 | 43 | 47; 1000 x 8 of 64 (1000 | 504 | 256) 190 | 127 | 125; 60 queries x 32 heads of 256 against 2060
+// keys, one block to a multiprocessor (256 | 128 | 64) 672 | 362 | 501; 100 against 9100 (416 | 224 | 128) 4395 | 3153 | 2213;
+// backward of 300 x 8 / 2 heads of 128 204 | 248 | 293 (the rule, which picks for each kernel: 184), of 1400 x 4 of 128
+// 749 | 549 | 450, of 700 x 4 of 128 230 | 170 | 215.  It is not the best of the three everywhere: the forward of 700 x 4 of
+// 128 takes one row a warp, 118 us, where four take 101; of 1000 x 8 / 2 of 96 four, 195, where two take 165.
+constexpr int64_t SMEM_PER_SM = 228 * 1024, SMEM_BESIDE = 2 * 1024;
 static int rows_per_warp(int64_t rows, int64_t heads, int d, int own, int probs) {
     for (int rpw = 1; rpw < 4; rpw *= 2) {
-        const int64_t blocks = (rows + WARPS * rpw - 1) / (WARPS * rpw) * heads, fit = (227 * 1024) / (int64_t)generic_smem(d, rpw, own, probs);
+        const int64_t blocks = (rows + WARPS * rpw - 1) / (WARPS * rpw) * heads, fit = SMEM_PER_SM / ((int64_t)generic_smem(d, rpw, own, probs) + SMEM_BESIDE);
         if (blocks <= std::min<int64_t>(148 * fit, 370)) return rpw;
     }
     return 4;
