@@ -9,8 +9,8 @@
 //          key), P^T = exp2(S^T sl - lse) and dS^T = P^T (dP^T - delta) elementwise, rounded to the
 //          input dtype back into tensor memory, then dV += P^T dO and dK += dS^T Q with the A
 //          operand read from tensor memory, accumulated in TMEM over the whole sweep.
-//   dq     one block per tile of 128 query rows (128 / P tokens x P heads of a group, see pack_log2).  Q_i and dO_i stay in shared memory; the block
-//          sweeps, in steps of 64, the keys its queries see.  Per step: S = Q_i K^T, dP = dO_i V^T,
+//   dq     one block per tile of 128 query rows (128 / P tokens x P heads of a group, see pack_log2).  Q_i and dO_i
+//          stay in shared memory; the block sweeps, in steps of 128, the keys its queries see.  Per step: S = Q_i K^T, dP = dO_i V^T,
 //          dS = P (dP - delta), then dQ += dS K.
 //
 // Both recompute the scores tile by tile from the saved log-sum-exp (no T x T anywhere): seven

@@ -113,7 +113,11 @@ typedef struct dash_attn_decode_params {
 
 /* Bytes of device scratch each call needs (0 is possible).  256-byte aligned workspace.  The forward
  * also runs without its scratch, or with less (it then does not split a tile's keys over blocks, and
- * a call of few queries against many keys takes longer). */
+ * a call of few queries against many keys takes longer).  Whether keys are split depends on the whole
+ * call, its batch and heads among it, and a split sums in another order: a sequence or a head computed
+ * alone can differ in its last bits from the same one in a larger call (packed batches and calls
+ * without scratch are never split).  So can key and value gradients at head dimension 256, where a
+ * small call's units are shared between two blocks.  The same call gives the same bits on every run. */
 size_t dash_attn_forward_workspace(const dash_attn_params *p);
 size_t dash_attn_backward_workspace(const dash_attn_params *p);
 size_t dash_attn_decode_workspace(const dash_attn_decode_params *p);
