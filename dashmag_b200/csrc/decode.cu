@@ -349,10 +349,9 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 //
 // WARPS warps to a block: eight, or two where blocks of eight would leave multiprocessors without one (a block is a
 // multiprocessor's worth of shared memory: 256 units of one sequence's 8 heads in blocks of eight are 32 blocks).  The warps
-// resident at a time are the same.  Blocks of two up to eight warps a multiprocessor, where they measured ahead (one sequence
-// of 2047 keys with rotation and append: 15.5 us with blocks of eight, 13.5 with two); beyond, eight (64 sequences of up to
-// 4096: 91 against 102 us; 40 of up to 6000 with one head, 1880 warps: 24.7 against 26.2): its warps read neighbouring heads
-// of the same keys at the same time.
+// resident at a time are the same.  Blocks of two up to two waves of warps, where they measured ahead (one sequence of 2047
+// keys with rotation and append: 15.5 us with blocks of eight, 13.5 with two); beyond, eight (64 sequences of up to 4096:
+// 91 against 102 us): its warps read neighbouring heads of the same keys at the same time.
 //
 // Two columns rotated in the dtype's own arithmetic, as rope_kernel does it (each product and the sum rounded once): `low` for
 // the first half of the rotated features, whose partner enters with its sign turned.
@@ -812,7 +811,7 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, cudaStream_
 template <typename T, int DFULL>
 static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream) {
     const long long warps = (long long)a.splits * a.hkv * (DFULL > 128 ? 2 : 1) * ((a.hq / a.hkv + 15) / 16);   // of one sequence
-    return warps * a.b < 148LL * 8 ? split_mma_w<T, DFULL, 2>(a, warps, stream) : split_mma_w<T, DFULL, 8>(a, warps, stream);
+    return warps * a.b < 148LL * 8 * 2 ? split_mma_w<T, DFULL, 2>(a, warps, stream) : split_mma_w<T, DFULL, 8>(a, warps, stream);
 }
 template <> cudaError_t split_mma<float, 128>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }   // never taken: 16-bit caches only
 template <> cudaError_t split_mma<float, 64>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }
@@ -852,12 +851,7 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
     *launches += 1;
     if (e != cudaSuccess) return e;
     *launches += 1;
-    // The merge comes in under the pass's end (one sequence of 4096 keys: 14.5 -> 12.5 us) while its parts are few: its blocks then
-    // gather on the multiprocessors that the pass has left first, which costs more than it hides where they have much to read
-    // (16 sequences of up to 20000 keys, 16 heads on one: 36.0 us after the pass, 38.2 under its end, 20 MB of parts; 25 of up
-    // to 19426, 31 MB, 42.2 and 42.7; but 20 of up to 8192, 10 MB, 22.7 and 21.7).
-    const bool under = (int64_t)sizeof(float) * a.b * a.hq * a.splits * a.d <= 12000000;
-    return launch_beside(decode_merge_kernel<T>, dim3(a.b * a.hq), 128, 0, stream, under, a);
+    return launch_beside(decode_merge_kernel<T>, dim3(a.b * a.hq), 128, 0, stream, true, a);
 }
 
 cudaError_t launch_decode(int dtype, const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches) {
