@@ -233,7 +233,7 @@ int forward_splits(const dash_attn_params *p) {
     };
     int best = 1;
     for (int s = 2; s <= 32 && l / s >= 2 && tiles * s <= 65535; ++s)
-        if (cost(s) < 0.93 * cost(1) && cost(s) < cost(best)) best = s;
+        if (cost(s) < 0.95 * cost(1) && cost(s) < cost(best)) best = s;
     return best;
 }
 static size_t split_rows(const dash_attn_params *p, int splits) { return (size_t)splits * p->b * p->tq * p->hq; }
