@@ -189,9 +189,9 @@ int check_decode(const dash_attn_decode_params *p, const char *op = "attention_d
     return DASH_ATTN_OK;
 }
 
-// Keys per split and splits per sequence: enough warps to fill the 148 multiprocessors of a B200
-// several times over (16 resident warps each, 4 waves), between 64 and 512 keys a split so that
-// the partial outputs stay a few percent of the cache traffic.  A pure function of the shape, so
+// Keys per split and splits per sequence: 64 to 512 keys a split.  Where the units (a split of a key-value head) are a few waves
+// at most, the length whose waves are shortest; else as long as still leaves units to fill the 148 multiprocessors of a B200
+// several times over, so that the partial outputs stay a few percent of the cache traffic.  A pure function of the shape, so
 // the workspace query and the launch agree without looking at the device.
 void decode_plan(const dash_attn_decode_params *p, int *chunk, int *splits) {
     // DASH_ATTN_DECODE_CHUNK (read once, when the first plan is made) fixes the chunk for comparison runs.

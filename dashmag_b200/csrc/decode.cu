@@ -349,9 +349,11 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 //
 // WARPS warps to a block: eight, or two where blocks of eight would leave multiprocessors without one (a block is a
 // multiprocessor's worth of shared memory: 256 units of one sequence's 8 heads in blocks of eight are 32 blocks).  The warps
-// resident at a time are the same.  Blocks of two up to two waves of warps, where they measured ahead (one sequence of 2047
-// keys with rotation and append: 15.5 us with blocks of eight, 13.5 with two); beyond, eight (64 sequences of up to 4096:
-// 91 against 102 us): its warps read neighbouring heads of the same keys at the same time.
+// resident at a time are the same.  Blocks of two up to sixteen warps a multiprocessor (at D 128 two waves of them, at D 64
+// one), where they measured ahead: one sequence of 2047 keys with rotation and append, 15.5 us with blocks of eight, 13.5 with
+// two; 56 sequences of up to 5136 with one head, 2296 warps, 36.9 and 33.3; 34 of up to 7657 under a window of 4096, 2040
+// warps, 24.8 and 23.0; but 40 of up to 6000, 1880 warps, 24.7 and 26.1, for which no rule was found.  Beyond, eight (64
+// sequences of up to 4096, 8 heads: 91 against 102 us): its warps read neighbouring heads of the same keys at the same time.
 //
 // Two columns rotated in the dtype's own arithmetic, as rope_kernel does it (each product and the sum rounded once): `low` for
 // the first half of the rotated features, whose partner enters with its sign turned.
@@ -851,6 +853,11 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
     *launches += 1;
     if (e != cudaSuccess) return e;
     *launches += 1;
+    // The merge comes in under the pass's end: one sequence of 4096 keys 14.5 -> 12.5 us, 64 of up to 5387 with one head 39.0 ->
+    // 37.0, 28 of up to 7754, 8 heads, 100.3 -> 98.6.  (Its blocks gather on the multiprocessors the pass leaves first, and a
+    // few calls of few blocks with much to read lose by it: 16 of up to 20000 keys, 16 heads on one, 36.0 us after the pass,
+    // 38.2 under its end; 25 of up to 19426 41.5 and 42.3.  Neither the parts' size nor the blocks' number tells them apart:
+    // with the line at 12 or 20 MB of parts more calls lost than won.)
     return launch_beside(decode_merge_kernel<T>, dim3(a.b * a.hq), 128, 0, stream, true, a);
 }
 
