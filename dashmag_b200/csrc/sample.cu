@@ -17,7 +17,7 @@
 //      Top-k leaves few tokens of many, and a lower bound of its threshold is cheap: the k-th largest of the THREADS' maxima
 //      is a token at least k tokens reach.  The tokens above the bound go into a list in shared memory, in the pass that sums
 //      the exponentials anyway, and the search and the draw look at the list; a list that would not fit leaves the passes over
-//      the row.  64 x 151936 bf16 logits, k = 50, p = 0.9: 74 -> 45 us side by side.  (A nucleus alone has no such bound
+//      the row.  64 x 151936 bf16 logits, k = 50, p = 0.9: 74 -> 41 us side by side.  (A nucleus alone has no such bound
 //      without one more pass over the row, which cost more than the list gave at every spread of the logits: N(0, 10) 67.8
 //      us with it, 63.8 without.)
 //   4. argmax over the kept tokens of s_i + g_i, ties to the lowest id, four tokens per Philox call;
