@@ -6,6 +6,8 @@ module raises at import time of the first call, naming the build command.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import pathlib
 import struct
@@ -13,6 +15,7 @@ import struct
 HERE = pathlib.Path(__file__).resolve().parent
 #: The built library; DASH_ATTN_LIBRARY names another build of the same sources (for experiments).
 LIB_PATH = pathlib.Path(os.environ.get("DASH_ATTN_LIBRARY", HERE / "csrc" / "libdash_attn_b200.so"))
+BINDING_PATH = HERE / "csrc" / "_binding.so"
 
 OK, INVALID, UNSUPPORTED, WORKSPACE, CUDA = 0, 1, 2, 3, 4
 MASK_NONE, MASK_KEY_PADDING, MASK_PACKED = 0, 1, 2
@@ -175,6 +178,30 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = handle
     return _lib
+
+
+_binding = None
+#: The functions the binding calls, in the order it takes them.
+BOUND = ("dash_attn_forward_workspace", "dash_attn_forward", "dash_attn_backward_workspace", "dash_attn_backward",
+         "dash_attn_decode_workspace", "dash_attn_decode", "dash_attn_decode_append",
+         "dash_attn_decode_append_rope_workspace", "dash_attn_decode_append_rope", "dash_sample_workspace", "dash_sample")
+
+
+def binding():
+    """The entry points' native host side (``csrc/binding.cpp``).  Raises if it has not been built."""
+    global _binding
+    if _binding is None:
+        if not BINDING_PATH.exists():
+            raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m dashmag_b200.build`.")
+        import torch  # noqa: F401  (the binding's symbols)
+
+        loader = importlib.machinery.ExtensionFileLoader("_binding", str(BINDING_PATH))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_binding", loader))
+        loader.exec_module(module)
+        handle = lib()
+        module.use(*(ctypes.cast(getattr(handle, name), vp).value for name in BOUND))
+        _binding = module
+    return _binding
 
 
 def last_error() -> str:

@@ -44,6 +44,13 @@ def _raise(code: int) -> None:
     raise RuntimeError(message)
 
 
+def _result(done):
+    """What the native host side returned: the outputs, or the C ABI's error code."""
+    if type(done) is int:
+        _raise(done)
+    return done
+
+
 def _ptr(t: Optional[torch.Tensor]):
     return None if t is None or t.numel() == 0 else t.data_ptr()
 
@@ -160,6 +167,9 @@ def attention_with_lse(query, key, value, mask: AttentionMask = AttentionMask.no
                        options: AttentionOptions = AttentionOptions()):
     """crates/dash-ops/src/attention.rs:660-682: the output ``[B,Tq,Hq,D]`` in the queries' dtype
     and the natural log-sum-exp ``[B,Tq,Hq]`` in f32 (``-inf`` for a query that sees no key)."""
+    done = _lib.binding().forward(query, key, value, mask, options)
+    if done is not None:
+        return _result(done)
     op = "attention"
     p, keep = make_params(op, query, key, value, mask, options)
     _check_device(op, query, key, value, *keep)
@@ -187,6 +197,9 @@ def attention_backward(query, key, value, output, lse, grad_output, mask: Attent
     """crates/dash-ops/src/attention.rs:689-724: the gradients of ``query``, ``key`` and ``value``,
     each in its input's shape and dtype, from the forward's ``output`` and ``lse`` and the
     gradient of the output."""
+    done = _lib.binding().backward(query, key, value, output, lse, grad_output, mask, options)
+    if done is not None:
+        return _result(done)
     op = "attention_backward"
     p, keep = make_params(op, query, key, value, mask, options, output, grad_output)
     if tuple(output.shape) != tuple(query.shape):
@@ -250,6 +263,9 @@ def attention_decode(query, key, value, cache_lengths=None, options: AttentionOp
     """crates/dash-ops/src/attention.rs:732-760: ``query`` ``[B,Hq,D]`` against the cache
     ``[B,S,Hkv,D]`` (a slice of a longer cache is read in place); ``cache_lengths`` ``[B]`` int or
     ``None`` for all ``S``; of the options the scale and the window's ``left`` apply."""
+    done = _lib.binding().decode(query, key, value, cache_lengths, options)
+    if done is not None:
+        return _result(done)
     op = "attention_decode"
     p, keep = make_decode_params(query, key, value, cache_lengths, options)
     _check_device(op, query, key, value, *keep)
@@ -271,6 +287,9 @@ def attention_decode_append(query, new_key, new_value, key, value, cache_lengths
     (crates/dash-mag/src/tensor.rs:732-744) followed by ``attention_decode`` with the lengths plus
     one (crates/dash-ops/src/attention.rs:732-760), in the decoding step's own launches.
     ``cache_lengths`` are the lengths before the step; a full cache gets no row."""
+    done = _lib.binding().decode_append(query, new_key, new_value, key, value, cache_lengths, options)
+    if done is not None:
+        return _result(done)
     op = "attention_decode_append"
     if cache_lengths is None:
         raise ValueError(f"{op}: the lengths are needed: they say where each sequence's new row goes")

@@ -3,7 +3,8 @@
 ``python -m dashmag_b200.build`` (or ``build()``) compiles every ``csrc/*.cu`` with nvcc and links
 them into one shared library with a static CUDA runtime, so that the library loads on a machine
 without a GPU (only launches need one).  Objects are rebuilt when their source or any header is
-newer.
+newer.  Then ``csrc/binding.cpp``, the entry points' host side over torch's tensors, is compiled with the host
+compiler into ``csrc/_binding.so``.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ HERE = pathlib.Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = CSRC / "build"
 LIB = CSRC / "libdash_attn_b200.so"
+BINDING = CSRC / "_binding.so"
 INCLUDE = HERE.parent / "include"
 
 NVCC_FLAGS = [
@@ -71,7 +73,28 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_binding(host_cc or "g++", force)
     return LIB
+
+
+def build_binding(cxx: str, force: bool = False) -> pathlib.Path:
+    source = CSRC / "binding.cpp"
+    newest = max(source.stat().st_mtime, *(h.stat().st_mtime for h in INCLUDE.glob("*.h")))
+    if not force and BINDING.exists() and BINDING.stat().st_mtime > newest:
+        return BINDING
+    import sysconfig
+
+    import torch
+
+    root = pathlib.Path(torch.__file__).resolve().parent
+    cuda = pathlib.Path(_nvcc()).resolve().parent.parent
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root}/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}", str(source), "-o", str(BINDING),
+           f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"the binding did not build:\n{r.stdout}\n{r.stderr}")
+    return BINDING
 
 
 if __name__ == "__main__":

@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .attention import (AttentionError, AttentionOptions, _check_device, _DTYPES, _index_bytes, _on, _ptr, _raise, _stream,
+from .attention import (AttentionError, AttentionOptions, _check_device, _DTYPES, _index_bytes, _on, _ptr, _raise, _result, _stream,
                         _workspace, make_decode_params)
 
 
@@ -146,6 +146,10 @@ def attention_decode_append_rope(rope: Rope, query, new_key, new_value, key, val
     including them - ``Rope::apply_at`` twice, ``put_along_axis_owned`` twice and
     ``attention_decode`` in the reference's caller (crates/dash-mag/tests/step.rs:200-217 is the
     prefill form of the same sequence), one call here."""
+    if positions is None:
+        done = _lib.binding().decode_append_rope(rope, query, new_key, new_value, key, value, cache_lengths, options)
+        if done is not None:
+            return _result(done)
     op = "attention_decode_append_rope"
     if cache_lengths is None:
         raise AttentionError(f"{op}: the lengths are needed: they say where each sequence's new row goes")

@@ -14,7 +14,7 @@ from typing import Sequence
 import torch
 
 from . import _lib
-from .attention import AttentionError, _check_device, _DTYPES, _on, _ptr, _raise, _stream, _workspace
+from .attention import AttentionError, _check_device, _DTYPES, _on, _ptr, _raise, _result, _stream, _workspace
 
 
 @dataclasses.dataclass(frozen=True)
@@ -64,6 +64,10 @@ def make_sample_params(logits: torch.Tensor, options: SampleOptions, token_dtype
 
 def sample(logits: torch.Tensor, options: SampleOptions = SampleOptions(), token_dtype=torch.int64) -> Sampled:
     """One token per row of ``logits [B, V]`` (crates/dash-ops/src/sample.rs ``sample``)."""
+    if token_dtype == torch.int64:
+        done = _lib.binding().sample(logits, options)
+        if done is not None:
+            return Sampled(*_result(done))
     if logits.dim() == 2 and logits.stride(1) != 1:
         logits = logits.contiguous()
     p, keep = make_sample_params(logits, options, token_dtype)

@@ -1,0 +1,113 @@
+"""The native host side makes the very call the Python side makes: the same bits out, the same refusals, and what it leaves to
+the Python side (other devices' streams, transforms, layouts to copy) still runs."""
+import pytest
+import torch
+
+from dashmag_b200 import _lib
+from dashmag_b200 import attention as A
+from dashmag_b200.contract import AttentionMask, AttentionOptions
+from dashmag_b200.rope import Rope, attention_decode_append_rope
+from dashmag_b200.sample import SampleOptions, sample
+
+pytestmark = pytest.mark.gpu
+
+
+class Nothing:
+    """Stands in for the binding and does nothing."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def randn(*shape, dtype=torch.bfloat16, seed=0):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed + sum(shape))
+    return torch.randn(shape, generator=g, device="cuda", dtype=dtype)
+
+
+def train(mask, options, dtype=torch.bfloat16, d=64, swap=False):
+    q, k, v, g = (randn(1 if mask.kind == "packed" else 2, 150, h, d, dtype=dtype, seed=i) for i, h in enumerate((4, 2, 2, 4)))
+    if swap:
+        q, g = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (q, g))
+    o, lse = A.attention_with_lse(q, k, v, mask, options)
+    return (o, lse, *A.attention_backward(q, k, v, o, lse, g, mask, options))
+
+
+def calls():
+    cu = torch.tensor([0, 70, 150], dtype=torch.int32, device="cuda")
+    pad = torch.arange(150, device="cuda")[None] >= torch.tensor([[150], [90]], device="cuda")
+    causal = AttentionOptions(causal=True)
+    yield "none", lambda: train(AttentionMask.none(), AttentionOptions())
+    yield "packed", lambda: train(AttentionMask.packed(cu, cu), causal.with_window(40, 0))
+    yield "packed i64", lambda: train(AttentionMask.packed(cu.long(), cu.long()), causal.with_scale(0.2))
+    yield "padding", lambda: train(AttentionMask.key_padding(pad), AttentionOptions(), torch.float16, 128)
+    yield "padding i32, strided", lambda: train(AttentionMask.key_padding(pad.int()), causal.with_deterministic(True), torch.float32, 64, True)
+    q, k, v = randn(3, 8, 128), randn(3, 300, 2, 128), randn(3, 300, 2, 128, seed=1)
+    nk, nv = randn(3, 2, 128), randn(3, 2, 128, seed=1)
+    lens = torch.tensor([299, 0, 41], dtype=torch.int32, device="cuda")
+    rope = Rope(64, 10000.0, 300, torch.bfloat16)
+    yield "decode", lambda: (A.attention_decode(q, k, v, lens, AttentionOptions().with_window(100, None)),)
+    yield "decode all", lambda: (A.attention_decode(q, k[:, :200], v[:, :200], None, AttentionOptions(scale=0.1)),)
+
+    def append(f):
+        kk, vv = k.clone(), v.clone()
+        return f(kk, vv), kk, vv
+
+    yield "append", lambda: append(lambda kk, vv: A.attention_decode_append(q, nk, nv, kk, vv, lens.long()))
+    yield "append rope", lambda: append(lambda kk, vv: attention_decode_append_rope(rope, q, nk, nv, kk, vv, lens))
+    yield "append rope at", lambda: append(lambda kk, vv: attention_decode_append_rope(rope, q, nk, nv, kk, vv, lens, positions=lens // 2))
+    z = randn(5, 3001, dtype=torch.float32)
+    for o in (SampleOptions.greedy(), SampleOptions(temperature=0.7, top_k=20, top_p=0.9, seed=2**64 - 1, offset=3), SampleOptions(masked=(1, 7))):
+        yield f"sample {o}", lambda o=o: (lambda r: (r.tokens, r.logprob, r.tempered_logprob, r.sampling_logprob))(sample(z, o))
+    yield "sample of columns", lambda: (sample(z.t().contiguous().t(), SampleOptions(seed=4)).tokens,)
+
+
+def test_same_results_as_the_python_side(monkeypatch):
+    made = [(name, [x.clone() for x in call()]) for name, call in calls()]
+    torch.cuda.synchronize()
+    monkeypatch.setattr(_lib, "_binding", Nothing())
+    for (name, got), (_, call) in zip(made, calls()):
+        want = call()
+        assert len(got) == len(want)
+        for x, y in zip(got, want):
+            assert x.dtype == y.dtype and x.shape == y.shape and x.stride() == y.stride() and torch.equal(x, y), name
+
+
+def test_runs_on_the_current_stream_and_in_a_graph():
+    q, k, v = randn(2, 8, 128), randn(2, 500, 2, 128), randn(2, 500, 2, 128, seed=1)
+    want = A.attention_decode(q, k, v)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        A.attention_decode(q, k, v)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = A.attention_decode(q, k, v)
+        out.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+
+
+def test_refusals_of_the_library_are_raised():
+    q, k = randn(1, 4, 3, 64), randn(1, 4, 2, 64)
+    with pytest.raises(A.AttentionError, match="multiple of the key-value heads"):
+        A.attention(q, k, k)
+    with pytest.raises(A.AttentionError, match="multiple of the key-value heads"):
+        A.attention_decode(q[0], randn(4, 5, 2, 64), randn(4, 5, 2, 64))
+
+
+def test_a_mode_that_watches_sees_the_allocations():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    q, k = randn(1, 4, 2, 64), randn(1, 4, 2, 64)
+    with Watch():
+        A.attention(q, k, k)
+    assert any("empty" in s for s in seen)
