@@ -17,7 +17,10 @@
 //      Top-k leaves few tokens of many, and a lower bound of its threshold is cheap: the k-th largest of the THREADS' maxima
 //      is a token at least k tokens reach.  The tokens above the bound go into a list in shared memory, in the pass that sums
 //      the exponentials anyway, and the search and the draw look at the list; a list that would not fit leaves the passes over
-//      the row.  64 x 151936 bf16 logits, k = 50, p = 0.9: 74 -> 41 us side by side.  (A nucleus alone has no such bound
+//      the row.  The first of the row's blocks takes the others' lists over and does the rest alone: a few hundred tokens are
+//      less work than the blocks' meetings over them (a dozen of the two dozen there were, each about half a microsecond).
+//      64 x 151936 bf16 logits, k = 50, p = 0.9: 74 us without the list, 41 with one a block, 34 with the first block's;
+//      2 x 55620 f32 over eight blocks, k = 20, p = 0.9, 42.3 and 26.9.  (A nucleus alone has no such bound
 //      without one more pass over the row, which cost more than the list gave at every spread of the logits: N(0, 10) 67.8
 //      us with it, 63.8 without.)
 //   4. argmax over the kept tokens of s_i + g_i, ties to the lowest id, four tokens per Philox call;
@@ -84,7 +87,8 @@ __device__ __forceinline__ X block_reduce(X x, Op op, X *scratch) {
 }
 
 // The row's reduction: the block's, then the cluster's blocks in rank order through distributed
-// shared memory (`slot` is one value per block).
+// shared memory.  `slot` is one value per block and the call's own: it is written once in a launch, so the blocks meet once and
+// not a second time to give it back.  (No block leaves while another may still read: the kernel's last meeting.)
 template <typename X, typename Op>
 __device__ __forceinline__ X row_reduce(X x, Op op, X *scratch, X *slot) {
     x = block_reduce(x, op, scratch);
@@ -95,7 +99,6 @@ __device__ __forceinline__ X row_reduce(X x, Op op, X *scratch, X *slot) {
     cluster.sync();
     X r = *cluster.map_shared_rank(slot, 0);
     for (unsigned b = 1; b < blocks; ++b) r = op(r, *cluster.map_shared_rank(slot, b));
-    cluster.sync();   // every block has read before a slot is written again
     return r;
 }
 
@@ -135,17 +138,26 @@ __device__ __forceinline__ float gumbel_of_word(uint32_t x) {
 
 // Every token of the row once, thread by thread: 16 bytes of logits a load where the rows allow it
 // (eight 16-bit logits or four f32 to a thread at a time), one logit a load otherwise.
-template <typename T, typename F>
+// `AHEAD` loads of a thread are in flight at a time: four for the rows that are listed (17 x 150873 bf16 logits 74.8 -> 47.1 us with the rest);
+// one elsewhere, where the passes are shorter and four cost registers (125 x 31416, p alone, 46.4 us and 52.2).
+template <int AHEAD, typename T, typename F>
 __device__ __forceinline__ void for_each_logit(const T *z, int v, int tid, int TS, bool vec, F f) {
     constexpr int E = 16 / sizeof(T);
     int done = 0;
     if (vec) {
         const int nv = v / E;
-        for (int j = tid; j < nv; j += TS) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(z + (size_t)j * E);
-            const T *e = reinterpret_cast<const T *>(&raw);
+        for (int j = tid; j < nv; j += AHEAD * TS) {
+            uint4 raw[AHEAD];
 #pragma unroll
-            for (int k = 0; k < E; ++k) f(j * E + k, e[k]);
+            for (int u = 0; u < AHEAD; ++u)
+                if (j + u * TS < nv) raw[u] = *reinterpret_cast<const uint4 *>(z + (size_t)(j + u * TS) * E);
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                if (j + u * TS >= nv) break;
+                const T *e = reinterpret_cast<const T *>(&raw[u]);
+#pragma unroll
+                for (int k = 0; k < E; ++k) f((j + u * TS) * E + k, e[k]);
+            }
         }
         done = nv * E;
     }
@@ -162,8 +174,12 @@ struct RadixSmem {
     // A mass (41 bits of fixed point) as three pieces of 14, 14 and 13 bits in three 32-bit words: 32-bit
     // shared-memory atomics are native, 64-bit ones are not, and a copy's few thousand tokens cannot overflow a piece.
     uint32_t mass[3][8][256][4];
-    uint32_t tcnt[256];
-    unsigned long long tmass[256];
+    // The block's totals, which the cluster's other blocks read: two sets in turn, so that the blocks meet once a level - the set is
+    // written again two levels on, behind the next level's meeting, which no block reaches before it has read.
+    uint32_t tcnt[2][256];
+    unsigned long long tmass[2][256];
+    uint32_t row_cnt[256];            // all blocks' totals
+    unsigned long long row_mass[256];
     uint32_t sel, above_cnt, reach;
     unsigned long long above_mass, target;
 };
@@ -176,12 +192,11 @@ constexpr float MASS_ONE = 1099511627776.0f;   // 2^40: a weight in (0, 1] as an
 // for top-k (they sort last, as in the reference) and take no part in the masses.
 //
 // `each(f)` calls f(token, logit, whether it is masked) for this thread's tokens; GROUPS of the copies of the bins are used
-// (eight for a row, one for a list's few tokens).  The search ends early, with the low bits of T zero, once no more than
+// (eight for a row, one for a list's few tokens); over the row's `blocks`, or with 1 over this block's tokens alone.  The search ends early, with the low bits of T zero, once no more than
 // `enough` tokens reach T; `reaching` is how many do.
 template <typename T, bool MASS, int GROUPS, typename Each>
-__device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uint32_t floor_key, RadixSmem &sm, uint32_t enough, uint32_t &reaching) {
+__device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uint32_t floor_key, RadixSmem &sm, int blocks, uint32_t enough, uint32_t &reaching) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int blocks = (int)cluster.num_blocks();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t key_ninf = Key<T>::of(Num<T>::from_f32(-INFINITY));
     uint32_t prefix = 0, above_cnt = 0;
@@ -219,28 +234,32 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
                 if (MASS) w += (unsigned long long)sm.mass[0][x >> 2][threadIdx.x][x & 3] + ((unsigned long long)sm.mass[1][x >> 2][threadIdx.x][x & 3] << 14) +
                                ((unsigned long long)sm.mass[2][x >> 2][threadIdx.x][x & 3] << 28);
             }
-            sm.tcnt[threadIdx.x] = c;
-            sm.tmass[threadIdx.x] = w;
+            sm.tcnt[level & 1][threadIdx.x] = c;
+            sm.tmass[level & 1][threadIdx.x] = w;
         }
+        const uint32_t *tcnt = sm.tcnt[level & 1];
+        const unsigned long long *tmass = sm.tmass[level & 1];
         if (blocks > 1) {
             cluster.sync();
-            uint32_t c = 0;
-            unsigned long long w = 0;
             if (threadIdx.x < 256) {
+                uint32_t c = 0;
+                unsigned long long w = 0;
                 for (int r = 0; r < blocks; ++r) {
-                    c += *cluster.map_shared_rank(&sm.tcnt[threadIdx.x], r);
-                    if (MASS) w += *cluster.map_shared_rank(&sm.tmass[threadIdx.x], r);
+                    c += *cluster.map_shared_rank(&sm.tcnt[level & 1][threadIdx.x], r);
+                    if (MASS) w += *cluster.map_shared_rank(&sm.tmass[level & 1][threadIdx.x], r);
                 }
+                sm.row_cnt[threadIdx.x] = c;
+                sm.row_mass[threadIdx.x] = w;
             }
-            cluster.sync();   // every block has read the others' totals
-            if (threadIdx.x < 256) { sm.tcnt[threadIdx.x] = c; sm.tmass[threadIdx.x] = w; }
+            tcnt = sm.row_cnt;
+            tmass = sm.row_mass;
         }
         __syncthreads();
         if (warp == 0) {
             // Lane l holds bins 255 - 8 l down to 248 - 8 l: the higher bins on the lower lanes.
             uint32_t c8 = 0;
             unsigned long long w8 = 0;
-            for (int x = 0; x < 8; ++x) { c8 += sm.tcnt[255 - 8 * lane - x]; w8 += sm.tmass[255 - 8 * lane - x]; }
+            for (int x = 0; x < 8; ++x) { c8 += tcnt[255 - 8 * lane - x]; if (MASS) w8 += tmass[255 - 8 * lane - x]; }
             uint32_t c_before = c8;
             unsigned long long w_before = w8;
             for (int o = 1; o < 32; o <<= 1) {   // inclusive sums over the lanes up to this one
@@ -259,8 +278,8 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
             unsigned long long hit_w = 0;
             for (int x = 0; x < 8 && hit < 0; ++x) {
                 const int d = 255 - 8 * lane - x;
-                const uint32_t nc = run_c + sm.tcnt[d];
-                const unsigned long long nw = run_w + sm.tmass[d];
+                const uint32_t nc = run_c + tcnt[d];
+                const unsigned long long nw = run_w + (MASS ? tmass[d] : 0ull);
                 if (MASS ? (nw >= target && nc >= 1u) : (nc >= (uint32_t)a.top_k)) { hit = d; hit_c = run_c; hit_w = run_w; }
                 run_c = nc;
                 run_w = nw;
@@ -307,12 +326,13 @@ template <typename T> __device__ __forceinline__ T from_bits(uint32_t u) {
 // 4 us for code they never took.)
 template <typename T, bool LIST>
 __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
-    __shared__ unsigned long long us[32], uslot;
+    __shared__ unsigned long long us[32];
     __shared__ int listed_here;   // tokens that asked for a place in the block's list
     __shared__ float fs[32];
     __shared__ int is[32];
-    __shared__ float fslot;
-    __shared__ int islot;
+    // What the row's blocks tell one another, each written once.
+    __shared__ float slot_m, slot_s1, slot_wu, slot_best, slot_wp;
+    __shared__ int slot_first, slot_best_i, slot_listed;
     extern __shared__ __align__(16) uint8_t radix_raw[];
     RadixSmem &radix = *reinterpret_cast<RadixSmem *>(radix_raw);
     TokenList &list = *reinterpret_cast<TokenList *>(radix_raw + sizeof(RadixSmem));
@@ -324,30 +344,34 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     const uint32_t *bits = a.masked_bits;
     auto masked = [&](int i) { return bits != nullptr && ((bits[i >> 5] >> (i & 31)) & 1u) != 0; };
     const uint32_t key_ninf = Key<T>::of(Num<T>::from_f32(-INFINITY));
+    constexpr int AHEAD = LIST ? 4 : 1;
 
     // 1. m = max over the unmasked tokens; 2. sum exp(z - m) (and, tempered, sum exp((z - m) tau)).
     float m = -INFINITY;
-    for_each_logit(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
+    for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
         if (!masked(i)) m = fmaxf(m, Num<T>::to_f32(zi));
     });
     const float mine = m;
-    m = row_reduce(m, MaxOp(), fs, &fslot);
+    m = row_reduce(m, MaxOp(), fs, &slot_m);
     const bool degenerate = m == -INFINITY;   // no finite unmasked logit: the lowest unmasked id, NaN
     const bool tempered_differs = !a.greedy && a.tau != 1.0f;
     const bool cut = a.top_k > 0 || a.has_p;
-    auto each_logit = [&](auto f) { for_each_logit(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) { f(i, zi, masked(i)); }); };
-    // Top-k's bound: the k-th largest of the threads' maxima (at least k of them reach it), as many bytes of it as it takes for no
-    // more than half the threads to reach it: the row's tokens that do are then about 0.7 of the threads' number, whatever the
+    auto each_logit = [&](auto f) { for_each_logit<1>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) { f(i, zi, masked(i)); }); };
+    // Top-k's bound: the k-th largest of the threads' maxima (at least k tokens reach it), as many bytes of it as it takes for no
+    // more than half the threads to reach it: the tokens that do are then about 0.7 of the threads' number, whatever the
     // logits' offset and spread - where all bytes leave more, ties crowd at the cut and no list is made.  (One byte of a bf16
     // key is a factor of four: of logits N(20, 3) it held nearly all.)  Below it -inf, which is never drawn and weighs nothing.
+    // Up to half a block's threads each block takes the bound of its own threads' maxima - no token of the row's k largest lies
+    // below its block's k largest - and the blocks need not meet for it; above that, of all the row's.
     bool listed = LIST && !degenerate;
     uint32_t bound = 0xffffffffu;
     if constexpr (LIST) {
         if (listed) {
+            const int of = a.top_k <= ST / 2 ? 1 : blocks;
             auto each_maximum = [&](auto f) { if (mine != -INFINITY) f(0, Num<T>::from_f32(mine), false); };
             uint32_t reaching = 0;
-            bound = max(radix_threshold<T, false, 1>(each_maximum, a, m, 0u, radix, TS / 2, reaching), key_ninf + 1);
-            listed = reaching <= TS / 2;
+            bound = max(radix_threshold<T, false, 1>(each_maximum, a, m, 0u, radix, of, of * ST / 2, reaching), key_ninf + 1);
+            listed = reaching <= of * ST / 2;
             if (!listed) bound = 0xffffffffu;
         }
         if (threadIdx.x == 0) listed_here = 0;
@@ -355,7 +379,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     }
     float s1 = 0.f, wu = 0.f;
     int first = a.v;   // the lowest unmasked id holding the maximum
-    for_each_logit(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
+    for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
         if (masked(i)) return;
         const float x = Num<T>::to_f32(zi);
         s1 += expf(x - m);
@@ -366,32 +390,76 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
             if (at < LIST_MAX) { list.id[at] = (uint32_t)i; list.bits[at] = bits_of(zi); }
         }
     });
-    s1 = row_reduce(s1, AddOp(), fs, &fslot);
-    if (tempered_differs) wu = row_reduce(wu, AddOp(), fs, &fslot);
+    // The sums, and what the blocks have listed, in one meeting.
+    s1 = block_reduce(s1, AddOp(), fs);
+    if (tempered_differs) wu = block_reduce(wu, AddOp(), fs);
+    if (a.greedy || degenerate) first = block_reduce(first, MinOp(), is);
+    int n_listed = 0;
+    if (LIST && listed) {
+        __syncthreads();
+        n_listed = listed_here;
+        listed = n_listed <= LIST_MAX;
+    }
+    if (blocks > 1) {
+        if (threadIdx.x == 0) {
+            slot_s1 = s1;
+            slot_wu = wu;
+            slot_first = first;
+            slot_listed = listed ? n_listed : -1;
+        }
+        cluster.sync();
+        s1 = *cluster.map_shared_rank(&slot_s1, 0);
+        wu = *cluster.map_shared_rank(&slot_wu, 0);
+        first = *cluster.map_shared_rank(&slot_first, 0);
+        n_listed = *cluster.map_shared_rank(&slot_listed, 0);
+        listed = n_listed >= 0;
+        for (int b = 1; b < blocks; ++b) {
+            s1 += *cluster.map_shared_rank(&slot_s1, b);
+            wu += *cluster.map_shared_rank(&slot_wu, b);
+            first = min(first, *cluster.map_shared_rank(&slot_first, b));
+            const int n = *cluster.map_shared_rank(&slot_listed, b);
+            listed = listed && n >= 0;
+            n_listed += n;
+        }
+    }
+    if constexpr (LIST) {
+        listed = listed && n_listed <= LIST_MAX && s1 == s1;   // (a NaN among the logits: the passes over the row)
+        if (listed && blocks > 1) {
+            // The first block takes the others' lists over and does the rest, a few hundred tokens, by itself.
+            if (cluster.block_rank() == 0) {
+                int at = listed_here;
+                for (int b = 1; b < blocks; ++b) {
+                    const TokenList &other = *cluster.map_shared_rank(&list, b);
+                    const int n = *cluster.map_shared_rank(&slot_listed, b);
+                    for (int j = threadIdx.x; j < n; j += ST) {
+                        list.id[at + j] = other.id[j];
+                        list.bits[at + j] = other.bits[j];
+                    }
+                    at += n;
+                }
+            }
+            cluster.sync();
+            if (cluster.block_rank() != 0) return;
+        }
+    }
     const float lse = m + logf(s1);
 
     int token = 0;
     float tempered = 0.f, sampling = 0.f;
     bool own_tempered = true, own_sampling = true;   // false: the value is another output's (same bits)
     if (a.greedy || degenerate) {
-        token = row_reduce(first, MinOp(), is, &islot);
+        token = first;
     } else {
         // 3. The cuts: one threshold T on the keys; 0 keeps every token.
         uint32_t t_keep = 0;
         uint32_t reaching = 0;
-        if constexpr (LIST) {
-            __syncthreads();
-            const int most = row_reduce(-listed_here, MinOp(), is, &islot);   // of any block of the row
-            listed = listed && s1 == s1 && -most <= LIST_MAX;   // (a NaN among the logits: the passes over the row)
-        }
         if (listed) {
-            const int n = listed_here;
-            auto each_listed = [&](auto f) { for (int j = threadIdx.x; j < n; j += ST) f((int)list.id[j], from_bits<T>(list.bits[j]), false); };
-            t_keep = radix_threshold<T, false, 1>(each_listed, a, m, 0u, radix, 0, reaching);
-            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 1>(each_listed, a, m, t_keep, radix, 0, reaching));
+            auto each_listed = [&](auto f) { for (int j = threadIdx.x; j < n_listed; j += ST) f((int)list.id[j], from_bits<T>(list.bits[j]), false); };
+            t_keep = radix_threshold<T, false, 1>(each_listed, a, m, 0u, radix, 1, 0, reaching);
+            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 1>(each_listed, a, m, t_keep, radix, 1, 0, reaching));
         } else {
-            if (a.top_k > 0) t_keep = radix_threshold<T, false, 8>(each_logit, a, m, 0u, radix, 0, reaching);
-            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 8>(each_logit, a, m, t_keep, radix, 0, reaching));
+            if (a.top_k > 0) t_keep = radix_threshold<T, false, 8>(each_logit, a, m, 0u, radix, blocks, 0, reaching);
+            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 8>(each_logit, a, m, t_keep, radix, blocks, 0, reaching));
         }
 
         // 4. argmax of s + g over the kept tokens, ties to the lowest id; the kept tokens' mass.
@@ -442,7 +510,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
         if (listed) {
             // One token at a time, in whatever order the list took them: the winner does not depend on it (the larger score,
             // then the lower id), and the mass is summed in fixed point.
-            for (int j = threadIdx.x; j < listed_here; j += ST) {
+            for (int j = threadIdx.x; j < n_listed; j += ST) {
                 const T zi = from_bits<T>(list.bits[j]);
                 if (Key<T>::of(zi) < t_keep) continue;
                 const int i = (int)list.id[j];
@@ -498,22 +566,23 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
                 const int ib = __shfl_xor_sync(0xffffffffu, best_i, o);
                 if (better(best, best_i, sb, ib)) { best = sb; best_i = ib; }
             }
-            if (blocks > 1) {
-                if (threadIdx.x == 0) { fslot = best; islot = best_i; }
+            if (cut && !listed) wp = block_reduce(wp, AddOp(), fs);
+            if (blocks > 1 && !listed) {
+                if (threadIdx.x == 0) { slot_best = best; slot_best_i = best_i; slot_wp = wp; }
                 cluster.sync();
-                best = *cluster.map_shared_rank(&fslot, 0);
-                best_i = *cluster.map_shared_rank(&islot, 0);
+                best = *cluster.map_shared_rank(&slot_best, 0);
+                best_i = *cluster.map_shared_rank(&slot_best_i, 0);
+                wp = *cluster.map_shared_rank(&slot_wp, 0);
                 for (int b = 1; b < blocks; ++b) {
-                    const float sb = *cluster.map_shared_rank(&fslot, b);
-                    const int ib = *cluster.map_shared_rank(&islot, b);
+                    const float sb = *cluster.map_shared_rank(&slot_best, b);
+                    const int ib = *cluster.map_shared_rank(&slot_best_i, b);
                     if (better(best, best_i, sb, ib)) { best = sb; best_i = ib; }
+                    wp += *cluster.map_shared_rank(&slot_wp, b);
                 }
-                cluster.sync();
             }
         }
         token = best_i == INT_MAX ? 0 : best_i;
-        if (listed) wp = (float)((double)row_reduce(wp_mass, AddOp(), us, &uslot) * (1.0 / (double)MASS_ONE));
-        else if (cut) wp = row_reduce(wp, AddOp(), fs, &fslot);
+        if (listed) wp = (float)((double)block_reduce(wp_mass, AddOp(), us) * (1.0 / (double)MASS_ONE));
         const float s_t = __fmul_rn(Num<T>::to_f32(z[token]) - m, a.tau);
         if (tempered_differs) tempered = s_t - logf(wu); else own_tempered = false;
         if (cut) sampling = s_t - logf(wp); else own_sampling = false;
@@ -531,6 +600,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
         a.tempered[row] = tempered;
         a.sampling[row] = sampling;
     }
+    if (blocks > 1 && !listed) cluster.sync();   // no block leaves while another may read what it has told
 }
 
 }  // namespace
