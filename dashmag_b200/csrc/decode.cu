@@ -27,6 +27,7 @@
 //
 // Inputs the vector path cannot read (head dimension not 64 / 128 / 256, last stride not 1, rows
 // not 16-byte aligned) go through a slower scalar kernel with the same arithmetic.
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -683,10 +684,14 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_scalar_kernel(Dec
 // shared memory, then every thread its head dimensions over the splits.
 constexpr int MERGE_MAX = 1024;  // splits whose weights fit the shared array; more are folded in passes
 
-template <typename T>
-__global__ void __launch_bounds__(128) decode_merge_kernel(DecodeArgs a) {
+constexpr int MERGE_EACH = 8;    // partials a thread asks for at once
+
+template <typename T, int TH>
+__global__ void __launch_bounds__(TH) decode_merge_kernel(DecodeArgs a) {
     __shared__ float w[MERGE_MAX];
-    __shared__ float red[4];
+    __shared__ float red[TH / 32];
+    __shared__ float4 part[TH];
+    __shared__ float dens[TH];
     wait_before();   // the split pass
     const int bh = blockIdx.x;
     const int b = bh / a.hq;
@@ -695,31 +700,88 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(DecodeArgs a) {
     const int n = (len - first + a.chunk - 1) / a.chunk;  // splits that hold keys
     T *out = static_cast<T *>(a.out) + (int64_t)bh * a.d;
     if (n <= 0) {
-        for (int c = threadIdx.x; c < a.d; c += blockDim.x) out[c] = Num<T>::from_f32(0.f);
+        for (int c = threadIdx.x; c < a.d; c += TH) out[c] = Num<T>::from_f32(0.f);
+        return;
+    }
+    // Four head dimensions a thread (16-byte loads of the partials), the splits dealt over the TH / (d / 4) groups of threads,
+    // whose sums meet in shared memory in group order.
+    const int ct = max(a.d / 4, 1), groups = TH / ct;
+    const int c4 = threadIdx.x % ct, sg = threadIdx.x / ct;
+    auto finish = [&](float4 num, float den) {
+        part[threadIdx.x] = num;
+        dens[threadIdx.x] = den;
+        __syncthreads();
+        if (sg != 0) return;
+        for (int g = 1; g < groups; ++g) {
+            const float4 x = part[g * ct + c4];
+            num.x += x.x; num.y += x.y; num.z += x.z; num.w += x.w;
+            den += dens[g * ct + c4];
+        }
+        const float inv = den > 0.f ? 1.f / den : 0.f;
+        T *o = out + 4 * c4;
+        o[0] = Num<T>::from_f32(num.x * inv);
+        o[1] = Num<T>::from_f32(num.y * inv);
+        o[2] = Num<T>::from_f32(num.z * inv);
+        o[3] = Num<T>::from_f32(num.w * inv);
+    };
+    const bool vec = a.d % 4 == 0;
+    if (vec && n <= MERGE_EACH * groups) {
+        // Few splits: a thread asks for its log-sum-exps and its partials at once and has the maximum worked out under their
+        // flight, one trip to memory where the passes below take one for the maximum, one for the weights and one for
+        // every four partials.
+        const float *lse = a.part_lse + (int64_t)bh * a.splits;
+        const float *po = a.part_o + (int64_t)bh * a.splits * a.d + 4 * c4;
+        float own[MERGE_EACH];
+        float4 x[MERGE_EACH];
+#pragma unroll
+        for (int e = 0; e < MERGE_EACH; ++e) {
+            const int i = sg + e * groups;
+            const bool in = sg < groups && i < n;
+            own[e] = in ? lse[i] : -INFINITY;
+            x[e] = in ? *reinterpret_cast<const float4 *>(po + (int64_t)i * a.d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float mx = own[0];
+#pragma unroll
+        for (int e = 1; e < MERGE_EACH; ++e) mx = fmaxf(mx, own[e]);
+        mx = warp_max(mx);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        mx = red[0];
+#pragma unroll
+        for (int i = 1; i < TH / 32; ++i) mx = fmaxf(mx, red[i]);
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+        float den = 0.f;
+#pragma unroll
+        for (int e = 0; e < MERGE_EACH; ++e) {
+            if (sg + e * groups >= n) break;
+            const float wi = expf(own[e] - mx);
+            den += wi;
+            num.x = fmaf(wi, x[e].x, num.x);
+            num.y = fmaf(wi, x[e].y, num.y);
+            num.z = fmaf(wi, x[e].z, num.z);
+            num.w = fmaf(wi, x[e].w, num.w);
+        }
+        finish(num, den);
         return;
     }
     const float *lse = a.part_lse + (int64_t)bh * a.splits;
     const float *po = a.part_o + (int64_t)bh * a.splits * a.d;
     float mx = -INFINITY;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmaxf(mx, lse[i]);
+    for (int i = threadIdx.x; i < n; i += TH) mx = fmaxf(mx, lse[i]);
     mx = warp_max(mx);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
-    mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    mx = red[0];
+#pragma unroll
+    for (int i = 1; i < TH / 32; ++i) mx = fmaxf(mx, red[i]);
 
-    if (a.d % 4 == 0) {
-        // Four head dimensions a thread (16-byte loads of the partials), the splits dealt over the
-        // 128 / (d / 4) groups of threads, whose sums meet in shared memory in group order.
-        __shared__ float4 part[128];
-        __shared__ float dens[128];
-        const int ct = a.d / 4, groups = 128 / ct;
-        const int c4 = threadIdx.x % ct, sg = threadIdx.x / ct;
+    if (vec) {
         float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
         float den = 0.f;
         for (int i0 = 0; i0 < n; i0 += MERGE_MAX) {
             const int m = min(MERGE_MAX, n - i0);
             __syncthreads();
-            for (int i = threadIdx.x; i < m; i += blockDim.x) w[i] = expf(lse[i0 + i] - mx);
+            for (int i = threadIdx.x; i < m; i += TH) w[i] = expf(lse[i0 + i] - mx);
             __syncthreads();
             if (sg < groups) {
 #pragma unroll 4
@@ -734,29 +796,14 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(DecodeArgs a) {
                 }
             }
         }
-        part[threadIdx.x] = num;
-        dens[threadIdx.x] = den;
-        __syncthreads();
-        if (sg == 0) {
-            for (int g = 1; g < groups; ++g) {
-                const float4 x = part[g * ct + c4];
-                num.x += x.x; num.y += x.y; num.z += x.z; num.w += x.w;
-                den += dens[g * ct + c4];
-            }
-            const float inv = den > 0.f ? 1.f / den : 0.f;
-            T *o = out + 4 * c4;
-            o[0] = Num<T>::from_f32(num.x * inv);
-            o[1] = Num<T>::from_f32(num.y * inv);
-            o[2] = Num<T>::from_f32(num.z * inv);
-            o[3] = Num<T>::from_f32(num.w * inv);
-        }
+        finish(num, den);
         return;
     }
-    float num[2] = {0.f, 0.f}, den = 0.f;  // a.d <= 256: two head dimensions per thread at most
+    float num[2] = {0.f, 0.f}, den = 0.f;  // a.d <= 256 <= 2 TH: two head dimensions per thread at most
     for (int i0 = 0; i0 < n; i0 += MERGE_MAX) {
         const int m = min(MERGE_MAX, n - i0);
         __syncthreads();
-        for (int i = threadIdx.x; i < m; i += blockDim.x) w[i] = expf(lse[i0 + i] - mx);
+        for (int i = threadIdx.x; i < m; i += TH) w[i] = expf(lse[i0 + i] - mx);
         __syncthreads();
 #pragma unroll 4
         for (int i = 0; i < m; ++i) {
@@ -765,14 +812,14 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(DecodeArgs a) {
             const float *row = po + (int64_t)(i0 + i) * a.d;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const int c = threadIdx.x + 128 * k;
+                const int c = threadIdx.x + TH * k;
                 if (c < a.d) num[k] = fmaf(wi, row[c], num[k]);
             }
         }
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const int c = threadIdx.x + 128 * k;
+        const int c = threadIdx.x + TH * k;
         if (c < a.d) out[c] = Num<T>::from_f32(den > 0.f ? num[k] / den : 0.f);
     }
 }
@@ -858,7 +905,19 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
     // few calls of few blocks with much to read lose by it: 16 of up to 20000 keys, 16 heads on one, 36.0 us after the pass,
     // 38.2 under its end; 25 of up to 19426 41.5 and 42.3.  Neither the parts' size nor the blocks' number tells them apart:
     // with the line at 12 or 20 MB of parts more calls lost than won.)
-    return launch_beside(decode_merge_kernel<T>, dim3(a.b * a.hq), 128, 0, stream, true, a);
+    // Threads of a merge block: 128, or where the blocks are at most two a multiprocessor the fewest (up to 512) with which every
+    // partial is asked for at once.  (Threads 128 / 256 / 512, and the merge as it was: one sequence of 4096 keys, 8 heads,
+    // 64 splits on 32 blocks, 13.3 / 11.9 / 12.1 us, 13.7; two of 5919 13.5 / 13.0 / 11.9, 14.4; eight of 6144, 2 heads of 256,
+    // 35 splits on 64 blocks, 21.6 / 22.2 / 21.1, 22.0; but 60 of up to 9557 on 1920 blocks 193.7 / 196.3 / 205.5, 193.4, and 61
+    // under a window on 976 37.1 / 38.1 / 42.8, 37.9.)
+    const int64_t blocks = (int64_t)a.b * a.hq;
+    int threads = 128;
+    if (blocks <= 2 * 148)
+        while (threads < 512 && (int64_t)a.splits * std::max(a.d / 4, 1) > (int64_t)MERGE_EACH * threads) threads *= 2;
+    const dim3 grid((unsigned)blocks);
+    if (threads == 512) return launch_beside(decode_merge_kernel<T, 512>, grid, 512, 0, stream, true, a);
+    if (threads == 256) return launch_beside(decode_merge_kernel<T, 256>, grid, 256, 0, stream, true, a);
+    return launch_beside(decode_merge_kernel<T, 128>, grid, 128, 0, stream, true, a);
 }
 
 cudaError_t launch_decode(int dtype, const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches) {
