@@ -165,10 +165,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) bwd_plan_kernel(const Sm100BwdAr
 }
 
 // Launches the plan into a.order, or clears a.order when there is nothing to rank or too much to rank
-// in one block (the units then run in index order).
-cudaError_t launch_bwd_plan(Sm100BwdArgs &a, cudaStream_t stream, int *launches) {
+// in one block (the units then run in index order).  Nothing to rank: up to `at_once` units, which start together whatever their
+// order, and would wait 5 to 7 us for it.
+cudaError_t launch_bwd_plan(Sm100BwdArgs &a, int at_once, cudaStream_t stream, int *launches) {
     const long long items = (long long)a.b * ((a.tk + BIG - 1) / BIG);
-    if (a.order && items > 1 && items <= PLAN_MAX && items * a.hkv <= 0x7fffffffLL / 4) {
+    if (a.order && items > 1 && items * a.hkv > at_once && items <= PLAN_MAX && items * a.hkv <= 0x7fffffffLL / 4) {
         bwd_plan_kernel<<<1, PLAN_THREADS, 0, stream>>>(a, (int)items);
         *launches += 1;
         return cudaGetLastError();
@@ -260,16 +261,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     Tail &sh = *reinterpret_cast<Tail *>(FUSED ? red_s + 2 * RED_SLOT : do_s + DOS * BIG_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if constexpr (!FUSED) allow_beside();   // dq
-    // Units are taken in the order the plan kernel left (without one: in index order, the heads of a
-    // key block side by side).
-    const int nkb = (a.tk + BIG - 1) / BIG;
-    const int unit = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
-    const int item = unit / a.hkv, hk = unit - item * a.hkv;
-    const int b = item / nkb, kt = item - b * nkb;
-    const int group = a.hq / a.hkv;
-    const int k0 = kt * BIG, k1 = min(k0 + BIG, a.tk);
     auto BAR = [&](uint64_t &x) { return smem_u32(&x); };
+    // The kernel comes in under delta's end (FUSED: behind it).  What it reads of the kernels before it is delta and the plan:
+    // with a plan every thread waits for them before it asks for its unit, without one only the warp that gathers delta
+    // does, while the block sets itself up and brings in its first tiles.  Behind the wait dq may start: it reads delta too.
+    const bool planned = a.order != nullptr;
 
     if (threadIdx.x == 0) {
         sh.abort = *reinterpret_cast<volatile unsigned int *>(&g_sm100_bwd_status);
@@ -299,6 +295,26 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_do);
         if constexpr (FUSED) prefetch_tensormap(&tm_dq_acc);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&sh.tmem_base), 512);
+        tmem_relinquish();
+    }
+    __syncwarp();
+    if (planned) {
+        wait_before();
+        if constexpr (!FUSED) allow_beside();
+    }
+    // Units are taken in the order the plan kernel left (without one: in index order, the heads of a
+    // key block side by side).
+    const int nkb = (a.tk + BIG - 1) / BIG;
+    const int unit = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
+    const int item = unit / a.hkv, hk = unit - item * a.hkv;
+    const int b = item / nkb, kt = item - b * nkb;
+    const int group = a.hq / a.hkv;
+    const int k0 = kt * BIG, k1 = min(k0 + BIG, a.tk);
+
+    if (threadIdx.x == 0) {
         // The resident tiles are on their way before the block knows which queries it sweeps: their
         // flight covers the rest of the setup.  (A block that turns out to have nothing to do waits
         // for them at the end: shared memory must not be written behind a block that has left.)
@@ -308,10 +324,6 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if constexpr (HD > 64) tma_load_4d(smem_u32(k_s + BIG_HALF), &tm_k, rfull, 64, hk, k0, b);
         tma_load_4d(smem_u32(v_s), &tm_v, rfull, 0, hk, k0, b);
         if constexpr (HD > 64) tma_load_4d(smem_u32(v_s + BIG_HALF), &tm_v, rfull, 64, hk, k0, b);
-    }
-    if (warp == 1) {
-        tmem_alloc(smem_u32(&sh.tmem_base), 512);
-        tmem_relinquish();
     }
     int qfirst, qend;
     query_range(a.mask, k0, k1, a.tq, a.tk, qfirst, qend);
@@ -386,6 +398,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 dl_n[i] = a.delta[at];
             }
         };
+        if (!planned) {
+            wait_before();
+            if constexpr (!FUSED) allow_beside();
+        }
         if (steps > 0) gather(0);
         for (int t = 0; t < steps; ++t) {
             const int st = t & 1, ph = (t >> 1) & 1;
@@ -1064,8 +1080,10 @@ static cudaError_t launch_dkdv(const Sm100BwdMaps &m, const Sm100BwdArgs &a, lon
     cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_sm100_kernel<T, HD, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 gk((unsigned)(items * a.hkv), 1, 1);
-    bwd_dkdv_sm100_kernel<T, HD, FUSED><<<gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream>>>(m.k128, m.v128, m.q128, m.do128, m.dq_acc, a);
-    return cudaGetLastError();
+    // Under delta's end (4 packed sequences, 2149 tokens, 16 / 4 heads, forward and backward: 104.3 -> 98.2 us with the plan left out
+    // too; 9 sequences, 1047 tokens, 48.3 -> 43.2; 10 padded ones of 224, 12 / 4 heads, 53.4 -> 49.0); the fused form behind the memset.
+    return launch_beside(bwd_dkdv_sm100_kernel<T, HD, FUSED>, gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream, !FUSED, m.k128, m.v128, m.q128,
+                         m.do128, m.dq_acc, a);
 }
 
 template <typename T, int HD>

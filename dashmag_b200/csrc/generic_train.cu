@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
+    allow_beside();
     const int lane = threadIdx.x & 31;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq;
     int64_t row = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
@@ -583,6 +584,7 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
 // request.
 template <typename T, int D>
 __global__ void __launch_bounds__(THREADS) delta_rows_kernel(TrainArgs a) {
+    allow_beside();   // the key and value gradients' kernel, which waits for delta where it reads it
     constexpr int LPR = D / 8, RPW = 32 / LPR;   // lanes per row, rows per warp
     const int lane = threadIdx.x & 31, sub = lane % LPR;
     const int64_t rows = (int64_t)a.b * a.tq * a.hq;

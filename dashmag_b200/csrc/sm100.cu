@@ -328,7 +328,7 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
     f.pack = pack;
     // The plan's one block and delta run side by side; then dkdv, and dq beside its last waves (neither reads what
     // the other writes).
-    cudaError_t e = launch_bwd_plan(f, stream, launches);
+    cudaError_t e = launch_bwd_plan(f, p->d == 256 ? 37 : 148, stream, launches);
     if (e == cudaSuccess) e = launch_generic_delta(p->dtype, a, stream, launches, f.order != nullptr);
     if (e != cudaSuccess) return e;
     if (p->d == 256) return launch_bwd256_sm100(p->dtype, m, f, stream, launches);

@@ -55,7 +55,7 @@ struct Sm100BwdMaps {
 // Adds the kernels it launched to *launches.
 cudaError_t launch_bwd_sm100(int dtype, const Sm100BwdMaps &m, const Sm100BwdArgs &a, cudaStream_t stream, int *launches);
 size_t bwd_sm100_order_bytes(int b, int tk, int hkv);
-cudaError_t launch_bwd_plan(Sm100BwdArgs &a, cudaStream_t stream, int *launches);
+cudaError_t launch_bwd_plan(Sm100BwdArgs &a, int at_once, cudaStream_t stream, int *launches);
 // Head dimension 256: the dq pass, the plan, and the dk and dv passes as one launch (bwd256_sm100.cu).
 cudaError_t launch_bwd256_sm100(int dtype, const Sm100BwdMaps &m, const Sm100BwdArgs &a, cudaStream_t stream, int *launches);
 cudaError_t read_sm100_bwd256_status(unsigned int *status, bool clear);
