@@ -19,8 +19,9 @@
 //      the exponentials anyway, and the search and the draw look at the list; a list that would not fit leaves the passes over
 //      the row.  The first of the row's blocks takes the others' lists over and does the rest alone: a few hundred tokens are
 //      less work than the blocks' meetings over them (a dozen of the two dozen there were, each about half a microsecond).
-//      64 x 151936 bf16 logits, k = 50, p = 0.9: 74 us without the list, 41 with one a block, 34 with the first block's;
-//      2 x 55620 f32 over eight blocks, k = 20, p = 0.9, 42.3 and 26.9.  (A nucleus alone has no such bound
+//      64 x 151936 bf16 logits, k = 50, p = 0.9: 74 us without the list, 41 with one a block, 34 with the first block's, 30 with
+//      the passes' questions asked once a pass (masked ids, the temperature) or as one comparison of numbers (the bound);
+//      2 x 55620 f32 over eight blocks, k = 20, p = 0.9, 42.3 and 26.7; greedy 110 x 151557 f32 64.6 and 26.8.  (A nucleus alone has no such bound
 //      without one more pass over the row, which cost more than the list gave at every spread of the logits: N(0, 10) 67.8
 //      us with it, 63.8 without.)
 //   4. argmax over the kept tokens of s_i + g_i, ties to the lowest id, four tokens per Philox call;
@@ -32,6 +33,8 @@
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "sample.h"
@@ -66,6 +69,16 @@ template <> struct Key<__half> {
         return (u & 0x8000u) ? (~u & 0xffffu) : (u | 0x8000u);
     }
 };
+
+// The number whose key this is.
+template <typename T> __device__ __forceinline__ float number_of(uint32_t key);
+template <> __device__ __forceinline__ float number_of<float>(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key); }
+template <> __device__ __forceinline__ float number_of<__nv_bfloat16>(uint32_t key) {
+    return __bfloat162float(__ushort_as_bfloat16((unsigned short)((key & 0x8000u) ? key & 0x7fffu : ~key & 0xffffu)));
+}
+template <> __device__ __forceinline__ float number_of<__half>(uint32_t key) {
+    return __half2float(__ushort_as_half((unsigned short)((key & 0x8000u) ? key & 0x7fffu : ~key & 0xffffu)));
+}
 
 struct MaxOp { __device__ float operator()(float a, float b) const { return fmaxf(a, b); } };
 struct AddOp { template <typename X> __device__ X operator()(X a, X b) const { return a + b; } };
@@ -348,9 +361,12 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
 
     // 1. m = max over the unmasked tokens; 2. sum exp(z - m) (and, tempered, sum exp((z - m) tau)).
     float m = -INFINITY;
-    for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
-        if (!masked(i)) m = fmaxf(m, Num<T>::to_f32(zi));
-    });
+    // (Whether ids are masked at all is asked once a pass and not once a token.)
+    auto each_open = [&](auto f) {
+        if (bits) for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) { if (!masked(i)) f(i, zi); });
+        else for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, f);
+    };
+    each_open([&](int, T zi) { m = fmaxf(m, Num<T>::to_f32(zi)); });
     const float mine = m;
     m = row_reduce(m, MaxOp(), fs, &slot_m);
     const bool degenerate = m == -INFINITY;   // no finite unmasked logit: the lowest unmasked id, NaN
@@ -364,7 +380,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     // Up to half a block's threads each block takes the bound of its own threads' maxima - no token of the row's k largest lies
     // below its block's k largest - and the blocks need not meet for it; above that, of all the row's.
     bool listed = LIST && !degenerate;
-    uint32_t bound = 0xffffffffu;
+    uint32_t bound = 0u;
     if constexpr (LIST) {
         if (listed) {
             const int of = a.top_k <= ST / 2 ? 1 : blocks;
@@ -372,24 +388,31 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
             uint32_t reaching = 0;
             bound = max(radix_threshold<T, false, 1>(each_maximum, a, m, 0u, radix, of, of * ST / 2, reaching), key_ninf + 1);
             listed = reaching <= of * ST / 2;
-            if (!listed) bound = 0xffffffffu;
         }
         if (threadIdx.x == 0) listed_here = 0;
         __syncthreads();
     }
+    // The bound as a number: a token that compares with it is listed (0 and -0 compare equal and their keys are neighbours: the lower
+    // one listed too does no harm; of NaNs the sums tell).
+    float least = INFINITY;
+    if (LIST && listed) least = number_of<T>(bound);
     float s1 = 0.f, wu = 0.f;
     int first = a.v;   // the lowest unmasked id holding the maximum
-    for_each_logit<AHEAD>(z, a.v, tid, TS, a.vec != 0, [&](int i, T zi) {
-        if (masked(i)) return;
-        const float x = Num<T>::to_f32(zi);
-        s1 += expf(x - m);
-        if (tempered_differs) wu += expf((x - m) * a.tau);
-        if (x == m && i < first) first = i;
-        if (LIST && Key<T>::of(zi) >= bound) {
-            const int at = atomicAdd(&listed_here, 1);
-            if (at < LIST_MAX) { list.id[at] = (uint32_t)i; list.bits[at] = bits_of(zi); }
-        }
-    });
+    auto sums = [&](auto tempered_) {
+        each_open([&](int i, T zi) {
+            const float x = Num<T>::to_f32(zi);
+            s1 += expf(x - m);
+            if (decltype(tempered_)::value) wu += expf((x - m) * a.tau);
+            if (!LIST && x == m && i < first) first = i;
+            if (LIST && x >= least) {
+                const int at = atomicAdd(&listed_here, 1);
+                if (at < LIST_MAX) { list.id[at] = (uint32_t)i; list.bits[at] = bits_of(zi); }
+            }
+        });
+    };
+    if (tempered_differs) sums(std::true_type{});
+    else sums(std::false_type{});
+    if (LIST && degenerate) each_open([&](int i, T zi) { if (Num<T>::to_f32(zi) == m) first = min(first, i); });
     // The sums, and what the blocks have listed, in one meeting.
     s1 = block_reduce(s1, AddOp(), fs);
     if (tempered_differs) wu = block_reduce(wu, AddOp(), fs);
