@@ -17,10 +17,13 @@
 //
 // RPW is four where the rows fill the GPU that way (a tile row read from shared memory then serves four
 // products), two or one where they do not (rows_per_warp): small calls are bound by the length of a block's chain of
-// tiles, not by throughput.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
+// tiles, not by throughput.  Where one would do and shared memory allows it the block takes its tiles two at a time (KS 2): a warp
+// has two rows and every second tile, and the two warps of the same rows add their sums at the end - half the links in the chain, and
+// half the reads of shared memory a product.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
 // Two packed sequences of 384 tokens, four heads of 64, f32: the step 254 ->
 // 61 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
-// another; launch and host time are most of what is left).
+// another), and 53 with the tiles two at a time; 381 tokens, 3 / 1 heads of 96, 74 -> 55, 590 148 -> 103, 1478 of 64 345 -> 246
+// (the sums of two halves are nearer to f64 than one: dk of that call 9.3e-7 -> 6.8e-7).
 #include <algorithm>
 
 #include "bwd_common.cuh"
@@ -142,6 +145,29 @@ __device__ __forceinline__ void put_weights(float *weight, const float (&w)[RPW]
     else weight[lane] = w[0];
 }
 
+// KS warps swept a step's KS tiles for the same rows: the sums of the first take the others' in order.  `box`: the tiles' shared memory.
+template <int RPW, int NI, int KS>
+__device__ __forceinline__ void gather_shares(float *box, float (&acc)[RPW][NI]) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert((KS - 1) * (WARPS / KS) * RPW * NI * 32 <= 4 * KS * TILE * (NI > 2 ? 68 : 4), "the shares fit where the tiles were");
+    __syncthreads();   // nobody reads the tiles (or the shares before) any more
+    if (w >= WARPS / KS) {
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+#pragma unroll
+            for (int i = 0; i < NI; ++i) box[(((w - WARPS / KS) * RPW + r) * NI + i) * 32 + lane] = acc[r][i];
+    }
+    __syncthreads();
+    if (w < WARPS / KS) {
+#pragma unroll
+        for (int o = 1; o < KS; ++o)
+#pragma unroll
+            for (int r = 0; r < RPW; ++r)
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[r][i] += box[((((o - 1) * (WARPS / KS) + w) * RPW + r) * NI + i) * 32 + lane];
+    }
+}
+
 // The block's first row, and what each of its rows sees: the queries' key intervals (warp 0 places them) and their union.
 struct RowSpans {
     int lo[32], hi[32];
@@ -162,18 +188,19 @@ __device__ __forceinline__ void place_rows(RowSpans &sp, const MaskArgs &m, int 
 // ---------------------------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI>
+template <typename T, int RPW, int NI, int KS>
 __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int ROWS = WARPS * RPW;
+    constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
     const int dp = padded_d(a.d), sp = tile_stride(a.d);
     float *qs = smem;                          // [ROWS][dp]
-    float *kv = qs + ROWS * dp;                // [2 buffers][K, V][32][sp]
-    float *ps = kv + 4 * TILE * sp;            // [8 warps][32 keys][RPW]
+    float *kv = qs + ROWS * dp;                // [2 buffers][K, V][STEP][sp]
+    float *ps = kv + 4 * STEP * sp;            // [8 warps][32 keys][RPW]
     __shared__ RowSpans rs;
-    __shared__ int pad[2][TILE];               // key padding flags of the tile
+    __shared__ int pad[2][STEP];               // key padding flags of the tile
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);   // the warp's rows; its tile of the step's KS
     const int qt = gridDim.x - 1 - blockIdx.x;  // long (late) causal rows first
     const int h = blockIdx.y, b = blockIdx.z;
     const int hk = h / (a.hq / a.hkv);
@@ -189,8 +216,8 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
     int wlo = a.tk, whi = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        lo[r] = rs.lo[w * RPW + r];
-        hi[r] = rs.hi[w * RPW + r];
+        lo[r] = rs.lo[wr * RPW + r];
+        hi[r] = rs.hi[wr * RPW + r];
         if (hi[r] > lo[r]) { wlo = min(wlo, lo[r]); whi = max(whi, hi[r]); }
     }
     float m[RPW], l[RPW], acc[RPW][NI];   // l: this lane's share of the row's sum
@@ -202,26 +229,27 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
         for (int i = 0; i < NI; ++i) acc[r][i] = 0.f;
     }
     auto stage = [&](int k0, int buf) {
-        stage_rows<T>(kv + (2 * buf) * TILE * sp, sp, a.k, b, hk, k0, TILE, a.tk, a.d, vec);
-        stage_rows<T>(kv + (2 * buf + 1) * TILE * sp, sp, a.v, b, hk, k0, TILE, a.tk, a.d, vec);
-        if (threadIdx.x < TILE) {
+        stage_rows<T>(kv + (2 * buf) * STEP * sp, sp, a.k, b, hk, k0, STEP, a.tk, a.d, vec);
+        stage_rows<T>(kv + (2 * buf + 1) * STEP * sp, sp, a.v, b, hk, k0, STEP, a.tk, a.d, vec);
+        if (threadIdx.x < STEP) {
             const int key = k0 + threadIdx.x;
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
     };
     const int first = kmin / TILE * TILE;
     if (kmax > kmin) stage(first, 0);
-    for (int k0 = first, buf = 0; k0 < kmax; k0 += TILE, buf ^= 1) {
+    for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();   // the tile is whole, and every warp is done with the other buffer
-        if (k0 + TILE < kmax) stage(k0 + TILE, buf ^ 1);
-        if (k0 + TILE <= wlo || k0 >= whi) continue;  // no row of this warp sees the tile
-        const float *ks = kv + (2 * buf) * TILE * sp, *vs = ks + TILE * sp;
+        if (k0 + STEP < kmax) stage(k0 + STEP, buf ^ 1);
+        const int t0 = k0 + sub * TILE;
+        if (t0 + TILE <= wlo || t0 >= whi) continue;  // no row of this warp sees the tile
+        const float *ks = kv + (2 * buf) * STEP * sp + sub * TILE * sp, *vs = ks + STEP * sp;
 
         float s[RPW];
-        dots<RPW>(qs + w * RPW * dp, dp, ks + lane * sp, dp, s);
-        const int key = k0 + lane;
-        const bool open = pad[buf][lane] == 0;
+        dots<RPW>(qs + wr * RPW * dp, dp, ks + lane * sp, dp, s);
+        const int key = t0 + lane;
+        const bool open = pad[buf][sub * TILE + lane] == 0;
         float *pw = ps + w * TILE * RPW, ps4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
@@ -245,11 +273,42 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
         __syncwarp();
     }
     copies_wait();
+    if constexpr (KS > 1) {
+        // The warps that swept the other tiles hand over what they have, through the tiles' shared memory (4 STEP rows of at least
+        // four floats).
+        static_assert((KS - 1) * (WARPS / KS) * RPW * (NI + 2) * 32 <= 4 * STEP * (NI > 2 ? 68 : 4), "the shares fit where the tiles were");
+        __syncthreads();
+        auto box_of = [&](int s) { return kv + ((s - 1) * (WARPS / KS) + wr) * RPW * (NI + 2) * 32 + lane; };
+        if (sub > 0) {
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                float *x = box_of(sub) + r * (NI + 2) * 32;
+                x[0] = m[r];
+                x[32] = l[r];
+#pragma unroll
+                for (int i = 0; i < NI; ++i) x[(2 + i) * 32] = acc[r][i];
+            }
+        }
+        __syncthreads();
+        if (sub > 0) return;
+#pragma unroll
+        for (int o = 1; o < KS; ++o)
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                const float *x = box_of(o) + r * (NI + 2) * 32;
+                const float mn = fmaxf(m[r], x[0]);
+                const float mine = mn == -INFINITY ? 1.f : expf(m[r] - mn), theirs = mn == -INFINITY ? 1.f : expf(x[0] - mn);
+                l[r] = l[r] * mine + x[32] * theirs;
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[r][i] = acc[r][i] * mine + x[(2 + i) * 32] * theirs;
+                m[r] = mn;
+            }
+    }
 
     T *out = static_cast<T *>(a.out);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        const int row = row0 + w * RPW + r;
+        const int row = row0 + wr * RPW + r;
         const float sum = warp_sum(l[r]);
         if (row >= a.tq) continue;
         const float inv = sum > 0.f ? 1.f / sum : 0.f;
@@ -287,19 +346,20 @@ __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
 // ---------------------------------------------------------------------------------------------
 // dQ: each block of queries sweeps, in order, the key tiles it sees.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI>
+template <typename T, int RPW, int NI, int KS>
 __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int ROWS = WARPS * RPW;
+    constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
     const int dp = padded_d(a.d), sp = tile_stride(a.d);
     float *qs = smem;                          // [ROWS][dp]
     float *gs = qs + ROWS * dp;                // [ROWS][dp]   dO
-    float *kv = gs + ROWS * dp;                // [2 buffers][K, V][32][sp]
-    float *ps = kv + 4 * TILE * sp;            // [8][32][RPW]  dS
+    float *kv = gs + ROWS * dp;                // [2 buffers][K, V][STEP][sp]
+    float *ps = kv + 4 * STEP * sp;            // [8][32][RPW]  dS
     __shared__ RowSpans rs;
-    __shared__ int pad[2][TILE];
+    __shared__ int pad[2][STEP];
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);
     const int qt = gridDim.x - 1 - blockIdx.x;
     const int h = blockIdx.y, b = blockIdx.z;
     const int hk = h / (a.hq / a.hkv);
@@ -317,9 +377,9 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
     int wlo = a.tk, whi = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        const int row = row0 + w * RPW + r;
-        lo[r] = rs.lo[w * RPW + r];
-        hi[r] = rs.hi[w * RPW + r];
+        const int row = row0 + wr * RPW + r;
+        lo[r] = rs.lo[wr * RPW + r];
+        hi[r] = rs.hi[wr * RPW + r];
         if (hi[r] > lo[r]) { wlo = min(wlo, lo[r]); whi = max(whi, hi[r]); }
         float x = INFINITY, dl = 0.f;
         if (row < a.tq) {
@@ -336,27 +396,28 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
 #pragma unroll
         for (int i = 0; i < NI; ++i) acc[r][i] = 0.f;
     auto stage = [&](int k0, int buf) {
-        stage_rows<T>(kv + (2 * buf) * TILE * sp, sp, a.k, b, hk, k0, TILE, a.tk, a.d, vec);
-        stage_rows<T>(kv + (2 * buf + 1) * TILE * sp, sp, a.v, b, hk, k0, TILE, a.tk, a.d, vec);
-        if (threadIdx.x < TILE) {
+        stage_rows<T>(kv + (2 * buf) * STEP * sp, sp, a.k, b, hk, k0, STEP, a.tk, a.d, vec);
+        stage_rows<T>(kv + (2 * buf + 1) * STEP * sp, sp, a.v, b, hk, k0, STEP, a.tk, a.d, vec);
+        if (threadIdx.x < STEP) {
             const int key = k0 + threadIdx.x;
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
     };
     const int first = kmin / TILE * TILE;
     if (kmax > kmin) stage(first, 0);
-    for (int k0 = first, buf = 0; k0 < kmax; k0 += TILE, buf ^= 1) {
+    for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();
-        if (k0 + TILE < kmax) stage(k0 + TILE, buf ^ 1);
-        if (k0 + TILE <= wlo || k0 >= whi) continue;
-        const float *ks = kv + (2 * buf) * TILE * sp, *vs = ks + TILE * sp;
+        if (k0 + STEP < kmax) stage(k0 + STEP, buf ^ 1);
+        const int t0 = k0 + sub * TILE;
+        if (t0 + TILE <= wlo || t0 >= whi) continue;
+        const float *ks = kv + (2 * buf) * STEP * sp + sub * TILE * sp, *vs = ks + STEP * sp;
 
         float s[RPW], dpv[RPW];
-        dots<RPW>(qs + w * RPW * dp, dp, ks + lane * sp, dp, s);
-        dots<RPW>(gs + w * RPW * dp, dp, vs + lane * sp, dp, dpv);
-        const int key = k0 + lane;
-        const bool open = pad[buf][lane] == 0;
+        dots<RPW>(qs + wr * RPW * dp, dp, ks + lane * sp, dp, s);
+        dots<RPW>(gs + wr * RPW * dp, dp, vs + lane * sp, dp, dpv);
+        const int key = t0 + lane;
+        const bool open = pad[buf][sub * TILE + lane] == 0;
         float *pw = ps + w * TILE * RPW, ds4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
@@ -370,12 +431,13 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
         __syncwarp();
     }
     copies_wait();
+    if constexpr (KS > 1) gather_shares<RPW, NI, KS>(kv, acc);
 
     T *dq = static_cast<T *>(a.dq);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        const int row = row0 + w * RPW + r;
-        if (row >= a.tq) continue;
+        const int row = row0 + wr * RPW + r;
+        if (row >= a.tq || sub > 0) continue;
         const int64_t base = (((int64_t)b * a.tq + row) * a.hq + h) * a.d;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -390,20 +452,21 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
 // dK, dV: each block of keys sweeps, in order, the query heads of its group and the query
 // tiles that see it; a warp owns RPW keys, a lane one query of the tile.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI>
+template <typename T, int RPW, int NI, int KS>
 __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int ROWS = WARPS * RPW;
+    constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
     const int dp = padded_d(a.d), sp = tile_stride(a.d);
     float *ks = smem;                          // [ROWS][dp]
     float *vs = ks + ROWS * dp;                // [ROWS][dp]
-    float *qg = vs + ROWS * dp;                // [2 buffers][Q, dO][32][sp]
-    float *ps = qg + 4 * TILE * sp;            // [8][32][RPW]  P
+    float *qg = vs + ROWS * dp;                // [2 buffers][Q, dO][STEP][sp]
+    float *ps = qg + 4 * STEP * sp;            // [8][32][RPW]  P
     float *ds = ps + WARPS * TILE * RPW;       // [8][32][RPW]  dS
-    __shared__ float lses[2][TILE], deltas[2][TILE];
+    __shared__ float lses[2][STEP], deltas[2][STEP];
     __shared__ int from[32], to[32];           // the queries that see each of the block's keys
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);
     const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
     const int group = a.hq / a.hkv;
     const int key0 = kt * ROWS;
@@ -426,8 +489,8 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
     int wfrom = a.tq, wto = 0;
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        qa[r] = from[w * RPW + r];
-        qb[r] = to[w * RPW + r];
+        qa[r] = from[wr * RPW + r];
+        qb[r] = to[wr * RPW + r];
         if (qb[r] > qa[r]) { wfrom = min(wfrom, qa[r]); wto = max(wto, qb[r]); }
     }
     float acck[RPW][NI], accv[RPW][NI];
@@ -436,33 +499,33 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
 #pragma unroll
         for (int i = 0; i < NI; ++i) { acck[r][i] = 0.f; accv[r][i] = 0.f; }
 
-    const int first = qfirst / TILE * TILE, tiles = qend > qfirst ? (qend - first + TILE - 1) / TILE : 0, steps = tiles * group;
+    const int first = qfirst / TILE * TILE, tiles = qend > qfirst ? (qend - first + STEP - 1) / STEP : 0, steps = tiles * group;
     auto stage = [&](int t, int buf) {
-        const int h = hk * group + t / tiles, q0 = first + t % tiles * TILE;
-        stage_rows<T>(qg + (2 * buf) * TILE * sp, sp, a.q, b, h, q0, TILE, a.tq, a.d, vec);
-        stage_rows<T>(qg + (2 * buf + 1) * TILE * sp, sp, a.dout, b, h, q0, TILE, a.tq, a.d, vec);
-        if (threadIdx.x < 2 * TILE) {
-            const int row = q0 + (threadIdx.x & 31);
+        const int h = hk * group + t / tiles, q0 = first + t % tiles * STEP;
+        stage_rows<T>(qg + (2 * buf) * STEP * sp, sp, a.q, b, h, q0, STEP, a.tq, a.d, vec);
+        stage_rows<T>(qg + (2 * buf + 1) * STEP * sp, sp, a.dout, b, h, q0, STEP, a.tq, a.d, vec);
+        if (threadIdx.x < 2 * STEP) {
+            const int row = q0 + (threadIdx.x & (STEP - 1));
             const bool in = row < a.tq;
             const int64_t at = ((int64_t)b * a.tq + (in ? row : 0)) * a.hq + h;
-            if (threadIdx.x < TILE) copy_async(&lses[buf][threadIdx.x], a.lse + at, in, 0);
-            else copy_async(&deltas[buf][threadIdx.x - TILE], a.delta + at, in, 0);
+            if (threadIdx.x < STEP) copy_async(&lses[buf][threadIdx.x], a.lse + at, in, 0);
+            else copy_async(&deltas[buf][threadIdx.x - STEP], a.delta + at, in, 0);
         }
     };
     if (steps > 0) stage(0, 0);
     for (int t = 0; t < steps; ++t) {
-        const int buf = t & 1, q0 = first + t % tiles * TILE;
+        const int buf = t & 1, q0 = first + t % tiles * STEP + sub * TILE;
         copies_wait();
         __syncthreads();
         if (t + 1 < steps) stage(t + 1, buf ^ 1);
         if (q0 + TILE <= wfrom || q0 >= wto) continue;   // no key of this warp is seen from the tile
-        const float *qs = qg + (2 * buf) * TILE * sp, *gs = qs + TILE * sp;
+        const float *qs = qg + (2 * buf) * STEP * sp + sub * TILE * sp, *gs = qs + STEP * sp;
 
         float s[RPW], dpv[RPW];
-        dots<RPW>(ks + w * RPW * dp, dp, qs + lane * sp, dp, s);
-        dots<RPW>(vs + w * RPW * dp, dp, gs + lane * sp, dp, dpv);
+        dots<RPW>(ks + wr * RPW * dp, dp, qs + lane * sp, dp, s);
+        dots<RPW>(vs + wr * RPW * dp, dp, gs + lane * sp, dp, dpv);
         const int row = q0 + lane;
-        const float x = lses[buf][lane], lse = x == -INFINITY ? INFINITY : x, delta = deltas[buf][lane];
+        const float x = lses[buf][sub * TILE + lane], lse = x == -INFINITY ? INFINITY : x, delta = deltas[buf][sub * TILE + lane];
         float *pw = ps + w * TILE * RPW, *dw = ds + w * TILE * RPW, ps4[RPW], ds4[RPW];
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
@@ -479,12 +542,16 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
         __syncwarp();
     }
     copies_wait();
+    if constexpr (KS > 1) {
+        gather_shares<RPW, NI, KS>(qg, acck);
+        gather_shares<RPW, NI, KS>(qg, accv);
+    }
 
     T *dk = static_cast<T *>(a.dk), *dv = static_cast<T *>(a.dv);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        const int key = key0 + w * RPW + r;
-        if (key >= a.tk) continue;
+        const int key = key0 + wr * RPW + r;
+        if (key >= a.tk || sub > 0) continue;
         const int64_t base = (((int64_t)b * a.tk + key) * a.hkv + hk) * a.d;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -509,8 +576,12 @@ static bool rows_readable(const View4 &v, int d) {
 }
 
 // `own`: tensors whose rows the block keeps; `probs`: arrays of a tile's weights.
+// SHARED_ROWS in the place of the rows per warp: two rows a warp, and each pair of rows two warps' (KS 2).
+constexpr int SHARED_ROWS = 0;
+static int block_rows(int rpw) { return rpw == SHARED_ROWS ? WARPS : WARPS * rpw; }
 static size_t generic_smem(int d, int rpw, int own, int probs) {
-    return sizeof(float) * ((size_t)own * WARPS * rpw * padded_d(d) + 4 * TILE * tile_stride(d) + (size_t)probs * WARPS * TILE * rpw);
+    const int each = rpw == SHARED_ROWS ? 2 : rpw, ks = rpw == SHARED_ROWS ? 2 : 1;
+    return sizeof(float) * ((size_t)own * block_rows(rpw) * padded_d(d) + 4 * ks * TILE * tile_stride(d) + (size_t)probs * WARPS * TILE * each);
 }
 
 // Rows per warp: the fewest of one, two and four whose blocks all run at once - as many to a multiprocessor as its shared
@@ -525,8 +596,9 @@ static size_t generic_smem(int d, int rpw, int own, int probs) {
 constexpr int64_t SMEM_PER_SM = 228 * 1024, SMEM_BESIDE = 2 * 1024;
 static int rows_per_warp(int64_t rows, int64_t heads, int d, int own, int probs) {
     for (int rpw = 1; rpw < 4; rpw *= 2) {
-        const int64_t blocks = (rows + WARPS * rpw - 1) / (WARPS * rpw) * heads, fit = SMEM_PER_SM / ((int64_t)generic_smem(d, rpw, own, probs) + SMEM_BESIDE);
-        if (blocks <= std::min<int64_t>(148 * fit, 370)) return rpw;
+        const int64_t blocks = (rows + WARPS * rpw - 1) / (WARPS * rpw) * heads;
+        auto fit = [&](int r) { return SMEM_PER_SM / ((int64_t)generic_smem(d, r, own, probs) + SMEM_BESIDE); };
+        if (blocks <= std::min<int64_t>(148 * fit(rpw), 370)) return rpw == 1 && d <= 128 && blocks <= 148 * fit(SHARED_ROWS) ? SHARED_ROWS : rpw;
     }
     return 4;
 }
@@ -539,13 +611,14 @@ static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, 
 }
 // The instance for the rows per warp and the head dimension.
 #define GENERIC_PICK(kernel, T, rpw, d)                                                                    \
-    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2> : (d) <= 128 ? kernel<T, 4, 4> : kernel<T, 4, 8>)           \
-     : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2> : (d) <= 128 ? kernel<T, 2, 4> : kernel<T, 2, 8>)         \
-                : ((d) <= 64 ? kernel<T, 1, 2> : (d) <= 128 ? kernel<T, 1, 4> : kernel<T, 1, 8>))
+    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2, 1> : (d) <= 128 ? kernel<T, 4, 4, 1> : kernel<T, 4, 8, 1>)  \
+     : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2, 1> : (d) <= 128 ? kernel<T, 2, 4, 1> : kernel<T, 2, 8, 1>) \
+     : (rpw) == 1 ? ((d) <= 64 ? kernel<T, 1, 2, 1> : (d) <= 128 ? kernel<T, 1, 4, 1> : kernel<T, 1, 8, 1>) \
+                : ((d) <= 64 ? kernel<T, 2, 2, 2> : kernel<T, 2, 4, 2>))
 
 template <typename T>
 static cudaError_t forward_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
-    const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 1, 1), rows = WARPS * rpw;
+    const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 1, 1), rows = block_rows(rpw);
     const bool vec = rows_readable<T>(a.q, a.d) && rows_readable<T>(a.k, a.d) && rows_readable<T>(a.v, a.d);
     *launches += 1;
     return launch_generic(GENERIC_PICK(generic_forward_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 1, 1), stream,
@@ -564,7 +637,7 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     {
-        const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b, a.d, 2, 2), rows = WARPS * rpw;
+        const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b, a.d, 2, 2), rows = block_rows(rpw);
         *launches += 1;
         e = launch_generic(GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3((a.tk + rows - 1) / rows, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
                            false, a, vec);
@@ -572,7 +645,7 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
     }
     {   // beside dkdv.  (dkdv itself brought in under delta's end, to wait there, made the whole twice as slow: 1000 tokens, 4 / 2
         // heads of 64 327 against 213 us.)
-        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), rows = WARPS * rpw;
+        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), rows = block_rows(rpw);
         *launches += 1;
         return launch_generic(GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
                               true, a, vec);
