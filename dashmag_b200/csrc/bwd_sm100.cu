@@ -66,26 +66,32 @@ template <bool POLY> __device__ __forceinline__ float exp2_mixed(float x) { retu
 // instructions for one (measured on config 2: 35 us of 1 370 slower with a quarter as cubics).
 template <typename T> constexpr int poly_of4() { return Pack<T>::FMT == 1 ? 1 : 0; }
 
-// `groups` x 32 f32 accumulator columns of this thread's TMEM lane, scaled, rounded and stored as
-// contiguous elements of the row.
-template <typename T>
-__device__ __forceinline__ void store_acc_cols(uint32_t taddr, T *dst, float scale, bool write, int groups) {
+// 32 f32 accumulator columns of this thread's TMEM lane - plus `theirs`, four to a 16-byte word, STRIDE words apart -
+// scaled, rounded and stored as contiguous elements of the row.
+template <typename T, int STRIDE>
+__device__ __forceinline__ void store_acc_cols(uint32_t taddr, T *dst, float scale, bool write, const uint4 *theirs) {
+    uint32_t o[32];
+    tmem_ld32(taddr, o);
+    tmem_ld_wait();
+    if (theirs) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        if (c >= groups) break;
-        uint32_t o[32];
-        tmem_ld32(taddr + c * 32, o);
-        tmem_ld_wait();
-        if (write) {
+        for (int e = 0; e < 8; ++e) {
+            const uint4 x = theirs[e * STRIDE];
+            o[4 * e + 0] = __float_as_uint(__uint_as_float(o[4 * e + 0]) + __uint_as_float(x.x));
+            o[4 * e + 1] = __float_as_uint(__uint_as_float(o[4 * e + 1]) + __uint_as_float(x.y));
+            o[4 * e + 2] = __float_as_uint(__uint_as_float(o[4 * e + 2]) + __uint_as_float(x.z));
+            o[4 * e + 3] = __float_as_uint(__uint_as_float(o[4 * e + 3]) + __uint_as_float(x.w));
+        }
+    }
+    if (write) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                uint4 v;
-                v.x = Pack<T>::two(__uint_as_float(o[8 * e + 0]) * scale, __uint_as_float(o[8 * e + 1]) * scale);
-                v.y = Pack<T>::two(__uint_as_float(o[8 * e + 2]) * scale, __uint_as_float(o[8 * e + 3]) * scale);
-                v.z = Pack<T>::two(__uint_as_float(o[8 * e + 4]) * scale, __uint_as_float(o[8 * e + 5]) * scale);
-                v.w = Pack<T>::two(__uint_as_float(o[8 * e + 6]) * scale, __uint_as_float(o[8 * e + 7]) * scale);
-                reinterpret_cast<uint4 *>(dst)[c * 4 + e] = v;
-            }
+        for (int e = 0; e < 4; ++e) {
+            uint4 v;
+            v.x = Pack<T>::two(__uint_as_float(o[8 * e + 0]) * scale, __uint_as_float(o[8 * e + 1]) * scale);
+            v.y = Pack<T>::two(__uint_as_float(o[8 * e + 2]) * scale, __uint_as_float(o[8 * e + 3]) * scale);
+            v.z = Pack<T>::two(__uint_as_float(o[8 * e + 4]) * scale, __uint_as_float(o[8 * e + 5]) * scale);
+            v.w = Pack<T>::two(__uint_as_float(o[8 * e + 6]) * scale, __uint_as_float(o[8 * e + 7]) * scale);
+            reinterpret_cast<uint4 *>(dst)[e] = v;
         }
     }
 }
@@ -228,6 +234,7 @@ template <bool FUSED> struct DkdvTail {
     QAux aux[2];
     uint32_t tmem_base;
     unsigned int abort;
+    uint32_t share_whole[4 * KCG];   // PAIR: whether the second block's warp got through its sweep (written by that block)
     int cu_q[cu_cache<FUSED>()], cu_k[cu_cache<FUSED>()];   // the packed sequences' offsets, when they fit
 };
 
@@ -243,7 +250,8 @@ template <int HD, bool FUSED> constexpr size_t smem_dkdv() {
                  : 1024 + 6 * tile_bytes<HD>() + dkdv_tail<false>();
 }
 
-template <typename T, int HD, bool FUSED>
+// PAIR: a cluster of two blocks a unit, each half of the unit's steps (bwd_sm100_pairs says which calls).
+template <typename T, int HD, bool FUSED, bool PAIR>
 __global__ void __launch_bounds__(FUSED ? KTHREADS_FUSED : KTHREADS, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -308,7 +316,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // Units are taken in the order the plan kernel left (without one: in index order, the heads of a
     // key block side by side).
     const int nkb = (a.tk + BIG - 1) / BIG;
-    const int unit = a.order ? a.order[blockIdx.x] : (int)blockIdx.x;
+    const int at = PAIR ? blockIdx.x >> 1 : blockIdx.x, share = PAIR ? (int)cluster_rank() : 0;
+    const int unit = a.order ? a.order[at] : at;
     const int item = unit / a.hkv, hk = unit - item * a.hkv;
     const int b = item / nkb, kt = item - b * nkb;
     const int group = a.hq / a.hkv;
@@ -350,13 +359,14 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     // A streamed tile of 128 rows: `qt` tokens of 1 << pack heads of the group, row = token << pack | head.
     const int pack = a.pack, qt = QS >> pack;
     const int tiles = (!aborted && any_open && qend > qfirst) ? (qend - qfirst + qt - 1) / qt : 0;
-    const int steps = tiles * (group >> pack);
+    const int all_steps = tiles * (group >> pack), first_share = PAIR ? (all_steps + 1) / 2 : all_steps;
+    const int from = share == 0 ? 0 : first_share, steps = share == 0 ? first_share : all_steps - first_share;
     // The last queries first: under causality a key's weights fall with the query, and an accumulator that took the large
     // terms first would round off a little of itself - always towards zero - with each of the small ones after them.  (dv of the
     // first 128 keys of 32768 tokens, 8 / 1 heads, f16, against 64 bits: off by 6.1e-4 from the first query on, 2.9e-4 from the
     // last, the rounding of P and of the result.  One head after the other from its first query on: 4.4e-4.)
-    auto step_head = [&](int t) { return hk * group + ((t / tiles) << pack); };
-    auto step_q0 = [&](int t) { return qfirst + (tiles - 1 - t % tiles) * qt; };
+    auto step_head = [&](int t) { return hk * group + (((from + t) / tiles) << pack); };
+    auto step_q0 = [&](int t) { return qfirst + (tiles - 1 - (from + t) % tiles) * qt; };
     bool failed = aborted;
     // TMEM columns: S^T at 0, dP^T at 128 (each with its 16-bit twin over the first half of every
     // group of 32 columns: columns 32 g + [0, 16) hold queries 32 g + [0, 32)), dV at 256, dK at 384.
@@ -684,25 +694,58 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 }
             }
         }
-        // ---------------- epilogue: 32 columns of the row per thread (HD = 64: the first two of the four warps of a quadrant) ----------------
-        constexpr int EC = 32;
-        const bool mine = cg < HD / EC;
-        T *dk = static_cast<T *>(a.dk) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + cg * EC;
-        T *dv = static_cast<T *>(a.dv) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + cg * EC;
-        if (steps == 0 || failed) {
+        if (steps > 0 && !failed && !__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.acc_ready), 0))) failed = true;   // the sums are complete
+    }
+    constexpr int EC = 32;   // columns of a row per elementwise thread (HD = 64: the first two of the four warps of a quadrant)
+    constexpr int EW_THREADS = 128 * (HD / EC);   // threads with columns of their own
+    const bool ew = warp >= 2 && warp < 2 + 4 * KCG;
+    const int ecg = (warp - 2) >> 2, key = k0 + 32 * (warp & 3) + lane;
+    const uint32_t t_sums = tmem + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + ecg * EC;
+    const bool mine = ew && ecg < HD / EC;
+    if constexpr (PAIR) {
+        // The second block's f32 sums go into the first one's shared memory, whose tiles are dead once both have got here: thread by
+        // thread, 16 bytes apart, so that a warp's stores are contiguous.  With each warp's share goes whether it is whole: where a
+        // wait of the second block ran out (or it found the status raised) the first stores nothing either.  Every thread of
+        // both blocks passes both meetings.
+        __syncwarp();
+        cluster_sync();
+        if (share == 1 && ew) {
+            if (lane == 0) cluster_store1(cluster_map(smem_u32(&sh.share_whole[warp - 2]), 0), failed ? 0u : 1u);
+            if (steps > 0 && mine) {
+                tc_fence_after_sync();
+                const uint32_t to = cluster_map(smem_u32(smem), 0) + (uint32_t)(threadIdx.x - 64) * 16;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(t_sums + (c == 0 ? COL_DV : COL_DK), o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        cluster_store4(to + (uint32_t)((c * 8 + e) * EW_THREADS * 16), o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+                }
+                tc_fence_before_sync();
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+    }
+    if (share == 0 && ew) {
+        // ---------------- epilogue ----------------
+        const bool shared_sweep = PAIR && all_steps > first_share;   // the second block had steps
+        if (shared_sweep && sh.share_whole[warp - 2] == 0) failed = true;
+        T *dk = static_cast<T *>(a.dk) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + ecg * EC;
+        T *dv = static_cast<T *>(a.dv) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + ecg * EC;
+        if (steps == 0) {
             if (key < a.tk && !failed && mine) {
                 store_zero_cols<T, EC / 8>(dk);
                 store_zero_cols<T, EC / 8>(dv);
             }
-        } else if (__all_sync(0xffffffffu, mbar_wait(BAR(sh.bar.acc_ready), 0))) {
+        } else if (!failed && mine) {
             tc_fence_after_sync();
-            if (mine) {
-                store_acc_cols<T>(t_lane + COL_DV + cg * EC, dv, 1.f, key < a.tk, 1);
-                store_acc_cols<T>(t_lane + COL_DK + cg * EC, dk, a.scale, key < a.tk, 1);
-            }
+            const uint4 *theirs = shared_sweep ? reinterpret_cast<const uint4 *>(smem) + (threadIdx.x - 64) : nullptr;
+            store_acc_cols<T, EW_THREADS>(t_sums + COL_DV, dv, 1.f, key < a.tk, theirs);
+            store_acc_cols<T, EW_THREADS>(t_sums + COL_DK, dk, a.scale, key < a.tk, theirs ? theirs + 8 * EW_THREADS : nullptr);
             tc_fence_before_sync();
-        } else {
-            failed = true;
         }
     }
 
@@ -1074,16 +1117,16 @@ __global__ void __launch_bounds__(256) bwd_dq_finish_kernel(const float *__restr
 }
 
 // -------------------------------------------------------------------------------------------------
-template <typename T, int HD, bool FUSED>
+template <typename T, int HD, bool FUSED, bool PAIR>
 static cudaError_t launch_dkdv(const Sm100BwdMaps &m, const Sm100BwdArgs &a, long long items, cudaStream_t stream) {
     constexpr size_t smem = smem_dkdv<HD, FUSED>();
-    cudaError_t e = cudaFuncSetAttribute(bwd_dkdv_sm100_kernel<T, HD, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const auto kernel = bwd_dkdv_sm100_kernel<T, HD, FUSED, PAIR>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 gk((unsigned)(items * a.hkv), 1, 1);
+    dim3 gk((unsigned)(items * a.hkv * (PAIR ? 2 : 1)), 1, 1);
     // Under delta's end (4 packed sequences, 2149 tokens, 16 / 4 heads, forward and backward: 104.3 -> 98.2 us with the plan left out
     // too; 9 sequences, 1047 tokens, 48.3 -> 43.2; 10 padded ones of 224, 12 / 4 heads, 53.4 -> 49.0); the fused form behind the memset.
-    return launch_beside(bwd_dkdv_sm100_kernel<T, HD, FUSED>, gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream, !FUSED, m.k128, m.v128, m.q128,
-                         m.do128, m.dq_acc, a);
+    return launch_clusters(kernel, gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream, !FUSED, PAIR ? 2u : 1u, m.k128, m.v128, m.q128, m.do128, m.dq_acc, a);
 }
 
 template <typename T, int HD>
@@ -1097,7 +1140,9 @@ static cudaError_t launch_t(const Sm100BwdMaps &m, Sm100BwdArgs a, cudaStream_t 
     }
     const long long items = (long long)a.b * ((a.tk + BIG - 1) / BIG);
     if (items * a.hkv > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    e = fused ? launch_dkdv<T, HD, true>(m, a, items, stream) : launch_dkdv<T, HD, false>(m, a, items, stream);
+    e = fused ? launch_dkdv<T, HD, true, false>(m, a, items, stream)
+        : a.pairs ? launch_dkdv<T, HD, false, true>(m, a, items, stream)
+                  : launch_dkdv<T, HD, false, false>(m, a, items, stream);
     *launches += 1;
     if (e != cudaSuccess) return e;
     if (!fused) {

@@ -225,18 +225,29 @@ __device__ __forceinline__ void end_beside() {
 __device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
-inline cudaError_t launch_beside(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool beside, A... args) {
+inline cudaError_t launch_clusters(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool beside, unsigned cluster, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    if (beside) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = beside ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_beside(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool beside, A... args) {
+    return launch_clusters(kernel, grid, threads, smem, stream, beside, 1u, args...);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -244,6 +244,23 @@ static size_t split_bytes(const dash_attn_params *p, int splits) {
 size_t sm100_forward_workspace(const dash_attn_params *p, bool any_size) {
     return parameters_taken(p, 0, any_size) ? split_bytes(p, forward_splits(p)) : 0;   // a call the generic kernels take is not split
 }
+// Whether two blocks share each unit (128 keys of a key-value head) of the key and value gradients, half its steps each (D 64 and
+// 128; D 256 has a rule of its own).  A unit sweeps the queries of all heads of its group that see it, and with few units the
+// longest sweep is the kernel's length; with two blocks to a unit it is half that, a second set-up and the meeting of the two.  The
+// rule looks at no number of heads, so that a head slice of a packed batch keeps the whole call's bits: key blocks so few that
+// with eight key-value heads (one, where groups are of eight) twice the units still start at once, and sweeps of five steps of
+// 128 rows or more.  Backward, one block | two (us): 500 tokens, 16 / 4 heads of 128, 36.7 | 28.4, 32 / 8 37.6 | 29.4; 1000 in four,
+// 32 / 8, 39.1 | 33.8, 16 / 8 24.3 | 24.4; 1152, 24 / 8, 56.6 | 43.9; 8 / 1: 500 62.8 | 41.7, 4700 in two 350 | 188; heads
+// of 64 the same.  Beyond it, 2420 tokens in three, 32 / 8 of 64, 152 units: 117 | 125.
+static bool backward_pairs(const dash_attn_params *p) {
+    if (p->d != 64 && p->d != 128) return false;
+    const int64_t blocks = (int64_t)p->b * ((p->tk + 127) / 128), group = p->hq / p->hkv;
+    const int64_t none = (int64_t)p->tq + p->tk + 1;
+    int64_t queries = p->mask_kind == DASH_ATTN_MASK_PACKED ? p->tq / std::max(p->cu_seqlens_q_len - 1, 1) : p->tq;
+    if (p->has_window && p->window_left >= 0 && p->window_left < none && (p->causal || (p->window_right >= 0 && p->window_right < none)))
+        queries = std::min(queries, p->window_left + (p->causal ? 0 : p->window_right) + 128);
+    return queries * group >= 5 * 128 && group >= 2 && blocks <= (group >= 8 ? 37 : 9);
+}
 // Whether the caller lets dQ be summed in any order, where a form exists that makes use of it (D 64, 128).
 static bool order_is_free(const dash_attn_params *p) { return !p->deterministic && (p->d == 128 || p->d == 64); }
 // Whether such a call does take that form, five products with dQ added by reductions in L2.  It shares the scores but not its
@@ -253,7 +270,7 @@ static bool order_is_free(const dash_attn_params *p) { return !p->deterministic 
 // 3072 units, 596 | 378.  D 128 packed, 1000 to 30000 tokens, 60 to 99.7 % of the speed; padded, 8 of 500, 12 / 12, 384 units,
 // 77 | 81, 16 of 1000, 12 / 4, 512 units, 309 | 293, 32 of 1000, 1024 units, 603 | 507.
 static bool fused_backward(const dash_attn_params *p) {
-    if (!order_is_free(p)) return false;
+    if (!order_is_free(p) || backward_pairs(p)) return false;
     const int64_t units = (int64_t)p->b * ((p->tk + 127) / 128) * p->hkv;
     const bool packed = p->mask_kind == DASH_ATTN_MASK_PACKED;
     return p->d == 64 ? units >= (packed ? 240 : 90) : !packed && units >= 500;
@@ -337,6 +354,7 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
     f.order = static_cast<int *>(workspace);
     f.dq_acc = dq_acc;
     f.pack = pack;
+    f.pairs = backward_pairs(p) ? 1 : 0;
     // The plan's one block and delta run side by side; then dkdv, and dq beside its last waves (neither reads what
     // the other writes).
     cudaError_t e = launch_bwd_plan(f, p->d == 256 ? 37 : 148, stream, launches);

@@ -43,6 +43,7 @@ struct Sm100BwdArgs {
     int *order;          // scratch: the (key block, key-value head) units in launch order, [B * ceil(Tk / 128) * Hkv]
     float *dq_acc;       // scratch [B,Tq,Hq,D] f32, or null: the query gradient summed by reductions in L2 (the fused form)
     int pack;            // a tile of 128 query rows is 128 >> pack tokens of 1 << pack heads of one group
+    int pairs;           // D 64, 128, fixed order: two blocks share a unit of dkdv
 };
 
 // Tensor maps of the backward: every tensor with boxes of 128 rows, resident or streamed.

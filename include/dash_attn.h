@@ -116,8 +116,9 @@ typedef struct dash_attn_decode_params {
  * a call of few queries against many keys takes longer).  Whether keys are split depends on the whole
  * call, its batch and heads among it, and a split sums in another order: a sequence or a head computed
  * alone can differ in its last bits from the same one in a larger call (packed batches and calls
- * without scratch are never split).  So can key and value gradients at head dimension 256, where a
- * small call's units are shared between two blocks.  The same call gives the same bits on every run. */
+ * without scratch are never split).  So can key and value gradients where a small call's units
+ * are shared between two blocks (at head dimension 256 by the units' number; at 64 and 128 by the batch's key blocks
+ * and the length of their sweeps, whatever the number of heads).  The same call gives the same bits on every run. */
 size_t dash_attn_forward_workspace(const dash_attn_params *p);
 size_t dash_attn_backward_workspace(const dash_attn_params *p);
 size_t dash_attn_decode_workspace(const dash_attn_decode_params *p);
