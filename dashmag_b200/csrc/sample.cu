@@ -319,6 +319,60 @@ __device__ uint32_t radix_threshold(Each each, const SampleArgs &a, float m, uin
     return prefix;
 }
 
+// The same over a block's own tokens whose keys lie within NARROW of `base` (those below it do not count: `base` is a lower bound
+// of the threshold): every key a bin of its own, one pass and one scan from the top where the radix search takes one for each
+// byte.  64 x 151936 bf16 logits, k = 50, p = 0.9: 28.5 -> 25.7 us on the device; 2 x 7631 14.6 -> 12.1.
+constexpr uint32_t NARROW = ST;
+template <typename T, bool MASS, typename Each>
+__device__ uint32_t narrow_threshold(Each each, const SampleArgs &a, float m, uint32_t base, uint32_t floor_key, RadixSmem &sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t *cnt = &sm.cnt[0][0][0];
+    auto mass = [&](int piece) { return &sm.mass[piece][0][0][0]; };
+    unsigned long long *warp_mass = sm.tmass[0];
+    uint32_t *warp_cnt = sm.tcnt[0];
+    __syncthreads();   // the bins of the search before are read
+    cnt[threadIdx.x] = 0;
+    if (MASS) { mass(0)[threadIdx.x] = 0; mass(1)[threadIdx.x] = 0; mass(2)[threadIdx.x] = 0; }
+    if (threadIdx.x == 0) sm.sel = base;
+    __syncthreads();
+    each([&](int, T zi, bool) {
+        const uint32_t key = Key<T>::of(zi);
+        if (key < base || key < floor_key) return;
+        const uint32_t d = min(key - base, NARROW - 1);
+        if (MASS) {
+            const unsigned long long w = __float2ull_rn(expf(__fmul_rn(Num<T>::to_f32(zi) - m, a.tau)) * MASS_ONE);
+            if (w == 0) return;
+            atomicAdd(&mass(0)[d], (uint32_t)(w & 0x3fffu));
+            if (w >> 14) atomicAdd(&mass(1)[d], (uint32_t)((w >> 14) & 0x3fffu));
+            if (w >> 28) atomicAdd(&mass(2)[d], (uint32_t)(w >> 28));
+        }
+        atomicAdd(&cnt[d], 1u);
+    });
+    __syncthreads();
+    const uint32_t d = NARROW - 1 - threadIdx.x, own = cnt[d];   // the highest key first
+    const unsigned long long own_mass = MASS ? (unsigned long long)mass(0)[d] + ((unsigned long long)mass(1)[d] << 14) + ((unsigned long long)mass(2)[d] << 28) : 0ull;
+    uint32_t c = own;
+    unsigned long long w = own_mass;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t cu = __shfl_up_sync(0xffffffffu, c, o);
+        const unsigned long long wu = MASS ? __shfl_up_sync(0xffffffffu, w, o) : 0ull;
+        if (lane >= o) { c += cu; w += wu; }
+    }
+    if (lane == 31) { warp_cnt[warp] = c; warp_mass[warp] = w; }
+    __syncthreads();
+    unsigned long long total = 0;
+    for (int i = 0; i < ST / 32; ++i) {
+        if (i < warp) { c += warp_cnt[i]; if (MASS) w += warp_mass[i]; }
+        if (MASS) total += warp_mass[i];
+    }
+    const unsigned long long target = MASS ? __double2ull_ru((double)a.p * (double)total) : 0ull;
+    auto reached = [&](uint32_t n, unsigned long long x) { return MASS ? x >= target && n >= 1u : n >= (uint32_t)a.top_k; };
+    if (reached(c, w) && !reached(c - own, w - own_mass)) sm.sel = base + d;   // one thread's
+    __syncthreads();
+    return sm.sel;
+}
+
 // The tokens above a bound of top-k's threshold: their ids and the bits of their logits.
 constexpr int LIST_MAX = 8192;   // per block
 struct TokenList {
@@ -478,8 +532,14 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
         uint32_t reaching = 0;
         if (listed) {
             auto each_listed = [&](auto f) { for (int j = threadIdx.x; j < n_listed; j += ST) f((int)list.id[j], from_bits<T>(list.bits[j]), false); };
-            t_keep = radix_threshold<T, false, 1>(each_listed, a, m, 0u, radix, 1, 0, reaching);
-            if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 1>(each_listed, a, m, t_keep, radix, 1, 0, reaching));
+            const uint32_t base = max(bound, key_ninf + 1);
+            if (Key<T>::BITS == 16 && Key<T>::of(Num<T>::from_f32(m)) - base < NARROW - 1) {
+                t_keep = narrow_threshold<T, false>(each_listed, a, m, base, 0u, radix);
+                if (a.has_p) t_keep = max(t_keep, narrow_threshold<T, true>(each_listed, a, m, base, t_keep, radix));
+            } else {
+                t_keep = radix_threshold<T, false, 1>(each_listed, a, m, 0u, radix, 1, 0, reaching);
+                if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 1>(each_listed, a, m, t_keep, radix, 1, 0, reaching));
+            }
         } else {
             if (a.top_k > 0) t_keep = radix_threshold<T, false, 8>(each_logit, a, m, 0u, radix, blocks, 0, reaching);
             if (a.has_p) t_keep = max(t_keep, radix_threshold<T, true, 8>(each_logit, a, m, t_keep, radix, blocks, 0, reaching));
