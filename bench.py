@@ -492,7 +492,7 @@ def main():
     if _lib.probe("atomic_runs") > a0:
         atf = w["bwd_flops"] / (ra["bwd_ms"] * 1e-3) / 1e12
         atomic_leg = {"ms": ra["bwd_ms"], "tflops": atf, "spread_ms": ra["bwd_spread_ms"],
-                      "roofline": tensor_roofline(atf / world, "backward pass with the query gradient added by atomics: five products", "bwd_atomic")}
+                      "roofline": tensor_roofline(atf / world, "backward pass with the order of the query gradient's sums left free", "bwd_atomic")}
     del wa
 
     # ---- end to end through the public API: host buffers in, results back to the host, every step ----
