@@ -48,6 +48,17 @@ struct Ref {   // an owned reference
     Ref &operator=(const Ref &) = delete;
 };
 
+// The call into the library without the interpreter's lock, as ctypes makes it: a launch may wait for room in the GPU's queue.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
+template <typename... P, typename... A> int unlocked(int (*call)(P...), A... args) {
+    Unlocked u;
+    return call(args...);
+}
+
 PyObject *nothing_done() {
     PyErr_Clear();
     Py_RETURN_NONE;
@@ -208,7 +219,7 @@ PyObject *forward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type()), lse = fresh(q->sizes().slice(0, 3), *q, at::kFloat);
     const size_t need = lib.forward_workspace(&p);
     at::Tensor ws = scratch(need, *q);
-    const int rc = lib.forward(&p, pointer(*q), pointer(*k), pointer(*v), pointer(out), static_cast<float *>(pointer(lse)),
+    const int rc = unlocked(lib.forward, &p, pointer(*q), pointer(*k), pointer(*v), pointer(out), static_cast<float *>(pointer(lse)),
                                      need ? ws.data_ptr() : nullptr, need, stream_of(*q));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({out, lse});
@@ -232,7 +243,7 @@ PyObject *backward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor dq = fresh(q->sizes(), *q, q->scalar_type()), dk = fresh(k->sizes(), *q, q->scalar_type()), dv = fresh(v->sizes(), *q, q->scalar_type());
     const size_t need = lib.backward_workspace(&p);
     at::Tensor ws = scratch(need, *q);
-    const int rc = lib.backward(&p, pointer(*q), pointer(*k), pointer(*v), pointer(*o), static_cast<const float *>(pointer(*lse)), pointer(*g),
+    const int rc = unlocked(lib.backward, &p, pointer(*q), pointer(*k), pointer(*v), pointer(*o), static_cast<const float *>(pointer(*lse)), pointer(*g),
                                       pointer(dq), pointer(dk), pointer(dv), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({dq, dk, dv});
@@ -280,7 +291,7 @@ PyObject *decode(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
     const size_t need = lib.decode_workspace(&p);
     at::Tensor ws = scratch(need, *q);
-    const int rc = lib.decode(&p, pointer(*q), pointer(*k), pointer(*v), pointer(out), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    const int rc = unlocked(lib.decode, &p, pointer(*q), pointer(*k), pointer(*v), pointer(out), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -296,7 +307,7 @@ PyObject *decode_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
     const size_t need = lib.decode_workspace(&p);
     at::Tensor ws = scratch(need, *q);
-    const int rc = lib.decode_append(&p, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
+    const int rc = unlocked(lib.decode_append, &p, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
                                            need ? ws.data_ptr() : nullptr, need, stream_of(*q));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
@@ -332,7 +343,7 @@ PyObject *decode_append_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
     const size_t need = lib.decode_append_rope_workspace(&p);
     at::Tensor ws = scratch(need, *q);
-    const int rc = lib.decode_append_rope(&p, &r, nullptr, 0, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
+    const int rc = unlocked(lib.decode_append_rope, &p, &r, nullptr, 0, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
                                                 need ? ws.data_ptr() : nullptr, need, stream_of(*q));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
@@ -370,7 +381,7 @@ PyObject *sample(PyObject *, PyObject *const *args, Py_ssize_t n) {
     at::Tensor logprob = fresh({p.b}, *z, at::kFloat), tempered = fresh({p.b}, *z, at::kFloat), sampling = fresh({p.b}, *z, at::kFloat);
     const size_t need = lib.sample_workspace(&p);
     at::Tensor ws = scratch(need, *z);
-    const int rc = lib.sample(&p, pointer(*z), pointer(tokens), static_cast<float *>(pointer(logprob)), static_cast<float *>(pointer(tempered)),
+    const int rc = unlocked(lib.sample, &p, pointer(*z), pointer(tokens), static_cast<float *>(pointer(logprob)), static_cast<float *>(pointer(tempered)),
                                static_cast<float *>(pointer(sampling)), need ? ws.data_ptr() : nullptr, need, stream_of(*z));
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({tokens, logprob, tempered, sampling});
