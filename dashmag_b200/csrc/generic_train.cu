@@ -256,7 +256,9 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
             const bool vis = open && key >= lo[r] && key < hi[r];
             const float sr = vis ? s[r] * a.scale : -INFINITY;
             const float mn = fmaxf(m[r], warp_max(sr));
-            float p = 0.f, alpha = 1.f;
+            // No maximum yet: the weights are zero, but for a NaN - no maximum shows it, and it is a NaN of the row whatever else the
+            // row sees, in this warp's tiles or in another's.
+            float p = sr == sr ? 0.f : sr, alpha = 1.f;
             if (mn != -INFINITY) {
                 alpha = expf(m[r] - mn);  // exp(-inf) = 0 on the first visible tile
                 p = expf(sr - mn);
