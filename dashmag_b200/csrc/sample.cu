@@ -466,7 +466,8 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     };
     if (tempered_differs) sums(std::true_type{});
     else sums(std::false_type{});
-    if (LIST && degenerate) each_open([&](int i, T zi) { if (Num<T>::to_f32(zi) == m) first = min(first, i); });
+    // (By the id alone: of logits that are all NaN none compares with the maximum.)
+    if (degenerate) each_open([&](int i, T) { first = min(first, i); });
     // The sums, and what the blocks have listed, in one meeting.
     s1 = block_reduce(s1, AddOp(), fs);
     if (tempered_differs) wu = block_reduce(wu, AddOp(), fs);

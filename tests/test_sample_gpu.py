@@ -2,6 +2,8 @@
 crates/dash-ops/tests/sample.rs holds the reference's kernel to it: the same tokens, the three
 log-probabilities within KERNEL_REFERENCE = 4e-6, identities and repeats bit for bit, draws that
 follow the kept set's distribution."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -106,6 +108,22 @@ def test_a_row_without_a_finite_logit():
     z[0, 5] = -np.inf   # a token the model rules out is never drawn
     for offset in range(20):
         assert 5 not in run(np.tile(z[:1], (32, 1)), "f32", SampleOptions(seed=3, offset=offset))[0]
+
+
+@pytest.mark.parametrize("b,v,dtype", [(3, 40, "f32"), (2, 40001, "bf16"), (160, 9000, "f16")])
+@pytest.mark.parametrize("options", [SampleOptions.greedy(), SampleOptions(), SampleOptions(temperature=0.7, top_p=0.9), SampleOptions(top_k=20, top_p=0.9)], ids=str)
+def test_a_row_of_nan(b, v, dtype, options):
+    """No logit compares with anything: the lowest id that is not ruled out, NaN for its log-probabilities."""
+    z = logits_of(b, v, dtype, 5)
+    for row in (0, b - 1):
+        z[row] = np.nan
+        z[row, 7] = -np.inf
+    z[b - 1, 7] = np.nan
+    for masked in ((), (0, 1)):
+        t, lp, tp, sp = run(z, dtype, dataclasses.replace(options, masked=masked))
+        for row in (0, b - 1):
+            assert t[row] == len(masked) and np.isnan([lp[row], tp[row], sp[row]]).all()
+        assert ((0 <= t) & (t < v)).all() and np.isfinite(np.delete(lp, [0, b - 1])).all()
 
 
 @pytest.mark.parametrize("name,options,kept", [
