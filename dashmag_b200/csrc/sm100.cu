@@ -261,16 +261,15 @@ static bool backward_pairs(const dash_attn_params *p) {
         queries = std::min(queries, p->window_left + (p->causal ? 0 : p->window_right) + 128);
     return queries * group >= 5 * 128 && group >= 2 && blocks <= (group >= 8 ? 37 : 9);
 }
-// Whether the caller lets dQ be summed in any order, where a form exists that makes use of it (D 64, 128).
-static bool order_is_free(const dash_attn_params *p) { return !p->deterministic && (p->d == 128 || p->d == 64); }
-// Whether such a call does take that form, five products with dQ added by reductions in L2.  It shares the scores but not its
+// Whether a call whose caller lets dQ be summed in any order takes the form that makes use of it, five products with dQ added by
+// reductions in L2 (D 64, 128).  It shares the scores but not its
 // units: the seven-product form fills what few units leave idle with dq's tiles, and at D 128 the reductions cost what the two products
 // do.  Backward, 170 calls (us, seven products | five): D 64 packed, 16 / 4 heads, 4000 tokens, 128 units, 71 | 87, 8000, 252 units,
 // 148 | 133, 30000 960 | 758; padded, 8 of 256, 12 / 4, 64 units, 24 | 25, 4 of 256, 12 / 12, 96 units, 19 | 17, 32 of 1000,
 // 3072 units, 596 | 378.  D 128 packed, 1000 to 30000 tokens, 60 to 99.7 % of the speed; padded, 8 of 500, 12 / 12, 384 units,
 // 77 | 81, 16 of 1000, 12 / 4, 512 units, 309 | 293, 32 of 1000, 1024 units, 603 | 507.
 static bool fused_backward(const dash_attn_params *p) {
-    if (!order_is_free(p) || backward_pairs(p)) return false;
+    if (p->deterministic || (p->d != 64 && p->d != 128) || backward_pairs(p)) return false;
     const int64_t units = (int64_t)p->b * ((p->tk + 127) / 128) * p->hkv;
     const bool packed = p->mask_kind == DASH_ATTN_MASK_PACKED;
     return p->d == 64 ? units >= (packed ? 240 : 90) : !packed && units >= 500;
@@ -326,7 +325,7 @@ cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *w
 cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *workspace, cudaStream_t stream, int *launches,
                            bool *atomic, std::string &err) {
     const bool fused = fused_backward(p);
-    *atomic = order_is_free(p);
+    *atomic = fused;
     Sm100BwdMaps m;
     float *dq_acc = fused ? reinterpret_cast<float *>(static_cast<char *>(workspace) + bwd_sm100_order_bytes(p->b, p->tk, p->hkv)) : nullptr;
     const void *q = a.q.ptr, *k = a.k.ptr, *v = a.v.ptr, *g = a.dout.ptr;

@@ -311,7 +311,7 @@ enum {
     DASH_ATTN_PROBE_KERNEL_LAUNCHES = 0, /* kernels this library launched */
     DASH_ATTN_PROBE_BACKWARD_RUNS = 1,   /* calls of dash_attn_backward that launched */
     DASH_ATTN_PROBE_INPUT_COPIES = 2,    /* always 0: every input is read in place */
-    DASH_ATTN_PROBE_ATOMIC_RUNS = 3,     /* backward passes free to sum dq with atomics (deterministic 0, D 64 / 128, 16-bit); they do where that is faster */
+    DASH_ATTN_PROBE_ATOMIC_RUNS = 3,     /* backward passes that summed dq with atomics (of those with deterministic 0: where that is faster) */
     DASH_ATTN_PROBE_TENSOR_CORE_RUNS = 4, /* calls that took the tcgen05 path */
     DASH_ATTN_PROBE_GENERIC_RUNS = 5,    /* calls that took the generic kernels */
     DASH_ATTN_PROBE_TENSOR_MAP_ENCODES = 6, /* TMA tensor maps encoded through the driver (repeated calls reuse theirs) */

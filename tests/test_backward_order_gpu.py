@@ -5,6 +5,7 @@ import math
 import pytest
 import torch
 
+from dashmag_b200 import _lib
 from dashmag_b200 import attention as A
 from dashmag_b200.contract import AttentionMask, AttentionOptions
 
@@ -14,14 +15,17 @@ pytestmark = pytest.mark.gpu
 BOUND = 2.0 ** -11 * math.sqrt(2 / 3)
 
 
-@pytest.mark.parametrize("d,deterministic", [(64, True), (128, True), (256, True), (128, False)])
-def test_small_terms_count(d, deterministic):
-    t, heads, first = 32768, 8, 128
+# (Heads of 128 take the five-product form, where dq may be summed in any order, from 500 blocks of 128 keys on: two key-value heads.)
+@pytest.mark.parametrize("d,deterministic,hkv", [(64, True, 1), (128, True, 1), (256, True, 1), (64, False, 1), (128, False, 2)])
+def test_small_terms_count(d, deterministic, hkv):
+    t, heads, first = 32768, 8, 128   # heads to a key-value head, whose first one is looked at
     g = torch.Generator(device="cuda").manual_seed(1)
-    q, k, v, w = (torch.randn(1, t, h, d, generator=g, device="cuda").half() for h in (heads, 1, 1, heads))
+    q, k, v, w = (torch.randn(1, t, h, d, generator=g, device="cuda").half() for h in (heads * hkv, hkv, hkv, heads * hkv))
     options = AttentionOptions(causal=True, deterministic=deterministic)
     o, lse = A.attention_with_lse(q, k, v, AttentionMask.none(), options)
+    five = _lib.probe("atomic_runs")
     _, dk, dv = A.attention_backward(q, k, v, o, lse, w, AttentionMask.none(), options)
+    assert _lib.probe("atomic_runs") == five + int(not deterministic)
     keys, values = k[0, :first, 0].double(), v[0, :first, 0].double()
     want_k, want_v = torch.zeros_like(keys), torch.zeros_like(values)
     hidden = torch.arange(first, device="cuda")[None] > torch.arange(t, device="cuda")[:, None]

@@ -1,5 +1,6 @@
-"""The backward where two blocks share a unit's steps (few key blocks, long sweeps), and on both sides of the lines between the forms
-of a call that leaves the order of dq's sums free, against the same sums in f64; the fixed order repeats to the bit."""
+"""The backward where two blocks share a unit's steps (few key blocks, long sweeps), and the forms of a call that leaves the order of
+dq's sums free - on both sides of the lines between them, and the five-product form (the probe says that it ran) over groups, masks,
+windows and dtypes - against the same sums in f64; the fixed order repeats to the bit."""
 import math
 
 import numpy as np
@@ -14,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 def reference(q, k, v, g, seen):
-    """dq, dk, dv in f64 of [T, H, D] tensors of one batch element; `seen` [T, T] or None.  And what an error in delta of all of
+    """dq, dk, dv in f64 of [T, H, D] tensors of one batch element; `seen` [Tq, Tk] or None.  And what an error in delta of all of
     sum |O| |dO| would make of them: a query that sees one key has dP = delta, gradients of zero and nothing but that error."""
     group = q.shape[1] // k.shape[1]
     q, g = q.double(), g.double()
@@ -32,11 +33,15 @@ def reference(q, k, v, g, seen):
             (fold(torch.einsum("hij,ihd->jhd", p, g)), torch.zeros(1)))
 
 
-def check(b, t, hkv, group, d, dtype, mask_kind, causal, window, deterministic):
+def check(b, t, hkv, group, d, dtype, mask_kind, causal, window, deterministic, five=False, tq=None):
+    """`five`: the call sums dq by reductions, five products a pair of tiles; `tq` queries (t, where not said) against t keys."""
+    tq = tq or t
     gen = torch.Generator(device="cuda").manual_seed(t)
-    q, k, v, g = (torch.randn((b, t, h, d), generator=gen, device="cuda").to(dtype) for h in (hkv * group, hkv, hkv, hkv * group))
+    q, k, v, g = (torch.randn((b, n, h, d), generator=gen, device="cuda").to(dtype)
+                  for n, h in ((tq, hkv * group), (t, hkv), (t, hkv), (tq, hkv * group)))
     i = torch.arange(t, device="cuda")
-    seen = [torch.ones(t, t, dtype=torch.bool, device="cuda") for _ in range(b)]
+    at = torch.arange(tq, device="cuda") + t - tq   # the queries' places among the keys
+    seen = [torch.ones(tq, t, dtype=torch.bool, device="cuda") for _ in range(b)]
     if mask_kind == "packed":
         cut = [0, t // 3, t // 3 + 1, t]
         cu = torch.tensor(cut, dtype=torch.int32, device="cuda")
@@ -51,15 +56,15 @@ def check(b, t, hkv, group, d, dtype, mask_kind, causal, window, deterministic):
     else:
         mask = AttentionMask.none()
     if causal:
-        seen = [s & (i[:, None] >= i[None]) for s in seen]
+        seen = [s & (at[:, None] >= i[None]) for s in seen]
     options = AttentionOptions(causal=causal, deterministic=deterministic)
     if window is not None:
         options = options.with_window(window, window)
-        seen = [s & ((i[:, None] - i[None]).abs() <= window) for s in seen]
+        seen = [s & ((at[:, None] - i[None]).abs() <= window) for s in seen]
     o, lse = A.attention_with_lse(q, k, v, mask, options)
     atomic = _lib.probe("atomic_runs")
     runs = [A.attention_backward(q, k, v, o, lse, g, mask, options) for _ in range(4)]
-    assert _lib.probe("atomic_runs") == atomic + (0 if deterministic else 4)
+    assert _lib.probe("atomic_runs") == atomic + (4 if five else 0)
     for run in runs[1:]:
         for x, y, fixed in zip(run, runs[0], (deterministic, True, True)):
             assert not fixed or torch.equal(x, y)
@@ -82,8 +87,9 @@ def test_shared_units(b, t, hkv, group, d, dtype, mask, causal, window):
     check(b, t, hkv, group, d, dtype, mask, causal, window, True)
 
 
-@pytest.mark.parametrize("b,t,hkv,group,d,mask", [
-    (30, 300, 1, 1, 64, "padding"), (29, 300, 1, 1, 64, "padding"), (1, 3840, 8, 1, 64, "packed"), (1, 3700, 8, 1, 64, "packed"),
-    (125, 260, 2, 1, 128, "padding"), (100, 200, 2, 1, 128, "padding"), (1, 1000, 2, 4, 128, "packed"), (2, 1000, 2, 4, 64, "none")])
-def test_free_order_on_both_sides(b, t, hkv, group, d, mask):
-    check(b, t, hkv, group, d, torch.bfloat16, mask, False, None, False)
+# Units (blocks of 128 keys by key-value heads by batch) on both sides of the lines: 90 (packed: 240) at heads of 64, 500 (packed: never) at 128.
+@pytest.mark.parametrize("b,t,hkv,group,d,mask,five", [
+    (30, 300, 1, 1, 64, "padding", True), (29, 300, 1, 1, 64, "padding", False), (1, 3840, 8, 1, 64, "packed", True), (1, 3700, 8, 1, 64, "packed", False),
+    (125, 260, 2, 1, 128, "padding", True), (100, 200, 2, 1, 128, "padding", False), (1, 1000, 2, 4, 128, "packed", False), (2, 1000, 2, 4, 64, "none", False)])
+def test_free_order_on_both_sides(b, t, hkv, group, d, mask, five):
+    check(b, t, hkv, group, d, torch.bfloat16, mask, False, None, False, five)

@@ -7,16 +7,19 @@ import numpy as np
 import pytest
 import torch
 
+from dashmag_b200 import _lib
 from dashmag_b200 import attention as A
 from dashmag_b200.contract import AttentionMask, AttentionOptions
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("blocks,hkv,group,d,deterministic", [
-    (1, 1, 1, 128, True), (74, 2, 2, 128, True), (75, 2, 2, 128, True), (148, 1, 4, 64, True), (149, 1, 1, 128, True), (37, 1, 2, 256, True),
-    (38, 1, 1, 256, True), (74, 2, 1, 128, False), (149, 1, 2, 64, False)])
-def test_both_sides(blocks, hkv, group, d, deterministic):
+# `five`: dq summed in any order and so by reductions, from 240 units on (never without a launch order in a packed batch).
+@pytest.mark.parametrize("blocks,hkv,group,d,five", [
+    (1, 1, 1, 128, None), (74, 2, 2, 128, None), (75, 2, 2, 128, None), (148, 1, 4, 64, None), (149, 1, 1, 128, None), (37, 1, 2, 256, None),
+    (38, 1, 1, 256, None), (74, 2, 1, 128, False), (149, 1, 2, 64, False), (240, 1, 2, 64, True), (80, 3, 4, 64, True)])
+def test_both_sides(blocks, hkv, group, d, five):
+    deterministic = five is None
     rng = np.random.default_rng(blocks)
     t = 128 * blocks - int(rng.integers(0, 128))
     lens = []
@@ -27,9 +30,11 @@ def test_both_sides(blocks, hkv, group, d, deterministic):
     cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
     mask, options = AttentionMask.packed(cu, cu), AttentionOptions(causal=True, deterministic=deterministic)
     o, lse = A.attention_with_lse(q, k, v, mask, options)
+    atomic = _lib.probe("atomic_runs")
     runs = [A.attention_backward(q, k, v, o, lse, go, mask, options) for _ in range(8)]
+    assert _lib.probe("atomic_runs") == atomic + (8 if five else 0)
     for run in runs[1:]:
-        for x, y, fixed in zip(run, runs[0], (deterministic, True, True)):
+        for x, y, fixed in zip(run, runs[0], (not five, True, True)):
             assert not fixed or torch.equal(x, y)
     want = [torch.empty(x.shape, dtype=torch.float64, device="cuda") for x in runs[0]]
     at = 0
