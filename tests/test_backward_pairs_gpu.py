@@ -93,3 +93,19 @@ def test_shared_units(b, t, hkv, group, d, dtype, mask, causal, window):
     (125, 260, 2, 1, 128, "padding", True), (100, 200, 2, 1, 128, "padding", False), (1, 1000, 2, 4, 128, "packed", False), (2, 1000, 2, 4, 64, "none", False)])
 def test_free_order_on_both_sides(b, t, hkv, group, d, mask, five):
     check(b, t, hkv, group, d, torch.bfloat16, mask, False, None, False, five)
+
+
+B, H = torch.bfloat16, torch.float16
+
+
+# Tiles of 128 / 2^p tokens by 2^p heads: p = 0 (groups 1, 3), 1 (2, 6), 2 (4, 12), 3 (8, 16).
+@pytest.mark.parametrize("b,tq,t,hkv,group,d,dtype,mask,causal,window", [
+    (12, 130, 130, 4, 2, 64, B, "none", True, None), (16, 257, 257, 2, 3, 64, H, "padding", False, None), (10, 300, 300, 3, 4, 64, B, "none", True, 60),
+    (13, 300, 300, 3, 8, 64, H, "none", True, None), (50, 129, 200, 1, 16, 64, B, "none", True, None), (45, 255, 131, 1, 6, 64, B, "none", True, None),
+    (24, 500, 500, 1, 12, 64, H, "padding", True, 100), (1, 3840, 3840, 8, 2, 64, B, "packed", True, None), (1, 3840, 3840, 8, 4, 64, H, "packed", True, 300),
+    (1, 5250, 5250, 6, 3, 64, B, "packed", False, 90), (45, 256, 256, 1, 1, 64, B, "none", True, None),
+    (50, 130, 130, 5, 2, 128, B, "none", True, None), (45, 260, 260, 4, 3, 128, H, "padding", False, None), (64, 140, 140, 4, 4, 128, H, "none", True, 40),
+    (32, 256, 256, 8, 8, 128, B, "none", True, None), (84, 129, 300, 2, 6, 128, B, "none", False, 70), (125, 5, 200, 2, 16, 128, H, "none", True, None),
+    (125, 257, 129, 2, 1, 128, H, "none", True, None), (64, 200, 200, 4, 12, 128, B, "padding", True, None)], ids=str)
+def test_five_products(b, tq, t, hkv, group, d, dtype, mask, causal, window):
+    check(b, t, hkv, group, d, dtype, mask, causal, window, False, True, tq)

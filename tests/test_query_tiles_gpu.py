@@ -1,6 +1,7 @@
 """Tiles of query rows that hold several heads of a group (128 / 2^p tokens x 2^p heads): every power of two a
 group can give (1, 2, 4, 8, and what is left of 3, 6, 12 and 16), with lengths on both sides of a tile's tokens,
-on the kernels of the three head dimensions, against the f64 oracle; repeats to the bit."""
+on the kernels of the three head dimensions, against the f64 oracle; repeats to the bit.  (These calls are too small for the
+five-product backward: test_backward_pairs_gpu.py has its tiles.)"""
 import numpy as np
 import pytest
 
@@ -52,4 +53,4 @@ def test_heads_share_tiles(adapter, case):
     for x, y in zip([a.out, a.lse, *a.grads], [b.out, b.lse, *b.grads]):
         assert np.array_equal(x, y, equal_nan=True), "two runs of the same call differ"
     c = run_case(adapter, case, DType.BF16, deterministic=False)
-    R.check(f"atomic {case.name}", [c.out, c.lse, *c.grads], want, bounds)
+    R.check(f"any order {case.name}", [c.out, c.lse, *c.grads], want, bounds)
