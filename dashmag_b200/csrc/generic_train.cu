@@ -595,6 +595,11 @@ static size_t generic_smem(int d, int rpw, int own, int probs) {
 // backward of 300 x 8 / 2 heads of 128 204 | 248 | 293 (the rule, which picks for each kernel: 184), of 1400 x 4 of 128
 // 749 | 549 | 450, of 700 x 4 of 128 230 | 170 | 215.  It is not the best of the three everywhere: the forward of 700 x 4 of
 // 128 takes one row a warp, 118 us, where four take 101; of 1000 x 8 / 2 of 96 four, 195, where two take 165.
+// Shared rows sum in another order (even and odd tiles apart), so a slice of a call's heads or batch, which may take them where the call
+// does not, can differ from it in the last bits.  What it would cost to keep them: every form with the two sums apart, 75 calls, f32,
+// 0 to 3 % on average, but 4 heads of 128, 1500 tokens, 146 -> 205 us forward and 368 -> 420 backward, 8 of 96, 900 tokens, 111 -> 128
+// and 214 -> 259 (the second set of sums in registers; in local memory 111 -> 133 and 214 -> 371); shared rows by the number of rows
+// alone, 32 heads of 64, 200 tokens, backward 48 -> 65, 32 of 128 79 -> 138; without them 3 / 1 heads of 96, 590 tokens, 103 -> 148.
 constexpr int64_t SMEM_PER_SM = 228 * 1024, SMEM_BESIDE = 2 * 1024;
 static int rows_per_warp(int64_t rows, int64_t heads, int d, int own, int probs) {
     for (int rpw = 1; rpw < 4; rpw *= 2) {

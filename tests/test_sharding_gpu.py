@@ -114,3 +114,47 @@ def test_head_slices_in_another_order(t, hkv, group, d, packed):
         share = step(q[:, :, qh], k[:, :, kv], v[:, :, kv], g[:, :, qh])
         for name, got, want, at in zip("o lse dq dk dv".split(), share, whole, (qh, qh, qh, kv, kv)):
             assert_rounding(name, got, want[:, :, at], "a head slice")
+
+
+# The CUDA-core kernels take another form as the rows, heads and batch of a call grow: one, two or four rows a warp, which sum in one order,
+# or (up to head dimension 128) two warps to a pair of rows, which sum in another.  dtype, batch, key-value heads, group, tokens, head dimension,
+# mask, with the whole call and its slices on both sides of the lines: slices agree to rounding, and to the bit beyond 128.
+@pytest.mark.parametrize("dtype,b,hkv,group,t,d,kind", [
+    (torch.float32, 1, 4, 1, 1000, 64, "packed"), (torch.float32, 1, 4, 2, 1500, 64, "packed"), (torch.float32, 1, 8, 4, 300, 128, "window"),
+    (torch.float32, 1, 16, 1, 700, 96, "packed"), (torch.float32, 1, 2, 8, 333, 40, "packed"), (torch.bfloat16, 2, 8, 2, 500, 80, "padding"),
+    (torch.float32, 12, 2, 2, 200, 64, "causal"), (torch.float16, 24, 3, 1, 170, 96, "padding"), (torch.float32, 3, 6, 1, 260, 200, "window")], ids=str)
+def test_slices_on_the_cuda_cores(dtype, b, hkv, group, t, d, kind):
+    q, k, v, g = (normal((b, t, h, d), i).to(dtype) for i, h in enumerate((hkv * group, hkv, hkv, hkv * group)))
+    options = AttentionOptions.causal_() if kind != "padding" else AttentionOptions()
+    if kind == "window":
+        options = options.with_window(t // 3, 0)
+    cu = torch.tensor([0, 1, t // 3 + 7, t], dtype=torch.int32, device=DEV)
+    pad = torch.arange(t, device=DEV)[None] >= t - 13 * torch.arange(b, device=DEV)[:, None] % t
+
+    def step(n, kv):
+        mask = AttentionMask.packed(cu, cu) if kind == "packed" else AttentionMask.key_padding(pad[n]) if kind == "padding" else AttentionMask.none()
+        qh = slice(kv.start * group, kv.stop * group)
+        qs, ks, vs, gs = q[n][:, :, qh], k[n][:, :, kv], v[n][:, :, kv], g[n][:, :, qh]
+        o, lse = A.attention_with_lse(qs, ks, vs, mask, options)
+        return (o, lse) + tuple(A.attention_backward(qs, ks, vs, o, lse, gs, mask, options))
+
+    before = _lib.probe("generic_runs")
+    whole = step(slice(0, b), slice(0, hkv))
+    assert _lib.probe("generic_runs") == before + 2
+    for n in (1, max(b // 3, 1)):
+        for heads in (1, max(hkv // 2, 1)):
+            at, kv = slice(b - n, b), slice(0, heads)
+            qh = slice(0, heads * group)
+            for name, got, want, h in zip("o lse dq dk dv".split(), step(at, kv), whole, (qh, qh, qh, kv, kv)):
+                want = want[at][:, :, h]
+                if d > 128:
+                    assert torch.equal(got, want), f"{name}: {n} sequences, {heads} key-value heads"
+                    continue
+                # Both lie within the f32 kernels' bound of the exact result (tests/test_kernels_gpu.py: 1e-5 of the largest value, the
+                # log-sum-exp 1e-6), so within twice that of each other; 16-bit results that straddle a rounding are neighbours.
+                near = (2e-6 if name == "lse" else 2e-5) * want.float().abs()[torch.isfinite(want)].max()
+                slack = 0.0 if name == "lse" else {torch.float32: 0.0, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}[dtype]
+                finite = torch.isfinite(want)
+                assert torch.equal(torch.isfinite(got), finite)
+                apart = (got.float() - want.float()).abs()[finite] - slack * want.float().abs()[finite]
+                assert float(apart.max()) <= float(near), f"{name}: {n} sequences, {heads} key-value heads"
