@@ -250,7 +250,7 @@ template <int HD, bool FUSED> constexpr size_t smem_dkdv() {
                  : 1024 + 6 * tile_bytes<HD>() + dkdv_tail<false>();
 }
 
-// PAIR: a cluster of two blocks a unit, each half of the unit's steps (bwd_sm100_pairs says which calls).
+// PAIR: a cluster of two blocks a unit, each half of the unit's steps (backward_pairs says which calls).
 template <typename T, int HD, bool FUSED, bool PAIR>
 __global__ void __launch_bounds__(FUSED ? KTHREADS_FUSED : KTHREADS, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,

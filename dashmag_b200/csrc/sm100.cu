@@ -248,10 +248,14 @@ size_t sm100_forward_workspace(const dash_attn_params *p, bool any_size) {
 // 128; D 256 has a rule of its own).  A unit sweeps the queries of all heads of its group that see it, and with few units the
 // longest sweep is the kernel's length; with two blocks to a unit it is half that, a second set-up and the meeting of the two.  The
 // rule looks at no number of heads, so that a head slice of a packed batch keeps the whole call's bits: key blocks so few that
-// with eight key-value heads (one, where groups are of eight) twice the units still start at once, and sweeps of five steps of
-// 128 rows or more.  Backward, one block | two (us): 500 tokens, 16 / 4 heads of 128, 36.7 | 28.4, 32 / 8 37.6 | 29.4; 1000 in four,
-// 32 / 8, 39.1 | 33.8, 16 / 8 24.3 | 24.4; 1152, 24 / 8, 56.6 | 43.9; 8 / 1: 500 62.8 | 41.7, 4700 in two 350 | 188; heads
-// of 64 the same.  Beyond it, 2420 tokens in three, 32 / 8 of 64, 152 units: 117 | 125.
+// with eight key-value heads (two, where groups are of eight) twice the units still start at once, and sweeps of five steps of
+// 128 rows or more.  Backward, one block | two (us): 500 tokens, 16 / 4 heads of 128, 36.7 | 28.4, 32 / 8 39.2 | 30.9; 1000 in three,
+// 32 / 8, 37.8 | 37.2, 16 / 8 24.9 | 26.8; 1152, 16 / 8, 42.6 | 36.0, 24 / 8 56.6 | 43.9; groups of eight, 8 / 1, 500 62.8 | 41.7, 4700 in two
+// 350 | 188, 16 / 2 4700 505 | 274, 32 / 4 2400 267 | 158, 64 / 8 1800 216 | 197; heads of 64 the same.
+// What the slices' bits cost: with more key-value heads the doubled blocks come in waves, and the pair loses what a line on the units
+// (about 100) would keep - 32 / 16 heads, 500 tokens, 26.8 | 26.8, 1000 45.9 | 59.5, 1152 53.4 | 67.8; 64 / 32, 500, 37.0 | 49.3; 64 / 16,
+// 500, 47.6 | 45.2, 1152 96.2 | 110; 64 / 8, 2400, 308 | 319, 4700 1145 | 1204, in four 411 | 441; 128 / 16, 4700 in four, 834 | 903.
+constexpr int64_t PAIR_BLOCKS = 9, PAIR_BLOCKS_GROUP8 = 37, PAIR_ROWS = 5 * 128;
 static bool backward_pairs(const dash_attn_params *p) {
     if (p->d != 64 && p->d != 128) return false;
     const int64_t blocks = (int64_t)p->b * ((p->tk + 127) / 128), group = p->hq / p->hkv;
@@ -259,7 +263,7 @@ static bool backward_pairs(const dash_attn_params *p) {
     int64_t queries = p->mask_kind == DASH_ATTN_MASK_PACKED ? p->tq / std::max(p->cu_seqlens_q_len - 1, 1) : p->tq;
     if (p->has_window && p->window_left >= 0 && p->window_left < none && (p->causal || (p->window_right >= 0 && p->window_right < none)))
         queries = std::min(queries, p->window_left + (p->causal ? 0 : p->window_right) + 128);
-    return queries * group >= 5 * 128 && group >= 2 && blocks <= (group >= 8 ? 37 : 9);
+    return queries * group >= PAIR_ROWS && group >= 2 && blocks <= (group >= 8 ? PAIR_BLOCKS_GROUP8 : PAIR_BLOCKS);
 }
 // Whether a call whose caller lets dQ be summed in any order takes the form that makes use of it, five products with dQ added by
 // reductions in L2 (D 64, 128).  It shares the scores but not its
@@ -268,11 +272,12 @@ static bool backward_pairs(const dash_attn_params *p) {
 // 148 | 133, 30000 960 | 758; padded, 8 of 256, 12 / 4, 64 units, 24 | 25, 4 of 256, 12 / 12, 96 units, 19 | 17, 32 of 1000,
 // 3072 units, 596 | 378.  D 128 packed, 1000 to 30000 tokens, 60 to 99.7 % of the speed; padded, 8 of 500, 12 / 12, 384 units,
 // 77 | 81, 16 of 1000, 12 / 4, 512 units, 309 | 293, 32 of 1000, 1024 units, 603 | 507.
+constexpr int64_t FIVE_UNITS_64 = 90, FIVE_UNITS_64_PACKED = 240, FIVE_UNITS_128 = 500;
 static bool fused_backward(const dash_attn_params *p) {
     if (p->deterministic || (p->d != 64 && p->d != 128) || backward_pairs(p)) return false;
     const int64_t units = (int64_t)p->b * ((p->tk + 127) / 128) * p->hkv;
     const bool packed = p->mask_kind == DASH_ATTN_MASK_PACKED;
-    return p->d == 64 ? units >= (packed ? 240 : 90) : !packed && units >= 500;
+    return p->d == 64 ? units >= (packed ? FIVE_UNITS_64_PACKED : FIVE_UNITS_64) : !packed && units >= FIVE_UNITS_128;
 }
 static size_t dq_acc_bytes(const dash_attn_params *p) {
     return (sizeof(float) * (size_t)p->b * p->tq * p->hq * p->d + 255) & ~size_t(255);
@@ -322,6 +327,11 @@ cudaError_t sm100_forward(const dash_attn_params *p, const TrainArgs &a, void *w
     return e;
 }
 
+// Units that need no launch order: one a multiprocessor, at D 256 (two passes, two blocks to a unit) a quarter of that.  Units shared by two
+// blocks take the first line too, though 75 to 148 of them do not all start at once: of 90 such calls the order gained 2 % in three and
+// cost up to 10 in the others (32 / 16 heads of 128, 700 tokens, 96 units, 41.1 us without, 45.2 with).
+constexpr int AT_ONCE = 148, AT_ONCE_256 = 37;
+
 cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *workspace, cudaStream_t stream, int *launches,
                            bool *atomic, std::string &err) {
     const bool fused = fused_backward(p);
@@ -356,7 +366,7 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
     f.pairs = backward_pairs(p) ? 1 : 0;
     // The plan's one block and delta run side by side; then dkdv, and dq beside its last waves (neither reads what
     // the other writes).
-    cudaError_t e = launch_bwd_plan(f, p->d == 256 ? 37 : 148, stream, launches);
+    cudaError_t e = launch_bwd_plan(f, p->d == 256 ? AT_ONCE_256 : AT_ONCE, stream, launches);
     if (e == cudaSuccess) e = launch_generic_delta(p->dtype, a, stream, launches, f.order != nullptr);
     if (e != cudaSuccess) return e;
     if (p->d == 256) return launch_bwd256_sm100(p->dtype, m, f, stream, launches);
