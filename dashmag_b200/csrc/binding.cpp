@@ -11,6 +11,7 @@
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -40,6 +41,10 @@ struct Library {
 } lib;
 
 // ---- what a call hands over ------------------------------------------------------------------------
+// The tensors a call's parameters point into that are not its arguments: an attribute may be a property whose tensor nobody else
+// holds, and what a mask or a Rope holds another thread may replace while the library is called without the interpreter's lock.
+using Held = c10::SmallVector<at::Tensor, 2>;
+
 struct Ref {   // an owned reference
     PyObject *p;
     explicit Ref(PyObject *o) : p(o) {}
@@ -160,8 +165,8 @@ PyObject *wrapped(std::initializer_list<at::Tensor> outs) {
 }
 
 // ---- training --------------------------------------------------------------------------------------
-// The parameters of a training call; `hold` keeps what they point to.  False: not for us.
-bool train_params(dash_attn_params &p, const at::Tensor &q, const at::Tensor &k, const at::Tensor &v, PyObject *mask, PyObject *options) {
+// The parameters of a training call; `held` keeps what they point to.  False: not for us.
+bool train_params(dash_attn_params &p, Held &held, const at::Tensor &q, const at::Tensor &k, const at::Tensor &v, PyObject *mask, PyObject *options) {
     if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || !fits32(q) || !fits32(k) || !fits32(v)) return false;
     const int code = code_of(q.scalar_type());
     if (code < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return false;
@@ -178,13 +183,14 @@ bool train_params(dash_attn_params &p, const at::Tensor &q, const at::Tensor &k,
     if (PyUnicode_CompareWithASCIIString(kind.p, "none") == 0) {
         p.mask_kind = DASH_ATTN_MASK_NONE;
     } else if (PyUnicode_CompareWithASCIIString(kind.p, "key_padding") == 0) {
-        Ref o(PyObject_GetAttrString(mask, "key_padding_mask"));   // (the mask object keeps the tensor)
+        Ref o(PyObject_GetAttrString(mask, "key_padding_mask"));
         const at::Tensor *m = o.p ? plain(o.p) : nullptr;
         if (!m || m->dim() != 2 || !fits32(*m) || m->get_device() != q.get_device()) return false;
         const at::ScalarType s = m->scalar_type();
         p.key_padding_elem_bytes = s == at::kBool || s == at::kByte || s == at::kChar ? 1 : s == at::kInt ? 4 : 0;
         if (p.key_padding_elem_bytes == 0) return false;
         p.mask_kind = DASH_ATTN_MASK_KEY_PADDING;
+        held.push_back(*m);
         p.key_padding = m->data_ptr();
         for (int i = 0; i < 2; ++i) {
             p.key_padding_shape[i] = (int32_t)m->size(i);
@@ -198,6 +204,8 @@ bool train_params(dash_attn_params &p, const at::Tensor &q, const at::Tensor &k,
         p.index_elem_bytes = index_bytes(cq->scalar_type());
         if (p.index_elem_bytes == 0) return false;
         p.mask_kind = DASH_ATTN_MASK_PACKED;
+        held.push_back(*cq);
+        held.push_back(*ck);
         p.cu_seqlens_q = cq->data_ptr();
         p.cu_seqlens_k = ck->data_ptr();
         p.cu_seqlens_q_len = (int32_t)cq->size(0);
@@ -215,7 +223,8 @@ PyObject *forward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (n != 5) return nothing_done();
     const at::Tensor *q = plain(args[0]), *k = plain(args[1]), *v = plain(args[2]);
     dash_attn_params p{};
-    if (!q || !k || !v || !train_params(p, *q, *k, *v, args[3], args[4])) return nothing_done();
+    Held held;
+    if (!q || !k || !v || !train_params(p, held, *q, *k, *v, args[3], args[4])) return nothing_done();
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type()), lse = fresh(q->sizes().slice(0, 3), *q, at::kFloat);
     const size_t need = lib.forward_workspace(&p);
     at::Tensor ws = scratch(need, *q);
@@ -232,7 +241,8 @@ PyObject *backward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (n != 8) return nothing_done();
     const at::Tensor *q = plain(args[0]), *k = plain(args[1]), *v = plain(args[2]), *o = plain(args[3]), *lse = plain(args[4]), *g = plain(args[5]);
     dash_attn_params p{};
-    if (!q || !k || !v || !o || !lse || !g || !train_params(p, *q, *k, *v, args[6], args[7])) return nothing_done();
+    Held held;
+    if (!q || !k || !v || !o || !lse || !g || !train_params(p, held, *q, *k, *v, args[6], args[7])) return nothing_done();
     const int device = (int)q->get_device();
     if (o->sizes() != q->sizes() || g->sizes() != q->sizes() || lse->sizes() != q->sizes().slice(0, 3) || o->scalar_type() != q->scalar_type() ||
         g->scalar_type() != q->scalar_type() || lse->scalar_type() != at::kFloat || !lse->is_contiguous() || o->get_device() != device ||
@@ -315,9 +325,9 @@ PyObject *decode_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 // A Rope's tables for tensors of `dtype` with `d` features; false: not for us.
-bool rope_tables(dash_rope_tables &r, PyObject *rope, at::ScalarType dtype, int64_t d, const at::Tensor &near) {
+bool rope_tables(dash_rope_tables &r, Held &held, PyObject *rope, at::ScalarType dtype, int64_t d, const at::Tensor &near) {
     Ref dt(PyObject_GetAttrString(rope, "dtype")), dim(PyObject_GetAttrString(rope, "dim")), len(PyObject_GetAttrString(rope, "_len"));
-    Ref oc(PyObject_GetAttrString(rope, "cos")), os(PyObject_GetAttrString(rope, "sin"));   // (the Rope keeps them)
+    Ref oc(PyObject_GetAttrString(rope, "cos")), os(PyObject_GetAttrString(rope, "sin"));
     if (!dt.p || !dim.p || !len.p || !oc.p || !os.p || !THPDtype_Check(dt.p)) return false;
     if (reinterpret_cast<THPDtype *>(dt.p)->scalar_type != dtype) return false;
     const at::Tensor *c = plain(oc.p), *s = plain(os.p);
@@ -326,6 +336,8 @@ bool rope_tables(dash_rope_tables &r, PyObject *rope, at::ScalarType dtype, int6
     if (c->get_device() != near.get_device() || s->get_device() != near.get_device()) return false;
     r.dtype = code_of(dtype);
     r.dim = (int32_t)features;
+    held.push_back(*c);
+    held.push_back(*s);
     r.cos = pointer(*c);
     r.sin = pointer(*s);
     return r.dtype >= 0;
@@ -338,8 +350,9 @@ PyObject *decode_append_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const at::Tensor *q = plain(args[1]), *nk = plain(args[2]), *nv = plain(args[3]), *k = plain(args[4]), *v = plain(args[5]);
     dash_attn_decode_params p{};
     dash_rope_tables r{};
+    Held held;
     if (!q || !k || !v || args[6] == Py_None || !decode_params(p, *q, *k, *v, args[6], args[7]) || !new_row(nk, *k) || !new_row(nv, *k)) return nothing_done();
-    if (q->stride(2) != 1 || !rope_tables(r, args[0], q->scalar_type(), q->size(2), *q)) return nothing_done();
+    if (q->stride(2) != 1 || !rope_tables(r, held, args[0], q->scalar_type(), q->size(2), *q)) return nothing_done();
     at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
     const size_t need = lib.decode_append_rope_workspace(&p);
     at::Tensor ws = scratch(need, *q);

@@ -111,3 +111,28 @@ def test_a_mode_that_watches_sees_the_allocations():
     with Watch():
         A.attention(q, k, k)
     assert any("empty" in s for s in seen)
+
+
+def test_what_only_an_attribute_holds_outlives_the_call():
+    """A mask whose tensor is made anew each time it is asked for: the call alone holds it, and must until its kernels are launched -
+    while the outputs are allocated, that is, the tensor's memory is not free."""
+    pad = torch.arange(60, device="cuda")[None] >= torch.tensor([[60], [31]], device="cuda")
+    size = []
+
+    class Fresh:
+        kind = "key_padding"
+
+        @property
+        def key_padding_mask(self):
+            large = pad.repeat(1, 1 << 16)
+            size.append(large.untyped_storage().nbytes())
+            return large[:, :60]
+
+    q, k, v = randn(2, 60, 1, 64), randn(2, 60, 1, 64, seed=1), randn(2, 60, 1, 64, seed=2)
+    want = A.attention_with_lse(q, k, v, AttentionMask.key_padding(pad), AttentionOptions())
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = A.attention_with_lse(q, k, v, Fresh(), AttentionOptions())
+    assert torch.cuda.max_memory_allocated() - before >= size[0] + sum(x.untyped_storage().nbytes() for x in got)
+    assert len(size) == 1 and all(torch.equal(x, y) for x, y in zip(got, want))
