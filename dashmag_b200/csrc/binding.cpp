@@ -7,6 +7,7 @@
 // anything, and the Python code it stands in front of makes the call or raises what there is to raise.  None is the answer to
 // everything out of the ordinary: a tensor of another kind or device, a shape or dtype the Python side would refuse or copy, a
 // number its C type does not hold, a mode or a transform that wants to see the allocations.
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -69,9 +70,10 @@ PyObject *nothing_done() {
     Py_RETURN_NONE;
 }
 
-// A plain strided CUDA tensor: torch.Tensor or Parameter itself, no wrapper, no mode that watches.
+// A plain strided CUDA tensor: torch.Tensor or Parameter itself, no wrapper, no mode that watches (of functions or of dispatch:
+// what the Python side asks torch for such a mode sees).
 const at::Tensor *plain(PyObject *o) {
-    if (!THPVariable_CheckExact(o)) return nullptr;
+    if (!THPVariable_CheckExact(o) || at::impl::torch_function_mode_enabled()) return nullptr;
     const at::Tensor &t = THPVariable_Unpack(o);
     if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || at::isTensorSubclassLike(t)) return nullptr;
     return &t;

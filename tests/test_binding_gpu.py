@@ -98,6 +98,7 @@ def test_refusals_of_the_library_are_raised():
 
 
 def test_a_mode_that_watches_sees_the_allocations():
+    from torch.overrides import TorchFunctionMode
     from torch.utils._python_dispatch import TorchDispatchMode
 
     seen = []
@@ -107,10 +108,17 @@ def test_a_mode_that_watches_sees_the_allocations():
             seen.append(str(func))
             return func(*args, **(kwargs or {}))
 
+    class WatchFunctions(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func.__name__)
+            return func(*args, **(kwargs or {}))
+
     q, k = randn(1, 4, 2, 64), randn(1, 4, 2, 64)
-    with Watch():
-        A.attention(q, k, k)
-    assert any("empty" in s for s in seen)
+    for mode in (Watch, WatchFunctions):
+        seen.clear()
+        with mode():
+            A.attention(q, k, k)
+        assert any("empty" in s for s in seen), mode
 
 
 def test_what_only_an_attribute_holds_outlives_the_call():
