@@ -54,15 +54,15 @@ struct Ref {   // an owned reference
     Ref &operator=(const Ref &) = delete;
 };
 
-// The call into the library without the interpreter's lock, as ctypes makes it: a launch may wait for room in the GPU's queue.
+// Allocations and the call into the library without the interpreter's lock, as torch.empty and ctypes make them: an allocation may
+// wait for the driver or for memory to be given back, a launch for room in the GPU's queue.
 struct Unlocked {
     PyThreadState *state = PyEval_SaveThread();
-    ~Unlocked() { PyEval_RestoreThread(state); }
+    ~Unlocked() { PyEval_RestoreThread(state); }   // on the way out of an exception too: it is raised with the lock
 };
-
-template <typename... P, typename... A> int unlocked(int (*call)(P...), A... args) {
+template <typename F> int unlocked(F call) {
     Unlocked u;
-    return call(args...);
+    return call();
 }
 
 PyObject *nothing_done() {
@@ -227,11 +227,15 @@ PyObject *forward(PyObject *, PyObject *const *args, Py_ssize_t n) {
     dash_attn_params p{};
     Held held;
     if (!q || !k || !v || !train_params(p, held, *q, *k, *v, args[3], args[4])) return nothing_done();
-    at::Tensor out = fresh(q->sizes(), *q, q->scalar_type()), lse = fresh(q->sizes().slice(0, 3), *q, at::kFloat);
-    const size_t need = lib.forward_workspace(&p);
-    at::Tensor ws = scratch(need, *q);
-    const int rc = unlocked(lib.forward, &p, pointer(*q), pointer(*k), pointer(*v), pointer(out), static_cast<float *>(pointer(lse)),
-                                     need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    at::Tensor out, lse;
+    const int rc = unlocked([&] {
+        out = fresh(q->sizes(), *q, q->scalar_type());
+        lse = fresh(q->sizes().slice(0, 3), *q, at::kFloat);
+        const size_t need = lib.forward_workspace(&p);
+        at::Tensor ws = scratch(need, *q);
+        return lib.forward(&p, pointer(*q), pointer(*k), pointer(*v), pointer(out), static_cast<float *>(pointer(lse)), need ? ws.data_ptr() : nullptr, need,
+                           stream_of(*q));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({out, lse});
     END_HANDLE_TH_ERRORS
@@ -252,11 +256,16 @@ PyObject *backward(PyObject *, PyObject *const *args, Py_ssize_t n) {
         return nothing_done();
     strides(p.o_stride, *o);
     strides(p.do_stride, *g);
-    at::Tensor dq = fresh(q->sizes(), *q, q->scalar_type()), dk = fresh(k->sizes(), *q, q->scalar_type()), dv = fresh(v->sizes(), *q, q->scalar_type());
-    const size_t need = lib.backward_workspace(&p);
-    at::Tensor ws = scratch(need, *q);
-    const int rc = unlocked(lib.backward, &p, pointer(*q), pointer(*k), pointer(*v), pointer(*o), static_cast<const float *>(pointer(*lse)), pointer(*g),
-                                      pointer(dq), pointer(dk), pointer(dv), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    at::Tensor dq, dk, dv;
+    const int rc = unlocked([&] {
+        dq = fresh(q->sizes(), *q, q->scalar_type());
+        dk = fresh(k->sizes(), *q, q->scalar_type());
+        dv = fresh(v->sizes(), *q, q->scalar_type());
+        const size_t need = lib.backward_workspace(&p);
+        at::Tensor ws = scratch(need, *q);
+        return lib.backward(&p, pointer(*q), pointer(*k), pointer(*v), pointer(*o), static_cast<const float *>(pointer(*lse)), pointer(*g), pointer(dq),
+                            pointer(dk), pointer(dv), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({dq, dk, dv});
     END_HANDLE_TH_ERRORS
@@ -300,10 +309,13 @@ PyObject *decode(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const at::Tensor *q = plain(args[0]), *k = plain(args[1]), *v = plain(args[2]);
     dash_attn_decode_params p{};
     if (!q || !k || !v || !decode_params(p, *q, *k, *v, args[3], args[4])) return nothing_done();
-    at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
-    const size_t need = lib.decode_workspace(&p);
-    at::Tensor ws = scratch(need, *q);
-    const int rc = unlocked(lib.decode, &p, pointer(*q), pointer(*k), pointer(*v), pointer(out), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    at::Tensor out;
+    const int rc = unlocked([&] {
+        out = fresh(q->sizes(), *q, q->scalar_type());
+        const size_t need = lib.decode_workspace(&p);
+        at::Tensor ws = scratch(need, *q);
+        return lib.decode(&p, pointer(*q), pointer(*k), pointer(*v), pointer(out), need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -316,11 +328,14 @@ PyObject *decode_append(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const at::Tensor *q = plain(args[0]), *nk = plain(args[1]), *nv = plain(args[2]), *k = plain(args[3]), *v = plain(args[4]);
     dash_attn_decode_params p{};
     if (!q || !k || !v || args[5] == Py_None || !decode_params(p, *q, *k, *v, args[5], args[6]) || !new_row(nk, *k) || !new_row(nv, *k)) return nothing_done();
-    at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
-    const size_t need = lib.decode_workspace(&p);
-    at::Tensor ws = scratch(need, *q);
-    const int rc = unlocked(lib.decode_append, &p, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
-                                           need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    at::Tensor out;
+    const int rc = unlocked([&] {
+        out = fresh(q->sizes(), *q, q->scalar_type());
+        const size_t need = lib.decode_workspace(&p);
+        at::Tensor ws = scratch(need, *q);
+        return lib.decode_append(&p, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out), need ? ws.data_ptr() : nullptr, need,
+                                 stream_of(*q));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -355,11 +370,14 @@ PyObject *decode_append_rope(PyObject *, PyObject *const *args, Py_ssize_t n) {
     Held held;
     if (!q || !k || !v || args[6] == Py_None || !decode_params(p, *q, *k, *v, args[6], args[7]) || !new_row(nk, *k) || !new_row(nv, *k)) return nothing_done();
     if (q->stride(2) != 1 || !rope_tables(r, held, args[0], q->scalar_type(), q->size(2), *q)) return nothing_done();
-    at::Tensor out = fresh(q->sizes(), *q, q->scalar_type());
-    const size_t need = lib.decode_append_rope_workspace(&p);
-    at::Tensor ws = scratch(need, *q);
-    const int rc = unlocked(lib.decode_append_rope, &p, &r, nullptr, 0, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
-                                                need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    at::Tensor out;
+    const int rc = unlocked([&] {
+        out = fresh(q->sizes(), *q, q->scalar_type());
+        const size_t need = lib.decode_append_rope_workspace(&p);
+        at::Tensor ws = scratch(need, *q);
+        return lib.decode_append_rope(&p, &r, nullptr, 0, pointer(*q), pointer(*nk), pointer(*nv), pointer(*k), pointer(*v), pointer(out),
+                                      need ? ws.data_ptr() : nullptr, need, stream_of(*q));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS
@@ -392,12 +410,17 @@ PyObject *sample(PyObject *, PyObject *const *args, Py_ssize_t n) {
     const uint32_t no_ids = 0;
     p.masked = &no_ids;
     p.token_elem_bytes = 8;
-    at::Tensor tokens = fresh({p.b}, *z, at::kLong);
-    at::Tensor logprob = fresh({p.b}, *z, at::kFloat), tempered = fresh({p.b}, *z, at::kFloat), sampling = fresh({p.b}, *z, at::kFloat);
-    const size_t need = lib.sample_workspace(&p);
-    at::Tensor ws = scratch(need, *z);
-    const int rc = unlocked(lib.sample, &p, pointer(*z), pointer(tokens), static_cast<float *>(pointer(logprob)), static_cast<float *>(pointer(tempered)),
-                               static_cast<float *>(pointer(sampling)), need ? ws.data_ptr() : nullptr, need, stream_of(*z));
+    at::Tensor tokens, logprob, tempered, sampling;
+    const int rc = unlocked([&] {
+        tokens = fresh({p.b}, *z, at::kLong);
+        logprob = fresh({p.b}, *z, at::kFloat);
+        tempered = fresh({p.b}, *z, at::kFloat);
+        sampling = fresh({p.b}, *z, at::kFloat);
+        const size_t need = lib.sample_workspace(&p);
+        at::Tensor ws = scratch(need, *z);
+        return lib.sample(&p, pointer(*z), pointer(tokens), static_cast<float *>(pointer(logprob)), static_cast<float *>(pointer(tempered)),
+                          static_cast<float *>(pointer(sampling)), need ? ws.data_ptr() : nullptr, need, stream_of(*z));
+    });
     if (rc != DASH_ATTN_OK) return PyLong_FromLong(rc);
     return wrapped({tokens, logprob, tempered, sampling});
     END_HANDLE_TH_ERRORS

@@ -1,5 +1,11 @@
 """The native host side makes the very call the Python side makes: the same bits out, the same refusals, and what it leaves to
 the Python side (other devices' streams, transforms, layouts to copy) still runs."""
+import ctypes
+import pathlib
+import subprocess
+import threading
+import time
+
 import pytest
 import torch
 
@@ -144,3 +150,86 @@ def test_what_only_an_attribute_holds_outlives_the_call():
     got = A.attention_with_lse(q, k, v, Fresh(), AttentionOptions())
     assert torch.cuda.max_memory_allocated() - before >= size[0] + sum(x.untyped_storage().nbytes() for x in got)
     assert len(size) == 1 and all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+WAITING_ALLOCATOR = r"""
+#include <cuda_runtime_api.h>
+#include <sys/types.h>
+#include <unistd.h>
+extern "C" {
+volatile int waiting = 0, go = 0, late = 0;
+void *take(ssize_t size, int, cudaStream_t) {
+    waiting = 1;
+    for (int i = 0; i < 3000 && !go; ++i) usleep(1000);
+    if (!go) late = 1;
+    void *p = nullptr;
+    return cudaMalloc(&p, size) == cudaSuccess ? p : nullptr;
+}
+void give(void *p, ssize_t, int, cudaStream_t) { cudaFree(p); }
+}
+"""
+
+
+def test_other_threads_run_while_the_outputs_are_allocated(tmp_path):
+    """An allocator that waits (three seconds at most) for another Python thread to let it go on."""
+    source, path = tmp_path / "waiting.cpp", tmp_path / "waiting.so"
+    source.write_text(WAITING_ALLOCATOR)
+    cuda = pathlib.Path("/usr/local/cuda")
+    subprocess.run(["g++", "-shared", "-fPIC", f"-I{cuda}/include", str(source), "-o", str(path), f"-L{cuda}/lib64", "-lcudart"], check=True)
+    flags = ctypes.CDLL(str(path))
+    waiting, go, late = (ctypes.c_int.in_dll(flags, n) for n in ("waiting", "go", "late"))
+    q, k = randn(2, 8, 128), randn(2, 500, 2, 128)
+    want = A.attention_decode(q, k, k)
+
+    def let_go():
+        for _ in range(5000):
+            if waiting.value:
+                break
+            time.sleep(0.001)
+        go.value = 1
+
+    pool = torch.cuda.MemPool(torch.cuda.memory.CUDAPluggableAllocator(str(path), "take", "give").allocator())
+    other = threading.Thread(target=let_go)
+    other.start()
+    with torch.cuda.use_mem_pool(pool):
+        got = A.attention_decode(q, k, k)
+    other.join()
+    assert waiting.value and not late.value
+    assert torch.equal(got, want)
+    torch.cuda.synchronize()
+
+
+def test_an_allocation_that_fails_is_raised():
+    q = torch.empty(1, 1, 1, 64, dtype=torch.bfloat16, device="cuda").expand(1, 1 << 20, 2048, 64)   # 256 GB of output
+    with pytest.raises(torch.OutOfMemoryError):
+        A.attention(q, q, q)
+    small = randn(1, 4, 2, 64)
+    assert torch.isfinite(A.attention(small, small, small)).all()
+
+
+def test_two_threads_on_two_streams():
+    """Each thread's calls are its own: parameters, outputs and scratch, on its own stream."""
+    def work(seed, out):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            q, k = randn(3, 8, 128, seed=seed), randn(3, 900, 2, 128, seed=seed)
+            tq, tk = randn(1, 200, 4, 64, seed=seed), randn(1, 200, 2, 64, seed=seed)
+            cu = torch.tensor([0, 90 + seed, 200], dtype=torch.int32, device="cuda")
+            mask, options = AttentionMask.packed(cu, cu), AttentionOptions(causal=True)
+            for _ in range(60):
+                o, lse = A.attention_with_lse(tq, tk, tk, mask, options)
+                out.append((A.attention_decode(q, k, k), o, lse, *A.attention_backward(tq, tk, tk, o, lse, tq, mask, options)))
+            torch.cuda.current_stream().synchronize()
+
+    alone = [[], []]
+    for seed in (0, 1):
+        work(seed, alone[seed])
+    both = [[], []]
+    threads = [threading.Thread(target=work, args=(seed, both[seed])) for seed in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for seed in (0, 1):
+        assert len(both[seed]) == 60
+        for made in both[seed]:
+            assert all(torch.equal(x, y) for x, y in zip(made, alone[seed][0]))
