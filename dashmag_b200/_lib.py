@@ -11,6 +11,7 @@ import importlib.util
 import os
 import pathlib
 import struct
+import warnings
 
 HERE = pathlib.Path(__file__).resolve().parent
 #: The built library; DASH_ATTN_LIBRARY names another build of the same sources (for experiments).
@@ -187,19 +188,42 @@ BOUND = ("dash_attn_forward_workspace", "dash_attn_forward", "dash_attn_backward
          "dash_attn_decode_append_rope_workspace", "dash_attn_decode_append_rope", "dash_sample_workspace", "dash_sample")
 
 
-def binding():
-    """The entry points' native host side (``csrc/binding.cpp``).  Raises if it has not been built."""
-    global _binding
-    if _binding is None:
-        if not BINDING_PATH.exists():
-            raise RuntimeError(f"{BINDING_PATH} is missing: build it with `python -m dashmag_b200.build`.")
-        import torch  # noqa: F401  (the binding's symbols)
+class _Declines:
+    """Stands in for the native host side where there is none: leaves every call to the Python side."""
 
-        loader = importlib.machinery.ExtensionFileLoader("_binding", str(BINDING_PATH))
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def _load_binding():
+    """The native host side, or why it cannot be used."""
+    if not BINDING_PATH.exists():
+        return None, f"{BINDING_PATH} is missing"
+    import torch  # (the binding's symbols)
+
+    loader = importlib.machinery.ExtensionFileLoader("_binding", str(BINDING_PATH))
+    try:
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_binding", loader))
         loader.exec_module(module)
+    except ImportError as e:
+        return None, str(e)
+    if getattr(module, "torch", None) != torch.__version__:
+        return None, f"{BINDING_PATH} was built for torch {getattr(module, 'torch', None)} and this is {torch.__version__}"
+    return module, None
+
+
+def binding():
+    """The entry points' native host side (``csrc/binding.cpp``).  Without one that was built for this torch the Python side makes
+    every call, which takes longer on the host: a warning says so, once."""
+    global _binding
+    if _binding is None:
         handle = lib()
-        module.use(*(ctypes.cast(getattr(handle, name), vp).value for name in BOUND))
+        module, why = _load_binding()
+        if module is None:
+            warnings.warn(f"{why}: calls go through the Python side; `python -m dashmag_b200.build` builds it.", RuntimeWarning, stacklevel=3)
+            module = _Declines()
+        else:
+            module.use(*(ctypes.cast(getattr(handle, name), vp).value for name in BOUND))
         _binding = module
     return _binding
 

@@ -80,8 +80,6 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
 def build_binding(cxx: str, force: bool = False) -> pathlib.Path:
     source = CSRC / "binding.cpp"
     newest = max(source.stat().st_mtime, *(h.stat().st_mtime for h in INCLUDE.glob("*.h")))
-    if not force and BINDING.exists() and BINDING.stat().st_mtime > newest:
-        return BINDING
     import sysconfig
 
     import torch
@@ -89,11 +87,16 @@ def build_binding(cxx: str, force: bool = False) -> pathlib.Path:
     root = pathlib.Path(torch.__file__).resolve().parent
     cuda = pathlib.Path(_nvcc()).resolve().parent.parent
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DDASH_BUILT_FOR_TORCH="{torch.__version__}"',
            f"-I{root}/include", f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}", str(source), "-o", str(BINDING),
            f"-L{root}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    made_by = OBJ / "binding.cmd"   # another torch, compiler or place of either: another command
+    if not force and BINDING.exists() and BINDING.stat().st_mtime > newest and made_by.exists() and made_by.read_text() == " ".join(cmd):
+        return BINDING
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"the binding did not build:\n{r.stdout}\n{r.stderr}")
+    made_by.write_text(" ".join(cmd))
     return BINDING
 
 

@@ -457,4 +457,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, n
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding(void) { return PyModule_Create(&module); }
+// `torch`: the version this was built for.  Nothing of torch's is touched until a function is called.
+PyMODINIT_FUNC PyInit__binding(void) {
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "torch", DASH_BUILT_FOR_TORCH) < 0) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

@@ -61,3 +61,43 @@ def test_the_binding_calls_the_library_that_is_loaded():
         b.use(*[0] * len(_lib.BOUND))
     for name in _lib.BOUND:
         assert ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value
+
+
+@pytest.mark.parametrize("what", ["missing", "another torch", "not an extension"])
+def test_without_a_native_host_side_the_python_side_makes_the_calls(what, monkeypatch, tmp_path):
+    monkeypatch.setattr(_lib, "_binding", None)
+    if what == "another torch":
+        monkeypatch.setattr(torch, "__version__", "2.0.0")
+    else:
+        path = tmp_path / "_binding.so"
+        if what == "not an extension":
+            path.write_bytes(b"no library")
+        monkeypatch.setattr(_lib, "BINDING_PATH", path)
+    with pytest.warns(RuntimeWarning, match="the Python side"):
+        b = _lib.binding()
+    assert _lib.binding() is b and b.forward(1, 2) is None
+    q, k, v = tensors()
+    with pytest.raises(Unsupported):
+        attention(q, k, v)
+
+
+def test_another_torch_builds_the_binding_anew(monkeypatch, tmp_path):
+    from dashmag_b200 import build
+
+    commands = []
+    monkeypatch.setattr(build, "BINDING", tmp_path / "_binding.so")
+    monkeypatch.setattr(build, "OBJ", tmp_path)
+
+    class Done:
+        returncode = 0
+
+    def compiler(cmd, **kwargs):
+        commands.append(cmd)
+        (tmp_path / "_binding.so").write_bytes(b"")
+        return Done
+
+    monkeypatch.setattr(build.subprocess, "run", compiler)
+    for version, made in (("2.0.0", 1), ("2.0.0", 1), ("2.0.1", 2), ("2.0.1", 2)):
+        monkeypatch.setattr(torch, "__version__", version)
+        build.build_binding("g++")
+        assert len(commands) == made
