@@ -22,7 +22,7 @@
 // half the reads of shared memory a product.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
 // Two packed sequences of 384 tokens, four heads of 64, f32: the step 254 ->
 // 61 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
-// another), and 53 with the tiles two at a time; 381 tokens, 3 / 1 heads of 96, 74 -> 55, 590 148 -> 103, 1478 of 64 345 -> 246
+// another), and 57 with the tiles two at a time; 381 tokens, 3 / 1 heads of 96, 74 -> 55, 590 148 -> 103, 1478 of 64 345 -> 246
 // (the sums of two halves are nearer to f64 than one: dk of that call 9.3e-7 -> 6.8e-7).
 #include <algorithm>
 
