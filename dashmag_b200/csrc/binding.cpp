@@ -15,6 +15,7 @@
 #include <c10/util/SmallVector.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cfloat>
@@ -70,10 +71,19 @@ PyObject *nothing_done() {
     Py_RETURN_NONE;
 }
 
-// A plain strided CUDA tensor: torch.Tensor or Parameter itself, no wrapper, no mode that watches (of functions or of dispatch:
-// what the Python side asks torch for such a mode sees).
+// Whether a torch-function mode would see what the Python side asks torch for.  A default device is such a mode too, but one that has
+// nothing to say about allocations whose device is given.
+PyObject *default_device_mode = nullptr;   // its type (use(), below)
+bool watched() {
+    if (!at::impl::torch_function_mode_enabled()) return false;
+    for (int64_t i = 0; i < at::impl::PythonTorchFunctionTLS::stack_len(); ++i)
+        if (reinterpret_cast<PyObject *>(Py_TYPE(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter()))) != default_device_mode) return true;
+    return false;
+}
+
+// A plain strided CUDA tensor: torch.Tensor or Parameter itself, no wrapper, no mode that watches, of functions or of dispatch.
 const at::Tensor *plain(PyObject *o) {
-    if (!THPVariable_CheckExact(o) || at::impl::torch_function_mode_enabled()) return nullptr;
+    if (!THPVariable_CheckExact(o) || watched()) return nullptr;
     const at::Tensor &t = THPVariable_Unpack(o);
     if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || at::isTensorSubclassLike(t)) return nullptr;
     return &t;
@@ -436,6 +446,11 @@ PyObject *use(PyObject *, PyObject *const *args, Py_ssize_t n) {
         if (!at[i]) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_ValueError, "use: address %zd is null", i);
     }
     memcpy(&lib, at, sizeof lib);
+    if (!default_device_mode) {
+        Ref module(PyImport_ImportModule("torch.utils._device"));
+        if (module.p) default_device_mode = PyObject_GetAttrString(module.p, "DeviceContext");
+        PyErr_Clear();   // (without it every mode watches)
+    }
     Py_RETURN_NONE;
 }
 

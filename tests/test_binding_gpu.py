@@ -152,6 +152,16 @@ def test_a_mode_that_watches_sees_the_allocations():
         assert any("empty" in s for s in seen), mode
 
 
+def test_a_default_device_does_not_watch(monkeypatch):
+    q, k = randn(1, 4, 2, 64), randn(1, 4, 2, 64)
+    want = A.attention(q, k, k)
+    noted = Noted(_lib.binding())
+    monkeypatch.setattr(_lib, "_binding", noted)
+    with torch.device("cpu"):
+        got = A.attention(q, k, k)
+    assert noted.made == [True] and torch.equal(got, want)
+
+
 def test_what_only_an_attribute_holds_outlives_the_call():
     """A mask whose tensor is made anew each time it is asked for: the call alone holds it, and must until its kernels are launched -
     while the outputs are allocated, that is, the tensor's memory is not free."""
