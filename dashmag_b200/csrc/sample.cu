@@ -466,8 +466,7 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     };
     if (tempered_differs) sums(std::true_type{});
     else sums(std::false_type{});
-    // (By the id alone: of logits that are all NaN none compares with the maximum.)
-    if (degenerate) each_open([&](int i, T) { first = min(first, i); });
+    if (LIST && degenerate) each_open([&](int i, T zi) { if (Num<T>::to_f32(zi) == m) first = min(first, i); });
     // The sums, and what the blocks have listed, in one meeting.
     s1 = block_reduce(s1, AddOp(), fs);
     if (tempered_differs) wu = block_reduce(wu, AddOp(), fs);
@@ -526,6 +525,8 @@ __global__ void __launch_bounds__(ST) sample_kernel(SampleArgs a) {
     float tempered = 0.f, sampling = 0.f;
     bool own_tempered = true, own_sampling = true;   // false: the value is another output's (same bits)
     if (a.greedy || degenerate) {
+        if (first == a.v)   // all NaN: none equals the maximum
+            for (first = 0; masked(first); ++first) {}
         token = first;
     } else {
         // 3. The cuts: one threshold T on the keys; 0 keeps every token.
