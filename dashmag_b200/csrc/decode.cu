@@ -90,6 +90,9 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool v
     const int bytes = valid ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -299,21 +302,40 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_kernel(DecodeArgs
 // The split pass on the tensor cores (16-bit cache, head dimension 64, 128 or 256, groups of two heads or more)
 // ---------------------------------------------------------------------------------------------
 // With several query heads to a key-value head the scalar pass spends its time on FMA issue,
-// not on HBM: a cache row of 512 bytes feeds 2048 multiply-adds.  Here the query heads of the group
-// are the M dimension of warp-level MMAs (m16n8k16): S = Q K^T with the 16 keys of a tile as two
-// N tiles, then O += P V with P taken straight from the accumulator registers of S as the A
-// operand.  One warp per (chunk, key-value head) as before, with a ring of its own in shared memory:
-// every lane copies 16-byte pieces of the tile's 16 key rows and 16 value rows asynchronously, two
-// tiles ahead, into rows (256 bytes at D = 128) whose 16-byte chunks are XOR-swizzled by the row, and ldmatrix
-// reads the fragments from there without bank conflicts (transposed for V).
+// not on HBM: a cache row of 512 bytes feeds 2048 multiply-adds.  Here warp-level MMAs (m16n8k16) do the products.  Groups of up to
+// eight heads are the N dimension of the transposed products, S^T = K Q^T with the 16 keys of a tile as M, then O^T += V^T P^T
+// with the features as M: half the MMAs, half the exponentials and half the accumulators of rows of sixteen heads, most of them
+// not there.  (D 128, a group of four: 24 MMAs a tile and not 48.)  Larger groups (WIDE) are the M dimension, S = Q K^T with the
+// 16 keys as two N tiles, then O += P V with P taken straight from the accumulator registers of S as the A operand: two column
+// tiles of eight heads in the other form measured slower by a tenth, its 8 x 8 transposes and its maxima over eight lanes cost more.
+// One warp per (share of the keys, key-value head), with a ring of its own in shared memory: every lane copies 16-byte pieces of
+// the tile's 16 key rows and 16 value rows asynchronously, two tiles ahead, into rows (256 bytes at D = 128) whose 16-byte chunks
+// are XOR-swizzled by the row, and ldmatrix reads the fragments from there without bank conflicts (transposed for V).  What a warp
+// waits for in a tile is its own chain, not memory (six stages for three change nothing, 0.8 us a tile where four warps are
+// alone on a multiprocessor): all fragments are fetched in front of the products, V's under the softmax, no product follows
+// the one it depends on, and a tile's copies go out from running addresses (0.5 us).  One sequence of 2047 keys, 32 / 8 heads of 128,
+// split and merge, 13.0 -> 12.5 us, 16 of 16384 104.9 -> 96.2, groups of sixteen, 40 sequences of 20000, 55.9 -> 53.5.
+//
+// CLUSTER: the blocks of a cluster take one (sequence, key-value head) together, its tiles dealt evenly over their warps by the
+// length the sequence really has, and meet in distributed shared memory: each block merges its warps' sums, hands every block of
+// the cluster the outputs that block finishes, and finishes its own.  No partials in HBM, no merge kernel behind the pass (3.3 us
+// of an 8 us step), no chunks past the lengths (figures at decode_cluster).
 constexpr int DM_STAGES = 3;    // tiles of the per-warp ring
 constexpr int DM_KEYS = 16;     // keys per tile
 
+// The 8 x 8 matrix of 16-bit values held two a lane (row lane / 4, columns 2 (lane % 4), + 1), transposed.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+    uint32_t r;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+
 template <typename T> struct MmaType;
 template <> struct MmaType<__nv_bfloat16> {
+    static constexpr bool NARROW = false;   // of exponents
     using Two = __nv_bfloat162;
     static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     }
     static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
@@ -324,9 +346,10 @@ template <> struct MmaType<__nv_bfloat16> {
     static __device__ __forceinline__ float hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 };
 template <> struct MmaType<__half> {
+    static constexpr bool NARROW = true;
     using Two = __half2;
     static __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
     }
     static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
@@ -366,10 +389,30 @@ __device__ __forceinline__ uint32_t rotate_two(uint32_t x, uint32_t partner, uin
     return *reinterpret_cast<uint32_t *>(&r);
 }
 
-template <typename T, int D, int PARTS, int WARPS, bool ROPE>
+// ---- the blocks of a cluster -------------------------------------------------------------------
+constexpr int MAX_CLUSTER = 16, CLUSTER_WARPS = 4;
+__device__ __forceinline__ uint32_t cluster_blocks() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// To the place that `mine` is in this block, in block `rank`.
+__device__ __forceinline__ uint32_t cluster_address(const void *mine, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(mine))), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(void *mine, int rank, float4 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_address(mine, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void cluster_store(void *mine, int rank, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_address(mine, rank)), "f"(v.x), "f"(v.y) : "memory");
+}
+
+template <typename T, int D, int PARTS, bool WIDE, int WARPS, bool ROPE, int TOGETHER>
 __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs a) {
     constexpr int DM_WARPS = WARPS;
-    allow_beside();   // the merge
+    constexpr bool CLUSTER = TOGETHER > 0, FOLDS = TOGETHER == 2;
+    if constexpr (!CLUSTER) allow_beside();   // the merge
     constexpr int DFULL = D * PARTS;            // the head dimension; D is what one warp takes of it
     constexpr int ROWB = 2 * D;                 // bytes of a warp's part of a cache row: 256 at D = 128, 128 at D = 64
     constexpr int CH = D / 8;                   // its 16-byte chunks
@@ -379,38 +422,99 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int group = a.hq / a.hkv;
     const int b = blockIdx.y;
-    const long long unit = ((long long)blockIdx.x * DM_WARPS + wib) / PARTS;
+    const int csize = CLUSTER ? (int)cluster_blocks() : 1, crank = CLUSTER ? (int)cluster_rank() : 0;
+    if constexpr (CLUSTER) cluster_arrive();   // (every block of the cluster runs before the first one's memory is written to)
+    const long long unit = CLUSTER ? blockIdx.x / csize : ((long long)blockIdx.x * DM_WARPS + wib) / PARTS;
     const int part = wib % PARTS, d0 = part * D;   // this warp's features [d0, d0 + D)
-    // A unit: sixteen query heads of a group (the M rows of the MMAs; a group of more takes several
+    // A unit: eight query heads of a group, or sixteen (WIDE; a group of more takes several
     // units side by side, whose warps read the same chunk of the cache at the same time: once from
     // HBM, the rest from L2), a key-value head, a chunk.
-    const int hblocks = (group + 15) / 16;
-    const int g_base = (int)(unit % hblocks) * 16;
+    constexpr int HEADS = WIDE ? 16 : 8;
+    static_assert(!(WIDE && CLUSTER), "sixteen heads meet in the merge");
+    const int hblocks = (group + HEADS - 1) / HEADS;
+    const int g_base = (int)(unit % hblocks) * HEADS;
     const int hk = (int)((unit / hblocks) % a.hkv);
-    const long long split = unit / hblocks / a.hkv;
-    if (split >= a.splits) return;
+    const long long split = CLUSTER ? 0 : unit / hblocks / a.hkv;
+    if (!CLUSTER && split >= a.splits) return;
     int first, len;
     decode_range(a, b, first, len);
-    const long long c0l = (long long)first + split * a.chunk;
-    if (c0l >= len) return;
-    const int c0 = (int)c0l, c1 = min(len, c0 + a.chunk);
-    const int iters = (c1 - c0 + DM_KEYS - 1) / DM_KEYS;
-
-    const int g = lane >> 2, t = lane & 3;   // fragment coordinates: row (head) g and g + 8, column pair t
-    // Q as the A operand of every score MMA: [16 heads x 16 d] per k-step, rows past the group zero.
-    uint32_t qa[D / 16][4];
-    {
-        const T *q0 = static_cast<const T *>(a.q) + (int64_t)b * a.q_sb + (int64_t)(hk * group + min(g_base + g, group - 1)) * a.q_sh + d0;
-        const T *q1 = static_cast<const T *>(a.q) + (int64_t)b * a.q_sb + (int64_t)(hk * group + min(g_base + g + 8, group - 1)) * a.q_sh + d0;
-        const bool live0 = g_base + g < group, live1 = g_base + g + 8 < group;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-            qa[ks][0] = live0 ? *reinterpret_cast<const uint32_t *>(q0 + ks * 16 + 2 * t) : 0u;
-            qa[ks][1] = live1 ? *reinterpret_cast<const uint32_t *>(q1 + ks * 16 + 2 * t) : 0u;
-            qa[ks][2] = live0 ? *reinterpret_cast<const uint32_t *>(q0 + ks * 16 + 8 + 2 * t) : 0u;
-            qa[ks][3] = live1 ? *reinterpret_cast<const uint32_t *>(q1 + ks * 16 + 8 + 2 * t) : 0u;
-        }
+    int c0, c1;
+    if constexpr (CLUSTER) {
+        // The tiles of what the sequence really sees, dealt evenly over the cluster's warps in order; some may get none.
+        constexpr int PER = DM_WARPS / PARTS;
+        const int tiles = (max(len - first, 0) + DM_KEYS - 1) / DM_KEYS, shares = csize * PER, mine = crank * PER + wib / PARTS;
+        c0 = first + (int)((long long)tiles * mine / shares) * DM_KEYS;
+        c1 = min(len, first + (int)((long long)tiles * (mine + 1) / shares) * DM_KEYS);
+    } else {
+        const long long c0l = (long long)first + split * a.chunk;
+        if (c0l >= len) return;
+        c0 = (int)c0l;
+        c1 = min(len, c0 + a.chunk);
     }
+    const int iters = max(c1 - c0 + DM_KEYS - 1, 0) / DM_KEYS;
+
+    const T *kbase = static_cast<const T *>(a.k.ptr) + (int64_t)b * a.k.sb + (int64_t)hk * a.k.sh + d0;
+    const T *vbase = static_cast<const T *>(a.v.ptr) + (int64_t)b * a.v.sb + (int64_t)hk * a.v.sh + d0;
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(dm_ring)) + (uint32_t)wib * DM_STAGES * 2 * DM_TILE;
+
+    // This lane's pieces of a tile: chunk (lane % 16) of rows (lane / 16) + 2 j.
+    const int cp_chunk = lane % CH, cp_row0 = lane / CH;
+    constexpr int RPP = 32 / CH;                // rows the warp copies per pass
+    // The appending step: the row at `pos` comes from the new rows, and the warp whose chunk holds it also writes it into the
+    // cache, below.
+    const int pos = decode_append_at(a, b);
+    const T *knew = static_cast<const T *>(a.k_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
+    const T *vnew = static_cast<const T *>(a.v_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
+    const int pos_it = (pos >= c0 && pos < c1) ? (pos - c0) / DM_KEYS : -1;   // the tile of the new row, if this chunk holds it
+    // (The rows of a lane differ from its first by whole multiples of a power of two above it, so their swizzles by one exclusive or.)
+    const uint32_t to0 = ring + (uint32_t)(cp_row0 * ROWB), sw0 = (uint32_t)((cp_chunk ^ cp_row0) << 4);
+    const int64_t k_hop = RPP * a.k.st, v_hop = RPP * a.v.st;
+    auto issue = [&](int it) {
+        if (it < iters) {
+            const uint32_t dst = to0 + (uint32_t)(it % DM_STAGES) * 2 * DM_TILE;
+            const int key0 = c0 + it * DM_KEYS + cp_row0;
+            const T *kp = kbase + (int64_t)key0 * a.k.st + cp_chunk * 8, *vp = vbase + (int64_t)key0 * a.v.st + cp_chunk * 8;
+            if (c0 + (it + 1) * DM_KEYS <= c1 && it != pos_it) {
+#pragma unroll
+                for (int j = 0; j < DM_KEYS / RPP; ++j) {
+                    const uint32_t at = dst + (uint32_t)(RPP * j * ROWB) + (sw0 ^ (uint32_t)(((RPP * j) & 7) << 4));
+                    cp_async16(at, kp);
+                    cp_async16(at + DM_TILE, vp);
+                    kp += k_hop;
+                    vp += v_hop;
+                }
+            } else {   // keys past the last are zeros; the new row comes from where it was given
+#pragma unroll
+                for (int j = 0; j < DM_KEYS / RPP; ++j) {
+                    const int key = key0 + RPP * j;
+                    const bool valid = key < c1, fresh = key == pos;
+                    const uint32_t at = dst + (uint32_t)(RPP * j * ROWB) + (sw0 ^ (uint32_t)(((RPP * j) & 7) << 4));
+                    cp_async16(at, fresh ? knew + cp_chunk * 8 : valid ? kp + j * k_hop : kbase + (int64_t)c0 * a.k.st, valid);
+                    cp_async16(at + DM_TILE, fresh ? vnew + cp_chunk * 8 : valid ? vp + j * v_hop : vbase + (int64_t)c0 * a.v.st, valid);
+                }
+            }
+        }
+        cp_async_commit();  // always, so that the group count stays in step with the tiles
+    };
+
+    const int g = lane >> 2, t = lane & 3;   // fragment coordinates
+    // Q as the operand of every score MMA.  Eight heads: the B operand, per k-step features 16 ks + 2 t, + 1 and those eight further
+    // on of head g.  Sixteen: the A operand [16 heads x 16 d], the same of heads g and g + 8.  Heads past the group are zero.
+    uint32_t qa[D / 16][WIDE ? 4 : 2];
+    const T *qg = static_cast<const T *>(a.q) + (int64_t)b * a.q_sb + (int64_t)(hk * group) * a.q_sh;
+    constexpr int QH = WIDE ? 2 : 1;   // heads a lane holds: g, and g + 8
+#pragma unroll
+    for (int x = 0; x < QH; ++x) {
+        const int head = g_base + g + 8 * x;
+        const T *row = qg + (int64_t)min(head, group - 1) * a.q_sh + d0 + 2 * t;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) qa[ks][j * QH + x] = head < group ? *reinterpret_cast<const uint32_t *>(row + ks * 16 + 8 * j) : 0u;
+    }
+    // The first tiles are on their way before the rotation's tables are asked for: that trip to memory falls under theirs.
+#pragma unroll
+    for (int s = 0; s < DM_STAGES - 1; ++s) issue(s);
     // The rotation's row of the tables (no such row: every rotated feature is a NaN, as rope_kernel has it).
     const int half = a.rope_dim / 2;
     const T *cos_row = nullptr, *sin_row = nullptr;
@@ -420,39 +524,26 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
             cos_row = static_cast<const T *>(a.rope_cos) + at * a.rope_dim;
             sin_row = static_cast<const T *>(a.rope_sin) + at * a.rope_dim;
         }
-        const T *qg = static_cast<const T *>(a.q) + (int64_t)b * a.q_sb + (int64_t)(hk * group) * a.q_sh;
-        const int64_t r0 = (int64_t)min(g_base + g, group - 1) * a.q_sh, r1 = (int64_t)min(g_base + g + 8, group - 1) * a.q_sh;
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
+        for (int x = 0; x < QH; ++x) {
+            const int head = g_base + g + 8 * x;
+            const T *row = qg + (int64_t)min(head, group - 1) * a.q_sh;
 #pragma unroll
-            for (int j = 0; j < 4; j += 2) {   // columns c, c + 1 of rows g and g + 8
-                const int c = d0 + ks * 16 + 4 * j + 2 * t;
-                if (c >= a.rope_dim) continue;
-                const bool low = c < half;
-                const int other = low ? c + half : c - half;
-                if (cos_row) {
-                    const uint32_t cs = *reinterpret_cast<const uint32_t *>(cos_row + c), sn = *reinterpret_cast<const uint32_t *>(sin_row + c);
-                    qa[ks][j] = rotate_two<T>(qa[ks][j], *reinterpret_cast<const uint32_t *>(qg + r0 + other), cs, sn, low);
-                    qa[ks][j + 1] = rotate_two<T>(qa[ks][j + 1], *reinterpret_cast<const uint32_t *>(qg + r1 + other), cs, sn, low);
-                } else {
-                    qa[ks][j] = qa[ks][j + 1] = 0x7fff7fffu;   // a NaN in either dtype
+            for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int c = d0 + ks * 16 + 8 * j + 2 * t;
+                    if (c >= a.rope_dim || head >= group) continue;
+                    const bool low = c < half;
+                    const int other = low ? c + half : c - half;
+                    uint32_t &q2 = qa[ks][j * QH + x];
+                    q2 = cos_row ? rotate_two<T>(q2, *reinterpret_cast<const uint32_t *>(row + other), *reinterpret_cast<const uint32_t *>(cos_row + c),
+                                                 *reinterpret_cast<const uint32_t *>(sin_row + c), low)
+                                 : 0x7fff7fffu;   // a NaN in either dtype
                 }
-                if (g_base + g >= group) qa[ks][j] = 0u;
-                if (g_base + g + 8 >= group) qa[ks][j + 1] = 0u;
-            }
+        }
     }
-    const T *kbase = static_cast<const T *>(a.k.ptr) + (int64_t)b * a.k.sb + (int64_t)hk * a.k.sh + d0;
-    const T *vbase = static_cast<const T *>(a.v.ptr) + (int64_t)b * a.v.sb + (int64_t)hk * a.v.sh + d0;
-    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(dm_ring)) + (uint32_t)wib * DM_STAGES * 2 * DM_TILE;
-
-    // This lane's pieces of a tile: chunk (lane % 16) of rows (lane / 16) + 2 j.
-    const int cp_chunk = lane % CH, cp_row0 = lane / CH;
-    constexpr int RPP = 32 / CH;                // rows the warp copies per pass
-    // The appending step: the row at `pos` comes from the new rows, and the warp whose chunk holds
-    // it also writes it into the cache (D / 8 lanes the key row, D / 8 the value row).
-    const int pos = decode_append_at(a, b);
-    const T *knew = static_cast<const T *>(a.k_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
-    const T *vnew = static_cast<const T *>(a.v_new) + ((int64_t)b * a.hkv + hk) * DFULL + d0;
+    // (D / 8 lanes the new key row, D / 8 the value row.)
     uint4 row_chunk = make_uint4(0, 0, 0, 0);   // lanes below CH: this lane's chunk of the new key row, rotated if the step rotates
     if (pos >= c0 && pos < c1 && lane < 2 * CH) {
         row_chunk = *reinterpret_cast<const uint4 *>((lane < CH ? knew : vnew) + cp_chunk * 8);
@@ -473,34 +564,29 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
             *reinterpret_cast<uint4 *>(dst) = row_chunk;
         }
     }
-    const int pos_it = (pos >= c0 && pos < c1) ? (pos - c0) / DM_KEYS : -1;   // the tile of the new row, if this chunk holds it
-    auto issue = [&](int it) {
-        if (it < iters) {
-            const uint32_t dst = ring + (uint32_t)(it % DM_STAGES) * 2 * DM_TILE;
-#pragma unroll
-            for (int j = 0; j < DM_KEYS / RPP; ++j) {
-                const int row = cp_row0 + RPP * j, key = c0 + it * DM_KEYS + row;
-                const bool valid = key < c1;
-                const uint32_t at = (uint32_t)(row * ROWB + ((cp_chunk ^ (row & 7)) << 4));
-                const T *kp = kbase + (int64_t)(valid ? key : c0) * a.k.st, *vp = vbase + (int64_t)(valid ? key : c0) * a.v.st;
-                if (it == pos_it && key == pos) { kp = knew; vp = vnew; }   // only the tile that holds the new row looks for it
-                cp_async16(dst + at, kp + cp_chunk * 8, valid);
-                cp_async16(dst + DM_TILE + at, vp + cp_chunk * 8, valid);
-            }
-        }
-        cp_async_commit();  // always, so that the group count stays in step with the tiles
-    };
-
     const float sl = a.scale * 1.4426950408889634f;   // scores are exponentiated in base 2
-    float o[D / 8][4];
+    // The largest probability of a head: 1, or at f16, in a cluster's longer sweeps, 2^8 - the second part of a small probability is then no
+    // subnormal number, whose rounding would be the largest error of the sum.
+    constexpr float LIFT = CLUSTER && MmaType<T>::NARROW ? 8.f : 0.f;
+    // From one maximum to another: the difference of the two offsets as the exponentials used them, each product rounded on its own,
+    // so that what was summed against either shares one reference.
+    auto between = [sl](float from, float to) { return exp2f(__fsub_rn(__fmul_rn(from, sl), __fmul_rn(to, sl))); };
+    // The accumulator: eight heads have it transposed (rows are features, columns heads), sixteen as rows of heads.
+    constexpr int ON = WIDE ? D / 8 : D / 16;
+    float o[ON][4];
 #pragma unroll
-    for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // rows g and g + 8; l is this lane's share
+    for (int n = 0; n < ON; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    // A warp that sweeps more keys than a long chunk (TOGETHER 2; 512, at f16, whose P is sharper, 256): a product's additions to an
+    // accumulator that has grown large lose a little of it each, so every 256 keys what has gathered moves to a second accumulator.  (An instance of its own: the code
+    // costs a call of few tiles 0.6 us.  f16, 3000 keys a sequence, error against f64 where the output is next to nothing, 2.3e-8
+    // in chunks of 256; 3.4e-8 in 750 without, 2.1e-8 with it and LIFT.)
+    constexpr int FOLD = 256 / DM_KEYS;
+    float old[FOLDS ? ON : 1][4] = {};
+    // This lane's two heads (2 t and 2 t + 1; of sixteen: g and g + 8); l is the lane's share of their sums.
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
     // ldmatrix rows: lane -> (matrix lane / 8, row lane % 8)
     const int lm = lane >> 3, lr = lane & 7;
 
-#pragma unroll
-    for (int s = 0; s < DM_STAGES - 1; ++s) issue(s);
     for (int it = 0; it < iters; ++it) {
         __syncwarp();   // every lane is done with the stage about to be refilled
         issue(it + DM_STAGES - 1);
@@ -515,29 +601,60 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
             __syncwarp();
         }
 
-        // S[16 heads x 16 keys] as two N tiles of 8 keys.
-        float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        float sc[WIDE ? 2 : 1][4] = {};
+        uint32_t kf[D / 16][4], vf[D / 16][4];   // the tile's fragments
+        if constexpr (WIDE) {
+            // S[16 heads x 16 keys] as two N tiles of 8 keys.
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const int row = nt * 8 + lr;
+            for (int ks = 0; ks < D / 16; ks += 2)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {   // b0, b1 of k-step ks, then of ks + 1
+                    const int row = nt * 8 + lr;
+                    ldmatrix_x4(kt + (uint32_t)(row * ROWB + (((2 * ks + lm) ^ (row & 7)) << 4)), kf[ks + nt]);
+                }
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ks += 2)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) MmaType<T>::mma(sc[nt], qa[ks + j], kf[ks + nt][2 * j], kf[ks + nt][2 * j + 1]);
+        } else {
+            // S transposed, [16 keys x 8 heads]; the even and the odd k-steps as two chains.
+            float odd[4] = {};
+            const int row = (lm & 1) * 8 + lr;
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks)   // keys 0-7 and 8-15 of the k-step's first eight features, then of the others
+                ldmatrix_x4(kt + (uint32_t)(row * ROWB + (((2 * ks + (lm >> 1)) ^ (row & 7)) << 4)), kf[ks]);
 #pragma unroll
             for (int ks = 0; ks < D / 16; ks += 2) {
-                uint32_t kb[4];   // b0, b1 of k-step ks, then of ks + 1
-                ldmatrix_x4(kt + (uint32_t)(row * ROWB + (((2 * ks + lm) ^ (row & 7)) << 4)), kb);
-                MmaType<T>::mma(sc[nt], qa[ks], kb[0], kb[1]);
-                MmaType<T>::mma(sc[nt], qa[ks + 1], kb[2], kb[3]);
+                MmaType<T>::mma(sc[0], kf[ks], qa[ks][0], qa[ks][1]);
+                MmaType<T>::mma(odd, kf[ks + 1], qa[ks + 1][0], qa[ks + 1][1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sc[0][e] += odd[e];
+        }
+        // V's fragments are fetched under the softmax.
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) {
+            if constexpr (WIDE) {   // b0, b1 of eight features, then of the next eight
+                const int row = (lm & 1) * 8 + lr, chunk = 2 * n + (lm >> 1);
+                ldmatrix_x4_trans(vt + (uint32_t)(row * ROWB + ((chunk ^ (row & 7)) << 4)), vf[n]);
+            } else {                // features 0-7 and 8-15 of keys 0-7, then of keys 8-15
+                const int row = (lm >> 1) * 8 + lr, chunk = 2 * n + (lm & 1);
+                ldmatrix_x4_trans(vt + (uint32_t)(row * ROWB + ((chunk ^ (row & 7)) << 4)), vf[n]);
             }
         }
         if constexpr (PARTS == 2) {
             // The other half of the sum over the features is the neighbouring warp's: both write theirs, meet,
             // and add part 0's and part 1's in that order.
-            float *mine = dm_exchange + ((size_t)wib * 32 + lane) * 8, *other = dm_exchange + ((size_t)(wib ^ 1) * 32 + lane) * 8;
+            constexpr int SN = WIDE ? 2 : 1;
+            float *mine = dm_exchange + ((size_t)wib * 32 + lane) * 4 * SN, *other = dm_exchange + ((size_t)(wib ^ 1) * 32 + lane) * 4 * SN;
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int nt = 0; nt < SN; ++nt)
                 *reinterpret_cast<float4 *>(mine + 4 * nt) = make_float4(sc[nt][0], sc[nt][1], sc[nt][2], sc[nt][3]);
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (wib >> 1)) : "memory");
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
+            for (int nt = 0; nt < SN; ++nt) {
                 const float4 o4 = *reinterpret_cast<const float4 *>(other + 4 * nt);
                 const float theirs[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
@@ -545,70 +662,232 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
             }
             asm volatile("bar.sync %0, 64;" ::"r"(1 + (wib >> 1)) : "memory");   // both have read before the next tile's are written
         }
-        // Online softmax of rows g (values 0, 1 of a tile) and g + 8 (values 2, 3); a tile's columns
-        // are keys key0 + 8 nt + 2 t + {0, 1}.
-        if (key0 + DM_KEYS > c1) {
+        // Online softmax.  P goes to the tensor cores as the sum of two 16-bit values (what the rounding of the first
+        // loses is the second), so that the products keep the f32 accuracy of the scalar pass.
+        if constexpr (WIDE) {
+            // Rows g (values 0, 1 of a tile) and g + 8 (values 2, 3); a tile's columns are keys key0 + 8 nt + 2 t + {0, 1}.
+            if (key0 + DM_KEYS > c1) {
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (key0 + nt * 8 + 2 * t + (j & 1) >= c1) sc[nt][j] = -INFINITY;
+            }
+            uint32_t pa[4], pl[4];
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+                float mx = fmaxf(fmaxf(sc[0][2 * rr], sc[0][2 * rr + 1]), fmaxf(sc[1][2 * rr], sc[1][2 * rr + 1]));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float mn = fmaxf(m[rr], mx);
+                if (__any_sync(0xffffffffu, mn > m[rr])) {
+                    // The row's maximum grew (in some row of the warp): bring the sum and the accumulator along.
+                    const float corr = mn == -INFINITY ? 1.f : between(m[rr], mn);   // exp2(-inf) = 0 for a first maximum
+                    l[rr] *= corr;
+#pragma unroll
+                    for (int n = 0; n < ON; ++n) { o[n][2 * rr] *= corr; o[n][2 * rr + 1] *= corr; }
+                    m[rr] = mn;
+                }
+                const float base = m[rr] == -INFINITY ? 0.f : __fmul_rn(m[rr], sl);
+                const float p00 = exp2f(fmaf(sc[0][2 * rr], sl, -base)), p01 = exp2f(fmaf(sc[0][2 * rr + 1], sl, -base));
+                const float p10 = exp2f(fmaf(sc[1][2 * rr], sl, -base)), p11 = exp2f(fmaf(sc[1][2 * rr + 1], sl, -base));
+                l[rr] += (p00 + p01) + (p10 + p11);
+                pa[rr] = MmaType<T>::pack(p00, p01);       // a0 / a1: keys 2t, 2t + 1
+                pa[2 + rr] = MmaType<T>::pack(p10, p11);   // a2 / a3: keys 8 + 2t, 8 + 2t + 1
+                pl[rr] = MmaType<T>::pack(p00 - MmaType<T>::lo(pa[rr]), p01 - MmaType<T>::hi(pa[rr]));
+                pl[2 + rr] = MmaType<T>::pack(p10 - MmaType<T>::lo(pa[2 + rr]), p11 - MmaType<T>::hi(pa[2 + rr]));
+            }
+            // O[16 heads x D] += P[16 x 16 keys] V[16 keys x D]: one part of P over all features, then the other, so that no
+            // product waits for the one before it.
+#pragma unroll
+            for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], pa, vf[n / 2][2 * (n & 1)], vf[n / 2][2 * (n & 1) + 1]);
+#pragma unroll
+            for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], pl, vf[n / 2][2 * (n & 1)], vf[n / 2][2 * (n & 1) + 1]);
+        } else {
+            // Heads 2 t (values 0 and 2: keys g and g + 8) and 2 t + 1 (values 1 and 3).
+            if (key0 + DM_KEYS > c1) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (key0 + nt * 8 + 2 * t + (j & 1) >= c1) sc[nt][j] = -INFINITY;
-        }
-        // P goes to the tensor cores as the sum of two 16-bit values (what the rounding of the first
-        // loses is the second), so that the products keep the f32 accuracy of the scalar pass.
-        uint32_t pa[4], pl[4];
-#pragma unroll
-        for (int rr = 0; rr < 2; ++rr) {
-            float mx = fmaxf(fmaxf(sc[0][2 * rr], sc[0][2 * rr + 1]), fmaxf(sc[1][2 * rr], sc[1][2 * rr + 1]));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            const float mn = fmaxf(m[rr], mx);
-            if (__any_sync(0xffffffffu, mn > m[rr])) {
-                // The row's maximum grew (in some row of the warp): bring the sum and the accumulator along.
-                const float corr = mn == -INFINITY ? 1.f : exp2f((m[rr] - mn) * sl);   // exp2(-inf) = 0 for a first maximum
-                l[rr] *= corr;
-#pragma unroll
-                for (int n = 0; n < D / 8; ++n) { o[n][2 * rr] *= corr; o[n][2 * rr + 1] *= corr; }
-                m[rr] = mn;
+                    if (key0 + g + 8 * (j >> 1) >= c1) sc[0][j] = -INFINITY;
             }
-            const float base = m[rr] == -INFINITY ? 0.f : m[rr] * sl;
-            const float p00 = exp2f(fmaf(sc[0][2 * rr], sl, -base)), p01 = exp2f(fmaf(sc[0][2 * rr + 1], sl, -base));
-            const float p10 = exp2f(fmaf(sc[1][2 * rr], sl, -base)), p11 = exp2f(fmaf(sc[1][2 * rr + 1], sl, -base));
-            l[rr] += (p00 + p01) + (p10 + p11);
-            pa[rr] = MmaType<T>::pack(p00, p01);       // a0 / a1: keys 2t, 2t + 1
-            pa[2 + rr] = MmaType<T>::pack(p10, p11);   // a2 / a3: keys 8 + 2t, 8 + 2t + 1
-            pl[rr] = MmaType<T>::pack(p00 - MmaType<T>::lo(pa[rr]), p01 - MmaType<T>::hi(pa[rr]));
-            pl[2 + rr] = MmaType<T>::pack(p10 - MmaType<T>::lo(pa[2 + rr]), p11 - MmaType<T>::hi(pa[2 + rr]));
-        }
-        // O[16 heads x 128 d] += P[16 x 16 keys] V[16 keys x 128 d], two N tiles of 8 d per load.
+            // A maximum moves in few tiles once some have been seen: a vote says whether one does in this, and only then the
+            // lanes tell one another theirs and bring the sums and the accumulator along.
+            const float mx0 = fmaxf(sc[0][0], sc[0][2]), mx1 = fmaxf(sc[0][1], sc[0][3]);
+            if (__any_sync(0xffffffffu, mx0 > m[0] || mx1 > m[1])) {
 #pragma unroll
-        for (int n = 0; n < D / 8; n += 2) {
-            uint32_t vb[4];   // b0, b1 of d-tile n, then of n + 1
-            const int row = (lm & 1) * 8 + lr, chunk = n + (lm >> 1);
-            ldmatrix_x4_trans(vt + (uint32_t)(row * ROWB + ((chunk ^ (row & 7)) << 4)), vb);
-            MmaType<T>::mma(o[n], pa, vb[0], vb[1]);
-            MmaType<T>::mma(o[n], pl, vb[0], vb[1]);
-            MmaType<T>::mma(o[n + 1], pa, vb[2], vb[3]);
-            MmaType<T>::mma(o[n + 1], pl, vb[2], vb[3]);
+                for (int e = 0; e < 2; ++e) {
+                    float mx = e == 0 ? mx0 : mx1;
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                    const float mn = fmaxf(m[e], mx);
+                    const float corr = mn == -INFINITY ? 1.f : between(m[e], mn);   // exp2(-inf) = 0 for a first maximum
+                    l[e] *= corr;
+#pragma unroll
+                    for (int n = 0; n < ON; ++n) { o[n][e] *= corr; o[n][2 + e] *= corr; }
+                    if constexpr (FOLDS) {
+                        if (it >= FOLD) {
+#pragma unroll
+                            for (int n = 0; n < ON; ++n) { old[n][e] *= corr; old[n][2 + e] *= corr; }
+                        }
+                    }
+                    m[e] = mn;
+                }
+            }
+            float p[4];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float base = m[e] == -INFINITY ? 0.f : __fmul_rn(m[e], sl);
+                if constexpr (LIFT > 0.f) base -= LIFT;
+                p[e] = exp2f(fmaf(sc[0][e], sl, -base));
+                p[2 + e] = exp2f(fmaf(sc[0][2 + e], sl, -base));
+                l[e] += p[e] + p[2 + e];
+            }
+            // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; the longer sweeps of a cluster have
+            // fewer of them, and at bf16 a third part of P makes up for it (8 sequences of 8766 keys, error against f64 where the output
+            // is next to nothing: 3.8e-8 in chunks, 4.4e-8 with two parts, 2.0e-8 with three).
+            constexpr bool THIRD = CLUSTER && !MmaType<T>::NARROW;
+            uint32_t pa[2], pl[2], pm[2];   // an 8 x 8 transpose each makes the accumulator's layout the B operand's
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {   // keys 0 to 7 of the tile, then 8 to 15
+                const uint32_t hi = MmaType<T>::pack(p[2 * j], p[2 * j + 1]);
+                const float r0 = p[2 * j] - MmaType<T>::lo(hi), r1 = p[2 * j + 1] - MmaType<T>::hi(hi);
+                const uint32_t low = MmaType<T>::pack(r0, r1);
+                pa[j] = transpose_8x8(hi);
+                pl[j] = transpose_8x8(low);
+                if constexpr (THIRD) pm[j] = transpose_8x8(MmaType<T>::pack(r0 - MmaType<T>::lo(low), r1 - MmaType<T>::hi(low)));
+            }
+            // O[D x 8 heads] += V^T[D x 16 keys] P^T[16 keys x 8 heads]
+#pragma unroll
+            for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], vf[n], pa[0], pa[1]);
+#pragma unroll
+            for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], vf[n], pl[0], pl[1]);
+            if constexpr (THIRD) {
+#pragma unroll
+                for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], vf[n], pm[0], pm[1]);
+            }
+            if constexpr (FOLDS) {
+                if (it % FOLD == FOLD - 1) {
+#pragma unroll
+                    for (int n = 0; n < ON; ++n)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) { old[n][e] += o[n][e]; o[n][e] = 0.f; }
+                }
+            }
         }
     }
     cp_async_wait<0>();
+    // Each head's sum over the lanes that share it.
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int x = WIDE ? 1 : 4; x < (WIDE ? 4 : 32); x *= 2) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
 
-    // Each row's sum over the four lanes that share it, then the normalised partial and its log-sum-exp.
+    if constexpr (FOLDS) {
 #pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-        l[rr] += __shfl_xor_sync(0xffffffffu, l[rr], 1);
-        l[rr] += __shfl_xor_sync(0xffffffffu, l[rr], 2);
-        const int hg = g_base + g + 8 * rr;
-        if (hg < group) {
-            const int h = hk * group + hg;
-            const float inv = l[rr] > 0.f ? 1.f / l[rr] : 0.f;
-            float *po = a.part_o + (((int64_t)b * a.hq + h) * a.splits + split) * DFULL + d0 + 2 * t;
+        for (int n = 0; n < ON; ++n)
 #pragma unroll
-            for (int n = 0; n < D / 8; ++n)
-                *reinterpret_cast<float2 *>(po + n * 8) = make_float2(o[n][2 * rr] * inv, o[n][2 * rr + 1] * inv);
-            if (t == 0 && part == 0) a.part_lse[((int64_t)b * a.hq + h) * a.splits + split] = l[rr] > 0.f ? m[rr] * a.scale + __logf(l[rr]) : -INFINITY;
+            for (int e = 0; e < 4; ++e) o[n][e] += old[n][e];
+    }
+    if constexpr (CLUSTER) {
+        constexpr int PER = DM_WARPS / PARTS;
+        float *const wide = reinterpret_cast<float *>(dm_ring);   // the warps' rings, from here on [PER][HEADS][DFULL]
+        float *const box = dm_exchange + (PARTS == 2 ? (size_t)DM_WARPS * 32 * 4 : 0);   // [block][this block's outputs], HEADS DFULL floats and a piece a block
+        float *const meets = box + HEADS * DFULL + 4 * MAX_CLUSTER;  // [block][HEADS][maximum, sum]
+        float *const own = meets + MAX_CLUSTER * 2 * HEADS;         // [warp of PER][HEADS][maximum, sum]
+        const int rows = min(HEADS, group - g_base), quads = rows * DFULL / 4;   // 16-byte pieces of the unit's output
+        __syncthreads();   // nobody's ring is read any more
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int row = 2 * t + e;
+            if (row < rows) {
+                float *po = wide + ((size_t)(wib / PARTS) * HEADS + row) * DFULL + d0 + g;
+#pragma unroll
+                for (int n = 0; n < ON; ++n) {
+                    po[n * 16] = o[n][e];
+                    po[n * 16 + 8] = o[n][2 + e];
+                }
+                if (g == 0 && part == 0) *reinterpret_cast<float2 *>(own + ((wib / PARTS) * HEADS + row) * 2) = make_float2(m[e], l[e]);
+            }
         }
+        __syncthreads();
+        // A part's weight against the maximum of all: where that is -inf nothing was seen (or nothing but NaN), and what is there
+        // is kept as it is.
+        auto weight = [&](float mine, float top) { return top == -INFINITY ? 1.f : between(mine, top); };
+        cluster_wait();
+        const int share = (quads + csize - 1) / csize;   // pieces a block finishes
+        for (int i = threadIdx.x; i < quads; i += DM_WARPS * 32) {
+            const int row = i / (DFULL / 4);
+            float top = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < PER; ++w) top = fmaxf(top, own[(w * HEADS + row) * 2]);
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < PER; ++w) {
+                const float wt = weight(own[(w * HEADS + row) * 2], top);
+                const float4 x = reinterpret_cast<const float4 *>(wide + (size_t)w * HEADS * DFULL)[i];
+                sum.x = fmaf(wt, x.x, sum.x);
+                sum.y = fmaf(wt, x.y, sum.y);
+                sum.z = fmaf(wt, x.z, sum.z);
+                sum.w = fmaf(wt, x.w, sum.w);
+            }
+            cluster_store(box + ((size_t)crank * share + i % share) * 4, i / share, sum);
+        }
+        for (int i = threadIdx.x; i < rows * csize; i += DM_WARPS * 32) {
+            const int row = i % rows, to = i / rows;
+            float top = -INFINITY, all = 0.f;
+#pragma unroll
+            for (int w = 0; w < PER; ++w) top = fmaxf(top, own[(w * HEADS + row) * 2]);
+#pragma unroll
+            for (int w = 0; w < PER; ++w) all = fmaf(weight(own[(w * HEADS + row) * 2], top), own[(w * HEADS + row) * 2 + 1], all);
+            cluster_store(meets + (crank * HEADS + row) * 2, to, make_float2(top, all));
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        const int at = crank * share + (int)threadIdx.x;
+        for (int i = at; i < min(quads, (crank + 1) * share); i += DM_WARPS * 32) {
+            const int row = i / (DFULL / 4);
+            float top = -INFINITY;
+            for (int c = 0; c < csize; ++c) top = fmaxf(top, meets[(c * HEADS + row) * 2]);
+            float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+            float den = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < csize; ++c) {
+                const float2 ml = *reinterpret_cast<const float2 *>(meets + (c * HEADS + row) * 2);
+                const float4 x = *reinterpret_cast<const float4 *>(box + ((size_t)c * share + i - crank * share) * 4);
+                const float wt = weight(ml.x, top);
+                den = fmaf(wt, ml.y, den);
+                num.x = fmaf(wt, x.x, num.x);
+                num.y = fmaf(wt, x.y, num.y);
+                num.z = fmaf(wt, x.z, num.z);
+                num.w = fmaf(wt, x.w, num.w);
+            }
+            const float inv = den > 0.f ? 1.f / den : 0.f;
+            const int64_t h = hk * group + g_base + row;
+            uint2 two = make_uint2(MmaType<T>::pack(num.x * inv, num.y * inv), MmaType<T>::pack(num.z * inv, num.w * inv));
+            reinterpret_cast<uint2 *>(static_cast<T *>(a.out) + ((int64_t)b * a.hq + h) * DFULL)[i % (DFULL / 4)] = two;
+        }
+        return;
+    }
+    // The normalised partial of each head and its log-sum-exp.
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int hg = g_base + (WIDE ? g + 8 * e : 2 * t + e);
+        if (hg >= group) continue;
+        const int64_t at = ((int64_t)b * a.hq + hk * group + hg) * a.splits + split;
+        const float inv = l[e] > 0.f ? 1.f / l[e] : 0.f;
+        float *po = a.part_o + at * DFULL + d0;
+#pragma unroll
+        for (int n = 0; n < ON; ++n) {
+            if constexpr (WIDE) {
+                *reinterpret_cast<float2 *>(po + n * 8 + 2 * t) = make_float2(o[n][2 * e] * inv, o[n][2 * e + 1] * inv);
+            } else {
+                po[n * 16 + g] = o[n][e] * inv;
+                po[n * 16 + 8 + g] = o[n][2 + e] * inv;
+            }
+        }
+        if ((WIDE ? t : g) == 0 && part == 0) a.part_lse[at] = l[e] > 0.f ? m[e] * a.scale + __logf(l[e]) : -INFINITY;
     }
 }
 
@@ -846,25 +1125,73 @@ static cudaError_t split_vec(const DecodeArgs &a, cudaStream_t stream) {
     return split_vec_g<T, D, 1>(a, grid, stream);
 }
 
-template <typename T, int DFULL, int WARPS>
-static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, cudaStream_t stream) {
+// Bytes of shared memory of a block of the tensor-core pass; `cluster`: with the boxes its cluster meets in (a share of the
+// outputs is rounded up to a piece a block).
+constexpr size_t mma_smem(int dfull, bool wide, int warps, bool cluster) {
+    const int parts = dfull > 128 ? 2 : 1, d = dfull / parts;
+    return (size_t)warps * DM_STAGES * 2 * DM_KEYS * 2 * d + (parts == 2 ? sizeof(float) * warps * 32 * (wide ? 8 : 4) : 0) +
+           (cluster ? sizeof(float) * (8 * dfull + MAX_CLUSTER * 4 + (MAX_CLUSTER + (size_t)warps / parts) * 16) : 0);
+}
+// `warps`: of one sequence.
+template <typename T, int DFULL, bool WIDE, int WARPS, int TOGETHER>
+static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster, cudaStream_t stream) {
     constexpr int PARTS = DFULL > 128 ? 2 : 1, D = DFULL / PARTS;
-    constexpr size_t smem = (size_t)WARPS * DM_STAGES * 2 * DM_KEYS * 2 * D + (PARTS == 2 ? (size_t)WARPS * 32 * 8 * sizeof(float) : 0);
-    const auto kernel = a.rope_cos ? decode_split_mma_kernel<T, D, PARTS, WARPS, true> : decode_split_mma_kernel<T, D, PARTS, WARPS, false>;
+    constexpr size_t smem = mma_smem(DFULL, WIDE, WARPS, TOGETHER > 0);
+    const auto kernel = a.rope_cos ? decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, true, TOGETHER> : decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, false, TOGETHER>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
-    dim3 grid((unsigned)((warps + WARPS - 1) / WARPS), a.b);
-    kernel<<<grid, WARPS * 32, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_clusters(kernel, dim3((unsigned)((warps + WARPS - 1) / WARPS), (unsigned)a.b), WARPS * 32, smem, stream, false, (unsigned)cluster, a);
+}
+// Blocks (of CLUSTER_WARPS warps) of the cluster that takes a key-value head of a sequence; 0: chunks, and the merge behind them.
+// Priced in tiles of a warp: its longest chain (a sequence may fill the cache), what a block costs whatever its share (eight
+// tiles' time), and where the blocks do not all run at once - two to a multiprocessor, four at D 64, less what larger clusters leave
+// idle of a GPU processing cluster - their waves, sequences with lengths at half the cache on average.  Few blocks leave
+// multiprocessors idle that the chunks would fill: then only chains of up to twenty tiles, and of five.  Chosen over 125 calls (1 to 64
+// sequences, 100 to 32768 keys, D 64 to 256, groups of 2 to 8) timed with every size of cluster and with chunks: within 1 % of the
+// best of them on average, slower than the chunks of before in four (eight of 6144, 2 heads of 256, 22.4 -> 22.9 were it
+// taken; D 256 and 64 have lines of their own for it).  us, chunks and merge as they were | now: 1 of 4096, 32 / 8 heads of 128 with
+// rotation and append 13.0 | 11.2, 4 17.7 | 13.1, 16 37.4 | 26.3, 16 of 16384 104.9 | 71.1; 12 of 8192 43.4 | 31.3, 64 of 32768 621 |
+// 579; 12 of 6000, 16 / 4 of 256, 33.2 | 25.4.  Caches of at most 512 keys keep the two launches
+// (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.6 where a cluster takes 5.4.
+static int decode_cluster(const DecodeArgs &a) {
+    if (a.s <= 512) return 0;
+    const int64_t units = (int64_t)a.hkv * a.b, shares = a.d > 128 ? CLUSTER_WARPS / 2 : CLUSTER_WARPS;
+    const bool window = a.left < a.s;
+    const int64_t tiles = ((window ? (int64_t)a.left + 1 : a.s) + DM_KEYS - 1) / DM_KEYS, fill = a.d == 128 ? 96 : 160;
+    const double mean = a.lengths && !window ? 0.5 : 1., fixed = 8.;
+    int best = 0;
+    double least = 0.;
+    for (int c = 1; c <= MAX_CLUSTER; c *= 2) {
+        const int64_t blocks = units * c, longest = (tiles + c * shares - 1) / (c * shares);
+        const double room = (c == 16 ? 128 : c == 8 ? 256 : c == 4 ? 272 : c == 2 ? 288 : 296) * (a.d == 64 ? 2 : 1);
+        if ((blocks < fill && longest > 5) || (blocks < 192 && longest > 20) || (c == 16 && blocks > room)) continue;
+        double cost = longest + fixed;
+        if (blocks > room) cost = std::max(cost, blocks * (mean * longest + fixed) / room) + 0.5 * (longest + fixed);
+        if (best == 0 || cost < least) { best = c; least = cost; }
+    }
+    return best;
 }
 template <typename T, int DFULL>
-static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream) {
-    const long long warps = (long long)a.splits * a.hkv * (DFULL > 128 ? 2 : 1) * ((a.hq / a.hkv + 15) / 16);   // of one sequence
-    return warps * a.b < 148LL * 8 * 2 ? split_mma_w<T, DFULL, 2>(a, warps, stream) : split_mma_w<T, DFULL, 8>(a, warps, stream);
+static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream, bool *merged) {
+    const int group = a.hq / a.hkv;
+    const bool wide = group > 8;
+    if (const int cluster = wide ? 0 : decode_cluster(a)) {
+        const long long warps = (long long)a.hkv * cluster * CLUSTER_WARPS, shares = cluster * CLUSTER_WARPS / (DFULL > 128 ? 2 : 1);
+        const cudaError_t e = std::min<long long>(a.s, (long long)a.left + 1) > (MmaType<T>::NARROW ? 256 : 512) * shares ? split_mma_w<T, DFULL, false, CLUSTER_WARPS, 2>(a, warps, cluster, stream)
+                                                                                          : split_mma_w<T, DFULL, false, CLUSTER_WARPS, 1>(a, warps, cluster, stream);
+        *merged = e == cudaSuccess;
+        if (*merged) return e;
+        cudaGetLastError();   // (a part of a GPU may have no room for such a cluster: the chunks go anywhere)
+    }
+    const long long warps = (long long)a.splits * a.hkv * (wide ? (group + 15) / 16 : 1) * (DFULL > 128 ? 2 : 1);   // of one sequence
+    const bool few = warps * a.b < 148LL * 8 * 2;
+    if (wide) return few ? split_mma_w<T, DFULL, true, 2, 0>(a, warps, 1, stream) : split_mma_w<T, DFULL, true, 8, 0>(a, warps, 1, stream);
+    return few ? split_mma_w<T, DFULL, false, 2, 0>(a, warps, 1, stream) : split_mma_w<T, DFULL, false, 8, 0>(a, warps, 1, stream);
 }
-template <> cudaError_t split_mma<float, 128>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }   // never taken: 16-bit caches only
-template <> cudaError_t split_mma<float, 64>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }
-template <> cudaError_t split_mma<float, 256>(const DecodeArgs &, cudaStream_t) { return cudaErrorInvalidValue; }
+template <> cudaError_t split_mma<float, 128>(const DecodeArgs &, cudaStream_t, bool *) { return cudaErrorInvalidValue; }   // never taken: 16-bit caches only
+template <> cudaError_t split_mma<float, 64>(const DecodeArgs &, cudaStream_t, bool *) { return cudaErrorInvalidValue; }
+template <> cudaError_t split_mma<float, 256>(const DecodeArgs &, cudaStream_t, bool *) { return cudaErrorInvalidValue; }
 
 // DASH_ATTN_DECODE_MMA=0 keeps the FMA pass (for comparison runs).
 static bool decode_force_scalar_pass() {
@@ -885,9 +1212,10 @@ template <typename T>
 static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches) {
     cudaError_t e;
     const bool mma = decode_uses_mma(sizeof(T), a, vector_ok);
-    if (mma && a.d == 128) e = split_mma<T, 128>(a, stream);
-    else if (mma && a.d == 64) e = split_mma<T, 64>(a, stream);
-    else if (mma && a.d == 256) e = split_mma<T, 256>(a, stream);
+    bool merged = false;
+    if (mma && a.d == 128) e = split_mma<T, 128>(a, stream, &merged);
+    else if (mma && a.d == 64) e = split_mma<T, 64>(a, stream, &merged);
+    else if (mma && a.d == 256) e = split_mma<T, 256>(a, stream, &merged);
     else if (vector_ok && a.d == 64) e = split_vec<T, 64>(a, stream);
     else if (vector_ok && a.d == 128) e = split_vec<T, 128>(a, stream);
     else if (vector_ok && a.d == 256) e = split_vec<T, 256>(a, stream);
@@ -898,7 +1226,7 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
         e = cudaGetLastError();
     }
     *launches += 1;
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || merged) return e;
     *launches += 1;
     // The merge comes in under the pass's end: one sequence of 4096 keys 14.5 -> 12.5 us, 64 of up to 5387 with one head 39.0 ->
     // 37.0, 28 of up to 7754, 8 heads, 100.3 -> 98.6.  (Its blocks gather on the multiprocessors the pass leaves first, and a
