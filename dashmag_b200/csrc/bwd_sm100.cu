@@ -791,6 +791,7 @@ struct DqTail {
     uint32_t tmem_base;
     unsigned int abort;
     int red_lo[4 * QCG], red_hi[4 * QCG];
+    OpenRun open[4 * QCG];
     int tile_bad;   // an elementwise warp gave up: dQ of the tile is not stored
 };
 
@@ -864,7 +865,12 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int lane_base = 32 * (warp & 3);
     const int r = lane_base + lane;
     int lo = a.tk, hi = 0;
+    const bool short_mask = a.mask.kind == 1 && a.tk <= OPEN_RUN_KEYS;
     if (warp >= 2) {
+        if (short_mask) {
+            const OpenRun mine = open_run_share(a.mask, b, a.tk, sw);
+            if (lane == 0) sh.open[sw] = mine;
+        }
         row_bounds_warp(a.mask, m0 + (r >> pack), a.tq, a.tk, lo, hi);
         int wlo = warp_min_i(hi > lo ? lo : a.tk), whi = warp_max_i(hi > lo ? hi : 0);
         if (lane == 0) { sh.red_lo[sw] = wlo; sh.red_hi[sw] = whi; }
@@ -877,7 +883,16 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     int kmin = a.tk, kmax = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }  // the first four warps cover every row
-    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
+    bool padded = a.mask.kind == 1;   // there are flags to look at in the sweep
+    if (short_mask) {
+        OpenRun run;
+        if (cut_to_open_run(sh.open, run, kmin, kmax)) {
+            padded = false;
+            lo = max(lo, run.first);
+            hi = min(hi, run.last + 1);
+        }
+    }
+    if (padded) trim_padded(a.mask, b, kmin, kmax);
     const int steps = (!aborted && kmax > kmin) ? (kmax - kmin + BIG - 1) / BIG : 0;
     bool failed = aborted;
     // TMEM columns: S at 0, dP[2] at 128 / 256 (dS over the first half of every group of 32 columns), dQ at 384.
@@ -965,7 +980,6 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const int row = m0 + (r >> pack), h = h0 + (r & ((1 << pack) - 1));
         const int cg = sw >> 2, col0 = cg * QW;
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
-        const bool padded = a.mask.kind == 1;
         float l2 = INFINITY, dl = 0.f;
         if (row < a.tq) {
             const int64_t at = ((int64_t)b * a.tq + row) * a.hq + h;

@@ -1147,7 +1147,7 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster
 // Priced in tiles of a warp: its longest chain (a sequence may fill the cache), what a block costs whatever its share (eight
 // tiles' time), and where the blocks do not all run at once - two to a multiprocessor, four at D 64, less what larger clusters leave
 // idle of a GPU processing cluster - their waves, sequences with lengths at half the cache on average.  Few blocks leave
-// multiprocessors idle that the chunks would fill: then only chains of up to twenty tiles, and of five.  Chosen over 125 calls (1 to 64
+// multiprocessors idle that the chunks would fill: then only chains of up to sixteen tiles, and of five.  Chosen over 125 calls (1 to 64
 // sequences, 100 to 32768 keys, D 64 to 256, groups of 2 to 8) timed with every size of cluster and with chunks: within 1 % of the
 // best of them on average, slower than the chunks of before in four (eight of 6144, 2 heads of 256, 22.4 -> 22.9 were it
 // taken; D 256 and 64 have lines of their own for it).  us, chunks and merge as they were | now: 1 of 4096, 32 / 8 heads of 128 with
@@ -1165,7 +1165,7 @@ static int decode_cluster(const DecodeArgs &a) {
     for (int c = 1; c <= MAX_CLUSTER; c *= 2) {
         const int64_t blocks = units * c, longest = (tiles + c * shares - 1) / (c * shares);
         const double room = (c == 16 ? 128 : c == 8 ? 256 : c == 4 ? 272 : c == 2 ? 288 : 296) * (a.d == 64 ? 2 : 1);
-        if ((blocks < fill && longest > 5) || (blocks < 192 && longest > 20) || (c == 16 && blocks > room)) continue;
+        if ((blocks < fill && longest > 5) || (blocks < 192 && longest > 16) || (c == 16 && blocks > room)) continue;
         double cost = longest + fixed;
         if (blocks > room) cost = std::max(cost, blocks * (mean * longest + fixed) / room) + 0.5 * (longest + fixed);
         if (best == 0 || cost < least) { best = c; least = cost; }

@@ -86,6 +86,7 @@ struct Shared {
     Barriers bar;
     uint32_t tmem_base;
     int red_lo[4 * NT], red_hi[4 * NT];
+    OpenRun open[4 * NT];
     unsigned int abort;
     int tile_bad[NT];   // a softmax warp of the tile gave up: its output is not stored
 };
@@ -200,7 +201,12 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int lane_base = 32 * (warp & 3);         // the TMEM lanes this warp may touch
     const int r = lane_base + lane;                // row of the tile
     int lo = a.tk, hi = 0;
+    const bool short_mask = a.mask.kind == 1 && a.tk <= OPEN_RUN_KEYS;
     if (warp >= 2 && warp < 2 + 4 * NT) {
+        if (short_mask) {
+            const OpenRun mine = open_run_share(a.mask, b, a.tk, sw);
+            if (lane == 0) sh.open[sw] = mine;
+        }
         row_bounds_warp(a.mask, tile_row0(tile) + (r >> pack), a.tq, a.tk, lo, hi);
         int wlo = warp_min_i(hi > lo ? lo : a.tk), whi = warp_max_i(hi > lo ? hi : 0);
         if (lane == 0) { sh.red_lo[sw] = wlo; sh.red_hi[sw] = whi; }
@@ -212,7 +218,17 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     int kmin = a.tk, kmax = 0;
 #pragma unroll
     for (int i = 0; i < 4 * NT; ++i) { kmin = min(kmin, sh.red_lo[i]); kmax = max(kmax, sh.red_hi[i]); }
-    if (a.mask.kind == 1) trim_padded(a.mask, b, kmin, kmax);
+    bool padded = a.mask.kind == 1;   // there are flags to look at in the sweep
+    const float rescale_at = hi - lo <= EXACT_KEYS ? 0.f : RESCALE_LOG2;   // (by what the row sees, padding or not)
+    if (short_mask) {
+        OpenRun run;
+        if (cut_to_open_run(sh.open, run, kmin, kmax)) {
+            padded = false;
+            lo = max(lo, run.first);
+            hi = min(hi, run.last + 1);
+        }
+    }
+    if (padded) trim_padded(a.mask, b, kmin, kmax);
     if constexpr (SPLIT) split_keys(split, a.splits, BN, kmin, kmax);
     const bool aborted = sh.abort != 0;
     const int subs = (!aborted && kmax > kmin) ? (kmax - kmin + SN - 1) / SN : 0;   // sub-steps of 64 keys
@@ -344,10 +360,8 @@ fwd2_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         const int t = tile, h = h0 + (r & ((1 << pack) - 1));
         const int row = tile_row0(t) + (r >> pack);
         const uint32_t t_lane = tmem + (static_cast<uint32_t>(lane_base) << 16);
-        const bool padded = a.mask.kind == 1;
         const float2 sl2 = make_float2(a.scale_log2, a.scale_log2);
         float m_ref = -INFINITY, l = 0.f;
-        const float rescale_at = hi - lo <= EXACT_KEYS ? 0.f : RESCALE_LOG2;
         // The padding flags of a sub-step are asked for one sub-step ahead: a trip to memory between the wait for S and
         // the maximum would be the longest link of the step.
         bool hidden[SN / 32] = {false, false};
