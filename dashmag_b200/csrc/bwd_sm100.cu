@@ -66,10 +66,11 @@ template <bool POLY> __device__ __forceinline__ float exp2_mixed(float x) { retu
 // instructions for one (measured on config 2: 35 us of 1 370 slower with a quarter as cubics).
 template <typename T> constexpr int poly_of4() { return Pack<T>::FMT == 1 ? 1 : 0; }
 
-// 32 f32 accumulator columns of this thread's TMEM lane - plus `theirs`, four to a 16-byte word, STRIDE words apart -
-// scaled, rounded and stored as contiguous elements of the row.
+// 32 f32 accumulator columns (the group `cols` of them) of this thread's TMEM lane - plus `theirs`, four to a 16-byte word, STRIDE
+// words apart - scaled, rounded and put into row r of a tile in the layout of a TMA box (64-column halves of 128-byte rows, 16-byte
+// chunks XOR-swizzled by the row).
 template <typename T, int STRIDE>
-__device__ __forceinline__ void store_acc_cols(uint32_t taddr, T *dst, float scale, bool write, const uint4 *theirs) {
+__device__ __forceinline__ void stage_acc_cols(uint32_t taddr, uint8_t *tile, int r, int cols, float scale, const uint4 *theirs) {
     uint32_t o[32];
     tmem_ld32(taddr, o);
     tmem_ld_wait();
@@ -83,16 +84,15 @@ __device__ __forceinline__ void store_acc_cols(uint32_t taddr, T *dst, float sca
             o[4 * e + 3] = __float_as_uint(__uint_as_float(o[4 * e + 3]) + __uint_as_float(x.w));
         }
     }
-    if (write) {
+    uint8_t *row = tile + (cols >> 1) * BIG_HALF + r * 128;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            uint4 v;
-            v.x = Pack<T>::two(__uint_as_float(o[8 * e + 0]) * scale, __uint_as_float(o[8 * e + 1]) * scale);
-            v.y = Pack<T>::two(__uint_as_float(o[8 * e + 2]) * scale, __uint_as_float(o[8 * e + 3]) * scale);
-            v.z = Pack<T>::two(__uint_as_float(o[8 * e + 4]) * scale, __uint_as_float(o[8 * e + 5]) * scale);
-            v.w = Pack<T>::two(__uint_as_float(o[8 * e + 6]) * scale, __uint_as_float(o[8 * e + 7]) * scale);
-            reinterpret_cast<uint4 *>(dst)[e] = v;
-        }
+    for (int e = 0; e < 4; ++e) {
+        uint4 v;
+        v.x = Pack<T>::two(__uint_as_float(o[8 * e + 0]) * scale, __uint_as_float(o[8 * e + 1]) * scale);
+        v.y = Pack<T>::two(__uint_as_float(o[8 * e + 2]) * scale, __uint_as_float(o[8 * e + 3]) * scale);
+        v.z = Pack<T>::two(__uint_as_float(o[8 * e + 4]) * scale, __uint_as_float(o[8 * e + 5]) * scale);
+        v.w = Pack<T>::two(__uint_as_float(o[8 * e + 6]) * scale, __uint_as_float(o[8 * e + 7]) * scale);
+        *reinterpret_cast<uint4 *>(row + ((((cols & 1) * 4 + e) ^ (r & 7)) << 4)) = v;
     }
 }
 
@@ -234,6 +234,7 @@ template <bool FUSED> struct DkdvTail {
     QAux aux[2];
     uint32_t tmem_base;
     unsigned int abort;
+    uint32_t tile_bad;                // an elementwise warp gave up: dK and dV of the unit are not stored
     uint32_t share_whole[4 * KCG];   // PAIR: whether the second block's warp got through its sweep (written by that block)
     int cu_q[cu_cache<FUSED>()], cu_k[cu_cache<FUSED>()];   // the packed sequences' offsets, when they fit
 };
@@ -255,7 +256,8 @@ template <typename T, int HD, bool FUSED, bool PAIR>
 __global__ void __launch_bounds__(FUSED ? KTHREADS_FUSED : KTHREADS, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                      const __grid_constant__ CUtensorMap tm_dq_acc, const Sm100BwdArgs a) {
+                      const __grid_constant__ CUtensorMap tm_dq_acc, const __grid_constant__ CUtensorMap tm_dk,
+                      const __grid_constant__ CUtensorMap tm_dv, const Sm100BwdArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     constexpr int BIG_BYTES = tile_bytes<HD>();
     constexpr int DOS = FUSED ? 1 : 2;        // stages of the dO ring
@@ -297,12 +299,15 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         mbar_init(BAR(sh.bar.acc_ready), 1);
         mbar_init(BAR(sh.bar.dq_done), 1);
         mbar_init(BAR(sh.bar.dq_taken), 4);          // one arrival per reduction warp
+        sh.tile_bad = 0;
         fence_mbar_init();
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_do);
         if constexpr (FUSED) prefetch_tensormap(&tm_dq_acc);
+        prefetch_tensormap(&tm_dk);
+        prefetch_tensormap(&tm_dv);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&sh.tmem_base), 512);
@@ -733,19 +738,39 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         // ---------------- epilogue ----------------
         const bool shared_sweep = PAIR && all_steps > first_share;   // the second block had steps
         if (shared_sweep && sh.share_whole[warp - 2] == 0) failed = true;
-        T *dk = static_cast<T *>(a.dk) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + ecg * EC;
-        T *dv = static_cast<T *>(a.dv) + (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + ecg * EC;
         if (steps == 0) {
+            const int64_t at = (((int64_t)b * a.tk + key) * a.hkv + hk) * HD + ecg * EC;
             if (key < a.tk && !failed && mine) {
-                store_zero_cols<T, EC / 8>(dk);
-                store_zero_cols<T, EC / 8>(dv);
+                store_zero_cols<T, EC / 8>(static_cast<T *>(a.dk) + at);
+                store_zero_cols<T, EC / 8>(static_cast<T *>(a.dv) + at);
             }
-        } else if (!failed && mine) {
-            tc_fence_after_sync();
-            const uint4 *theirs = shared_sweep ? reinterpret_cast<const uint4 *>(smem) + (threadIdx.x - 64) : nullptr;
-            store_acc_cols<T, EW_THREADS>(t_sums + COL_DV, dv, 1.f, key < a.tk, theirs);
-            store_acc_cols<T, EW_THREADS>(t_sums + COL_DK, dk, a.scale, key < a.tk, theirs ? theirs + 8 * EW_THREADS : nullptr);
-            tc_fence_before_sync();
+        } else {
+            // Every MMA has completed, so the streamed tiles are dead: the rows of dV and dK are staged over two of them (fused: of
+            // the Q ring; else of the dO ring, behind what the second block of a pair left) and leave as bulk stores - whole lines
+            // instead of 16 bytes per thread and row, 32 lines an instruction: from the last product on a unit took 5000 (D 64) to
+            // 7000 cycles - which drop the rows past the last key.  (16 x 509, 12 heads of 64, any order, backward 99.1 -> 94.4 us; 26 x
+            // 193 67.0 -> 63.6; 27161 packed tokens, 16 / 4 heads of 128, 1008 -> 981; long sequences the same.)
+            uint8_t *dv_tile = FUSED ? q_s : do_s, *dk_tile = dv_tile + BIG_BYTES;
+            if (!failed && mine) {
+                tc_fence_after_sync();
+                const int r = 32 * (warp & 3) + lane;
+                const uint4 *theirs = shared_sweep ? reinterpret_cast<const uint4 *>(smem) + (threadIdx.x - 64) : nullptr;
+                stage_acc_cols<T, EW_THREADS>(t_sums + COL_DV, dv_tile, r, ecg, 1.f, theirs);
+                stage_acc_cols<T, EW_THREADS>(t_sums + COL_DK, dk_tile, r, ecg, a.scale, theirs ? theirs + 8 * EW_THREADS : nullptr);
+                tc_fence_before_sync();
+            }
+            if (failed && lane == 0) sh.tile_bad = 1;
+            fence_proxy_async_smem();
+            named_barrier(2, 32 * 4 * KCG);   // the elementwise warps, all of which get here
+            if (warp == 2 && lane == 0 && sh.tile_bad == 0) {
+#pragma unroll
+                for (int half = 0; half < HD / 64; ++half) {
+                    tma_store_4d(&tm_dv, smem_u32(dv_tile + half * BIG_HALF), 64 * half, hk, k0, b);
+                    tma_store_4d(&tm_dk, smem_u32(dk_tile + half * BIG_HALF), 64 * half, hk, k0, b);
+                }
+                tma_store_commit();
+                tma_store_wait_read();
+            }
         }
     }
 
@@ -1140,7 +1165,7 @@ static cudaError_t launch_dkdv(const Sm100BwdMaps &m, const Sm100BwdArgs &a, lon
     dim3 gk((unsigned)(items * a.hkv * (PAIR ? 2 : 1)), 1, 1);
     // Under delta's end (4 packed sequences, 2149 tokens, 16 / 4 heads, forward and backward: 104.3 -> 98.2 us with the plan left out
     // too; 9 sequences, 1047 tokens, 48.3 -> 43.2; 10 padded ones of 224, 12 / 4 heads, 53.4 -> 49.0); the fused form behind the memset.
-    return launch_clusters(kernel, gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream, !FUSED, PAIR ? 2u : 1u, m.k128, m.v128, m.q128, m.do128, m.dq_acc, a);
+    return launch_clusters(kernel, gk, FUSED ? KTHREADS_FUSED : KTHREADS, smem, stream, !FUSED, PAIR ? 2u : 1u, m.k128, m.v128, m.q128, m.do128, m.dq_acc, m.dk128, m.dv128, a);
 }
 
 template <typename T, int HD>

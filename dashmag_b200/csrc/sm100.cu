@@ -346,6 +346,9 @@ cudaError_t sm100_backward(const dash_attn_params *p, const TrainArgs &a, void *
               encode(&m.do128, p->dtype, g, p->b, p->tq, p->hq, p->do_stride, 128, p->d, heads) &&
               encode(&m.k128, p->dtype, k, p->b, p->tk, p->hkv, p->k_stride, 128, p->d) &&
               encode(&m.v128, p->dtype, v, p->b, p->tk, p->hkv, p->v_stride, 128, p->d);
+    const int64_t dkv_stride[4] = {(int64_t)p->tk * p->hkv * p->d, (int64_t)p->hkv * p->d, p->d, 1};
+    if (p->d != 256) ok = ok && encode(&m.dk128, p->dtype, a.dk, p->b, p->tk, p->hkv, dkv_stride, 128, p->d) &&
+                          encode(&m.dv128, p->dtype, a.dv, p->b, p->tk, p->hkv, dkv_stride, 128, p->d);
     if (ok && fused) ok = encode(&m.dq_acc, DASH_ATTN_F32, dq_acc, p->b, p->tq, p->hq, dq_stride, 128, p->d, heads);
     else if (ok) m.dq_acc = m.dq128;   // not read
     if (!ok) {

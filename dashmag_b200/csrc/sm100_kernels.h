@@ -50,6 +50,7 @@ struct Sm100BwdArgs {
 struct Sm100BwdMaps {
     CUtensorMap q128, do128, k128, v128;
     CUtensorMap dq128;                   // dq kernel's output
+    CUtensorMap dk128, dv128;            // D 64, 128: dkdv's outputs, boxes of one head
     CUtensorMap dq_acc;                  // the fused form's f32 accumulator, boxes of 32 columns x 128 rows
 };
 
