@@ -19,7 +19,8 @@
 // products), two or one where they do not (rows_per_warp): small calls are bound by the length of a block's chain of
 // tiles, not by throughput.  Where one would do and shared memory allows it the block takes its tiles two at a time (KS 2): a warp
 // has two rows and every second tile, and the two warps of the same rows add their sums at the end - half the links in the chain, and
-// half the reads of shared memory a product.  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
+// half the reads of shared memory a product.  Blocks of a cluster share rows likewise, a run of the sweep each (SHARE: forward_cluster, dq_cluster,
+// dkdv_cluster).  NI is the number of head dimensions a lane owns (2, 4, 8 for D up to 64, 128, 256).
 // Two packed sequences of 384 tokens, four heads of 64, f32: the step 254 ->
 // 61 us side by side (three kernels of 105-113 us each, most of it scalar copies with a division an element, one after
 // another), and 57 with the tiles two at a time; 381 tokens, 3 / 1 heads of 96, 74 -> 55, 590 148 -> 103, 1478 of 64 345 -> 246
@@ -168,6 +169,46 @@ __device__ __forceinline__ void gather_shares(float *box, float (&acc)[RPW][NI])
     }
 }
 
+// ---- the blocks of a cluster (forward) -----------------------------------------------------------
+__device__ __forceinline__ int cluster_blocks() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r)); return (int)r; }
+__device__ __forceinline__ int cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return (int)r; }
+__device__ __forceinline__ void cluster_meet() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// What is in block `rank`'s shared memory where `mine` is in this one's.
+__device__ __forceinline__ float cluster_read(const float *mine, int rank) {
+    uint32_t at;
+    float x;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(mine))), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(at) : "memory");
+    return x;
+}
+
+// The sums of the cluster's first block take the others' in order, through the tiles' shared memory of each (from 32 features on).
+template <int RPW, int NI, int KS>
+__device__ __forceinline__ void gather_cluster(float *box, float (&acc)[RPW][NI], int csize, int crank) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    static_assert((WARPS / KS) * RPW * NI * 32 <= 4 * KS * TILE * (NI > 2 ? 68 : 36), "the shares fit where the tiles were");
+    float *mine = box + w * RPW * NI * 32 + lane;
+    __syncthreads();   // nobody reads the tiles (or the shares before) any more
+    if (crank > 0 && w < WARPS / KS) {
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+#pragma unroll
+            for (int i = 0; i < NI; ++i) mine[(r * NI + i) * 32] = acc[r][i];
+    }
+    cluster_meet();
+    if (crank == 0 && w < WARPS / KS) {
+        for (int o = 1; o < csize; ++o)
+#pragma unroll
+            for (int r = 0; r < RPW; ++r)
+#pragma unroll
+                for (int i = 0; i < NI; ++i) acc[r][i] += cluster_read(mine + (r * NI + i) * 32, o);
+    }
+    cluster_meet();   // the others' shared memory stays until it has been read
+}
+
 // The block's first row, and what each of its rows sees: the queries' key intervals (warp 0 places them) and their union.
 struct RowSpans {
     int lo[32], hi[32];
@@ -188,7 +229,7 @@ __device__ __forceinline__ void place_rows(RowSpans &sp, const MaskArgs &m, int 
 // ---------------------------------------------------------------------------------------------
 // Forward
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI, int KS>
+template <typename T, int RPW, int NI, int KS, bool SHARE>
 __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
@@ -201,7 +242,8 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);   // the warp's rows; its tile of the step's KS
-    const int qt = gridDim.x - 1 - blockIdx.x;  // long (late) causal rows first
+    const int csize = SHARE ? cluster_blocks() : 1, crank = SHARE ? cluster_rank() : 0;   // blocks that share the rows, each a run of their keys
+    const int qt = (gridDim.x - 1 - blockIdx.x) / csize;  // long (late) causal rows first
     const int h = blockIdx.y, b = blockIdx.z;
     const int hk = h / (a.hq / a.hkv);
     const int row0 = qt * ROWS;
@@ -236,8 +278,14 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
     };
-    const int first = kmin / TILE * TILE;
-    if (kmax > kmin) stage(first, 0);
+    int first = kmin / TILE * TILE;
+    if (SHARE && kmax > kmin) {   // (tiles are whole, so only the last of the runs ends inside one)
+        const int per = ((kmax - first + TILE - 1) / TILE + csize - 1) / csize * TILE;
+        first += crank * per;
+        kmax = min(kmax, first + per);
+        whi = min(whi, kmax);
+    }
+    if (kmax > first) stage(first, 0);
     for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();   // the tile is whole, and every warp is done with the other buffer
@@ -292,11 +340,12 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
             }
         }
         __syncthreads();
-        if (sub > 0) return;
+        if (sub > 0 && !SHARE) return;
 #pragma unroll
         for (int o = 1; o < KS; ++o)
 #pragma unroll
             for (int r = 0; r < RPW; ++r) {
+                if (sub > 0) break;
                 const float *x = box_of(o) + r * (NI + 2) * 32;
                 const float mn = fmaxf(m[r], x[0]);
                 const float mine = mn == -INFINITY ? 1.f : expf(m[r] - mn), theirs = mn == -INFINITY ? 1.f : expf(x[0] - mn);
@@ -305,6 +354,43 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
                 for (int i = 0; i < NI; ++i) acc[r][i] = acc[r][i] * mine + x[(2 + i) * 32] * theirs;
                 m[r] = mn;
             }
+    }
+    if constexpr (SHARE) {
+        // The cluster's blocks hand over what they have in the same way, block after block in order, through the tiles' shared
+        // memory of each; the first block finishes the rows.
+        static_assert((WARPS / KS) * RPW * (NI + 2) * 32 <= 4 * STEP * (NI > 2 ? 68 : 36), "the shares fit where the tiles were, from 32 features on");
+        float *box = kv + wr * RPW * (NI + 2) * 32 + lane;
+        __syncthreads();   // no warp is at its last tile any more, nor at the shares above
+        if (sub == 0 && crank > 0) {
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                float *x = box + r * (NI + 2) * 32;
+                x[0] = m[r];
+                x[32] = l[r];
+#pragma unroll
+                for (int i = 0; i < NI; ++i) x[(2 + i) * 32] = acc[r][i];
+            }
+        }
+        cluster_meet();
+        if (sub == 0 && crank == 0) {
+            for (int o = 1; o < csize; ++o)
+#pragma unroll
+                for (int r = 0; r < RPW; ++r) {
+                    const float *x = box + r * (NI + 2) * 32;
+                    float theirs_acc[NI];
+                    const float tm = cluster_read(x, o), tl = cluster_read(x + 32, o);
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) theirs_acc[i] = cluster_read(x + (2 + i) * 32, o);
+                    const float mn = fmaxf(m[r], tm);
+                    const float mine = mn == -INFINITY ? 1.f : expf(m[r] - mn), theirs = mn == -INFINITY ? 1.f : expf(tm - mn);
+                    l[r] = l[r] * mine + tl * theirs;
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) acc[r][i] = acc[r][i] * mine + theirs_acc[i] * theirs;
+                    m[r] = mn;
+                }
+        }
+        cluster_meet();   // the others' shared memory stays until it has been read
+        if (crank > 0 || sub > 0) return;
     }
 
     T *out = static_cast<T *>(a.out);
@@ -348,8 +434,9 @@ __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
 // ---------------------------------------------------------------------------------------------
 // dQ: each block of queries sweeps, in order, the key tiles it sees.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI, int KS>
-__global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int vec) {
+// (Four rows a warp at D 128: with more than 128 registers a thread a block would be alone on its multiprocessor.)
+template <typename T, int RPW, int NI, int KS, bool SHARE>
+__global__ void __launch_bounds__(THREADS, RPW == 4 && NI == 4 ? 2 : 0) generic_dq_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
     const int dp = padded_d(a.d), sp = tile_stride(a.d);
@@ -362,7 +449,8 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);
-    const int qt = gridDim.x - 1 - blockIdx.x;
+    const int csize = SHARE ? cluster_blocks() : 1, crank = SHARE ? cluster_rank() : 0;
+    const int qt = (gridDim.x - 1 - blockIdx.x) / csize;
     const int h = blockIdx.y, b = blockIdx.z;
     const int hk = h / (a.hq / a.hkv);
     const int row0 = qt * ROWS;
@@ -405,8 +493,14 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
             pad[buf][threadIdx.x] = key >= a.tk || key_padded(a.mask, b, key) ? 1 : 0;
         }
     };
-    const int first = kmin / TILE * TILE;
-    if (kmax > kmin) stage(first, 0);
+    int first = kmin / TILE * TILE;
+    if (SHARE && kmax > kmin) {   // as in the forward
+        const int per = ((kmax - first + TILE - 1) / TILE + csize - 1) / csize * TILE;
+        first += crank * per;
+        kmax = min(kmax, first + per);
+        whi = min(whi, kmax);
+    }
+    if (kmax > first) stage(first, 0);
     for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();
@@ -434,12 +528,13 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
     }
     copies_wait();
     if constexpr (KS > 1) gather_shares<RPW, NI, KS>(kv, acc);
+    if constexpr (SHARE) gather_cluster<RPW, NI, KS>(kv, acc, csize, crank);
 
     T *dq = static_cast<T *>(a.dq);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
         const int row = row0 + wr * RPW + r;
-        if (row >= a.tq || sub > 0) continue;
+        if (row >= a.tq || sub > 0 || crank > 0) continue;
         const int64_t base = (((int64_t)b * a.tq + row) * a.hq + h) * a.d;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -454,7 +549,7 @@ __global__ void __launch_bounds__(THREADS) generic_dq_kernel(TrainArgs a, int ve
 // dK, dV: each block of keys sweeps, in order, the query heads of its group and the query
 // tiles that see it; a warp owns RPW keys, a lane one query of the tile.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int RPW, int NI, int KS>
+template <typename T, int RPW, int NI, int KS, bool SHARE>
 __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
@@ -469,7 +564,8 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wr = w % (WARPS / KS), sub = w / (WARPS / KS);
-    const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+    const int csize = SHARE ? cluster_blocks() : 1, crank = SHARE ? cluster_rank() : 0;   // blocks that share the keys, each a run of the steps
+    const int kt = blockIdx.x / csize, hk = blockIdx.y, b = blockIdx.z;
     const int group = a.hq / a.hkv;
     const int key0 = kt * ROWS;
 
@@ -501,7 +597,8 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
 #pragma unroll
         for (int i = 0; i < NI; ++i) { acck[r][i] = 0.f; accv[r][i] = 0.f; }
 
-    const int first = qfirst / TILE * TILE, tiles = qend > qfirst ? (qend - first + STEP - 1) / STEP : 0, steps = tiles * group;
+    const int first = qfirst / TILE * TILE, tiles = qend > qfirst ? (qend - first + STEP - 1) / STEP : 0, all_steps = tiles * group;
+    const int begin = all_steps * crank / csize, steps = all_steps * (crank + 1) / csize;   // this block's [begin, steps)
     auto stage = [&](int t, int buf) {
         const int h = hk * group + t / tiles, q0 = first + t % tiles * STEP;
         stage_rows<T>(qg + (2 * buf) * STEP * sp, sp, a.q, b, h, q0, STEP, a.tq, a.d, vec);
@@ -514,8 +611,8 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
             else copy_async(&deltas[buf][threadIdx.x - STEP], a.delta + at, in, 0);
         }
     };
-    if (steps > 0) stage(0, 0);
-    for (int t = 0; t < steps; ++t) {
+    if (steps > begin) stage(begin, begin & 1);
+    for (int t = begin; t < steps; ++t) {
         const int buf = t & 1, q0 = first + t % tiles * STEP + sub * TILE;
         copies_wait();
         __syncthreads();
@@ -548,12 +645,16 @@ __global__ void __launch_bounds__(THREADS) generic_dkdv_kernel(TrainArgs a, int 
         gather_shares<RPW, NI, KS>(qg, acck);
         gather_shares<RPW, NI, KS>(qg, accv);
     }
+    if constexpr (SHARE) {
+        gather_cluster<RPW, NI, KS>(qg, acck, csize, crank);
+        gather_cluster<RPW, NI, KS>(qg, accv, csize, crank);
+    }
 
     T *dk = static_cast<T *>(a.dk), *dv = static_cast<T *>(a.dv);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
         const int key = key0 + wr * RPW + r;
-        if (key >= a.tk || sub > 0) continue;
+        if (key >= a.tk || sub > 0 || crank > 0) continue;
         const int64_t base = (((int64_t)b * a.tk + key) * a.hkv + hk) * a.d;
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
@@ -611,25 +712,56 @@ static int rows_per_warp(int64_t rows, int64_t heads, int d, int own, int probs)
 }
 
 using GenericKernel = void (*)(TrainArgs, int);
-static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, cudaStream_t stream, bool beside, const TrainArgs &a, bool vec) {
+static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, cudaStream_t stream, bool beside, const TrainArgs &a, bool vec,
+                                  unsigned cluster = 1) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_beside(kernel, grid, THREADS, smem, stream, beside, a, (int)vec);
+    return launch_clusters(kernel, grid, THREADS, smem, stream, beside, cluster, a, (int)vec);
 }
 // The instance for the rows per warp and the head dimension.
-#define GENERIC_PICK(kernel, T, rpw, d)                                                                    \
-    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2, 1> : (d) <= 128 ? kernel<T, 4, 4, 1> : kernel<T, 4, 8, 1>)  \
-     : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2, 1> : (d) <= 128 ? kernel<T, 2, 4, 1> : kernel<T, 2, 8, 1>) \
-     : (rpw) == 1 ? ((d) <= 64 ? kernel<T, 1, 2, 1> : (d) <= 128 ? kernel<T, 1, 4, 1> : kernel<T, 1, 8, 1>) \
-                : ((d) <= 64 ? kernel<T, 2, 2, 2> : kernel<T, 2, 4, 2>))
+#define GENERIC_PICK(kernel, T, rpw, d)                                                                                                \
+    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2, 1, false> : (d) <= 128 ? kernel<T, 4, 4, 1, false> : kernel<T, 4, 8, 1, false>)         \
+     : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2, 1, false> : (d) <= 128 ? kernel<T, 2, 4, 1, false> : kernel<T, 2, 8, 1, false>)       \
+     : (rpw) == 1 ? ((d) <= 64 ? kernel<T, 1, 2, 1, false> : (d) <= 128 ? kernel<T, 1, 4, 1, false> : kernel<T, 1, 8, 1, false>)       \
+                  : ((d) <= 64 ? kernel<T, 2, 2, 2, false> : kernel<T, 2, 4, 2, false>))
+#define GENERIC_PICK_SHARED(kernel, T, rpw, d)                                                                                         \
+    ((rpw) == 4 ? ((d) <= 64 ? kernel<T, 4, 2, 1, true> : kernel<T, 4, 4, 1, true>) : (rpw) == 2 ? ((d) <= 64 ? kernel<T, 2, 2, 1, true> : kernel<T, 2, 4, 1, true>) \
+     : (rpw) == 1 ? ((d) <= 64 ? kernel<T, 1, 2, 1, true> : kernel<T, 1, 4, 1, true>) : ((d) <= 64 ? kernel<T, 2, 2, 2, true> : kernel<T, 2, 4, 2, true>))
+
+// Blocks of the cluster that shares a block's rows, each a run of what they sweep.  Small calls wait for the chain of a block's
+// tiles, and where multiprocessors have room a second block halves it; causal calls gain by it beyond that, whose long chains end alone.
+// What it costs is the meeting (3 to 5 us with the first block's reads) and, packed, sweeps too short to share: `sweep` is the
+// mean sequence.  Measured (us, one block | two | four): forward of 16 queries against 4000 keys, 32 / 8 heads of 64, bf16, 64 blocks,
+// 168 | 97 | 69, 39 against 4783, 16 heads, 80 blocks, 201 | 152 | 107; f32, 450 tokens, 4 heads of 128, 228 blocks, 56 | 38 | 45, 1500, 8 heads,
+// 376 blocks, 398 | 297 | 305, 900 in four, 4 heads of 128, 228 blocks (two to a multiprocessor), 39 | 42 | 48, 384 in two 16.6 | 16.6 | 20.7.  (Heads
+// of 256, 64 queries against 128 keys, 64 blocks, 25 | 17 | 21, 60 against 2060, 128 blocks, 376 | 389 | 402.)  Backward (one | dq's two | dkdv's
+// two too): 39 against 4783 602 | 379 | 443; 590 in two, 3 / 1 heads of 96, 96 | 93 | 64; 300, 8 / 2 of 96, 124 | 122 | 81; 1000 in three, 4 / 2 of 64,
+// 91 | 79 | 84; 130, 4 heads, 20.7 | 21.2 | 27; dkdv's blocks sweep the whole group, so they gain where groups are large and
+// blocks few.
+static int64_t mean_sweep(const TrainArgs &a, int64_t rows) { return a.mask.kind == 2 ? rows / std::max(a.mask.seqs, 1) : rows; }
+static unsigned forward_cluster(const TrainArgs &a, int rpw, int64_t blocks) {
+    const int64_t room = 148 * (SMEM_PER_SM / ((int64_t)generic_smem(a.d, rpw, 1, 1) + SMEM_BESIDE)), sweep = mean_sweep(a, a.tk);
+    // Below 32 features a tile has no room for a block's sums; above 128 a head's bits do not depend on the others, and a rule
+    // that does not look at them would cost the calls of many heads a few per cent.
+    if (a.d < 32 || a.d > 128 || sweep < (a.d > 64 ? 64 : 128)) return 1;   // (302 in three, 4 heads of 64: 10.3 us alone, 12.3 shared; 202, 3 of 96: 12.4, 10.3)
+    if (blocks * 4 <= 330 && sweep >= 128) return 4;
+    return blocks <= 400 && (sweep >= 250 || blocks * 2 <= room) ? 2 : 1;
+}
+static unsigned dq_cluster(const TrainArgs &a, int64_t blocks) { return a.d >= 32 && a.d <= 128 && blocks <= 400 && mean_sweep(a, a.tk) >= 190 ? 2 : 1; }
+static unsigned dkdv_cluster(const TrainArgs &a, int64_t blocks) {
+    const int64_t group = a.hq / a.hkv;
+    return a.d >= 32 && a.d <= 128 && group >= 2 && blocks <= (group >= 3 ? 190 : 100) && mean_sweep(a, a.tq) * group >= 256 ? 2 : 1;
+}
 
 template <typename T>
 static cudaError_t forward_t(const TrainArgs &a, cudaStream_t stream, int *launches) {
     const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 1, 1), rows = block_rows(rpw);
     const bool vec = rows_readable<T>(a.q, a.d) && rows_readable<T>(a.k, a.d) && rows_readable<T>(a.v, a.d);
+    const int tiles = (a.tq + rows - 1) / rows;
+    const unsigned cluster = forward_cluster(a, rpw, (int64_t)tiles * a.hq * a.b);
     *launches += 1;
-    return launch_generic(GENERIC_PICK(generic_forward_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 1, 1), stream,
-                          false, a, vec);
+    return launch_generic(cluster > 1 ? GENERIC_PICK_SHARED(generic_forward_kernel, T, rpw, a.d) : GENERIC_PICK(generic_forward_kernel, T, rpw, a.d), dim3(tiles * cluster, a.hq, a.b), generic_smem(a.d, rpw, 1, 1), stream, false, a,
+                          vec, cluster);
 }
 
 template <typename T>
@@ -645,17 +777,21 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
     }
     {
         const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b, a.d, 2, 2), rows = block_rows(rpw);
+        const int tiles = (a.tk + rows - 1) / rows;
+        const unsigned cluster = dkdv_cluster(a, (int64_t)tiles * a.hkv * a.b);
         *launches += 1;
-        e = launch_generic(GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3((a.tk + rows - 1) / rows, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
-                           false, a, vec);
+        e = launch_generic(cluster > 1 ? GENERIC_PICK_SHARED(generic_dkdv_kernel, T, rpw, a.d) : GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3(tiles * cluster, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
+                           false, a, vec, cluster);
         if (e != cudaSuccess) return e;
     }
     {   // beside dkdv.  (dkdv itself brought in under delta's end, to wait there, made the whole twice as slow: 1000 tokens, 4 / 2
         // heads of 64 327 against 213 us.)
         const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), rows = block_rows(rpw);
+        const int tiles = (a.tq + rows - 1) / rows;
+        const unsigned cluster = dq_cluster(a, (int64_t)tiles * a.hq * a.b);
         *launches += 1;
-        return launch_generic(GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3((a.tq + rows - 1) / rows, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
-                              true, a, vec);
+        return launch_generic(cluster > 1 ? GENERIC_PICK_SHARED(generic_dq_kernel, T, rpw, a.d) : GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3(tiles * cluster, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
+                              true, a, vec, cluster);
     }
 }
 
