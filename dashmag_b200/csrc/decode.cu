@@ -21,9 +21,10 @@
 //     and rounds to the queries' dtype.  Chunks past a sequence's length or before its window are
 //     never touched.
 //
-// With 16-bit caches, head dimension 128 and four to sixteen query heads per key-value head the
-// split pass runs on the tensor cores instead (decode_split_mma_kernel below): at that much
-// arithmetic per cache row the FMA pipe, not HBM, bounds the pass above.
+// With 16-bit caches and two query heads or more per key-value head the pass runs on the tensor cores
+// instead (decode_split_mma_kernel below): at that much arithmetic per cache row the FMA pipe, not HBM,
+// bounds the pass above.  Above 512 keys its groups of up to eight heads need neither chunks nor merge: the
+// blocks of a cluster take a (sequence, key-value head) together (decode_cluster says which calls).
 //
 // Inputs the vector path cannot read (head dimension not 64 / 128 / 256, last stride not 1, rows
 // not 16-byte aligned) go through a slower scalar kernel with the same arithmetic.

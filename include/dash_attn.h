@@ -119,7 +119,7 @@ typedef struct dash_attn_decode_params {
  * without scratch are never split).  So can key and value gradients where a small call's units
  * are shared between two blocks (at head dimension 256 by the units' number; at 64 and 128 by the batch's key blocks
  * and the length of their sweeps, whatever the number of heads), every result of the CUDA-core kernels (f32, and what the
- * tensor-core kernels do not take) up to head dimension 128, packed or not, where two warps share a small call's rows, and a
+ * tensor-core kernels do not take) up to head dimension 128, packed or not, where warps and blocks share a small call's rows, and a
  * decoding step, whose cache is cut and merged by the size of the call.  The same call gives the same bits on every run. */
 size_t dash_attn_forward_workspace(const dash_attn_params *p);
 size_t dash_attn_backward_workspace(const dash_attn_params *p);
