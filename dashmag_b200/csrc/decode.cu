@@ -1156,7 +1156,8 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster
 // 579; 12 of 6000, 16 / 4 of 256, 33.2 | 25.4.  Caches of at most 512 keys keep the two launches
 // (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.6 where a cluster takes 5.4.
 static int decode_cluster(const DecodeArgs &a) {
-    if (a.s <= 512) return 0;
+    static const bool chunks = std::getenv("DASH_ATTN_DECODE_CHUNK") != nullptr;   // a comparison run fixes the chunk (api.cu)
+    if (chunks || a.s <= 512) return 0;
     const int64_t units = (int64_t)a.hkv * a.b, shares = a.d > 128 ? CLUSTER_WARPS / 2 : CLUSTER_WARPS;
     const bool window = a.left < a.s;
     const int64_t tiles = ((window ? (int64_t)a.left + 1 : a.s) + DM_KEYS - 1) / DM_KEYS, fill = a.d == 128 ? 96 : 160;
