@@ -309,6 +309,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_kernel(DecodeArgs
 // not there.  (D 128, a group of four: 24 MMAs a tile and not 48.)  Larger groups (WIDE) are the M dimension, S = Q K^T with the
 // 16 keys as two N tiles, then O += P V with P taken straight from the accumulator registers of S as the A operand: two column
 // tiles of eight heads in the other form measured slower by a tenth, its 8 x 8 transposes and its maxima over eight lanes cost more.
+// In chunks both forms sum in one order, so that a head's bits do not depend on how many others share its key-value head; that costs
+// the narrow one at most 2 % (16 of 200 keys, 16 / 4 heads of 128, split and merge, 7.8 -> 7.9 us; with sixteen rows 8.6).
 // One warp per (share of the keys, key-value head), with a ring of its own in shared memory: every lane copies 16-byte pieces of
 // the tile's 16 key rows and 16 value rows asynchronously, two tiles ahead, into rows (256 bytes at D = 128) whose 16-byte chunks
 // are XOR-swizzled by the row, and ldmatrix reads the fragments from there without bank conflicts (transposed for V).  What a warp
@@ -569,8 +571,8 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
     // The largest probability of a head: 1, or at f16, in a cluster's longer sweeps, 2^8 - the second part of a small probability is then no
     // subnormal number, whose rounding would be the largest error of the sum.
     constexpr float LIFT = CLUSTER && MmaType<T>::NARROW ? 8.f : 0.f;
-    // From one maximum to another: the difference of the two offsets as the exponentials used them, each product rounded on its own,
-    // so that what was summed against either shares one reference.
+    // From one maximum to another, in clusters: the difference of the two offsets as the exponentials used them, each product rounded on
+    // its own, so that what was summed against either shares one reference.
     auto between = [sl](float from, float to) { return exp2f(__fsub_rn(__fmul_rn(from, sl), __fmul_rn(to, sl))); };
     // The accumulator: eight heads have it transposed (rows are features, columns heads), sixteen as rows of heads.
     constexpr int ON = WIDE ? D / 8 : D / 16;
@@ -620,8 +622,9 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
 #pragma unroll
                     for (int nt = 0; nt < 2; ++nt) MmaType<T>::mma(sc[nt], qa[ks + j], kf[ks + nt][2 * j], kf[ks + nt][2 * j + 1]);
         } else {
-            // S transposed, [16 keys x 8 heads]; the even and the odd k-steps as two chains.
+            // S transposed, [16 keys x 8 heads]; in clusters the even and the odd k-steps as two chains, in chunks one, as sixteen heads have it.
             float odd[4] = {};
+            auto &second = CLUSTER ? odd : sc[0];
             const int row = (lm & 1) * 8 + lr;
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks)   // keys 0-7 and 8-15 of the k-step's first eight features, then of the others
@@ -629,10 +632,12 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
 #pragma unroll
             for (int ks = 0; ks < D / 16; ks += 2) {
                 MmaType<T>::mma(sc[0], kf[ks], qa[ks][0], qa[ks][1]);
-                MmaType<T>::mma(odd, kf[ks + 1], qa[ks + 1][0], qa[ks + 1][1]);
+                MmaType<T>::mma(second, kf[ks + 1], qa[ks + 1][0], qa[ks + 1][1]);
             }
+            if constexpr (CLUSTER) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) sc[0][e] += odd[e];
+                for (int e = 0; e < 4; ++e) sc[0][e] += odd[e];
+            }
         }
         // V's fragments are fetched under the softmax.
 #pragma unroll
@@ -683,7 +688,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                 const float mn = fmaxf(m[rr], mx);
                 if (__any_sync(0xffffffffu, mn > m[rr])) {
                     // The row's maximum grew (in some row of the warp): bring the sum and the accumulator along.
-                    const float corr = mn == -INFINITY ? 1.f : between(m[rr], mn);   // exp2(-inf) = 0 for a first maximum
+                    const float corr = mn == -INFINITY ? 1.f : exp2f((m[rr] - mn) * sl);   // exp2(-inf) = 0 for a first maximum
                     l[rr] *= corr;
 #pragma unroll
                     for (int n = 0; n < ON; ++n) { o[n][2 * rr] *= corr; o[n][2 * rr + 1] *= corr; }
@@ -722,7 +727,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
                     const float mn = fmaxf(m[e], mx);
-                    const float corr = mn == -INFINITY ? 1.f : between(m[e], mn);   // exp2(-inf) = 0 for a first maximum
+                    const float corr = mn == -INFINITY ? 1.f : CLUSTER ? between(m[e], mn) : exp2f((m[e] - mn) * sl);   // exp2(-inf) = 0 for a first maximum
                     l[e] *= corr;
 #pragma unroll
                     for (int n = 0; n < ON; ++n) { o[n][e] *= corr; o[n][2 + e] *= corr; }
@@ -742,7 +747,13 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                 if constexpr (LIFT > 0.f) base -= LIFT;
                 p[e] = exp2f(fmaf(sc[0][e], sl, -base));
                 p[2 + e] = exp2f(fmaf(sc[0][2 + e], sl, -base));
-                l[e] += p[e] + p[2 + e];
+            }
+            // The lane's share of the sums: in clusters its own two keys; in chunks those of its pair of lanes (keys g and g ^ 1, then the two
+            // eight further on), which is what a lane has of sixteen heads' rows: the sums are the same to the bit.
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if constexpr (CLUSTER) l[e] += p[e] + p[2 + e];
+                else l[e] += (p[e] + __shfl_xor_sync(0xffffffffu, p[e], 4)) + (p[2 + e] + __shfl_xor_sync(0xffffffffu, p[2 + e], 4));
             }
             // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; the longer sweeps of a cluster have
             // fewer of them, and at bf16 a third part of P makes up for it (8 sequences of 8766 keys, error against f64 where the output
@@ -782,7 +793,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int x = WIDE ? 1 : 4; x < (WIDE ? 4 : 32); x *= 2) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
+        for (int x = WIDE ? 1 : CLUSTER ? 4 : 8; x < (WIDE ? 4 : 32); x *= 2) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
 
     if constexpr (FOLDS) {
 #pragma unroll
