@@ -1192,7 +1192,9 @@ template <typename T, int DFULL>
 static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream, bool *merged) {
     const int group = a.hq / a.hkv;
     const bool wide = group > 8;
-    if (const int cluster = wide ? 0 : decode_cluster(a)) {
+    // (A cluster stores its outputs eight bytes at a time, the merge one element: it takes any address.)
+    const bool whole = reinterpret_cast<uintptr_t>(a.out) % 8 == 0;
+    if (const int cluster = wide || !whole ? 0 : decode_cluster(a)) {
         const long long warps = (long long)a.hkv * cluster * CLUSTER_WARPS, shares = cluster * CLUSTER_WARPS / (DFULL > 128 ? 2 : 1);
         const cudaError_t e = std::min<long long>(a.s, (long long)a.left + 1) > (MmaType<T>::NARROW ? 256 : 512) * shares ? split_mma_w<T, DFULL, false, CLUSTER_WARPS, 2>(a, warps, cluster, stream)
                                                                                           : split_mma_w<T, DFULL, false, CLUSTER_WARPS, 1>(a, warps, cluster, stream);
