@@ -579,6 +579,7 @@ int dash_attn_decode_append_rope(const dash_attn_decode_params *p, const dash_ro
     // Where the split pass can rotate on its way, the step is that pass and the merge; else a launch of the rotation goes first.
     dash::DecodeArgs f{};
     f.hq = p->hq; f.hkv = p->hkv; f.d = p->d;
+    f.scale = scale_for(p->has_scale, p->scale, p->d);
     f.rope_cos = r->cos; f.rope_sin = r->sin; f.rope_dim = r->dim; f.rope_len = r->len;
     f.rope_pos = positions ? positions : p->lengths;
     f.rope_pos_bytes = positions ? positions_elem_bytes : p->lengths_elem_bytes;

@@ -29,6 +29,7 @@
 // Inputs the vector path cannot read (head dimension not 64 / 128 / 256, last stride not 1, rows
 // not 16-byte aligned) go through a slower scalar kernel with the same arithmetic.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 
@@ -1217,8 +1218,10 @@ static bool decode_force_scalar_pass() {
     return off;
 }
 
+// (The tensor-core pass keeps maxima of scores that have not been scaled yet: a scale of zero or below would turn their order round, and
+// what is not finite would meet their first -inf.  The FMA pass scales first.)
 static bool decode_uses_mma(size_t elem, const DecodeArgs &a, bool vector_ok) {
-    return vector_ok && elem == 2 && a.hq / a.hkv >= 2 && !decode_force_scalar_pass();
+    return vector_ok && elem == 2 && a.hq / a.hkv >= 2 && a.scale > 0.f && std::isfinite(a.scale) && !decode_force_scalar_pass();
 }
 bool decode_fuses_rope(int dtype, const DecodeArgs &a, bool vector_ok) {
     auto aligned = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
