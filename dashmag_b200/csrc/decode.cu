@@ -23,8 +23,8 @@
 //
 // With 16-bit caches and two query heads or more per key-value head the pass runs on the tensor cores
 // instead (decode_split_mma_kernel below): at that much arithmetic per cache row the FMA pipe, not HBM,
-// bounds the pass above.  Above 512 keys its groups of up to eight heads need neither chunks nor merge: the
-// blocks of a cluster take a (sequence, key-value head) together (decode_cluster says which calls).
+// bounds the pass above.  Groups of up to eight heads with more than 512 keys need neither chunks nor merge where
+// their shares are short: the blocks of a cluster take a (sequence, key-value head) together (decode_cluster says which calls).
 //
 // Inputs the vector path cannot read (head dimension not 64 / 128 / 256, last stride not 1, rows
 // not 16-byte aligned) go through a slower scalar kernel with the same arithmetic.
@@ -412,10 +412,9 @@ __device__ __forceinline__ void cluster_store(void *mine, int rank, float2 v) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_address(mine, rank)), "f"(v.x), "f"(v.y) : "memory");
 }
 
-template <typename T, int D, int PARTS, bool WIDE, int WARPS, bool ROPE, int TOGETHER>
+template <typename T, int D, int PARTS, bool WIDE, int WARPS, bool ROPE, bool CLUSTER>
 __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs a) {
     constexpr int DM_WARPS = WARPS;
-    constexpr bool CLUSTER = TOGETHER > 0, FOLDS = TOGETHER == 2;
     if constexpr (!CLUSTER) allow_beside();   // the merge
     constexpr int DFULL = D * PARTS;            // the head dimension; D is what one warp takes of it
     constexpr int ROWB = 2 * D;                 // bytes of a warp's part of a cache row: 256 at D = 128, 128 at D = 64
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
         }
     }
     const float sl = a.scale * 1.4426950408889634f;   // scores are exponentiated in base 2
-    // The largest probability of a head: 1, or at f16, in a cluster's longer sweeps, 2^8 - the second part of a small probability is then no
+    // The largest probability of a head: 1, or at f16, in a cluster's sweeps, 2^8 - the second part of a small probability is then no
     // subnormal number, whose rounding would be the largest error of the sum.
     constexpr float LIFT = CLUSTER && MmaType<T>::NARROW ? 8.f : 0.f;
     // From one maximum to another, in clusters: the difference of the two offsets as the exponentials used them, each product rounded on
@@ -580,12 +579,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
     float o[ON][4];
 #pragma unroll
     for (int n = 0; n < ON; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    // A warp that sweeps more keys than a long chunk (TOGETHER 2; 512, at f16, whose P is sharper, 256): a product's additions to an
-    // accumulator that has grown large lose a little of it each, so every 256 keys what has gathered moves to a second accumulator.  (An instance of its own: the code
-    // costs a call of few tiles 0.6 us.  f16, 3000 keys a sequence, error against f64 where the output is next to nothing, 2.3e-8
-    // in chunks of 256; 3.4e-8 in 750 without, 2.1e-8 with it and LIFT.)
-    constexpr int FOLD = 256 / DM_KEYS;
-    float old[FOLDS ? ON : 1][4] = {};
     // This lane's two heads (2 t and 2 t + 1; of sixteen: g and g + 8); l is the lane's share of their sums.
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
     // ldmatrix rows: lane -> (matrix lane / 8, row lane % 8)
@@ -732,12 +725,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                     l[e] *= corr;
 #pragma unroll
                     for (int n = 0; n < ON; ++n) { o[n][e] *= corr; o[n][2 + e] *= corr; }
-                    if constexpr (FOLDS) {
-                        if (it >= FOLD) {
-#pragma unroll
-                            for (int n = 0; n < ON; ++n) { old[n][e] *= corr; old[n][2 + e] *= corr; }
-                        }
-                    }
                     m[e] = mn;
                 }
             }
@@ -756,7 +743,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                 if constexpr (CLUSTER) l[e] += p[e] + p[2 + e];
                 else l[e] += (p[e] + __shfl_xor_sync(0xffffffffu, p[e], 4)) + (p[2 + e] + __shfl_xor_sync(0xffffffffu, p[2 + e], 4));
             }
-            // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; the longer sweeps of a cluster have
+            // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; the sweeps of a cluster have
             // fewer of them, and at bf16 a third part of P makes up for it (8 sequences of 8766 keys, error against f64 where the output
             // is next to nothing: 3.8e-8 in chunks, 4.4e-8 with two parts, 2.0e-8 with three).
             constexpr bool THIRD = CLUSTER && !MmaType<T>::NARROW;
@@ -779,14 +766,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
 #pragma unroll
                 for (int n = 0; n < ON; ++n) MmaType<T>::mma(o[n], vf[n], pm[0], pm[1]);
             }
-            if constexpr (FOLDS) {
-                if (it % FOLD == FOLD - 1) {
-#pragma unroll
-                    for (int n = 0; n < ON; ++n)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) { old[n][e] += o[n][e]; o[n][e] = 0.f; }
-                }
-            }
         }
     }
     cp_async_wait<0>();
@@ -796,12 +775,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
 #pragma unroll
         for (int x = WIDE ? 1 : CLUSTER ? 4 : 8; x < (WIDE ? 4 : 32); x *= 2) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
 
-    if constexpr (FOLDS) {
-#pragma unroll
-        for (int n = 0; n < ON; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[n][e] += old[n][e];
-    }
     if constexpr (CLUSTER) {
         constexpr int PER = DM_WARPS / PARTS;
         float *const wide = reinterpret_cast<float *>(dm_ring);   // the warps' rings, from here on [PER][HEADS][DFULL]
@@ -1146,45 +1119,64 @@ constexpr size_t mma_smem(int dfull, bool wide, int warps, bool cluster) {
            (cluster ? sizeof(float) * (8 * dfull + MAX_CLUSTER * 4 + (MAX_CLUSTER + (size_t)warps / parts) * 16) : 0);
 }
 // `warps`: of one sequence.
-template <typename T, int DFULL, bool WIDE, int WARPS, int TOGETHER>
+template <typename T, int DFULL, bool WIDE, int WARPS, bool CLUSTER>
 static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster, cudaStream_t stream) {
     constexpr int PARTS = DFULL > 128 ? 2 : 1, D = DFULL / PARTS;
-    constexpr size_t smem = mma_smem(DFULL, WIDE, WARPS, TOGETHER > 0);
-    const auto kernel = a.rope_cos ? decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, true, TOGETHER> : decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, false, TOGETHER>;
+    constexpr size_t smem = mma_smem(DFULL, WIDE, WARPS, CLUSTER);
+    const auto kernel = a.rope_cos ? decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, true, CLUSTER> : decode_split_mma_kernel<T, D, PARTS, WIDE, WARPS, false, CLUSTER>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     return launch_clusters(kernel, dim3((unsigned)((warps + WARPS - 1) / WARPS), (unsigned)a.b), WARPS * 32, smem, stream, false, (unsigned)cluster, a);
 }
 // Blocks (of CLUSTER_WARPS warps) of the cluster that takes a key-value head of a sequence; 0: chunks, and the merge behind them.
-// Priced in tiles of a warp: its longest chain (a sequence may fill the cache), what a block costs whatever its share (eight
-// tiles' time), and where the blocks do not all run at once - two to a multiprocessor, four at D 64, less what larger clusters leave
-// idle of a GPU processing cluster - their waves, sequences with lengths at half the cache on average.  Few blocks leave
-// multiprocessors idle that the chunks would fill: then only chains of up to sixteen tiles, and of five.  Chosen over 125 calls (1 to 64
-// sequences, 100 to 32768 keys, D 64 to 256, groups of 2 to 8) timed with every size of cluster and with chunks: within 1 % of the
-// best of them on average, slower than the chunks of before in four (eight of 6144, 2 heads of 256, 22.4 -> 22.9 were it
-// taken; D 256 and 64 have lines of their own for it).  us, chunks and merge as they were | now: 1 of 4096, 32 / 8 heads of 128 with
-// rotation and append 13.0 | 11.2, 4 17.7 | 13.1, 16 37.4 | 26.3, 16 of 16384 104.9 | 71.1; 12 of 8192 43.4 | 31.3, 64 of 32768 621 |
-// 579; 12 of 6000, 16 / 4 of 256, 33.2 | 25.4.  Caches of at most 512 keys keep the two launches
-// (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.6 where a cluster takes 5.4.
-static int decode_cluster(const DecodeArgs &a) {
+// A cluster saves the merge and its launch, 3 to 5 us; what it costs is the chain of a warp's tiles (0.4 us a tile at D 64, 0.6 at 128,
+// 0.7 at 256), which nobody else shortens: where one sequence is much longer than the others, or the last blocks start when the first have
+// ended, the GPU waits for it, and chunks spread over all multiprocessors.  So: the blocks run at once, and the longest share that a sequence may
+// give a warp (it may fill the cache) is short - five tiles where few blocks run, whose multiprocessors would stand idle beside them, more where
+// they nearly fill the GPU; of several sizes the one with the shortest share.  Lengths given, blocks for 1.4 times to nearly twice the room still
+// pay, in clusters of up to four with shares of 8 to 16 tiles: not all of them last.  (`room`: blocks that run at once, two of 104 KB to a multiprocessor and
+// four at D 64, less what the clusters leave idle of GPU processing clusters; the runtime says 296, 296, 284, 264 and 224 for 1 to 16 blocks where
+// nothing else runs, the lines lie a few clusters below.)
+// Under a window of at most half the cache every longer sequence has the same share, and most chunks are empty: any number of blocks, priced
+// in tiles - the longest share and eight tiles' time that a block costs, or the waves of that and half of it again.
+// Chosen over 864 shapes (1 to 64 sequences, 530 to 32768 keys, D 64 to 256, groups of 2 to 8), each with whole caches and with lengths
+// spread evenly, all short, a few long and one long, timed with chunks and with every size of cluster, and tried on 837 others with and without
+// rotation and append, bf16 and f16: against chunks and merge with heads as rows the mean of those is 1.12 (whole), 1.17 (even), 1.25 (short), 1.18 (one
+// long), 1.16 (a few long), the worst 0.94, under 0.97 in 5 of 3521.  (Clusters wherever a price that takes lengths at half the cache says so:
+// 1.12, 1.20, 1.37, 1.13, 1.13, but under 0.97 in 237, the worst 0.52.)  1202 windows of 60 to 4096 keys: whole caches 1.93, even lengths 1.87, none slower.
+// us, heads as rows | clusters wherever | now: 9 whole caches of 20576 keys, 16 / 4 heads of 128, 67 | 87 | 65; 18 of 6156, 8 / 2 of 256, 41 | 56 |
+// 41; 23 of up to 32768, 32 / 8, one of them long, 59 | 123 | 57; 16 of up to 4096, one long, 19.5 | 24.9 | 16.0, evenly spread 35.5 | 30.7 | 31.4;
+// 4 of up to 10006, evenly spread, 30.5 | 21.2 | 28.7; one of 2947 with rotation and append 12.6 | 10.7 | 10.7.
+// A share is at most 512 keys, at f16 256, as a chunk: one accumulator loses a little of each addition to a long sum, at f16, whose P is
+// sharper, first (error against f64 where the output is next to nothing, 3000 keys a sequence: 2.3e-8 in chunks of 256, 3.4e-8 in shares of 750).
+// Caches of at most 512 keys keep the two launches (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.9 where a
+// cluster takes 5.4.
+static int decode_cluster(const DecodeArgs &a, bool narrow) {
     static const bool chunks = std::getenv("DASH_ATTN_DECODE_CHUNK") != nullptr;   // a comparison run fixes the chunk (api.cu)
     if (chunks || a.s <= 512) return 0;
     const int64_t units = (int64_t)a.hkv * a.b, shares = a.d > 128 ? CLUSTER_WARPS / 2 : CLUSTER_WARPS;
-    const bool window = a.left < a.s;
-    const int64_t tiles = ((window ? (int64_t)a.left + 1 : a.s) + DM_KEYS - 1) / DM_KEYS, fill = a.d == 128 ? 96 : 160;
-    const double mean = a.lengths && !window ? 0.5 : 1., fixed = 8.;
-    // Rows of 64 are arithmetic more than bytes, and long sweeps of many heads pay for the third part of P: 14 of 32768 keys, 8 heads,
-    // 77.1 us in chunks, 85.1 together, 31 of 18651 188 and 214, 64 of 16384 190 and 201; 9 of 32000 78.2 and 76.8, 60 of 4000 58.4 and 52.1.
-    if (a.d == 64 && units * tiles * DM_KEYS * mean > 1.6e6) return 0;
+    const int64_t seen = std::min<int64_t>(a.s, (int64_t)a.left + 1), tiles = (seen + DM_KEYS - 1) / DM_KEYS, few = a.d == 128 ? 96 : 160;
+    const bool window = 2 * seen <= a.s;
     int best = 0;
     double least = 0.;
     for (int c = 1; c <= MAX_CLUSTER; c *= 2) {
         const int64_t blocks = units * c, longest = (tiles + c * shares - 1) / (c * shares);
-        const double room = (c == 16 ? 128 : c == 8 ? 256 : c == 4 ? 272 : c == 2 ? 288 : 296) * (a.d == 64 ? 2 : 1);
-        if ((blocks < fill && longest > 5) || (blocks < 192 && longest > 16) || (c == 16 && blocks > room)) continue;
-        double cost = longest + fixed;
-        if (blocks > room) cost = std::max(cost, blocks * (mean * longest + fixed) / room) + 0.5 * (longest + fixed);
+        const double full = blocks / ((c == 16 ? 128. : c == 8 ? 256. : c == 4 ? 272. : c == 2 ? 288. : 296.) * (a.d == 64 ? 2 : 1));   // of the room
+        double cost = longest;
+        if (longest > (narrow ? 16 : 32) || (c == 16 && full > 1.)) continue;
+        if (window) {
+            if ((blocks < few && longest > 5) || (blocks < 192 && longest > 16)) continue;
+            cost += 8.;
+            if (full > 1.) cost *= full + 0.5;
+        } else if (full <= 1.) {
+            // (Clusters of sixteen leave half the multiprocessors without a block, which a cache that is not in L2 is read slower by.)
+            const double most = a.d <= 128 ? 5. + 18. * full * full : 4. + 18. * full * full;
+            if (longest > (c < 16 ? most : a.d <= 128 ? std::min(most, 12.) : 3. + full * full)) continue;
+        } else {
+            if (!a.lengths || full < 1.4 || full > 1.95 || c > 4 || a.d > 128 || longest < 8 || longest > 16) continue;
+            cost += 64.;   // whatever runs at once first
+        }
         if (best == 0 || cost < least) { best = c; least = cost; }
     }
     return best;
@@ -1195,18 +1187,17 @@ static cudaError_t split_mma(const DecodeArgs &a, cudaStream_t stream, bool *mer
     const bool wide = group > 8;
     // (A cluster stores its outputs eight bytes at a time, the merge one element: it takes any address.)
     const bool whole = reinterpret_cast<uintptr_t>(a.out) % 8 == 0;
-    if (const int cluster = wide || !whole ? 0 : decode_cluster(a)) {
-        const long long warps = (long long)a.hkv * cluster * CLUSTER_WARPS, shares = cluster * CLUSTER_WARPS / (DFULL > 128 ? 2 : 1);
-        const cudaError_t e = std::min<long long>(a.s, (long long)a.left + 1) > (MmaType<T>::NARROW ? 256 : 512) * shares ? split_mma_w<T, DFULL, false, CLUSTER_WARPS, 2>(a, warps, cluster, stream)
-                                                                                          : split_mma_w<T, DFULL, false, CLUSTER_WARPS, 1>(a, warps, cluster, stream);
+    if (const int cluster = wide || !whole ? 0 : decode_cluster(a, MmaType<T>::NARROW)) {
+        const long long warps = (long long)a.hkv * cluster * CLUSTER_WARPS;
+        const cudaError_t e = split_mma_w<T, DFULL, false, CLUSTER_WARPS, true>(a, warps, cluster, stream);
         *merged = e == cudaSuccess;
         if (*merged) return e;
         cudaGetLastError();   // (a part of a GPU may have no room for such a cluster: the chunks go anywhere)
     }
     const long long warps = (long long)a.splits * a.hkv * (wide ? (group + 15) / 16 : 1) * (DFULL > 128 ? 2 : 1);   // of one sequence
     const bool few = warps * a.b < 148LL * 8 * 2;
-    if (wide) return few ? split_mma_w<T, DFULL, true, 2, 0>(a, warps, 1, stream) : split_mma_w<T, DFULL, true, 8, 0>(a, warps, 1, stream);
-    return few ? split_mma_w<T, DFULL, false, 2, 0>(a, warps, 1, stream) : split_mma_w<T, DFULL, false, 8, 0>(a, warps, 1, stream);
+    if (wide) return few ? split_mma_w<T, DFULL, true, 2, false>(a, warps, 1, stream) : split_mma_w<T, DFULL, true, 8, false>(a, warps, 1, stream);
+    return few ? split_mma_w<T, DFULL, false, 2, false>(a, warps, 1, stream) : split_mma_w<T, DFULL, false, 8, false>(a, warps, 1, stream);
 }
 template <> cudaError_t split_mma<float, 128>(const DecodeArgs &, cudaStream_t, bool *) { return cudaErrorInvalidValue; }   // never taken: 16-bit caches only
 template <> cudaError_t split_mma<float, 64>(const DecodeArgs &, cudaStream_t, bool *) { return cudaErrorInvalidValue; }
