@@ -4,7 +4,6 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <initializer_list>
 #include <algorithm>
@@ -194,11 +193,7 @@ int check_decode(const dash_attn_decode_params *p, const char *op = "attention_d
 // several times over, so that the partial outputs stay a few percent of the cache traffic.  A pure function of the shape, so
 // the workspace query and the launch agree without looking at the device.
 void decode_plan(const dash_attn_decode_params *p, int *chunk, int *splits) {
-    // DASH_ATTN_DECODE_CHUNK (read once, when the first plan is made) fixes the chunk for comparison runs.
-    static const long long fixed = [] {
-        const char *env = std::getenv("DASH_ATTN_DECODE_CHUNK");
-        return env ? std::atoll(env) : 0LL;
-    }();
+    const long long fixed = dash::decode_fixed_chunk();   // a comparison run's
     // Units a multiprocessor works on at a time: warps of the tensor-core pass (two a unit at D 256), or of the FMA pass.
     const int group = p->hkv > 0 ? p->hq / p->hkv : 1;
     const bool mma = p->dtype != DASH_ATTN_F32 && group >= 2 && (p->d == 64 || p->d == 128 || p->d == 256);

@@ -38,6 +38,15 @@
 
 namespace dash {
 
+// DASH_ATTN_DECODE_CHUNK (read once) fixes the chunk for comparison runs, whose calls are then all in chunks; 0 and less: the planner's.
+long long decode_fixed_chunk() {
+    static const long long fixed = [] {
+        const char *env = std::getenv("DASH_ATTN_DECODE_CHUNK");
+        return env ? std::atoll(env) : 0LL;
+    }();
+    return fixed;
+}
+
 constexpr int DEC_WARPS = 4;    // warps per block, each with its own (chunk, key-value head)
 constexpr int DEC_UNROLL = 4;   // keys per group of D / 8 lanes in one step
 constexpr int DEC_STAGES = 4;   // steps of the per-lane ring (16-bit dtypes; two for f32)
@@ -1153,8 +1162,7 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster
 // Caches of at most 512 keys keep the two launches (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.9 where a
 // cluster takes 5.4.
 static int decode_cluster(const DecodeArgs &a, bool narrow) {
-    static const bool chunks = std::getenv("DASH_ATTN_DECODE_CHUNK") != nullptr;   // a comparison run fixes the chunk (api.cu)
-    if (chunks || a.s <= 512) return 0;
+    if (decode_fixed_chunk() > 0 || a.s <= 512) return 0;
     const int64_t units = (int64_t)a.hkv * a.b, shares = a.d > 128 ? CLUSTER_WARPS / 2 : CLUSTER_WARPS;
     const int64_t seen = std::min<int64_t>(a.s, (int64_t)a.left + 1), tiles = (seen + DM_KEYS - 1) / DM_KEYS, few = a.d == 128 ? 96 : 160;
     const bool window = 2 * seen <= a.s;

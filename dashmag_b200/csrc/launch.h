@@ -15,6 +15,7 @@ cudaError_t launch_generic_delta(int dtype, const TrainArgs &a, cudaStream_t str
 // Whether launch_decode rotates on its way (DecodeArgs::rope_*): a 16-bit cache on the tensor-core pass, rotated features and
 // tables readable 16 bytes at a time.  Other calls rotate with a launch of their own first.
 bool decode_fuses_rope(int dtype, const DecodeArgs &a, bool vector_ok);
+long long decode_fixed_chunk();
 cudaError_t launch_decode(int dtype, const DecodeArgs &a, bool vector_ok, cudaStream_t stream, int *launches);
 // The library's own decode scratch: its size in floats, and its address on the current device.
 size_t decode_static_capacity_floats();
