@@ -190,7 +190,7 @@ static __device__ __noinline__ int2 trim_padded_span(const void *kp, int kp_byte
         first = warp_min_i(first);
         kmin = first != 2147483647 ? first : kmin + 256;
     }
-    return make_int2(kmin, kmax);
+    return kmax > kmin ? make_int2(kmin, kmax) : make_int2(0, 0);   // (nothing: no tile starts below the span's end)
 }
 __device__ __forceinline__ void trim_padded(const MaskArgs &m, int b, int &kmin, int &kmax) {
     const int2 span = trim_padded_span(m.kp, m.kp_bytes, m.kp_sb, m.kp_st, b, kmin, kmax);

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(THREADS) generic_forward_kernel(TrainArgs a, i
         kmax = min(kmax, first + per);
         whi = min(whi, kmax);
     }
-    if (kmax > first) stage(first, 0);
+    if (SHARE ? kmax > first : kmax > kmin) stage(first, 0);
     for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();   // the tile is whole, and every warp is done with the other buffer
@@ -434,9 +434,10 @@ __global__ void __launch_bounds__(THREADS) generic_delta_kernel(TrainArgs a) {
 // ---------------------------------------------------------------------------------------------
 // dQ: each block of queries sweeps, in order, the key tiles it sees.
 // ---------------------------------------------------------------------------------------------
-// (Four rows a warp at D 128: with more than 128 registers a thread a block would be alone on its multiprocessor.)
+// (Four rows a warp at D 128, shared: with more than 128 registers a thread a block would be alone on its multiprocessor.  One row a warp: 64
+// registers, where ptxas left to itself takes 72 - 333 tokens in six, 8 / 2 heads of 80, backward 95 and 112 us.)
 template <typename T, int RPW, int NI, int KS, bool SHARE>
-__global__ void __launch_bounds__(THREADS, RPW == 4 && NI == 4 ? 2 : 0) generic_dq_kernel(TrainArgs a, int vec) {
+__global__ void __launch_bounds__(THREADS, RPW == 4 && NI == 4 && SHARE ? 2 : RPW == 1 && NI == 4 ? 4 : 0) generic_dq_kernel(TrainArgs a, int vec) {
     extern __shared__ __align__(16) float smem[];
     constexpr int ROWS = WARPS * RPW / KS, STEP = TILE * KS;
     const int dp = padded_d(a.d), sp = tile_stride(a.d);
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(THREADS, RPW == 4 && NI == 4 ? 2 : 0) generic_
         kmax = min(kmax, first + per);
         whi = min(whi, kmax);
     }
-    if (kmax > first) stage(first, 0);
+    if (SHARE ? kmax > first : kmax > kmin) stage(first, 0);
     for (int k0 = first, buf = 0; k0 < kmax; k0 += STEP, buf ^= 1) {
         copies_wait();
         __syncthreads();
@@ -729,28 +730,44 @@ static cudaError_t launch_generic(GenericKernel kernel, dim3 grid, size_t smem, 
      : (rpw) == 1 ? ((d) <= 64 ? kernel<T, 1, 2, 1, true> : kernel<T, 1, 4, 1, true>) : ((d) <= 64 ? kernel<T, 2, 2, 2, true> : kernel<T, 2, 4, 2, true>))
 
 // Blocks of the cluster that shares a block's rows, each a run of what they sweep.  Small calls wait for the chain of a block's
-// tiles, and where multiprocessors have room a second block halves it; causal calls gain by it beyond that, whose long chains end alone.
-// What it costs is the meeting (3 to 5 us with the first block's reads) and, packed, sweeps too short to share: `sweep` is the
-// mean sequence.  Measured (us, one block | two | four): forward of 16 queries against 4000 keys, 32 / 8 heads of 64, bf16, 64 blocks,
-// 168 | 97 | 69, 39 against 4783, 16 heads, 80 blocks, 201 | 152 | 107; f32, 450 tokens, 4 heads of 128, 228 blocks, 56 | 38 | 45, 1500, 8 heads,
-// 376 blocks, 398 | 297 | 305, 900 in four, 4 heads of 128, 228 blocks (two to a multiprocessor), 39 | 42 | 48, 384 in two 16.6 | 16.6 | 20.7.  (Heads
-// of 256, 64 queries against 128 keys, 64 blocks, 25 | 17 | 21, 60 against 2060, 128 blocks, 376 | 389 | 402.)  Backward (one | dq's two | dkdv's
-// two too): 39 against 4783 602 | 379 | 443; 590 in two, 3 / 1 heads of 96, 96 | 93 | 64; 300, 8 / 2 of 96, 124 | 122 | 81; 1000 in three, 4 / 2 of 64,
-// 91 | 79 | 84; 130, 4 heads, 20.7 | 21.2 | 27; dkdv's blocks sweep the whole group, so they gain where groups are large and
-// blocks few.
-static int64_t mean_sweep(const TrainArgs &a, int64_t rows) { return a.mask.kind == 2 ? rows / std::max(a.mask.seqs, 1) : rows; }
-static unsigned forward_cluster(const TrainArgs &a, int rpw, int64_t blocks) {
-    const int64_t room = 148 * (SMEM_PER_SM / ((int64_t)generic_smem(a.d, rpw, 1, 1) + SMEM_BESIDE)), sweep = mean_sweep(a, a.tk);
-    // Below 32 features a tile has no room for a block's sums; above 128 a head's bits do not depend on the others, and a rule
-    // that does not look at them would cost the calls of many heads a few per cent.
-    if (a.d < 32 || a.d > 128 || sweep < (a.d > 64 ? 64 : 128)) return 1;   // (302 in three, 4 heads of 64: 10.3 us alone, 12.3 shared; 202, 3 of 96: 12.4, 10.3)
-    if (blocks * 4 <= 330 && sweep >= 128) return 4;
-    return blocks <= 400 && (sweep >= 250 || blocks * 2 <= room) ? 2 : 1;
+// tiles, and where multiprocessors have room a second block halves it.  What it costs is the meeting (3 to 5 us with the first block's
+// reads), and where multiprocessors have none the other blocks' time.  So by the blocks there are and the steps of a block's sweep:
+// the more blocks, the longer the sweep.  Lines drawn from 2338 calls (f32 and bf16, 32 to 128 features, 60 to 4000 keys, packed, padded, plain,
+// fewer queries than keys), each timed with one, two and four blocks, backward with each pair, and tried on 875 others, against one block: forward
+// mean 1.07 times as fast, 13 calls slower by more than 3 %, the worst 0.89; backward 1.09, 9, 0.85.  (By sweeps of 190 keys and 400 blocks alone:
+// the same means, 130 and 37 calls, the worst 0.36 and 0.65.)  us, one block | two | four, forward: 16 queries against 4000 keys, 32 / 8
+// heads of 64, bf16, 64 blocks, 168 | 97 | 69; 450 tokens, 4 heads of 128, 228 blocks, 56 | 38 | 45; 384 in two, 4 heads of 64, 192 blocks, 16.6 | 16.6 | 20.7; 154, 2 heads of 128, 40 blocks, 10 | - | 20.
+// Backward (one | dq's two | dkdv's two | both): 474, 3 / 1 heads of 80, 126 | 126 | 72 | 69; 649 in two, 2 / 1 of 80, 112 | 108 | 81 | 68; but 294, 4 of 64,
+// whole rows, 43 | 43 | 61 | 48, and 161 queries against 294 keys, 39 | - | 51 | 46: dkdv's alone only where the keys' sweeps are a triangle.
+// (`room`: blocks that fit at once.)  Below 32 features a tile has no room for a block's sums; above 128 a head's bits do not depend on
+// the others, and a rule that does not look at them would cost the calls of many heads a few per cent.
+static double block_steps(const TrainArgs &a, int64_t swept, int rpw) {
+    const int64_t mean = a.mask.kind == 2 ? swept / std::max(a.mask.seqs, 1) : swept;
+    return (double)std::min(mean, (int64_t)a.mask.left + a.mask.right + block_rows(rpw)) / (rpw == SHARED_ROWS ? 2 * TILE : TILE);
 }
-static unsigned dq_cluster(const TrainArgs &a, int64_t blocks) { return a.d >= 32 && a.d <= 128 && blocks <= 400 && mean_sweep(a, a.tk) >= 190 ? 2 : 1; }
-static unsigned dkdv_cluster(const TrainArgs &a, int64_t blocks) {
-    const int64_t group = a.hq / a.hkv;
-    return a.d >= 32 && a.d <= 128 && group >= 2 && blocks <= (group >= 3 ? 190 : 100) && mean_sweep(a, a.tq) * group >= 256 ? 2 : 1;
+static bool shareable(const TrainArgs &a) { return a.d >= 32 && a.d <= 128; }
+static int64_t room_for(const TrainArgs &a, int rpw, int own, int probs) { return 148 * (SMEM_PER_SM / ((int64_t)generic_smem(a.d, rpw, own, probs) + SMEM_BESIDE)); }
+static unsigned forward_cluster(const TrainArgs &a, int rpw, int64_t blocks) {
+    const int64_t room = room_for(a, rpw, 1, 1);
+    const double steps = block_steps(a, a.tk, rpw);
+    const bool causal = a.mask.right == 0;
+    if (!shareable(a)) return 1;
+    if (blocks * 4 <= room && ((blocks <= 37 && steps >= 3) || (blocks <= 74 && steps >= 4))) return 4;
+    if (blocks * 2 > room) return causal && blocks <= 296 && steps >= 16 ? 2 : 1;
+    if (blocks > 222) return causal && rpw < 4 && blocks <= 400 && steps >= 9 ? 2 : 1;
+    return steps >= (rpw == 4 ? 9 : blocks > 148 ? 3 : 2.1) ? 2 : 1;
+}
+static unsigned dq_cluster(const TrainArgs &a, int rpw, int64_t blocks) {
+    const bool roomy = rpw < 4 && blocks * 2 <= room_for(a, rpw, 2, 1);
+    return shareable(a) && blocks <= 400 && block_steps(a, a.tk, rpw) >= (blocks <= 74 ? 3 : blocks <= 148 ? 6 : blocks <= 222 && roomy ? 3 : 9) ? 2 : 1;
+}
+static unsigned dkdv_cluster(const TrainArgs &a, int rpw, int64_t blocks, bool dq_shared) {
+    const double steps = block_steps(a, a.tq, rpw) * (a.hq / a.hkv);   // a block sweeps its whole group
+    if (!shareable(a)) return 1;
+    if (blocks <= 37) return steps >= 1.5 ? 2 : 1;
+    const bool triangle = a.mask.right == 0 && a.tq >= a.tk;
+    if (blocks <= 148 && (dq_shared || triangle) && steps >= (blocks <= 74 ? 4 : 6)) return 2;
+    return dq_shared && blocks <= 400 && steps >= 48 ? 2 : 1;
 }
 
 template <typename T>
@@ -775,10 +792,12 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
         generic_delta_kernel<T><<<blocks, THREADS, 0, stream>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
+    const int q_rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), q_rows = block_rows(q_rpw), q_tiles = (a.tq + q_rows - 1) / q_rows;
+    const unsigned q_cluster = dq_cluster(a, q_rpw, (int64_t)q_tiles * a.hq * a.b);
     {
         const int rpw = rows_per_warp(a.tk, (int64_t)a.hkv * a.b, a.d, 2, 2), rows = block_rows(rpw);
         const int tiles = (a.tk + rows - 1) / rows;
-        const unsigned cluster = dkdv_cluster(a, (int64_t)tiles * a.hkv * a.b);
+        const unsigned cluster = dkdv_cluster(a, rpw, (int64_t)tiles * a.hkv * a.b, q_cluster > 1);
         *launches += 1;
         e = launch_generic(cluster > 1 ? GENERIC_PICK_SHARED(generic_dkdv_kernel, T, rpw, a.d) : GENERIC_PICK(generic_dkdv_kernel, T, rpw, a.d), dim3(tiles * cluster, a.hkv, a.b), generic_smem(a.d, rpw, 2, 2), stream,
                            false, a, vec, cluster);
@@ -786,12 +805,9 @@ static cudaError_t backward_t(const TrainArgs &a, cudaStream_t stream, int *laun
     }
     {   // beside dkdv.  (dkdv itself brought in under delta's end, to wait there, made the whole twice as slow: 1000 tokens, 4 / 2
         // heads of 64 327 against 213 us.)
-        const int rpw = rows_per_warp(a.tq, (int64_t)a.hq * a.b, a.d, 2, 1), rows = block_rows(rpw);
-        const int tiles = (a.tq + rows - 1) / rows;
-        const unsigned cluster = dq_cluster(a, (int64_t)tiles * a.hq * a.b);
         *launches += 1;
-        return launch_generic(cluster > 1 ? GENERIC_PICK_SHARED(generic_dq_kernel, T, rpw, a.d) : GENERIC_PICK(generic_dq_kernel, T, rpw, a.d), dim3(tiles * cluster, a.hq, a.b), generic_smem(a.d, rpw, 2, 1), stream,
-                              true, a, vec, cluster);
+        return launch_generic(q_cluster > 1 ? GENERIC_PICK_SHARED(generic_dq_kernel, T, q_rpw, a.d) : GENERIC_PICK(generic_dq_kernel, T, q_rpw, a.d), dim3(q_tiles * q_cluster, a.hq, a.b), generic_smem(a.d, q_rpw, 2, 1), stream,
+                              true, a, vec, q_cluster);
     }
 }
 
