@@ -577,9 +577,6 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
         }
     }
     const float sl = a.scale * 1.4426950408889634f;   // scores are exponentiated in base 2
-    // The largest probability of a head: 1, or at f16, in a cluster's sweeps, 2^8 - the second part of a small probability is then no
-    // subnormal number, whose rounding would be the largest error of the sum.
-    constexpr float LIFT = CLUSTER && MmaType<T>::NARROW ? 8.f : 0.f;
     // From one maximum to another, in clusters: the difference of the two offsets as the exponentials used them, each product rounded on
     // its own, so that what was summed against either shares one reference.
     auto between = [sl](float from, float to) { return exp2f(__fsub_rn(__fmul_rn(from, sl), __fmul_rn(to, sl))); };
@@ -740,8 +737,7 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
             float p[4];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                float base = m[e] == -INFINITY ? 0.f : __fmul_rn(m[e], sl);
-                if constexpr (LIFT > 0.f) base -= LIFT;
+                const float base = m[e] == -INFINITY ? 0.f : __fmul_rn(m[e], sl);
                 p[e] = exp2f(fmaf(sc[0][e], sl, -base));
                 p[2 + e] = exp2f(fmaf(sc[0][2 + e], sl, -base));
             }
@@ -752,9 +748,10 @@ __global__ void __launch_bounds__(WARPS * 32) decode_split_mma_kernel(DecodeArgs
                 if constexpr (CLUSTER) l[e] += p[e] + p[2 + e];
                 else l[e] += (p[e] + __shfl_xor_sync(0xffffffffu, p[e], 4)) + (p[2 + e] + __shfl_xor_sync(0xffffffffu, p[2 + e], 4));
             }
-            // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; the sweeps of a cluster have
-            // fewer of them, and at bf16 a third part of P makes up for it (8 sequences of 8766 keys, error against f64 where the output
-            // is next to nothing: 3.8e-8 in chunks, 4.4e-8 with two parts, 2.0e-8 with three).
+            // A chunk's largest probability is 1 and has no error, and it is much of the chunk's sum; a cluster's shares go against one
+            // maximum at the end and have fewer of them, and at bf16 a third part of P makes up for it, and more (8 of 2000 keys, 32 / 8 heads of
+            // 128, error against f64 where the output is next to nothing: 6.3e-8 in chunks, 6.9e-8 with two parts, 2.4e-8 with three; under a window of 4096
+            // keys, shares of 512, 5.3e-8, 5.8e-8, 3.2e-8).
             constexpr bool THIRD = CLUSTER && !MmaType<T>::NARROW;
             uint32_t pa[2], pl[2], pm[2];   // an 8 x 8 transpose each makes the accumulator's layout the B operand's
 #pragma unroll
@@ -1157,8 +1154,9 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster
 // us, heads as rows | clusters wherever | now: 9 whole caches of 20576 keys, 16 / 4 heads of 128, 67 | 87 | 65; 18 of 6156, 8 / 2 of 256, 41 | 56 |
 // 41; 23 of up to 32768, 32 / 8, one of them long, 59 | 123 | 57; 16 of up to 4096, one long, 19.5 | 24.9 | 16.0, evenly spread 35.5 | 30.7 | 31.4;
 // 4 of up to 10006, evenly spread, 30.5 | 21.2 | 28.7; one of 2947 with rotation and append 12.6 | 10.7 | 10.7.
-// A share is at most 512 keys, at f16 256, as a chunk: one accumulator loses a little of each addition to a long sum, at f16, whose P is
-// sharper, first (error against f64 where the output is next to nothing, 3000 keys a sequence: 2.3e-8 in chunks of 256, 3.4e-8 in shares of 750).
+// A share is at most 512 keys; at f16, whose P is sharper in two parts than bf16's, no longer than the chunk would be, or 192: one accumulator loses a
+// little of each addition to a long sum, which shows there first (error against f64 where the output is next to nothing, 32 of 1000 keys, 32 / 8 heads
+// of 128: 2.46e-8 in chunks of 128, 2.63e-8 in shares of 256, 2.14e-8 in shares of 128; 16 of 3000, 2.07e-8 in chunks, 2.02e-8 in shares of 192).
 // Caches of at most 512 keys keep the two launches (tests/test_decode_rotates_gpu.py counts them): 16 of 200, 16 / 4 heads, 7.9 where a
 // cluster takes 5.4.
 static int decode_cluster(const DecodeArgs &a, bool narrow) {
@@ -1166,13 +1164,14 @@ static int decode_cluster(const DecodeArgs &a, bool narrow) {
     const int64_t units = (int64_t)a.hkv * a.b, shares = a.d > 128 ? CLUSTER_WARPS / 2 : CLUSTER_WARPS;
     const int64_t seen = std::min<int64_t>(a.s, (int64_t)a.left + 1), tiles = (seen + DM_KEYS - 1) / DM_KEYS, few = a.d == 128 ? 96 : 160;
     const bool window = 2 * seen <= a.s;
+    const int64_t most_keys = narrow ? std::max(a.chunk, 192) : 512;
     int best = 0;
     double least = 0.;
     for (int c = 1; c <= MAX_CLUSTER; c *= 2) {
         const int64_t blocks = units * c, longest = (tiles + c * shares - 1) / (c * shares);
         const double full = blocks / ((c == 16 ? 128. : c == 8 ? 256. : c == 4 ? 272. : c == 2 ? 288. : 296.) * (a.d == 64 ? 2 : 1));   // of the room
         double cost = longest;
-        if (longest > (narrow ? 16 : 32) || (c == 16 && full > 1.)) continue;
+        if (longest * DM_KEYS > most_keys || (c == 16 && full > 1.)) continue;
         if (window) {
             if ((blocks < few && longest > 5) || (blocks < 192 && longest > 16)) continue;
             cost += 8.;

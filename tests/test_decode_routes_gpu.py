@@ -19,8 +19,8 @@ pytestmark = pytest.mark.gpu
     (3, 20000, 32, 8, 128, -1, "bf16", 2, 2),
     (4, 11776, 32, 8, 128, -1, "bf16", 1, 1),      # eight blocks a head, all of the room: 23 tiles a share, then 24
     (4, 11792, 32, 8, 128, -1, "bf16", 2, 2),
-    (4, 8192, 32, 8, 128, -1, "f16", 1, 1),        # f16: 16 tiles, then 17
-    (4, 8208, 32, 8, 128, -1, "f16", 2, 2),
+    (4, 6144, 32, 8, 128, -1, "f16", 1, 1),        # f16: 12 tiles, the most where the chunk is no longer, then 13
+    (4, 6160, 32, 8, 128, -1, "f16", 2, 2),
     (1, 12288, 32, 8, 128, -1, "bf16", 1, 1),      # sixteen blocks a head: 12 tiles, then 13
     (1, 12304, 32, 8, 128, -1, "bf16", 2, 2),
     (1, 6144, 4, 2, 128, -1, "bf16", 1, 1),        # two heads: 6 tiles, then 7
