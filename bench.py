@@ -686,7 +686,7 @@ def main():
                          "frac": gbs / world / pk["hbm"], "frac_of_nominal_8TBs": gbs / world / 8000.0,
                          "traffic": None if scale is None else dec_bytes / world * scale,
                          "traffic_unit": "DRAM bytes per pass: the profiler's ratio of traffic to algorithmic bytes at batch 8, times this pass's bytes",
-                         "kernels": "decode_split_mma_kernel, its clusters merging (pass-level)"},
+                         "kernels": "decode_split_mma_kernel + decode_merge_kernel (pass-level)"},
         }
         del kc, vc
         # Host overhead of a short decoding step (crates/dash-ops/src/attention.rs:123-127,

@@ -14,9 +14,8 @@
 //   * scores are reduced across the D / 8 lanes with shuffles, the softmax is kept online in f32
 //     per query head, lane groups are merged with shuffles at the end, and each warp writes one
 //     normalised partial output and its log-sum-exp;
-//     (dash_attn_decode_append_rope: the pass also rotates the queries and the new key as it reads them;
-//     one sequence of 2047 keys, the whole step on the device 19.2 -> 13.5 us with that, the chunk of 64
-//     keys the planner now picks and the merge brought in under the pass's end);
+//     (dash_attn_decode_append_rope: the pass also rotates the queries and the new key as it reads them, where it runs on the
+//     tensor cores, below: a launch less);
 //   * the merge kernel combines the partials of each (sequence, query head) by their log-sum-exp
 //     and rounds to the queries' dtype.  Chunks past a sequence's length or before its window are
 //     never touched.
@@ -326,8 +325,9 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) decode_split_kernel(DecodeArgs
 // are XOR-swizzled by the row, and ldmatrix reads the fragments from there without bank conflicts (transposed for V).  What a warp
 // waits for in a tile is its own chain, not memory (six stages for three change nothing, 0.8 us a tile where four warps are
 // alone on a multiprocessor): all fragments are fetched in front of the products, V's under the softmax, no product follows
-// the one it depends on, and a tile's copies go out from running addresses (0.5 us).  One sequence of 2047 keys, 32 / 8 heads of 128,
-// split and merge, 13.0 -> 12.5 us, 16 of 16384 104.9 -> 96.2, groups of sixteen, 40 sequences of 20000, 55.9 -> 53.5.
+// the one it depends on, and a tile's copies go out from running addresses (0.5 us).  Split and merge, against
+// heads as rows with each fragment fetched where it is used: 16 of 200 keys, 16 / 4 heads of 128, 9.0 -> 7.9 us, 64 of up to 16384, 32 / 8 of 64, 176 -> 166;
+// groups of sixteen, 40 sequences of 20000, 56.2 -> 53.8.
 //
 // CLUSTER: the blocks of a cluster take one (sequence, key-value head) together, its tiles dealt evenly over their warps by the
 // length the sequence really has, and meet in distributed shared memory: each block merges its warps' sums, hands every block of
@@ -387,10 +387,11 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 // WARPS warps to a block: eight, or two where blocks of eight would leave multiprocessors without one (a block is a
 // multiprocessor's worth of shared memory: 256 units of one sequence's 8 heads in blocks of eight are 32 blocks).  The warps
 // resident at a time are the same.  Blocks of two up to sixteen warps a multiprocessor (at D 128 two waves of them, at D 64
-// one), where they measured ahead: one sequence of 2047 keys with rotation and append, 15.5 us with blocks of eight, 13.5 with
-// two; 56 sequences of up to 5136 with one head, 2296 warps, 36.9 and 33.3; 34 of up to 7657 under a window of 4096, 2040
-// warps, 24.8 and 23.0; but 40 of up to 6000, 1880 warps, 24.7 and 26.1, for which no rule was found.  Beyond, eight (64
-// sequences of up to 4096, 8 heads: 91 against 102 us): its warps read neighbouring heads of the same keys at the same time.
+// one), where they measured ahead (us, eight | two): one sequence of 300 keys with rotation and append, 12.2 | 10.1; 16 of up to 500, 16 / 4 heads,
+// 10.2 | 8.8; 56 of up to 5136 with one head, 26.3 | 22.0; but 34 of up to 7657, 16 heads on one, 22.9 | 24.2, for which no rule was found.  Beyond,
+// eight: its warps read neighbouring heads of the same keys at the same time (20 sequences of up to 8192, 32 / 2 heads, 23.0 | 26.1; 16 of up to 20000, 16
+// on one, 22.0 | 24.1).  With heads as columns groups of four are ahead in twos there as well (64 of up to 4096, 8 heads, 92.3 | 88.4): the line
+// was drawn before that.
 //
 // Two columns rotated in the dtype's own arithmetic, as rope_kernel does it (each product and the sum rounded once): `low` for
 // the first half of the rotated features, whose partner enters with its sign turned.
@@ -1247,16 +1248,14 @@ static cudaError_t decode_t(const DecodeArgs &a, bool vector_ok, cudaStream_t st
     *launches += 1;
     if (e != cudaSuccess || merged) return e;
     *launches += 1;
-    // The merge comes in under the pass's end: one sequence of 4096 keys 14.5 -> 12.5 us, 64 of up to 5387 with one head 39.0 ->
-    // 37.0, 28 of up to 7754, 8 heads, 100.3 -> 98.6.  (Its blocks gather on the multiprocessors the pass leaves first, and a
-    // few calls of few blocks with much to read lose by it: 16 of up to 20000 keys, 16 heads on one, 36.0 us after the pass,
-    // 38.2 under its end; 25 of up to 19426 41.5 and 42.3.  Neither the parts' size nor the blocks' number tells them apart:
-    // with the line at 12 or 20 MB of parts more calls lost than won.)
+    // The merge comes in under the pass's end (us, after it | under it): 16 of up to 500 keys, 16 / 4 heads, 9.0 | 8.8; two of 8192, 8 on one, 9.5 | 8.9; eight
+    // of 6144, 8 / 2 of 128, 14.8 | 14.3; 60 of up to 9557, 8 heads, 184.2 | 183.7.  (Its blocks gather on the multiprocessors the pass leaves first, and
+    // a few calls lose by it: eight of 6144, 8 / 2 of 256, 22.6 | 23.0, one of up to 20000, 8 heads, 18.0 | 18.2.  Neither the parts' size nor the blocks'
+    // number tells them apart.)
     // Threads of a merge block: 128, or where the blocks are at most two a multiprocessor the fewest (up to 512) with which every
-    // partial is asked for at once.  (Threads 128 / 256 / 512, and the merge as it was: one sequence of 4096 keys, 8 heads,
-    // 64 splits on 32 blocks, 13.3 / 11.9 / 12.1 us, 13.7; two of 5919 13.5 / 13.0 / 11.9, 14.4; eight of 6144, 2 heads of 256,
-    // 35 splits on 64 blocks, 21.6 / 22.2 / 21.1, 22.0; but 60 of up to 9557 on 1920 blocks 193.7 / 196.3 / 205.5, 193.4, and 61
-    // under a window on 976 37.1 / 38.1 / 42.8, 37.9.)
+    // partial is asked for at once.  (Threads 128 / 256 / 512: eight of 6144, 8 / 2 heads of 128, 15.7 / 14.3 / 15.3 us; one of up to 20000, 32 / 8, 20.0 / 18.5 / 18.2;
+    // two of 8192, 8 on one, 10.6 / 9.5 / 8.9; eight of 6144, 8 / 2 of 256, 23.7 / 22.8 / 22.9; but 60 of up to 9557 on 1920 blocks 183.6 / 186.4 / 195.9, and 64 of up to
+    // 4096 on 2048 92.5 / 96.3 / 105.8.)
     const int64_t blocks = (int64_t)a.b * a.hq;
     int threads = 128;
     if (blocks <= 2 * 148)
