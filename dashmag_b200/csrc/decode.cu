@@ -1154,7 +1154,7 @@ static cudaError_t split_mma_w(const DecodeArgs &a, long long warps, int cluster
 // 1.12, 1.20, 1.37, 1.13, 1.13, but under 0.97 in 237, the worst 0.52.)  1202 windows of 60 to 4096 keys: whole caches 1.93, even lengths 1.87, none slower.
 // us, heads as rows | clusters wherever | now: 9 whole caches of 20576 keys, 16 / 4 heads of 128, 67 | 87 | 65; 18 of 6156, 8 / 2 of 256, 41 | 56 |
 // 41; 23 of up to 32768, 32 / 8, one of them long, 59 | 123 | 57; 16 of up to 4096, one long, 19.5 | 24.9 | 16.0, evenly spread 35.5 | 30.7 | 31.4;
-// 4 of up to 10006, evenly spread, 30.5 | 21.2 | 28.7; one of 2947 with rotation and append 12.6 | 10.7 | 10.7.
+// 4 of up to 10006, evenly spread, 30.5 | 21.2 | 21.2, but 8 of up to 7537 42.2 | 31.5 | 39.4; one of 2947 with rotation and append 12.6 | 10.7 | 10.7.
 // A share is at most 512 keys; at f16, whose P is sharper in two parts than bf16's, no longer than the chunk would be, or 192: one accumulator loses a
 // little of each addition to a long sum, which shows there first (error against f64 where the output is next to nothing, 32 of 1000 keys, 32 / 8 heads
 // of 128: 2.46e-8 in chunks of 128, 2.63e-8 in shares of 256, 2.14e-8 in shares of 128; 16 of 3000, 2.07e-8 in chunks, 2.02e-8 in shares of 192).
